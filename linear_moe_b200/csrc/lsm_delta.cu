@@ -257,9 +257,13 @@ __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
 // ---------------------------------------------------------------------------------------------------------------
 // Chunk-parallel construction of the tiles (forward): one CTA per (batch, head, chunk).
 //   b_i = inclusive cumulative log decay inside the chunk,  Gamma_ij = e^{b_i - b_j}
-//   A   = strictly-lower(diag(beta) (K K^T . Gamma)),   T = (I + A)^{-1}   (column c of T lives in the registers of
-//         thread c: row i needs only rows < i of the same column, so the substitution runs without any barrier)
+//   A   = strictly-lower(diag(beta) (K K^T . Gamma)),   T = (I + A)^{-1}
 //   W = T (beta e^{b} K),  U = T (beta V),  Aqk = scale tril((Q K^T) . Gamma),  Qd = scale e^{b} Q,  Kd = e^{b_C - b} K
+// The inverse is taken in fp32 by halves: the four 16 x 16 diagonal blocks by substitution, one column per thread, then
+// [[T0, 0], [-T1 (A10 T0), T1]] twice, with all threads on the small products.  A substitution over the whole chunk, one
+// column per thread, is a chain of 2016 multiply-adds on two warps; it was most of this kernel's time.
+// What bounds the kernel is the traffic of its five tiles (112 KB in and out per chunk at D = 128); three CTAs of eight
+// warps per SM overlap one chunk's loads with another's products.
 // ---------------------------------------------------------------------------------------------------------------
 struct PrepArgs {
     const bf16 *q, *k, *v;             // [B,T,H,D] with the strides below (elements)
@@ -270,29 +274,94 @@ struct PrepArgs {
     float* gamma;                      // [BH, N]
     int B, T, H, N;
     float scale;
+    bf16* Tinv;                        // [BH, N, C, C] the inverse, or null
 };
 
+constexpr int NTP = 256;               // threads of the chunk-parallel tile kernel
+constexpr int LDF = C + 4;             // row stride of the fp32 matrix (16-byte rows)
+
+// X = A B for fp32 matrices of N x N (N = 16 or 32) inside arrays of row stride LDF; NTP threads, `sign` on the result.
+// Four neighbouring columns per thread; `count` independent products, `step` elements apart.
+template <int N>
+__device__ __forceinline__ void small_product(const float* A, const float* B, float* X, float sign, int count, int step) {
+    constexpr int PER = N * N / 4;                            // threads of one product
+    for (int i = threadIdx.x; i < PER * count; i += NTP) {
+        const int m = i / PER, r = (i % PER) / (N / 4), c = (i % (N / 4)) * 4;
+        const float *a = A + m * step + r * LDF, *b = B + m * step + c;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < N; k += 4) {
+            const float4 av = *reinterpret_cast<const float4*>(a + k);
+            const float* ap = reinterpret_cast<const float*>(&av);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 bv = *reinterpret_cast<const float4*>(b + (k + e) * LDF);
+                x.x += ap[e] * bv.x; x.y += ap[e] * bv.y; x.z += ap[e] * bv.z; x.w += ap[e] * bv.w;
+            }
+        }
+        *reinterpret_cast<float4*>(X + m * step + r * LDF + c) = make_float4(sign * x.x, sign * x.y, sign * x.z, sign * x.w);
+    }
+}
+
+// F holds a strictly lower triangular A (zeros elsewhere); on return its lower blocks hold T = (I + A)^{-1}.  The blocks above the
+// diagonal are scratch.  Called by all NTP threads with A visible; ends with a barrier.
+__device__ __forceinline__ void unit_lower_inverse(float* F) {
+    if (threadIdx.x < C) {
+        const int blk = threadIdx.x >> 4, c = threadIdx.x & 15;
+        float* D = F + (blk * 16) * LDF + blk * 16;
+        float t[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float acc = (i == c) ? 1.f : 0.f;
+#pragma unroll
+            for (int j = 0; j < i; ++j) acc -= D[i * LDF + j] * t[j];
+            t[i] = acc;
+        }
+        __syncwarp();                                        // both blocks of this warp have been read
+#pragma unroll
+        for (int i = 0; i < 16; ++i) D[i * LDF + c] = t[i];
+    }
+    __syncthreads();
+    constexpr int S2 = 32 * LDF + 32;                        // from one half of the diagonal to the other
+    // the (1,0) and (3,2) blocks
+    small_product<16>(F + 16 * LDF, F, F + 16, 1.f, 2, S2);                       // A10 T0 -> above the diagonal
+    __syncthreads();
+    small_product<16>(F + 16 * LDF + 16, F + 16, F + 16 * LDF, -1.f, 2, S2);      // -T1 (A10 T0)
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * 16 * 4; i += NTP) {                          // the scratch blocks are zeros of T
+        const int m = i >> 6, r = (i >> 2) & 15, c = (i & 3) * 4;
+        *reinterpret_cast<float4*>(F + m * S2 + r * LDF + 16 + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    // the lower left quarter
+    small_product<32>(F + 32 * LDF, F, F + 32, 1.f, 1, 0);
+    __syncthreads();
+    small_product<32>(F + 32 * LDF + 32, F + 32, F + 32 * LDF, -1.f, 1, 0);
+    __syncthreads();
+}
+
 template <int D>
-__global__ void __launch_bounds__(NT) delta_prep_fwd_kernel(PrepArgs a) {
-    constexpr int LD = D + 8, LDC = C + 8, LDA = C + 1;
+__global__ void __launch_bounds__(NTP, 3) delta_prep_fwd_kernel(PrepArgs a) {
+    constexpr int LD = D + 8, LDC = C + 8, NH = D / 16;      // NH: n-tiles of a warp's half of D columns
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* Ks = reinterpret_cast<bf16*>(smem_raw);            // [C][LD]
     bf16* Vs = Ks + C * LD;                                  // [C][LD]  V, then beta V
-    bf16* Qs = Vs + C * LD;                                  // [C][LD]
-    bf16* Kb = Qs + C * LD;                                  // [C][LD]  beta e^b K
-    bf16* Tb = Kb + C * LD;                                  // [C][LDC] T in bf16
-    float* A32 = reinterpret_cast<float*>(Tb + C * LDC);     // [C][LDA] strictly lower A
-    float* bcum = A32 + C * LDA;                             // [C]
+    bf16* Qs = Vs + C * LD;                                  // [C][LD]  Q, then beta e^b K
+    float* F = reinterpret_cast<float*>(Qs + C * LD);        // [C][LDF] strictly lower A, then T
+    bf16* Tb = reinterpret_cast<bf16*>(F);                   // [C][LDC] T in bf16 (over F)
+    float* bcum = F + C * LDF;                               // [C]
     float* bet = bcum + C;                                   // [C]
     const int n = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int m0 = 16 * (w & 3), half = w >> 2;
     const int t0 = n * C;
     const int valid = min(C, a.T - t0);
     const long long cn = (long long)bh * a.N + n;
 
     load_tile_async<C, D, LD>(Ks, a.k + b * a.ks_b + h * a.ks_h + (long long)t0 * a.ks_t, a.ks_t, valid);
-    load_tile_async<C, D, LD>(Vs, a.v + b * a.vs_b + h * a.vs_h + (long long)t0 * a.vs_t, a.vs_t, valid);
     load_tile_async<C, D, LD>(Qs, a.q + b * a.qs_b + h * a.qs_h + (long long)t0 * a.qs_t, a.qs_t, valid);
+    cp_async_commit();
+    load_tile_async<C, D, LD>(Vs, a.v + b * a.vs_b + h * a.vs_h + (long long)t0 * a.vs_t, a.vs_t, valid);
     cp_async_commit();
     if (w == 0) {                                            // decay table: two tokens per lane, warp scan
         const int i0 = 2 * l, i1 = 2 * l + 1;
@@ -318,94 +387,94 @@ __global__ void __launch_bounds__(NT) delta_prep_fwd_kernel(PrepArgs a) {
         bet[i0] = be0;
         bet[i1] = be1;
     }
-    cp_async_wait<0>();
+    cp_async_wait<1>();
     __syncthreads();
     const float btot = bcum[C - 1];
-    // ---- K K^T -> A (fp32, strictly lower) and Q K^T -> Aqk (bf16, to global); warp w owns rows 16w .. 16w+15
+    // ---- K K^T -> A (fp32, strictly lower) and Q K^T -> Aqk (bf16, to global); warp: 16 rows x 32 columns, tiles above the
+    //      diagonal are only zeroed
     {
-        float kk[8][4], qk[8][4];
-        zero_acc<8>(kk);
-        zero_acc<8>(qk);
-        warp_gemm<8, D, false, false>(kk, Ks, LD, 16 * w, Ks, LD, 0);
-        warp_gemm<8, D, false, false>(qk, Qs, LD, 16 * w, Ks, LD, 0);
+        const int nc = 32 * half;
+        float kk[4][4], qk[4][4];
+        zero_acc<4>(kk);
+        zero_acc<4>(qk);
+        if (nc <= m0) {
+            warp_gemm<4, D, false, false>(kk, Ks, LD, m0, Ks, LD, nc);
+            warp_gemm<4, D, false, false>(qk, Qs, LD, m0, Ks, LD, nc);
+        }
         bf16* Ag = a.A + cn * C * C;
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+        for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                const int i = 16 * w + (l >> 2) + 8 * hh;
-                const int j = nt * 8 + (l & 3) * 2;
+                const int i = m0 + (l >> 2) + 8 * hh;
+                const int j = nc + nt * 8 + (l & 3) * 2;
                 const float bi = bcum[i], be = bet[i];
                 const float d0 = __expf(bi - bcum[j]), d1 = __expf(bi - bcum[j + 1]);
-                A32[i * LDA + j] = i > j ? be * d0 * kk[nt][2 * hh] : 0.f;
-                A32[i * LDA + j + 1] = i > j + 1 ? be * d1 * kk[nt][2 * hh + 1] : 0.f;
+                *reinterpret_cast<float2*>(F + i * LDF + j) = make_float2(i > j ? be * d0 * kk[nt][2 * hh] : 0.f,
+                                                                          i > j + 1 ? be * d1 * kk[nt][2 * hh + 1] : 0.f);
                 const float a0 = i >= j ? a.scale * d0 * qk[nt][2 * hh] : 0.f;
                 const float a1 = i >= j + 1 ? a.scale * d1 * qk[nt][2 * hh + 1] : 0.f;
                 *reinterpret_cast<__nv_bfloat162*>(Ag + i * C + j) = __floats2bfloat162_rn(a0, a1);
             }
     }
+    cp_async_wait<0>();
     __syncthreads();
-    // ---- threads 0..63: column c of T = (I + A)^{-1} by forward substitution, entirely in registers;
-    //      threads 64..127: the elementwise tiles (beta e^b K -> Kb, beta V in place, Qd and Kd to global)
-    if (threadIdx.x < C) {
-        const int c = threadIdx.x;
-        float t[C];
-#pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float acc = (i == c) ? 1.f : 0.f;
-#pragma unroll
-            for (int j = 0; j < i; ++j) acc -= A32[i * LDA + j] * t[j];
-            t[i] = acc;
-        }
-#pragma unroll
-        for (int i = 0; i < C; ++i) Tb[i * LDC + c] = __float2bfloat16(t[i]);
-    } else {
-        const int tid = threadIdx.x - C;                      // 0..63: one row each
-        const int i = tid;
+    // ---- the elementwise tiles: Qd and Kd to global, beta e^b K over Q, beta V in place
+    for (int x = threadIdx.x; x < C * (D / 8); x += NTP) {
+        const int i = x / (D / 8), c = (x % (D / 8)) * 8;
         const float bi = bcum[i], be = bet[i];
         const float fk = be * __expf(bi), fq = a.scale * __expf(bi), fd = __expf(btot - bi);
-        bf16* Qg = a.Qd + (cn * C + i) * D;
-        bf16* Kg = a.Kd + (cn * C + i) * D;
-#pragma unroll 4
-        for (int c = 0; c < D; c += 8) {
-            Vec<bf16> kx, vx, qx, o1, o2, o3, o4;
-            kx.load(Ks + i * LD + c);
-            vx.load(Vs + i * LD + c);
-            qx.load(Qs + i * LD + c);
+        Vec<bf16> kx, vx, qx, o1, o2, o3, o4;
+        kx.load(Ks + i * LD + c);
+        vx.load(Vs + i * LD + c);
+        qx.load(Qs + i * LD + c);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                o1.set(e, kx.get(e) * fk);
-                o2.set(e, vx.get(e) * be);
-                o3.set(e, qx.get(e) * fq);
-                o4.set(e, kx.get(e) * fd);
-            }
-            o1.store(Kb + i * LD + c);
-            o2.store(Vs + i * LD + c);
-            o3.store(Qg + c);
-            o4.store(Kg + c);
+        for (int e = 0; e < 8; ++e) {
+            o1.set(e, kx.get(e) * fk);
+            o2.set(e, vx.get(e) * be);
+            o3.set(e, qx.get(e) * fq);
+            o4.set(e, kx.get(e) * fd);
         }
-        if (tid == 0) a.gamma[cn] = __expf(btot);
+        o1.store(Qs + i * LD + c);
+        o2.store(Vs + i * LD + c);
+        o3.store(a.Qd + (cn * C + i) * D + c);
+        o4.store(a.Kd + (cn * C + i) * D + c);
+    }
+    if (threadIdx.x == 0) a.gamma[cn] = __expf(btot);
+    unit_lower_inverse(F);
+    {                                                        // T to bf16: read everything, then write over it
+        const int i = threadIdx.x >> 2, c = (threadIdx.x & 3) * 16;
+        float t[16];
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4*>(t + e) = *reinterpret_cast<const float4*>(F + i * LDF + c + e);
+        __syncthreads();
+        Vec<bf16> lo, hi;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            lo.set(e, c + e <= i ? t[e] : 0.f);              // above the diagonal is scratch
+            hi.set(e, c + 8 + e <= i ? t[8 + e] : 0.f);
+        }
+        lo.store(Tb + i * LDC + c);
+        hi.store(Tb + i * LDC + c + 8);
+        if (a.Tinv != nullptr) {
+            lo.store(a.Tinv + (cn * C + i) * C + c);
+            hi.store(a.Tinv + (cn * C + i) * C + c + 8);
+        }
     }
     __syncthreads();
-    // ---- W = T Kb, U = T (beta V): warp w -> rows 16w .. 16w+15, all D columns
-    {
-        float acc[D / 8][4];
-        zero_acc<D / 8>(acc);
-        warp_gemm<D / 8, C, false, true>(acc, Tb, LDC, 16 * w, Kb, LD, 0);
-        bf16* Wg = a.W + cn * C * D;
-        const int r = 16 * w + (l >> 2), cc = (l & 3) * 2;
+    // ---- W = T Kb, U = T (beta V): warp -> 16 rows, half of the columns; T is lower triangular
 #pragma unroll
-        for (int nt = 0; nt < D / 8; ++nt) {
-            *reinterpret_cast<__nv_bfloat162*>(Wg + r * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
-            *reinterpret_cast<__nv_bfloat162*>(Wg + (r + 8) * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
-        }
-        zero_acc<D / 8>(acc);
-        warp_gemm<D / 8, C, false, true>(acc, Tb, LDC, 16 * w, Vs, LD, 0);
-        bf16* Ug = a.U + cn * C * D;
+    for (int which = 0; which < 2; ++which) {
+        const bf16* X = which == 0 ? Qs : Vs;
+        bf16* Y = (which == 0 ? a.W : a.U) + cn * C * D + half * (D / 2);
+        float acc[NH][4];
+        zero_acc<NH>(acc);
+        for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<NH, 16, false, true>(acc, Tb + k0, LDC, m0, X + k0 * LD, LD, half * (D / 2));
+        const int r = m0 + (l >> 2), cc = (l & 3) * 2;
 #pragma unroll
-        for (int nt = 0; nt < D / 8; ++nt) {
-            *reinterpret_cast<__nv_bfloat162*>(Ug + r * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
-            *reinterpret_cast<__nv_bfloat162*>(Ug + (r + 8) * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
+        for (int nt = 0; nt < NH; ++nt) {
+            *reinterpret_cast<__nv_bfloat162*>(Y + r * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
+            *reinterpret_cast<__nv_bfloat162*>(Y + (r + 8) * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
         }
     }
 }
@@ -787,9 +856,7 @@ template <int D> constexpr size_t prep_bwd_smem() {
     return (size_t)(6 * C * (D + 8) + D * (D + 8) + 4 * C * (C + 8)) * 2 + (size_t)(C * (C + 1) + 4 * C + 4) * 4;
 }
 
-template <int D> constexpr size_t prep_smem() {
-    return (size_t)(4 * C * (D + 8) + C * (C + 8)) * 2 + (size_t)(C * (C + 1) + 2 * C) * 4;
-}
+template <int D> constexpr size_t prep_smem() { return (size_t)3 * C * (D + 8) * 2 + (size_t)(C * LDF + 2 * C) * 4; }
 
 }  // namespace dr
 }  // namespace lmoe
@@ -821,11 +888,11 @@ LMOE_API int lmoe_delta_prepare(int D, const dr::PrepArgs* ap, cudaStream_t st) 
     if (D == 128) {
         cudaError_t e = cudaFuncSetAttribute(dr::delta_prep_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dr::prep_smem<128>());
         if (e != cudaSuccess) return (int)e;
-        dr::delta_prep_fwd_kernel<128><<<grid, dr::NT, dr::prep_smem<128>(), st>>>(a);
+        dr::delta_prep_fwd_kernel<128><<<grid, dr::NTP, dr::prep_smem<128>(), st>>>(a);
     } else if (D == 64) {
         cudaError_t e = cudaFuncSetAttribute(dr::delta_prep_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dr::prep_smem<64>());
         if (e != cudaSuccess) return (int)e;
-        dr::delta_prep_fwd_kernel<64><<<grid, dr::NT, dr::prep_smem<64>(), st>>>(a);
+        dr::delta_prep_fwd_kernel<64><<<grid, dr::NTP, dr::prep_smem<64>(), st>>>(a);
     } else return -2;
     return (int)cudaGetLastError();
 }

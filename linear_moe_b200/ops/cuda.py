@@ -1410,13 +1410,13 @@ class _DeltaPrepArgs(ctypes.Structure):
     _fields_ = ([(n, ctypes.c_void_p) for n in ("q", "k", "v")] +
                 [(n, ctypes.c_longlong) for n in ("qs_b", "qs_t", "qs_h", "ks_b", "ks_t", "ks_h", "vs_b", "vs_t", "vs_h")] +
                 [(n, ctypes.c_void_p) for n in ("beta", "g", "W", "U", "Qd", "Kd", "A", "gamma")] +
-                [(n, ctypes.c_int) for n in ("B", "T", "H", "N")] + [("scale", ctypes.c_float)])
+                [(n, ctypes.c_int) for n in ("B", "T", "H", "N")] + [("scale", ctypes.c_float), ("Tinv", ctypes.c_void_p)])
 
 
-def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64):
+def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64, inverse=None):
     """The tiles of :func:`_delta_prepare` from one chunk-parallel kernel (``delta_prep_fwd_kernel``, csrc/lsm_delta.cu):
-    K K^T, the triangular inverse (forward substitution in registers), W, U, Q K^T and the decay-scaled copies of Q, K.
-    No autograd: used by the forward pass, which keeps only the inputs."""
+    K K^T, the triangular inverse (in fp32, by blocks), W, U, Q K^T and the decay-scaled copies of Q, K.
+    ``inverse``: a bf16 ``[B,H,N,C,C]`` buffer for the inverse.  No autograd: the forward pass keeps only the inputs."""
     B, T, H, D = q.shape
     N = (T + C - 1) // C
     q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
@@ -1434,6 +1434,7 @@ def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64):
     a.beta, a.g = bt.data_ptr(), 0 if gt is None else gt.data_ptr()
     a.W, a.U, a.Qd, a.Kd, a.A, a.gamma = (t.data_ptr() for t in (W, U, Qd, Kd, A, gamma))
     a.B, a.T, a.H, a.N, a.scale = B, T, H, N, float(scale)
+    a.Tinv = 0 if inverse is None else inverse.data_ptr()
     _check(lib().lmoe_delta_prepare(_i32(D), ctypes.byref(a), _st()), "delta_prepare")
     return W, U, Qd, Kd, A, gamma
 
