@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
 // The inverse is taken in fp32 by halves: the four 16 x 16 diagonal blocks by substitution, one column per thread, then
 // [[T0, 0], [-T1 (A10 T0), T1]] twice, with all threads on the small products.  A substitution over the whole chunk, one
 // column per thread, is a chain of 2016 multiply-adds on two warps; it was most of this kernel's time.
-// What bounds the kernel is the traffic of its five tiles (112 KB in and out per chunk at D = 128); three CTAs of eight
-// warps per SM overlap one chunk's loads with another's products.
+// What bounds the kernel is the traffic of its tiles (120 KB in and out per chunk at D = 128); three CTAs of eight warps per SM
+// overlap one chunk's loads with another's products.  2 x 4096 tokens, 16 heads of 128: 110 -> 88 us (floor 37).
 // ---------------------------------------------------------------------------------------------------------------
 struct PrepArgs {
     const bf16 *q, *k, *v;             // [B,T,H,D] with the strides below (elements)
@@ -483,9 +483,8 @@ __global__ void __launch_bounds__(NTP, 3) delta_prep_fwd_kernel(PrepArgs a) {
 // ---------------------------------------------------------------------------------------------------------------
 // Chunk-parallel backward of everything that is not the state recurrence: one CTA per (batch, head, chunk).
 // Inputs: q, k, v, beta, g (to rebuild the tiles), the entering state S_n and the gradient dS'_n of the leaving state,
-// Vn, dVn (= dU) and dO of the chunk (written by the two scan kernels).  The gradient of the chunk's total decay,
-// dgamma_n = <dS'_n, S_n> (gated case), is formed here too: every thread keeps its share of S_n in registers while the
-// state buffer is refilled with dS'_n.
+// Vn, dVn (= dU) and dO of the chunk (written by the two scan kernels), T from the tile kernel.  The gradient of the chunk's total
+// decay, dgamma_n = <dS'_n, S_n> (gated case), is formed here too.
 //
 //   through the scan equations      dW = -dVn S^T,  dQd = dO S^T,  dKd = Vn dS'^T,  dAqk = tril(dO Vn^T)
 //   through W = T Kb, U = T Vb      dKb = T^T dW,  dVb = T^T dU,  dT = dW Kb^T + dU Vb^T,  dA = -strict_lower(T^T dT T^T)
@@ -505,19 +504,21 @@ struct PrepBwdArgs {
     const float* beta;
     const float* g;                    // or null
     const bf16 *Sn, *dSn;              // [BH, N, D, D]
-    const bf16 *Vn, *dVn, *dO;         // [BH, N, C, D]
+    const bf16 *Vn, *dVn;              // [BH, N, C, D]
+    const bf16* dO;                    // strides below (elements; batch, token, head)
+    long long gs_b, gs_t, gs_h;
+    const bf16* Tinv;                  // [BH, N, C, C] from the tile kernel
     bf16 *dq, *dk, *dv;                // contiguous [B, T, H, D]
     float *dbeta, *dg;                 // [B, T, H]
     int B, T, H, N;
     float scale;
 };
 
-// sum over the thread's columns of acc[row][col] * tile[row][col] for its two rows (r, r + 8), reduced over the quad
+// lo / hi += sum over the thread's columns of acc[row][col] * tile[row][col] for its two rows (r, r + 8)
 template <int NTL>
 __device__ __forceinline__ void row_dot(const float (&acc)[NTL][4], const bf16* tile, int ld, int m0, float& lo, float& hi) {
     const int l = threadIdx.x & 31;
     const int r = m0 + (l >> 2), c = (l & 3) * 2;
-    lo = 0.f; hi = 0.f;
 #pragma unroll
     for (int nt = 0; nt < NTL; ++nt) {
         const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(tile + r * ld + c + nt * 8);
@@ -525,8 +526,12 @@ __device__ __forceinline__ void row_dot(const float (&acc)[NTL][4], const bf16* 
         lo += acc[nt][0] * __bfloat162float(a.x) + acc[nt][1] * __bfloat162float(a.y);
         hi += acc[nt][2] * __bfloat162float(b.x) + acc[nt][3] * __bfloat162float(b.y);
     }
-    lo += __shfl_xor_sync(0xffffffffu, lo, 1); lo += __shfl_xor_sync(0xffffffffu, lo, 2);
-    hi += __shfl_xor_sync(0xffffffffu, hi, 1); hi += __shfl_xor_sync(0xffffffffu, hi, 2);
+}
+
+template <int NTL>
+__device__ __forceinline__ void scale_rows(float (&acc)[NTL][4], float lo, float hi) {
+#pragma unroll
+    for (int nt = 0; nt < NTL; ++nt) { acc[nt][0] *= lo; acc[nt][1] *= lo; acc[nt][2] *= hi; acc[nt][3] *= hi; }
 }
 
 // write a warp's [16 x 8 NTL] accumulator rows to global rows (bf16), rows >= valid skipped
@@ -541,48 +546,59 @@ __device__ __forceinline__ void store_rows_global(const float (&acc)[NTL][4], bf
     }
 }
 
-// 256 threads: warp w works on rows 16 (w & 3) .. +15 and on column half (w >> 2) of every product, so that eight
-// warps per SM hide each other's shared-memory and tensor-pipe latencies (the tiles allow one CTA per SM only).
-constexpr int NTB = 256;
+// 512 threads: warp w works on rows 16 (w & 3) .. +15 and on column quarter (w >> 2) of every product (the tiles allow one CTA
+// per SM only, so sixteen warps hide each other's shared-memory and tensor-pipe latencies).  Of the C x C products only
+// the blocks on and below the diagonal are computed or read.  Sums over rows and columns stay in registers until the end: a
+// shared atomic per element and the substitution for T were two thirds of this kernel's time, T now comes from the tile kernel
+// that has just run.  Tiles arrive in the order they are needed.  Bound by shared-memory reads of the fragments (about 3 cycles per
+// 2 cycles of tensor pipe).  2 x 4096 tokens, 16 heads of 128: 580 -> 221 us.
+constexpr int NTB = 512;
 
 template <int D>
-__global__ void __launch_bounds__(NTB) delta_prep_bwd_kernel(PrepBwdArgs a) {
-    constexpr int LD = D + 8, LDC = C + 8, LDA = C + 1, NTH = D / 16, HD = D / 2;
+__global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
+    constexpr int LD = D + 8, LDC = C + 8, NQ = D / 32, QD = D / 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* Ks = reinterpret_cast<bf16*>(smem_raw);            // [C][LD]
     bf16* Qs = Ks + C * LD;                                  // [C][LD]
-    bf16* Vs = Qs + C * LD;                                  // [C][LD]  V, later beta V
+    bf16* Vs = Qs + C * LD;                                  // [C][LD]
     bf16* Gs = Vs + C * LD;                                  // [C][LD]  dO, later dW
     bf16* Ns = Gs + C * LD;                                  // [C][LD]  Vn
     bf16* Us = Ns + C * LD;                                  // [C][LD]  dVn = dU
-    bf16* Sb = Us + C * LD;                                  // [D][LD]  S_n, then dS'_n, then Kb (first C rows)
-    bf16* Tb = Sb + D * LD;                                  // [C][LDC] T
+    bf16* Sb = Us + C * LD;                                  // [D][LD]  S_n
+    bf16* Db = Sb + D * LD;                                  // [D][LD]  dS'_n
+    bf16* Tb = Db + D * LD;                                  // [C][LDC] T
     bf16* Ps = Tb + C * LDC;                                 // [C][LDC] P, later M
     bf16* X1 = Ps + C * LDC;                                 // [C][LDC] dT
     bf16* X2 = X1 + C * LDC;                                 // [C][LDC] T^T dT
-    float* GK = reinterpret_cast<float*>(X2 + C * LDC);      // [C][LDA] Gamma_ij (k_i.k_j), strictly lower
-    float* bcum = GK + C * LDA;                              // [C]
+    float* bcum = reinterpret_cast<float*>(X2 + C * LDC);    // [C]
     float* bet = bcum + C;                                   // [C]
-    float* db = bet + C;                                     // [C] gradient of the cumulative log decay
-    float* dbe = db + C;                                     // [C] gradient of beta
-    float* dgam = dbe + C;                                   // [1] <dS'_n, S_n>
+    float* rdb = bet + C;                                    // [4][C] row sums of the decay gradient, by column quarter
+    float* rbe = rdb + 4 * C;                                // [4][C] ... of the gradient of beta
+    float* cdb = rbe + 4 * C;                                // [4][C] column sums, by row block
+    float* tot = cdb + 4 * C;                                // [2][16] per warp: <dS'_n, S_n>, sum of <dKd_j, Kd_j>
     const int n = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int t0 = n * C;
     const int valid = min(C, a.T - t0);
     const long long cn = (long long)bh * a.N + n;
-    const int m0 = 16 * (w & 3), r0 = m0 + (l >> 2), c0 = (l & 3) * 2;
+    const int qd = w >> 2, m0 = 16 * (w & 3), r0 = m0 + (l >> 2), c0 = (l & 3) * 2;
     const bool gated = a.g != nullptr;
-    const int nd = (w >> 2) * HD;                            // first column of this warp's half of a D-wide product
-    const int nc = (w >> 2) * (C / 2);                       // ... of a C-wide product
+    const int nd = qd * QD;                                  // first column of this warp's quarter of a D-wide product
+    const int nc = qd * 16;                                  // ... of a C-wide product
+    const bool lower = nc <= m0;                             // does the warp's C x C block touch the lower triangle?
 
     load_tile_async<C, D, LD>(Ks, a.k + b * a.ks_b + h * a.ks_h + (long long)t0 * a.ks_t, a.ks_t, valid);
     load_tile_async<C, D, LD>(Qs, a.q + b * a.qs_b + h * a.qs_h + (long long)t0 * a.qs_t, a.qs_t, valid);
-    load_tile_async<C, D, LD>(Vs, a.v + b * a.vs_b + h * a.vs_h + (long long)t0 * a.vs_t, a.vs_t, valid);
-    load_tile_async<C, D, LD>(Gs, a.dO + cn * C * D, D, C);
+    cp_async_commit();
+    load_tile_async<C, D, LD>(Gs, a.dO + b * a.gs_b + h * a.gs_h + (long long)t0 * a.gs_t, a.gs_t, valid);
     load_tile_async<C, D, LD>(Ns, a.Vn + cn * C * D, D, C);
-    load_tile_async<C, D, LD>(Us, a.dVn + cn * C * D, D, C);
+    cp_async_commit();
     load_tile_async<D, D, LD>(Sb, a.Sn + cn * D * D, D, D);
+    load_tile_async<C, D, LD>(Us, a.dVn + cn * C * D, D, C);
+    cp_async_commit();
+    load_tile_async<C, C, LDC>(Tb, a.Tinv + cn * C * C, C, C);
+    load_tile_async<C, D, LD>(Vs, a.v + b * a.vs_b + h * a.vs_h + (long long)t0 * a.vs_t, a.vs_t, valid);
+    load_tile_async<D, D, LD>(Db, a.dSn + cn * D * D, D, D);
     cp_async_commit();
     if (w == 0) {
         const int i0 = 2 * l, i1 = 2 * l + 1;
@@ -593,267 +609,215 @@ __global__ void __launch_bounds__(NTB) delta_prep_bwd_kernel(PrepBwdArgs a) {
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const float x = __shfl_up_sync(0xffffffffu, s, o); if (l >= o) s += x; }
         bcum[i1] = s; bcum[i0] = s - g1; bet[i0] = be0; bet[i1] = be1;
-        db[i0] = db[i1] = 0.f; dbe[i0] = dbe[i1] = 0.f;
-        if (l == 0) dgam[0] = 0.f;
     }
-    cp_async_wait<0>();
+    cp_async_wait<3>();
     __syncthreads();
     const float btot = bcum[C - 1];
     const float b_lo = bcum[r0], b_hi = bcum[r0 + 8], be_lo = bet[r0], be_hi = bet[r0 + 8];
+    // this thread's sums: rows r0 and r0 + 8 over its columns, its four columns over its rows
+    float db_lo = 0.f, db_hi = 0.f, dbe_lo = 0.f, dbe_hi = 0.f, kd = 0.f, col[4] = {0.f, 0.f, 0.f, 0.f};
 
-    // ---- (1) K K^T -> GK (fp32), T by substitution (threads 0..63) ---------------------------------------------
-    {
-        float kk[4][4];
-        zero_acc<4>(kk);
-        warp_gemm<4, D, false, false>(kk, Ks, LD, m0, Ks, LD, nc);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + 8 * hh, j = nc + nt * 8 + c0;
-                const float bi = hh ? b_hi : b_lo;
-                GK[i * LDA + j] = i > j ? __expf(bi - bcum[j]) * kk[nt][2 * hh] : 0.f;
-                GK[i * LDA + j + 1] = i > j + 1 ? __expf(bi - bcum[j + 1]) * kk[nt][2 * hh + 1] : 0.f;
-            }
+    // ---- (1) K K^T and Q K^T, kept in registers ------------------------------------------------------------------
+    float kk[2][4], qk[2][4], gam[2][4];
+    zero_acc<2>(kk);
+    zero_acc<2>(qk);
+    if (lower) {
+        warp_gemm<2, D, false, false>(kk, Ks, LD, m0, Ks, LD, nc);
+        warp_gemm<2, D, false, false>(qk, Qs, LD, m0, Ks, LD, nc);
     }
-    __syncthreads();
-    if (threadIdx.x < C) {
-        const int c = threadIdx.x;
-        float t[C];
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-            float acc = 0.f;
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-            for (int j = 0; j < i; ++j) acc += GK[i * LDA + j] * t[j];
-            t[i] = ((i == c) ? 1.f : 0.f) - bet[i] * acc;
+        for (int e = 0; e < 4; ++e) {
+            const int i = r0 + 8 * (e >> 1), j = nc + nt * 8 + c0 + (e & 1);
+            gam[nt][e] = i >= j ? __expf(((e >> 1) ? b_hi : b_lo) - bcum[j]) : 0.f;             // Gamma_ij
         }
+    cp_async_wait<2>();
+    __syncthreads();
+    // ---- (2) dAqk = tril(dO Vn^T); P = scale Gamma . dAqk; decay gradients of Aqk ------------------------------------
+    if (lower) {
+        float da[2][4];
+        zero_acc<2>(da);
+        warp_gemm<2, D, false, false>(da, Gs, LD, m0, Ns, LD, nc);
 #pragma unroll
-        for (int i = 0; i < C; ++i) Tb[i * LDC + c] = __float2bfloat16(t[i]);
-    }
-    // ---- (2) dAqk = tril(dO Vn^T), Q K^T again for Aqk; P = scale Gamma . dAqk; decay gradients of Aqk ---------------
-    {
-        float da[4][4], qk[4][4];
-        zero_acc<4>(da);
-        zero_acc<4>(qk);
-        warp_gemm<4, D, false, false>(da, Gs, LD, m0, Ns, LD, nc);
-        warp_gemm<4, D, false, false>(qk, Qs, LD, m0, Ks, LD, nc);
-        float rs_lo = 0.f, rs_hi = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
+        for (int nt = 0; nt < 2; ++nt) {
             float pv[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int i = r0 + 8 * (e >> 1), j = nc + nt * 8 + c0 + (e & 1);
-                const float gam = i >= j ? a.scale * __expf((e >> 1 ? b_hi : b_lo) - bcum[j]) : 0.f;
-                pv[e] = gam * da[nt][e];                              // P_ij
+                pv[e] = a.scale * gam[nt][e] * da[nt][e];             // P_ij
                 const float t_ = pv[e] * qk[nt][e];                   // dAqk_ij Aqk_ij
-                if (e >> 1) rs_hi += t_; else rs_lo += t_;
-                if (i >= j) atomicAdd(&db[j], -t_);
+                if (e >> 1) db_hi += t_; else db_lo += t_;
+                col[2 * nt + (e & 1)] -= t_;
             }
             *reinterpret_cast<__nv_bfloat162*>(Ps + r0 * LDC + nc + nt * 8 + c0) = __floats2bfloat162_rn(pv[0], pv[1]);
             *reinterpret_cast<__nv_bfloat162*>(Ps + (r0 + 8) * LDC + nc + nt * 8 + c0) = __floats2bfloat162_rn(pv[2], pv[3]);
         }
-        rs_lo += __shfl_xor_sync(0xffffffffu, rs_lo, 1); rs_lo += __shfl_xor_sync(0xffffffffu, rs_lo, 2);
-        rs_hi += __shfl_xor_sync(0xffffffffu, rs_hi, 1); rs_hi += __shfl_xor_sync(0xffffffffu, rs_hi, 2);
-        if ((l & 3) == 0) { atomicAdd(&db[r0], rs_lo); atomicAdd(&db[r0 + 8], rs_hi); }
     }
-    __syncthreads();                                                   // Ps, Tb complete
-    // ---- (3) dq = scale e^b (dO S^T) + P K; its decay gradient <dQd_i, Qd_i> ----------------------------------------
-    float acc_dk[NTH][4];
-    zero_acc<NTH>(acc_dk);
-    {
-        float acc[NTH][4];
-        zero_acc<NTH>(acc);
-        warp_gemm<NTH, D, false, false>(acc, Gs, LD, m0, Sb, LD, nd); // dQd = dO S^T  (S stored [dk][dv] = [n][k])
-        const float f_lo = a.scale * __expf(b_lo), f_hi = a.scale * __expf(b_hi);
-#pragma unroll
-        for (int nt = 0; nt < NTH; ++nt) { acc[nt][0] *= f_lo; acc[nt][1] *= f_lo; acc[nt][2] *= f_hi; acc[nt][3] *= f_hi; }
-        float d_lo, d_hi;
-        row_dot<NTH>(acc, Qs + nd, LD, m0, d_lo, d_hi);               // = <dQd_i, Qd_i> over this warp's columns
-        if ((l & 3) == 0) { atomicAdd(&db[r0], d_lo); atomicAdd(&db[r0 + 8], d_hi); }
-        warp_gemm<NTH, C, false, true>(acc, Ps, LDC, m0, Ks, LD, nd); // + P K
-        store_rows_global<NTH>(acc, a.dq + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
-        // dk += P^T Q
-        warp_gemm<NTH, C, true, true>(acc_dk, Ps, LDC, m0, Qs, LD, nd);
-    }
-    // ---- (4) dW = -dVn S^T -> shared (in dO's buffer once every warp is done with dO) --------------------------------
-    {
-        float acc[NTH][4];
-        zero_acc<NTH>(acc);
-        warp_gemm<NTH, D, false, false>(acc, Us, LD, m0, Sb, LD, nd);
-#pragma unroll
-        for (int nt = 0; nt < NTH; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[nt][e] = -acc[nt][e];
-        __syncthreads();                                               // all reads of dO (Gs) and S_n (Sb) are done
-        store_acc_bf16<NTH>(acc, Gs, LD, m0, nd);                      // Gs now holds dW
-    }
-    // ---- (5) dS'_n into the state buffer; dgamma = <dS'_n, S_n>; dKd = Vn dS'^T --------------------------------------
-    constexpr int SPT = D * D / 8 / NTB;                               // 16-byte pieces of the state per thread
-    uint4 keep[SPT];
-    if (gated) {
-#pragma unroll
-        for (int i = 0; i < SPT; ++i) {
-            const int idx = threadIdx.x + i * NTB;
-            keep[i] = *reinterpret_cast<const uint4*>(Sb + (idx / (D / 8)) * LD + (idx % (D / 8)) * 8);
-        }
-        __syncthreads();                                               // every thread has its share before the refill
-    }
-    load_tile_async<D, D, LD>(Sb, a.dSn + cn * D * D, D, D);
-    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();                                                   // Ps, S_n, dVn
+    // ---- (3) dq = scale e^b (dO S^T) + P K; its decay gradient <dQd_i, Qd_i>; dk += P^T Q -----------------------------
+    float acc_dk[NQ][4], acc[NQ][4];
+    zero_acc<NQ>(acc_dk);
+    zero_acc<NQ>(acc);
+    warp_gemm<NQ, D, false, false>(acc, Gs, LD, m0, Sb, LD, nd);      // dQd = dO S^T  (S stored [dk][dv] = [n][k])
+    scale_rows<NQ>(acc, a.scale * __expf(b_lo), a.scale * __expf(b_hi));
+    row_dot<NQ>(acc, Qs + nd, LD, m0, db_lo, db_hi);                  // <dQd_i, Qd_i> over this thread's columns
+    for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<NQ, 16, false, true>(acc, Ps + k0, LDC, m0, Ks + k0 * LD, LD, nd);
+    store_rows_global<NQ>(acc, a.dq + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
+    for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<NQ, 16, true, true>(acc_dk, Ps + k0 * LDC, LDC, m0, Qs + k0 * LD, LD, nd);
+    // ---- (4) dW = -dVn S^T -> shared, in dO's buffer once every warp is done with dO ---------------------------------
+    zero_acc<NQ>(acc);
+    warp_gemm<NQ, D, false, false>(acc, Us, LD, m0, Sb, LD, nd);
+    scale_rows<NQ>(acc, -1.f, -1.f);
     cp_async_wait<0>();
-    __syncthreads();
+    __syncthreads();                                                   // dO is free; T, V, dS'_n are here
+    store_acc_bf16<NQ>(acc, Gs, LD, m0, nd);                           // Gs now holds dW
+    // ---- (5) dgamma = <dS'_n, S_n>; dKd = Vn dS'^T -------------------------------------------------------------------
+    float dgam = 0.f;
     if (gated) {
-        float dot = 0.f;
-#pragma unroll
-        for (int i = 0; i < SPT; ++i) {
-            const int idx = threadIdx.x + i * NTB;
-            const uint4 d = *reinterpret_cast<const uint4*>(Sb + (idx / (D / 8)) * LD + (idx % (D / 8)) * 8);
-            const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&keep[i]);
-            const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&d);
+        for (int i = threadIdx.x; i < D * D / 8; i += NTB) {
+            const int o = (i / (D / 8)) * LD + (i % (D / 8)) * 8;
+            const uint4 x4 = *reinterpret_cast<const uint4*>(Sb + o), y4 = *reinterpret_cast<const uint4*>(Db + o);
+            const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&x4), *y = reinterpret_cast<const __nv_bfloat162*>(&y4);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float2 fx = __bfloat1622float2(x[e]), fy = __bfloat1622float2(y[e]);
-                dot += fx.x * fy.x + fx.y * fy.y;
+                dgam += fx.x * fy.x + fx.y * fy.y;
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (l == 0) atomicAdd(dgam, dot);
     }
+    zero_acc<NQ>(acc);
+    warp_gemm<NQ, D, false, false>(acc, Ns, LD, m0, Db, LD, nd);      // dKd_j = Vn_j dS'^T
+    scale_rows<NQ>(acc, __expf(btot - b_lo), __expf(btot - b_hi));
     {
-        float acc[NTH][4];
-        zero_acc<NTH>(acc);
-        warp_gemm<NTH, D, false, false>(acc, Ns, LD, m0, Sb, LD, nd); // dKd_j = Vn_j dS'^T
-        const float f_lo = __expf(btot - b_lo), f_hi = __expf(btot - b_hi);
-#pragma unroll
-        for (int nt = 0; nt < NTH; ++nt) { acc[nt][0] *= f_lo; acc[nt][1] *= f_lo; acc[nt][2] *= f_hi; acc[nt][3] *= f_hi; }
-        float d_lo, d_hi;
-        row_dot<NTH>(acc, Ks + nd, LD, m0, d_lo, d_hi);               // <dKd_j, Kd_j>
-        if ((l & 3) == 0) {
-            atomicAdd(&db[r0], -d_lo); atomicAdd(&db[r0 + 8], -d_hi);
-            atomicAdd(&db[C - 1], d_lo + d_hi);
-        }
-#pragma unroll
-        for (int nt = 0; nt < NTH; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc_dk[nt][e] += acc[nt][e];
+        float d_lo = 0.f, d_hi = 0.f;
+        row_dot<NQ>(acc, Ks + nd, LD, m0, d_lo, d_hi);                // <dKd_j, Kd_j>
+        db_lo -= d_lo; db_hi -= d_hi;
+        kd = d_lo + d_hi;
     }
-    __syncthreads();                                                   // dS'_n no longer needed: Sb becomes Kb
-    // ---- (6) dVb = T^T dU: dv, dbeta; then Kb = beta e^b K and Vb = beta V in shared -------------------------------
-    {
-        float acc[NTH][4];
-        zero_acc<NTH>(acc);
-        warp_gemm<NTH, C, true, true>(acc, Tb, LDC, m0, Us, LD, nd);
-        float d_lo, d_hi;
-        row_dot<NTH>(acc, Vs + nd, LD, m0, d_lo, d_hi);               // <dVb_i, v_i>
-        if ((l & 3) == 0) { atomicAdd(&dbe[r0], d_lo); atomicAdd(&dbe[r0 + 8], d_hi); }
 #pragma unroll
-        for (int nt = 0; nt < NTH; ++nt) { acc[nt][0] *= be_lo; acc[nt][1] *= be_lo; acc[nt][2] *= be_hi; acc[nt][3] *= be_hi; }
-        store_rows_global<NTH>(acc, a.dv + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
-    }
-    __syncthreads();                                                   // every warp has read raw V
-    for (int i = threadIdx.x; i < C * (D / 8); i += NTB) {
-        const int r = i / (D / 8), c = (i % (D / 8)) * 8;
-        const float be = bet[r], fk = be * __expf(bcum[r]);
-        Vec<bf16> kx, vx, o1, o2;
-        kx.load(Ks + r * LD + c);
-        vx.load(Vs + r * LD + c);
+    for (int nt = 0; nt < NQ; ++nt)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { o1.set(e, kx.get(e) * fk); o2.set(e, vx.get(e) * be); }
-        o1.store(Sb + r * LD + c);                                     // Kb
-        o2.store(Vs + r * LD + c);                                     // Vb
-    }
-    __syncthreads();
+        for (int e = 0; e < 4; ++e) acc_dk[nt][e] += acc[nt][e];
+    // ---- (6) dVb = T^T dU: dv, dbeta --------------------------------------------------------------------------------
+    zero_acc<NQ>(acc);
+    for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<NQ, 16, true, true>(acc, Tb + k0 * LDC, LDC, m0, Us + k0 * LD, LD, nd);
+    row_dot<NQ>(acc, Vs + nd, LD, m0, dbe_lo, dbe_hi);                // <dVb_i, v_i>
+    scale_rows<NQ>(acc, be_lo, be_hi);
+    store_rows_global<NQ>(acc, a.dv + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
+    __syncthreads();                                                   // dW complete
     // ---- (7) dKb = T^T dW: its part of dk, dbeta and db -------------------------------------------------------------
+    zero_acc<NQ>(acc);
+    for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<NQ, 16, true, true>(acc, Tb + k0 * LDC, LDC, m0, Gs + k0 * LD, LD, nd);
     {
-        float acc[NTH][4];
-        zero_acc<NTH>(acc);
-        warp_gemm<NTH, C, true, true>(acc, Tb, LDC, m0, Gs, LD, nd);
-        float d_lo, d_hi;
-        row_dot<NTH>(acc, Ks + nd, LD, m0, d_lo, d_hi);               // <dKb_i, k_i>
-        const float e_lo = __expf(b_lo), e_hi = __expf(b_hi);
-        if ((l & 3) == 0) {
-            atomicAdd(&dbe[r0], e_lo * d_lo); atomicAdd(&dbe[r0 + 8], e_hi * d_hi);
-            atomicAdd(&db[r0], be_lo * e_lo * d_lo); atomicAdd(&db[r0 + 8], be_hi * e_hi * d_hi);
-        }
+        float d_lo = 0.f, d_hi = 0.f;
+        row_dot<NQ>(acc, Ks + nd, LD, m0, d_lo, d_hi);                // <dKb_i, k_i>
+        const float e_lo = __expf(b_lo), e_hi = __expf(b_hi), f_lo = be_lo * e_lo, f_hi = be_hi * e_hi;
+        dbe_lo += e_lo * d_lo; dbe_hi += e_hi * d_hi;
+        db_lo += f_lo * d_lo; db_hi += f_hi * d_hi;
 #pragma unroll
-        for (int nt = 0; nt < NTH; ++nt) {
-            acc_dk[nt][0] += be_lo * e_lo * acc[nt][0]; acc_dk[nt][1] += be_lo * e_lo * acc[nt][1];
-            acc_dk[nt][2] += be_hi * e_hi * acc[nt][2]; acc_dk[nt][3] += be_hi * e_hi * acc[nt][3];
+        for (int nt = 0; nt < NQ; ++nt) {
+            acc_dk[nt][0] += f_lo * acc[nt][0]; acc_dk[nt][1] += f_lo * acc[nt][1];
+            acc_dk[nt][2] += f_hi * acc[nt][2]; acc_dk[nt][3] += f_hi * acc[nt][3];
         }
     }
-    // ---- (8) dT = dW Kb^T + dU Vb^T -> X1;  X2 = T^T dT;  dA = -(X2 T^T), strictly lower ------------------------------
-    {
-        float acc[4][4];
-        zero_acc<4>(acc);
-        warp_gemm<4, D, false, false>(acc, Gs, LD, m0, Sb, LD, nc);
-        warp_gemm<4, D, false, false>(acc, Us, LD, m0, Vs, LD, nc);
-        store_acc_bf16<4>(acc, X1, LDC, m0, nc);
-    }
-    __syncthreads();
-    {
-        float acc[4][4];
-        zero_acc<4>(acc);
-        warp_gemm<4, C, true, true>(acc, Tb, LDC, m0, X1, LDC, nc);
-        store_acc_bf16<4>(acc, X2, LDC, m0, nc);
-    }
-    __syncthreads();
-    {
-        float acc[4][4];
-        zero_acc<4>(acc);
-        warp_gemm<4, C, false, false>(acc, X2, LDC, m0, Tb, LDC, nc); // (X2 T^T)_ij = sum_k X2_ik T_jk
-        float rb_lo = 0.f, rb_hi = 0.f, rd_lo = 0.f, rd_hi = 0.f;
+    // ---- (8) dT_ij = beta_j e^{b_j} (dW_i . k_j) + beta_j (dU_i . v_j) -> X1;  X2 = T^T dT;  dA = -(X2 T^T), strictly lower
+    if (lower) {
+        float x[2][4], y[2][4];
+        zero_acc<2>(x);
+        zero_acc<2>(y);
+        warp_gemm<2, D, false, false>(x, Gs, LD, m0, Ks, LD, nc);
+        warp_gemm<2, D, false, false>(y, Us, LD, m0, Vs, LD, nc);
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int j = nc + nt * 8 + c0 + (e & 1);
+                x[nt][e] = bet[j] * (__expf(bcum[j]) * x[nt][e] + y[nt][e]);
+            }
+        store_acc_bf16<2>(x, X1, LDC, m0, nc);
+    }
+    __syncthreads();
+    if (lower) {
+        float x[2][4];
+        zero_acc<2>(x);
+        for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<2, 16, true, true>(x, Tb + k0 * LDC, LDC, m0, X1 + k0 * LDC, LDC, nc);
+        store_acc_bf16<2>(x, X2, LDC, m0, nc);
+    }
+    __syncthreads();
+    if (lower) {
+        float x[2][4];
+        zero_acc<2>(x);
+        for (int k0 = 0; k0 <= nc; k0 += 16) warp_gemm<2, 16, false, false>(x, X2 + k0, LDC, m0, Tb + k0, LDC, nc);   // (X2 T^T)_ij = sum_k X2_ik T_jk
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
             float mv[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int i = r0 + 8 * (e >> 1), j = nc + nt * 8 + c0 + (e & 1);
-                const float dA = i > j ? -acc[nt][e] : 0.f;
-                const float gk = GK[i * LDA + j];                      // Gamma_ij (k_i.k_j), zero on and above the diagonal
+                const float dA = i > j ? -x[nt][e] : 0.f;
                 const float be = (e >> 1) ? be_hi : be_lo;
-                const float t1 = dA * gk;                              // -> dbeta_i
+                const float t1 = dA * gam[nt][e] * kk[nt][e];          // dA_ij Gamma_ij (k_i.k_j) -> dbeta_i
                 const float t2 = t1 * be;                              // dA_ij A_ij -> db_i, -db_j
-                if (e >> 1) { rb_hi += t1; rd_hi += t2; } else { rb_lo += t1; rd_lo += t2; }
-                if (i > j) atomicAdd(&db[j], -t2);
-                mv[e] = i > j ? dA * be * __expf(((e >> 1) ? b_hi : b_lo) - bcum[j]) : 0.f;      // M_ij
+                if (e >> 1) { dbe_hi += t1; db_hi += t2; } else { dbe_lo += t1; db_lo += t2; }
+                col[2 * nt + (e & 1)] -= t2;
+                mv[e] = dA * be * gam[nt][e];                          // M_ij
             }
             *reinterpret_cast<__nv_bfloat162*>(Ps + r0 * LDC + nc + nt * 8 + c0) = __floats2bfloat162_rn(mv[0], mv[1]);
             *reinterpret_cast<__nv_bfloat162*>(Ps + (r0 + 8) * LDC + nc + nt * 8 + c0) = __floats2bfloat162_rn(mv[2], mv[3]);
         }
-#pragma unroll
-        for (int o = 1; o <= 2; o <<= 1) {
-            rb_lo += __shfl_xor_sync(0xffffffffu, rb_lo, o); rb_hi += __shfl_xor_sync(0xffffffffu, rb_hi, o);
-            rd_lo += __shfl_xor_sync(0xffffffffu, rd_lo, o); rd_hi += __shfl_xor_sync(0xffffffffu, rd_hi, o);
-        }
-        if ((l & 3) == 0) {
-            atomicAdd(&dbe[r0], rb_lo); atomicAdd(&dbe[r0 + 8], rb_hi);
-            atomicAdd(&db[r0], rd_lo); atomicAdd(&db[r0 + 8], rd_hi);
-        }
     }
-    __syncthreads();                                                   // Ps holds M
+    // the sums of this warp: rows over the four lanes that share them, columns over the eight
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+        db_lo += __shfl_xor_sync(0xffffffffu, db_lo, o); db_hi += __shfl_xor_sync(0xffffffffu, db_hi, o);
+        dbe_lo += __shfl_xor_sync(0xffffffffu, dbe_lo, o); dbe_hi += __shfl_xor_sync(0xffffffffu, dbe_hi, o);
+    }
+#pragma unroll
+    for (int o = 4; o <= 16; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) col[i] += __shfl_xor_sync(0xffffffffu, col[i], o);
+    kd = warp_sum(kd);
+    dgam = warp_sum(dgam);
+    if ((l & 3) == 0) {
+        rdb[qd * C + r0] = db_lo; rdb[qd * C + r0 + 8] = db_hi;
+        rbe[qd * C + r0] = dbe_lo; rbe[qd * C + r0 + 8] = dbe_hi;
+    }
+    if (l < 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cdb[(w & 3) * C + nc + (i >> 1) * 8 + c0 + (i & 1)] = col[i];
+    }
+    if (l == 0) { tot[w] = dgam; tot[16 + w] = kd; }
+    __syncthreads();                                                   // Ps holds M; the sums are in
     // ---- (9) dk += M K + M^T K; store ---------------------------------------------------------------------------------
-    warp_gemm<NTH, C, false, true>(acc_dk, Ps, LDC, m0, Ks, LD, nd);
-    warp_gemm<NTH, C, true, true>(acc_dk, Ps, LDC, m0, Ks, LD, nd);
-    store_rows_global<NTH>(acc_dk, a.dk + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
-    __syncthreads();                                                   // all contributions to db / dbeta are in
-    // ---- (10) dbeta; dg_s = sum_{i >= s} db_i (+ dgamma gamma on the last position) -----------------------------------
+    for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<NQ, 16, false, true>(acc_dk, Ps + k0, LDC, m0, Ks + k0 * LD, LD, nd);
+    for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<NQ, 16, true, true>(acc_dk, Ps + k0 * LDC, LDC, m0, Ks + k0 * LD, LD, nd);
+    store_rows_global<NQ>(acc_dk, a.dk + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
+    // ---- (10) dbeta; dg_s = sum_{i >= s} db_i (b_C also gets the sum of <dKd_j, Kd_j> and dgamma gamma) -------------------
     if (w == 0) {
         const int i0 = 2 * l, i1 = 2 * l + 1;
-        float x0 = db[i0], x1 = db[i1];
-        if (gated && l == 31) x1 += dgam[0] * __expf(btot);             // gamma = e^{b_C}: d b_C += dgamma gamma
+        float x0 = 0.f, x1 = 0.f, be0 = 0.f, be1 = 0.f, last = 0.f;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            x0 += rdb[p * C + i0] + cdb[p * C + i0]; x1 += rdb[p * C + i1] + cdb[p * C + i1];
+            be0 += rbe[p * C + i0]; be1 += rbe[p * C + i1];
+        }
+        if (l == 31) {
+            const float gamma = __expf(btot);                          // gamma = e^{b_C}: d b_C += dgamma gamma
+            for (int p = 0; p < NTB / 32; ++p) last += tot[p] * gamma + tot[16 + p];
+            x1 += last;
+        }
         float s = x0 + x1;                                             // suffix sums over lane pairs
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const float y = __shfl_down_sync(0xffffffffu, s, o); if (l + o < 32) s += y; }
         const long long o0 = ((long long)b * a.T + t0 + i0) * a.H + h, o1 = o0 + a.H;
-        if (i0 < valid) { a.dbeta[o0] = dbe[i0]; if (a.dg != nullptr) a.dg[o0] = s; }
-        if (i1 < valid) { a.dbeta[o1] = dbe[i1]; if (a.dg != nullptr) a.dg[o1] = s - x0; }
+        if (i0 < valid) { a.dbeta[o0] = be0; if (a.dg != nullptr) a.dg[o0] = s; }
+        if (i1 < valid) { a.dbeta[o1] = be1; if (a.dg != nullptr) a.dg[o1] = s - x0; }
     }
 }
 
 template <int D> constexpr size_t prep_bwd_smem() {
-    return (size_t)(6 * C * (D + 8) + D * (D + 8) + 4 * C * (C + 8)) * 2 + (size_t)(C * (C + 1) + 4 * C + 4) * 4;
+    return (size_t)(6 * C * (D + 8) + 2 * D * (D + 8) + 4 * C * (C + 8)) * 2 + (size_t)(14 * C + 32) * 4;
 }
 
 template <int D> constexpr size_t prep_smem() { return (size_t)3 * C * (D + 8) * 2 + (size_t)(C * LDF + 2 * C) * 4; }

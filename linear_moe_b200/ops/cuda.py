@@ -1513,11 +1513,13 @@ class _DeltaChunkScan(torch.autograd.Function):
 class _DeltaPrepBwdArgs(ctypes.Structure):
     _fields_ = ([(n, ctypes.c_void_p) for n in ("q", "k", "v")] +
                 [(n, ctypes.c_longlong) for n in ("qs_b", "qs_t", "qs_h", "ks_b", "ks_t", "ks_h", "vs_b", "vs_t", "vs_h")] +
-                [(n, ctypes.c_void_p) for n in ("beta", "g", "Sn", "dSn", "Vn", "dVn", "dO", "dq", "dk", "dv", "dbeta", "dg")] +
+                [(n, ctypes.c_void_p) for n in ("beta", "g", "Sn", "dSn", "Vn", "dVn", "dO")] +
+                [(n, ctypes.c_longlong) for n in ("gs_b", "gs_t", "gs_h")] +
+                [(n, ctypes.c_void_p) for n in ("Tinv", "dq", "dk", "dv", "dbeta", "dg")] +
                 [(n, ctypes.c_int) for n in ("B", "T", "H", "N")] + [("scale", ctypes.c_float)])
 
 
-def _delta_prepare_bwd_kernel(q, k, v, beta, g, scale, Sn, dSn, Vn, dVn, dO):
+def _delta_prepare_bwd_kernel(q, k, v, beta, g, scale, Sn, dSn, Vn, dVn, dO, Tinv):
     """Gradients of ``q, k, v, beta, g`` from what the two scan kernels wrote, one chunk-parallel kernel
     (``delta_prep_bwd_kernel``, csrc/lsm_delta.cu): the chunk-local scan equations, ``W = T Kb`` / ``U = T Vb``, the
     triangular inverse and the decay factors are differentiated in shared memory on the tensor cores."""
@@ -1536,7 +1538,8 @@ def _delta_prepare_bwd_kernel(q, k, v, beta, g, scale, Sn, dSn, Vn, dVn, dO):
     a.ks_b, a.ks_t, a.ks_h = k.stride(0), k.stride(1), k.stride(2)
     a.vs_b, a.vs_t, a.vs_h = v.stride(0), v.stride(1), v.stride(2)
     a.beta, a.g = bt.data_ptr(), 0 if gt is None else gt.data_ptr()
-    a.Sn, a.dSn, a.Vn, a.dVn, a.dO = (t.data_ptr() for t in (Sn, dSn, Vn, dVn, dO))
+    a.Sn, a.dSn, a.Vn, a.dVn, a.dO, a.Tinv = (t.data_ptr() for t in (Sn, dSn, Vn, dVn, dO, Tinv))
+    a.gs_b, a.gs_h, a.gs_t = dO.stride(0), dO.stride(1), dO.stride(3)      # [B,H,N,C,D], the chunks of a head one behind the other
     a.dq, a.dk, a.dv, a.dbeta = dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dbeta.data_ptr()
     a.dg = 0 if dg is None else dg.data_ptr()
     a.B, a.T, a.H, a.N, a.scale = B, T, H, N, float(scale)
@@ -1601,15 +1604,16 @@ def _delta_backward_kernels(ctx, do, dS):
     q, k, v, beta, g, s0 = ctx.saved_tensors
     B, T, H, D = q.shape
     with torch.no_grad():
-        W, U, Qd, Kd, A, gamma = _delta_prepare_kernel(q, k, v, beta, g, ctx.scale)
-        N, C = W.shape[2], W.shape[3]
+        N, C = (T + 63) // 64, 64
+        Tinv = torch.empty(B, H, N, C, C, dtype=torch.bfloat16, device=q.device)
+        W, U, Qd, Kd, A, gamma = _delta_prepare_kernel(q, k, v, beta, g, ctx.scale, inverse=Tinv)
         _, Vn, Sn, _ = _delta_scan_fwd(W, U, Qd, Kd, A, gamma, s0)
         dO = do.to(torch.bfloat16)
         if N * C != T:
             dO = F.pad(dO, (0, 0, 0, 0, 0, N * C - T))
         dO = dO.reshape(B, N, C, H, D).permute(0, 3, 1, 2, 4).contiguous()
         dVn, dSn, dS0 = _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dS)
-        dq, dk, dv, dbeta, dg = _delta_prepare_bwd_kernel(q, k, v, beta, g, ctx.scale, Sn, dSn, Vn, dVn, dO)
+        dq, dk, dv, dbeta, dg = _delta_prepare_bwd_kernel(q, k, v, beta, g, ctx.scale, Sn, dSn, Vn, dVn, dO, Tinv)
     need = ctx.needs_input_grad
     return (dq.to(q.dtype) if need[0] else None, dk.to(k.dtype) if need[1] else None, dv.to(v.dtype) if need[2] else None,
             dbeta.to(beta.dtype) if need[3] else None, (dg.to(g.dtype) if (g is not None and need[4]) else None),
