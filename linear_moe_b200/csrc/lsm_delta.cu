@@ -26,43 +26,51 @@ namespace dr {
 
 constexpr int C = 64;            // chunk length
 constexpr int DVS = 32;          // value columns per CTA
-constexpr int NT = 128;          // threads
+constexpr int NT = 256;          // threads
 
 struct Args {
     const bf16 *W, *U, *Qd, *Kd, *A;   // [BH, N, C, dk] / [BH, N, C, dv] / [BH, N, C, C]
     const float* gamma;                // [BH, N]
     const float* S0;                   // [BH, dk, dv] or null
-    const bf16* dO;                    // backward: [BH, N, C, dv]
+    const bf16* dO;                    // backward: [B, T, H, dv] with the strides gs_*
     const float* dSfinal;              // backward: [BH, dk, dv] or null
-    bf16* O;                           // forward: [BH, N, C, dv]
-    bf16* Vn;                          // forward out / backward in: [BH, N, C, dv]
+    bf16* O;                           // forward: [B, T, H, dv] with the strides os_*, or null (not wanted)
+    bf16* Vn;                          // forward out: [BH, N, C, dv], or null (neither Vn nor Sn is kept)
     bf16* Sn;                          // forward out: state entering chunk n, [BH, N, dk, dv]
     float* Sfinal;                     // forward out: [BH, dk, dv]
     bf16* dVn;                         // backward out: [BH, N, C, dv]
     bf16* dSn;                         // backward out: gradient of the state leaving chunk n, [BH, N, dk, dv]
     float* dS0;                        // backward out: [BH, dk, dv]
-    int N, dv;
+    long long os_b, os_t, os_h, gs_b, gs_t, gs_h;
+    int N, dv, T, H;
 };
 
+// Both walks are chains over the chunks, bound by the latency of a step: two products with a barrier behind each.  Eight warps
+// share a step's tiles, everything that does not depend on the state is taken off the chain (the outputs by four warps beside
+// the other four's pseudo values; Qd^T dO ahead of the barrier), and the next chunk's tiles arrive during the step.
+// 2 x 4096 tokens, 16 heads of 128 (64 chunks, 128 CTAs): forward 169 -> 142 us, without outputs 107, reverse 150 -> 140.
 template <int DK> struct Cfg {
     static constexpr int LDK = DK + 8;
     static constexpr int LDC = C + 8;
     static constexpr int LDV = DVS + 8;
-    static constexpr int RB = DK / 64;              // 16-row blocks of the state per warp (4 warps)
-    // shared memory (bf16 elements): 2 x {W, Qd, Kd: C x LDK; A: C x LDC; X (U or dO): C x LDV} + Sb [DK x LDV] + Vb [C x LDV] (+ Gb)
-    static constexpr int STAGE = 3 * C * LDK + C * LDC + C * LDV;
-    static constexpr size_t SMEM = (size_t)(2 * STAGE + DK * LDV + 2 * C * LDV) * 2;
+    static constexpr int SN = DK == 128 ? 4 : 2;    // the state's n-tiles per warp: 16 rows x 32 columns (dk = 128) or x 16 (dk = 64)
+    // a stage (bf16 elements): W, Kd: C x LDK; X (U or dO): C x LDV; Qd: C x LDK; A: C x LDC (the last two not where no output is wanted)
+    static constexpr int QD = 2 * C * LDK + C * LDV, AQ = QD + C * LDK;
+    static constexpr int FULL = AQ + C * LDC;
+    static constexpr size_t smem(bool out) { return (size_t)(2 * (out ? FULL : QD) + DK * LDV + 2 * C * LDV) * 2; }      // + state, Vn, O
 };
 
-template <int DK>
-__device__ __forceinline__ void issue_chunk(bf16* st, const Args& a, const bf16* xsrc, long long bh, int n, int col0) {
+template <int DK, bool FULL>
+__device__ __forceinline__ void issue_chunk(bf16* st, const Args& a, const bf16* x, long long xs_t, int x_rows, long long bh, int n) {
     using F = Cfg<DK>;
     const long long cn = bh * a.N + n;
     load_tile_async<C, DK, F::LDK>(st, a.W + cn * C * DK, DK, C);
-    load_tile_async<C, DK, F::LDK>(st + C * F::LDK, a.Qd + cn * C * DK, DK, C);
-    load_tile_async<C, DK, F::LDK>(st + 2 * C * F::LDK, a.Kd + cn * C * DK, DK, C);
-    load_tile_async<C, C, F::LDC>(st + 3 * C * F::LDK, a.A + cn * C * C, C, C);
-    load_tile_async<C, DVS, F::LDV>(st + 3 * C * F::LDK + C * F::LDC, xsrc + cn * C * a.dv + col0, a.dv, C);
+    load_tile_async<C, DK, F::LDK>(st + C * F::LDK, a.Kd + cn * C * DK, DK, C);
+    load_tile_async<C, DVS, F::LDV>(st + 2 * C * F::LDK, x + (long long)n * C * xs_t, xs_t, x_rows - n * C);
+    if (FULL) {
+        load_tile_async<C, DK, F::LDK>(st + F::QD, a.Qd + cn * C * DK, DK, C);
+        load_tile_async<C, C, F::LDC>(st + F::AQ, a.A + cn * C * C, C, C);
+    }
 }
 
 // write a [rows x DVS] bf16 tile held in shared memory (row stride LDV) to global rows of stride `gld`
@@ -74,183 +82,166 @@ __device__ __forceinline__ void store_rows(const bf16* s, bf16* g, int rows, lon
     }
 }
 
-template <int DK>
+// this warp's tile of an fp32 state [dk][dv] (null: zeros), to registers and in bf16 to shared memory; and back
+template <int SN>
+__device__ __forceinline__ void load_state(float (&S)[SN][4], const float* src, int dv, int col0, bf16* Sb, int ldv, int m0, int n0) {
+    const int l = threadIdx.x & 31, r = m0 + (l >> 2);
+#pragma unroll
+    for (int nt = 0; nt < SN; ++nt) {
+        const int c = col0 + n0 + nt * 8 + (l & 3) * 2;
+        if (src != nullptr) {
+            const float* p = src + (long long)r * dv + c;
+            S[nt][0] = p[0]; S[nt][1] = p[1];
+            S[nt][2] = p[8 * dv]; S[nt][3] = p[8 * dv + 1];
+        } else {
+            S[nt][0] = S[nt][1] = S[nt][2] = S[nt][3] = 0.f;
+        }
+    }
+    store_acc_bf16<SN>(S, Sb, ldv, m0, n0);
+}
+template <int SN>
+__device__ __forceinline__ void save_state(const float (&S)[SN][4], float* dst, int dv, int col0, int m0, int n0) {
+    const int l = threadIdx.x & 31, r = m0 + (l >> 2);
+#pragma unroll
+    for (int nt = 0; nt < SN; ++nt) {
+        float* p = dst + (long long)r * dv + col0 + n0 + nt * 8 + (l & 3) * 2;
+        p[0] = S[nt][0]; p[1] = S[nt][1];
+        p[8 * dv] = S[nt][2]; p[8 * dv + 1] = S[nt][3];
+    }
+}
+
+// OUT: the outputs O are wanted (the forward pass); without: Vn and the entering states only (what the backward pass rebuilds).
+template <int DK, bool OUT>
 __global__ void __launch_bounds__(NT) delta_scan_fwd_kernel(Args a) {
     using F = Cfg<DK>;
+    constexpr int STAGE = OUT ? F::FULL : F::QD, VN = OUT ? 4 : 2;   // VN: n-tiles of Vn per warp (four warps or all eight)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* stage = reinterpret_cast<bf16*>(smem_raw);
-    bf16* Sb = stage + 2 * F::STAGE;                 // [DK][LDV]
+    bf16* Sb = stage + 2 * STAGE;                    // [DK][LDV]
     bf16* Vb = Sb + DK * F::LDV;                     // [C][LDV]  Vn of the chunk
     bf16* Ob = Vb + C * F::LDV;                      // [C][LDV]  output staging
     const int col0 = blockIdx.x * DVS;
     const long long bh = blockIdx.y;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int s_m0 = DK == 128 ? 16 * w : 16 * (w & 3), s_n0 = DK == 128 ? 0 : 16 * (w >> 2);
+    const int m0 = 16 * (w & 3), v_n0 = OUT ? 0 : 16 * (w >> 2);
+    const bool outs = OUT && w >= 4;                 // these warps make O = Qd S + A Vn while the others make Vn = U - W S
+    const bf16* u = a.U + (bh * a.N) * C * a.dv + col0;
+    bf16* og = OUT ? a.O + (bh / a.H) * a.os_b + (bh % a.H) * a.os_h + col0 : nullptr;
 
-    // state slice: warp w owns rows [w*16*RB, +16*RB) x 32 columns
-    float S[F::RB][4][4];
-#pragma unroll
-    for (int rb = 0; rb < F::RB; ++rb) {
-        const int r = (w * F::RB + rb) * 16 + (l >> 2);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int c = col0 + nt * 8 + (l & 3) * 2;
-            if (a.S0 != nullptr) {
-                const float* p = a.S0 + (bh * DK + r) * a.dv + c;
-                S[rb][nt][0] = p[0]; S[rb][nt][1] = p[1];
-                S[rb][nt][2] = p[8 * a.dv]; S[rb][nt][3] = p[8 * a.dv + 1];
-            } else {
-                S[rb][nt][0] = S[rb][nt][1] = S[rb][nt][2] = S[rb][nt][3] = 0.f;
-            }
-        }
-        store_acc_bf16<4>(S[rb], Sb, F::LDV, (w * F::RB + rb) * 16, 0);
-    }
-    if (a.N > 0) issue_chunk<DK>(stage, a, a.U, bh, 0, col0);
+    float S[F::SN][4];
+    load_state<F::SN>(S, a.S0 == nullptr ? nullptr : a.S0 + bh * DK * a.dv, a.dv, col0, Sb, F::LDV, s_m0, s_n0);
+    if (a.N > 0) issue_chunk<DK, OUT>(stage, a, u, a.dv, a.N * C, bh, 0);
     cp_async_commit();
     for (int n = 0; n < a.N; ++n) {
-        bf16* st = stage + (n & 1) * F::STAGE;
-        if (n + 1 < a.N) issue_chunk<DK>(stage + ((n + 1) & 1) * F::STAGE, a, a.U, bh, n + 1, col0);
+        const bf16* Wt = stage + (n & 1) * STAGE;
+        const bf16* Kt = Wt + C * F::LDK;
+        const bf16* Ut = Wt + 2 * C * F::LDK;
+        const bf16* Qt = Wt + F::QD;
+        const bf16* At = Wt + F::AQ;
+        cp_async_wait<0>();
+        __syncthreads();                                           // tiles of chunk n and Sb visible; chunk n - 1 is done with its stage
+        if (n + 1 < a.N) issue_chunk<DK, OUT>(stage + ((n + 1) & 1) * STAGE, a, u, a.dv, a.N * C, bh, n + 1);
         cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();                                           // tiles of chunk n and Sb visible
-        const bf16* Wt = st;
-        const bf16* Qt = st + C * F::LDK;
-        const bf16* Kt = st + 2 * C * F::LDK;
-        const bf16* At = st + 3 * C * F::LDK;
-        const bf16* Ut = At + C * F::LDC;
         const float gamma = a.gamma[bh * a.N + n];
-        // entering state of this chunk (bf16), for the backward pass
-        store_rows<F::LDV>(Sb, a.Sn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
-        // Vn = U - W S   (warp w: rows 16w .. 16w+15)
-        float acc[4][4];
-        zero_acc<4>(acc);
-        warp_gemm<4, DK, false, true>(acc, Wt, F::LDK, 16 * w, Sb, F::LDV, 0);
-        {
-            const int r = 16 * w + (l >> 2);
+        if (a.Vn != nullptr) store_rows<F::LDV>(Sb, a.Sn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
+        float acc[VN][4];
+        zero_acc<VN>(acc);
+        if (!outs) {
+            warp_gemm<VN, DK, false, true>(acc, Wt, F::LDK, m0, Sb, F::LDV, v_n0);
+            const int r = m0 + (l >> 2);
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int c = nt * 8 + (l & 3) * 2;
+            for (int nt = 0; nt < VN; ++nt) {
+                const int c = v_n0 + nt * 8 + (l & 3) * 2;
                 const __nv_bfloat162 u0 = *reinterpret_cast<const __nv_bfloat162*>(Ut + r * F::LDV + c);
                 const __nv_bfloat162 u1 = *reinterpret_cast<const __nv_bfloat162*>(Ut + (r + 8) * F::LDV + c);
                 acc[nt][0] = __bfloat162float(u0.x) - acc[nt][0]; acc[nt][1] = __bfloat162float(u0.y) - acc[nt][1];
                 acc[nt][2] = __bfloat162float(u1.x) - acc[nt][2]; acc[nt][3] = __bfloat162float(u1.y) - acc[nt][3];
             }
+            store_acc_bf16<VN>(acc, Vb, F::LDV, m0, v_n0);
+        } else {
+            warp_gemm<VN, DK, false, true>(acc, Qt, F::LDK, m0, Sb, F::LDV, 0);
         }
-        store_acc_bf16<4>(acc, Vb, F::LDV, 16 * w, 0);
-        // O = Qd S (needs only Sb) ...
-        float acc_o[4][4];
-        zero_acc<4>(acc_o);
-        warp_gemm<4, DK, false, true>(acc_o, Qt, F::LDK, 16 * w, Sb, F::LDV, 0);
         __syncthreads();                                           // Vb complete; every read of Sb done
-        // ... + A Vn
-        warp_gemm<4, C, false, true>(acc_o, At, F::LDC, 16 * w, Vb, F::LDV, 0);
-        store_acc_bf16<4>(acc_o, Ob, F::LDV, 16 * w, 0);
         // S <- gamma S + Kd^T Vn
 #pragma unroll
-        for (int rb = 0; rb < F::RB; ++rb) {
+        for (int nt = 0; nt < F::SN; ++nt)
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) S[rb][nt][e] *= gamma;
-            warp_gemm<4, C, true, true>(S[rb], Kt, F::LDK, (w * F::RB + rb) * 16, Vb, F::LDV, 0);
-            store_acc_bf16<4>(S[rb], Sb, F::LDV, (w * F::RB + rb) * 16, 0);
-        }
-        __syncthreads();                                           // Ob, Vb, new Sb complete
-        store_rows<F::LDV>(Ob, a.O + ((bh * a.N + n) * C) * a.dv + col0, C, a.dv);
-        store_rows<F::LDV>(Vb, a.Vn + ((bh * a.N + n) * C) * a.dv + col0, C, a.dv);
-        __syncthreads();                                           // staging drained before the next chunk rewrites it
-    }
-#pragma unroll
-    for (int rb = 0; rb < F::RB; ++rb) {
-        const int r = (w * F::RB + rb) * 16 + (l >> 2);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int c = col0 + nt * 8 + (l & 3) * 2;
-            float* p = a.Sfinal + (bh * DK + r) * a.dv + c;
-            p[0] = S[rb][nt][0]; p[1] = S[rb][nt][1];
-            p[8 * a.dv] = S[rb][nt][2]; p[8 * a.dv + 1] = S[rb][nt][3];
+            for (int e = 0; e < 4; ++e) S[nt][e] *= gamma;
+        warp_gemm<F::SN, C, true, true>(S, Kt, F::LDK, s_m0, Vb, F::LDV, s_n0);
+        store_acc_bf16<F::SN>(S, Sb, F::LDV, s_m0, s_n0);
+        if (a.Vn != nullptr) store_rows<F::LDV>(Vb, a.Vn + ((bh * a.N + n) * C) * a.dv + col0, C, a.dv);
+        if (outs) {
+            for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<VN, 16, false, true>(acc, At + k0, F::LDC, m0, Vb + k0 * F::LDV, F::LDV, 0);
+            store_acc_bf16<VN>(acc, Ob, F::LDV, m0, 0);
+            __syncwarp();
+            for (int i = l; i < 16 * (DVS / 8); i += 32) {         // the warp's own 16 rows
+                const int r = m0 + i / (DVS / 8), c = (i % (DVS / 8)) * 8, t = n * C + r;
+                if (t < a.T) *reinterpret_cast<uint4*>(og + (long long)t * a.os_t + c) = *reinterpret_cast<const uint4*>(Ob + r * F::LDV + c);
+            }
+            __syncwarp();
         }
     }
+    save_state<F::SN>(S, a.Sfinal + bh * DK * a.dv, a.dv, col0, s_m0, s_n0);
 }
 
 // Reverse walk: dS' enters from the right (gradient of the state leaving the chunk).
 template <int DK>
 __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
     using F = Cfg<DK>;
+    constexpr int STAGE = F::FULL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* stage = reinterpret_cast<bf16*>(smem_raw);
-    bf16* Sb = stage + 2 * F::STAGE;                 // [DK][LDV]  bf16 copy of dS'
+    bf16* Sb = stage + 2 * STAGE;                    // [DK][LDV]  bf16 copy of dS'
     bf16* Vb = Sb + DK * F::LDV;                     // [C][LDV]   dVn of the chunk
     const int col0 = blockIdx.x * DVS;
     const long long bh = blockIdx.y;
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    const int s_m0 = DK == 128 ? 16 * w : 16 * (w & 3), s_n0 = DK == 128 ? 0 : 16 * (w >> 2);
+    const int m0 = 16 * (w & 3), v_n0 = 16 * (w >> 2);
+    const bf16* dO = a.dO + (bh / a.H) * a.gs_b + (bh % a.H) * a.gs_h + col0;
 
-    float S[F::RB][4][4];
-#pragma unroll
-    for (int rb = 0; rb < F::RB; ++rb) {
-        const int r = (w * F::RB + rb) * 16 + (l >> 2);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int c = col0 + nt * 8 + (l & 3) * 2;
-            if (a.dSfinal != nullptr) {
-                const float* p = a.dSfinal + (bh * DK + r) * a.dv + c;
-                S[rb][nt][0] = p[0]; S[rb][nt][1] = p[1];
-                S[rb][nt][2] = p[8 * a.dv]; S[rb][nt][3] = p[8 * a.dv + 1];
-            } else {
-                S[rb][nt][0] = S[rb][nt][1] = S[rb][nt][2] = S[rb][nt][3] = 0.f;
-            }
-        }
-        store_acc_bf16<4>(S[rb], Sb, F::LDV, (w * F::RB + rb) * 16, 0);
-    }
-    if (a.N > 0) issue_chunk<DK>(stage, a, a.dO, bh, a.N - 1, col0);
+    float S[F::SN][4];
+    load_state<F::SN>(S, a.dSfinal == nullptr ? nullptr : a.dSfinal + bh * DK * a.dv, a.dv, col0, Sb, F::LDV, s_m0, s_n0);
+    if (a.N > 0) issue_chunk<DK, true>(stage, a, dO, a.gs_t, a.T, bh, a.N - 1);
     cp_async_commit();
     for (int i = 0; i < a.N; ++i) {
         const int n = a.N - 1 - i;
-        bf16* st = stage + (i & 1) * F::STAGE;
-        if (n > 0) issue_chunk<DK>(stage + ((i + 1) & 1) * F::STAGE, a, a.dO, bh, n - 1, col0);
-        cp_async_commit();
-        cp_async_wait<1>();
+        const bf16* Wt = stage + (i & 1) * STAGE;
+        const bf16* Kt = Wt + C * F::LDK;
+        const bf16* Gt = Wt + 2 * C * F::LDK;         // dO slice
+        const bf16* Qt = Wt + F::QD;
+        const bf16* At = Wt + F::AQ;
+        cp_async_wait<0>();
         __syncthreads();
-        const bf16* Wt = st;
-        const bf16* Qt = st + C * F::LDK;
-        const bf16* Kt = st + 2 * C * F::LDK;
-        const bf16* At = st + 3 * C * F::LDK;
-        const bf16* Gt = At + C * F::LDC;             // dO slice
+        if (n > 0) issue_chunk<DK, true>(stage + ((i + 1) & 1) * STAGE, a, dO, a.gs_t, a.T, bh, n - 1);
+        cp_async_commit();
         const float gamma = a.gamma[bh * a.N + n];
         store_rows<F::LDV>(Sb, a.dSn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
         // dVn = A^T dO + Kd dS'
-        float acc[4][4];
-        zero_acc<4>(acc);
-        warp_gemm<4, C, true, true>(acc, At, F::LDC, 16 * w, Gt, F::LDV, 0);
-        warp_gemm<4, DK, false, true>(acc, Kt, F::LDK, 16 * w, Sb, F::LDV, 0);
-        store_acc_bf16<4>(acc, Vb, F::LDV, 16 * w, 0);
+        float acc[2][4];
+        zero_acc<2>(acc);
+        for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<2, 16, true, true>(acc, At + k0 * F::LDC, F::LDC, m0, Gt + k0 * F::LDV, F::LDV, v_n0);
+        warp_gemm<2, DK, false, true>(acc, Kt, F::LDK, m0, Sb, F::LDV, v_n0);
+        store_acc_bf16<2>(acc, Vb, F::LDV, m0, v_n0);
+        // dS = gamma dS' + Qd^T dO - W^T dVn; what does not wait for dVn first
+#pragma unroll
+        for (int nt = 0; nt < F::SN; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[nt][e] *= gamma;
+        warp_gemm<F::SN, C, true, true>(S, Qt, F::LDK, s_m0, Gt, F::LDV, s_n0);
         __syncthreads();                                           // Vb complete; reads of Sb done
-        // dS = gamma dS' + Qd^T dO - W^T dVn
+        float t[F::SN][4];
+        zero_acc<F::SN>(t);
+        warp_gemm<F::SN, C, true, true>(t, Wt, F::LDK, s_m0, Vb, F::LDV, s_n0);
 #pragma unroll
-        for (int rb = 0; rb < F::RB; ++rb) {
-            float t[4][4];
-            zero_acc<4>(t);
-            warp_gemm<4, C, true, true>(t, Wt, F::LDK, (w * F::RB + rb) * 16, Vb, F::LDV, 0);
+        for (int nt = 0; nt < F::SN; ++nt)
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) S[rb][nt][e] = S[rb][nt][e] * gamma - t[nt][e];
-            warp_gemm<4, C, true, true>(S[rb], Qt, F::LDK, (w * F::RB + rb) * 16, Gt, F::LDV, 0);
-            store_acc_bf16<4>(S[rb], Sb, F::LDV, (w * F::RB + rb) * 16, 0);
-        }
+            for (int e = 0; e < 4; ++e) S[nt][e] -= t[nt][e];
+        store_acc_bf16<F::SN>(S, Sb, F::LDV, s_m0, s_n0);
         store_rows<F::LDV>(Vb, a.dVn + ((bh * a.N + n) * C) * a.dv + col0, C, a.dv);
-        __syncthreads();
     }
-#pragma unroll
-    for (int rb = 0; rb < F::RB; ++rb) {
-        const int r = (w * F::RB + rb) * 16 + (l >> 2);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int c = col0 + nt * 8 + (l & 3) * 2;
-            float* p = a.dS0 + (bh * DK + r) * a.dv + c;
-            p[0] = S[rb][nt][0]; p[1] = S[rb][nt][1];
-            p[8 * a.dv] = S[rb][nt][2]; p[8 * a.dv + 1] = S[rb][nt][3];
-        }
-    }
+    save_state<F::SN>(S, a.dS0 + bh * DK * a.dv, a.dv, col0, s_m0, s_n0);
 }
 
 
@@ -830,16 +821,19 @@ using namespace lmoe;
 // dir 0: forward, dir 1: backward.  dk in {64, 128}; dv a multiple of 32.  Grid = (dv / 32, B*H).
 LMOE_API int lmoe_delta_scan(int dir, int dk, int BH, const dr::Args* ap, cudaStream_t st) {
     const dr::Args a = *ap;
-    if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0) return -1;
+    if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0 || a.H <= 0) return -1;
     dim3 grid(a.dv / dr::DVS, BH);
+    const bool out = dir != 0 || a.O != nullptr;
 #define LMOE_DR_LAUNCH(KERNEL, DK)                                                                                     \
     do {                                                                                                               \
-        cudaError_t e = cudaFuncSetAttribute(KERNEL<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dr::Cfg<DK>::SMEM); \
+        auto kernel = KERNEL;                                                                                          \
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dr::Cfg<DK>::smem(out)); \
         if (e != cudaSuccess) return (int)e;                                                                           \
-        KERNEL<DK><<<grid, dr::NT, dr::Cfg<DK>::SMEM, st>>>(a);                                                        \
+        kernel<<<grid, dr::NT, dr::Cfg<DK>::smem(out), st>>>(a);                                                       \
     } while (0)
-    if (dir == 0) { if (dk == 128) LMOE_DR_LAUNCH(dr::delta_scan_fwd_kernel, 128); else LMOE_DR_LAUNCH(dr::delta_scan_fwd_kernel, 64); }
-    else { if (dk == 128) LMOE_DR_LAUNCH(dr::delta_scan_bwd_kernel, 128); else LMOE_DR_LAUNCH(dr::delta_scan_bwd_kernel, 64); }
+    if (dir != 0) { if (dk == 128) LMOE_DR_LAUNCH(dr::delta_scan_bwd_kernel<128>, 128); else LMOE_DR_LAUNCH(dr::delta_scan_bwd_kernel<64>, 64); }
+    else if (out) { if (dk == 128) LMOE_DR_LAUNCH((dr::delta_scan_fwd_kernel<128, true>), 128); else LMOE_DR_LAUNCH((dr::delta_scan_fwd_kernel<64, true>), 64); }
+    else { if (dk == 128) LMOE_DR_LAUNCH((dr::delta_scan_fwd_kernel<128, false>), 128); else LMOE_DR_LAUNCH((dr::delta_scan_fwd_kernel<64, false>), 64); }
 #undef LMOE_DR_LAUNCH
     return (int)cudaGetLastError();
 }

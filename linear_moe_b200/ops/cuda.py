@@ -1362,7 +1362,9 @@ class _tf32:
 
 class _DeltaArgs(ctypes.Structure):
     _fields_ = ([(n, ctypes.c_void_p) for n in ("W", "U", "Qd", "Kd", "A", "gamma", "S0", "dO", "dSfinal", "O", "Vn", "Sn",
-                                                 "Sfinal", "dVn", "dSn", "dS0")] + [("N", ctypes.c_int), ("dv", ctypes.c_int)])
+                                                 "Sfinal", "dVn", "dSn", "dS0")] +
+                [(n, ctypes.c_longlong) for n in ("os_b", "os_t", "os_h", "gs_b", "gs_t", "gs_h")] +
+                [(n, ctypes.c_int) for n in ("N", "dv", "T", "H")])
 
 
 def _delta_prepare(q, k, v, beta, g, scale, C=64):
@@ -1439,32 +1441,43 @@ def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64, inverse=None):
     return W, U, Qd, Kd, A, gamma
 
 
-def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0):
+def _time_major(x):
+    """``[B,H,N,C,d]`` (the chunks of a head one behind the other) as ``[B,N*C,H,d]``."""
+    B, H, N, C, d = x.shape
+    return x.view(B, H, N * C, d).transpose(1, 2)
+
+
+def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, out=None, keep=True):
     """``delta_scan_fwd_kernel``: ``Vn = U - W S``, ``O = Qd S + A Vn``, ``S' = gamma S + Kd^T Vn`` over the chunks.
-    Returns ``O, Vn`` ``[B,H,N,C,dv]`` bf16, the state entering every chunk ``Sn`` ``[B,H,N,dk,dv]`` bf16 and the final
-    state in fp32."""
+    ``out``: a bf16 ``[B,T,H,dv]`` buffer (unit stride along ``dv``) for ``O``, or ``None`` where nobody needs it.  Returns ``Vn``
+    ``[B,H,N,C,dv]`` bf16 and the state entering every chunk ``Sn`` ``[B,H,N,dk,dv]`` bf16 (both ``None`` without ``keep``)
+    and the final state in fp32."""
     B, H, N, C, dk = W.shape
     dv = U.shape[-1]
     dev = W.device
     bf = torch.bfloat16
-    O = torch.empty(B, H, N, C, dv, dtype=bf, device=dev)
-    Vn = torch.empty(B, H, N, C, dv, dtype=bf, device=dev)
-    Sn = torch.empty(B, H, N, dk, dv, dtype=bf, device=dev)
+    Vn = torch.empty(B, H, N, C, dv, dtype=bf, device=dev) if keep else None
+    Sn = torch.empty(B, H, N, dk, dv, dtype=bf, device=dev) if keep else None
     Sf = torch.empty(B, H, dk, dv, dtype=torch.float32, device=dev)
     s0 = None if S0 is None else S0.float().contiguous()
     a = _DeltaArgs()
     a.W, a.U, a.Qd, a.Kd, a.A, a.gamma = (t.data_ptr() for t in (W, U, Qd, Kd, A, gamma))
     a.S0 = 0 if s0 is None else s0.data_ptr()
-    a.O, a.Vn, a.Sn, a.Sfinal = O.data_ptr(), Vn.data_ptr(), Sn.data_ptr(), Sf.data_ptr()
-    a.N, a.dv = N, dv
+    a.Sfinal = Sf.data_ptr()
+    if keep:
+        a.Vn, a.Sn = Vn.data_ptr(), Sn.data_ptr()
+    if out is not None:
+        a.O, a.T = out.data_ptr(), out.shape[1]
+        a.os_b, a.os_t, a.os_h = out.stride(0), out.stride(1), out.stride(2)
+    a.N, a.dv, a.H = N, dv, H
     _check(lib().lmoe_delta_scan(_i32(0), _i32(dk), _i32(B * H), ctypes.byref(a), _st()), "delta_scan_fwd")
-    return O, Vn, Sn, Sf
+    return Vn, Sn, Sf
 
 
 def _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf):
-    """``delta_scan_bwd_kernel``: the reverse recurrence ``dVn = A^T dO + Kd dS'``, ``dS = gamma dS' + Qd^T dO - W^T dVn``.
-    Returns ``dVn`` ``[B,H,N,C,dv]``, the gradient of the state leaving every chunk ``dSn`` ``[B,H,N,dk,dv]`` (bf16) and the
-    gradient of the initial state (fp32)."""
+    """``delta_scan_bwd_kernel``: the reverse recurrence ``dVn = A^T dO + Kd dS'``, ``dS = gamma dS' + Qd^T dO - W^T dVn`` for ``dO``
+    ``[B,T,H,dv]`` (:func:`_inner_contig`).  Returns ``dVn`` ``[B,H,N,C,dv]``, the gradient of the state leaving every chunk
+    ``dSn`` ``[B,H,N,dk,dv]`` (bf16) and the gradient of the initial state (fp32)."""
     B, H, N, C, dk = W.shape
     dv = dO.shape[-1]
     dev = W.device
@@ -1477,8 +1490,9 @@ def _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf):
     a.W, a.Qd, a.Kd, a.A, a.gamma = (t.data_ptr() for t in (W, Qd, Kd, A, gamma))
     a.U = 0
     a.dO, a.dSfinal = dO.data_ptr(), 0 if dsf is None else dsf.data_ptr()
+    a.gs_b, a.gs_t, a.gs_h = dO.stride(0), dO.stride(1), dO.stride(2)
     a.dVn, a.dSn, a.dS0 = dVn.data_ptr(), dSn.data_ptr(), dS0.data_ptr()
-    a.N, a.dv = N, dv
+    a.N, a.dv, a.T, a.H = N, dv, dO.shape[1], H
     _check(lib().lmoe_delta_scan(_i32(1), _i32(dk), _i32(B * H), ctypes.byref(a), _st()), "delta_scan_bwd")
     return dVn, dSn, dS0
 
@@ -1491,7 +1505,8 @@ class _DeltaChunkScan(torch.autograd.Function):
     @staticmethod
     def forward(ctx, W, U, Qd, Kd, A, gamma, S0):
         W, U, Qd, Kd, A, gamma = (t.contiguous() for t in (W, U, Qd, Kd, A, gamma))
-        O, Vn, Sn, Sf = _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0)
+        O = torch.empty_like(U)
+        Vn, Sn, Sf = _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, _time_major(O))
         ctx.save_for_backward(W, Qd, Kd, A, gamma, Vn, Sn)
         ctx.has_s0 = S0 is not None
         return O, Sf
@@ -1500,7 +1515,7 @@ class _DeltaChunkScan(torch.autograd.Function):
     def backward(ctx, dO, dSf):
         W, Qd, Kd, A, gamma, Vn, Sn = ctx.saved_tensors
         dO = dO.to(torch.bfloat16).contiguous()
-        dVn, dSn, dS0 = _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf)
+        dVn, dSn, dS0 = _delta_scan_bwd(W, Qd, Kd, A, gamma, _time_major(dO), dSf)
         SnT = Sn.transpose(-1, -2)
         dW = -(dVn @ SnT)
         dQd = dO @ SnT
@@ -1539,7 +1554,7 @@ def _delta_prepare_bwd_kernel(q, k, v, beta, g, scale, Sn, dSn, Vn, dVn, dO, Tin
     a.vs_b, a.vs_t, a.vs_h = v.stride(0), v.stride(1), v.stride(2)
     a.beta, a.g = bt.data_ptr(), 0 if gt is None else gt.data_ptr()
     a.Sn, a.dSn, a.Vn, a.dVn, a.dO, a.Tinv = (t.data_ptr() for t in (Sn, dSn, Vn, dVn, dO, Tinv))
-    a.gs_b, a.gs_h, a.gs_t = dO.stride(0), dO.stride(1), dO.stride(3)      # [B,H,N,C,D], the chunks of a head one behind the other
+    a.gs_b, a.gs_t, a.gs_h = dO.stride(0), dO.stride(1), dO.stride(2)
     a.dq, a.dk, a.dv, a.dbeta = dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dbeta.data_ptr()
     a.dg = 0 if dg is None else dg.data_ptr()
     a.B, a.T, a.H, a.N, a.scale = B, T, H, N, float(scale)
@@ -1564,10 +1579,10 @@ class _DeltaRuleScan(torch.autograd.Function):
                 tiles = _delta_prepare_kernel(q, k, v, beta, g, scale)
             else:
                 tiles = _delta_prepare(q, k, v, beta, g, scale)
-            O, S = _DeltaChunkScan.apply(*tiles, initial_state)
+            o = torch.empty(B, T, H, v.shape[-1], dtype=torch.bfloat16, device=q.device)
+            S = _delta_scan_fwd(*tiles, initial_state, o, keep=False)[2]     # the backward pass rebuilds Vn and the states
         ctx.save_for_backward(q, k, v, beta, g, initial_state)
         ctx.scale = scale
-        o = O.permute(0, 2, 3, 1, 4).reshape(B, -1, H, v.shape[-1])[:, :T]
         return o.to(q.dtype), S
 
     @staticmethod
@@ -1607,11 +1622,8 @@ def _delta_backward_kernels(ctx, do, dS):
         N, C = (T + 63) // 64, 64
         Tinv = torch.empty(B, H, N, C, C, dtype=torch.bfloat16, device=q.device)
         W, U, Qd, Kd, A, gamma = _delta_prepare_kernel(q, k, v, beta, g, ctx.scale, inverse=Tinv)
-        _, Vn, Sn, _ = _delta_scan_fwd(W, U, Qd, Kd, A, gamma, s0)
-        dO = do.to(torch.bfloat16)
-        if N * C != T:
-            dO = F.pad(dO, (0, 0, 0, 0, 0, N * C - T))
-        dO = dO.reshape(B, N, C, H, D).permute(0, 3, 1, 2, 4).contiguous()
+        Vn, Sn, _ = _delta_scan_fwd(W, U, Qd, Kd, A, gamma, s0)
+        dO = _inner_contig(do.to(torch.bfloat16))
         dVn, dSn, dS0 = _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dS)
         dq, dk, dv, dbeta, dg = _delta_prepare_bwd_kernel(q, k, v, beta, g, ctx.scale, Sn, dSn, Vn, dVn, dO, Tinv)
     need = ctx.needs_input_grad
