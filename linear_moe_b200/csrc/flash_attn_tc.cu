@@ -1,17 +1,18 @@
 // Flash-attention forward on the 5th-generation tensor cores: S = Q K^T and O_j = P_j V_j are tcgen05.mma instructions
 // with accumulators in tensor memory, operands staged by TMA (4-D tensor maps over [B, T, H, D], 128-byte swizzle).
 //
-// One CTA = 128 queries of one head.  128 + 128 * SPLIT threads (warps 0-1: TMA / MMA, warps 2-3 idle, warps 4.. softmax):
+// One CTA = 128 queries of one head.  640 threads:
 //   warp 0      TMA producer: Q once, then K_j / V_j tiles of 128 keys through two 2-stage rings
-//   warp 1      MMA issuer:   S_{j+1} = Q K_{j+1}^T is issued before P_j V_j, so the tensor core works on the next
-//               score tile while the softmax warps are busy with the current one
-//   warps 4..   softmax: the SPLIT warps with equal (w & 3) own the 32 query rows of that TMEM lane quarter and split
-//               the columns: one tensor-memory load of the scores, row max (exchanged between the parts through
-//               shared memory and a named barrier), exp2 / sum / bf16 pack, P_j written to shared memory in
-//               the K-major 128-byte-swizzle layout the MMA reads; O += P_j V_j is folded into registers
-//               (o = o * corr + O_j) one iteration later, so that it overlaps the next tile's math.  SPLIT warps per
-//               scheduler hide the tensor-memory latency; no tensor-memory stores, no shuffles.
-// Tensor memory: 2 x 128 columns of scores + 2 x D columns of partial outputs.
+//   warp 1      MMA issuer:   S_{j+1} = Q K_{j+1}^T is issued before O += P_j V_j
+//   warps 4..19 softmax, two groups of eight: group g works on the tiles j = g (mod 2), so that one group's exponentials run while the
+//               other one waits for its scores, exchanges maxima or hands over P.  (With all warps on the same tile every stage of
+//               it was exposed: 3900 cycles a tile against 1024 of exponentials.)  Inside a group the two warps with equal (w & 3) own the 32 rows
+//               of a tensor-memory lane quarter and half of the columns each.
+// Each group has its own running maximum, sum and output, which are joined at the end.  Its output accumulates in tensor memory in
+// units of a maximum that may lag behind by up to 2^LAG; only when a row runs ahead of that the output is rescaled there.  P_j goes
+// back over its scores in bf16 and is read as the A operand from tensor memory.
+// Tensor memory: 2 x 128 columns of scores, 2 x D of outputs.
+// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 190 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 66 us.
 // Masking (causal with a query offset, sliding window, key length) is applied only on tiles that cross a boundary.
 // Every mbarrier wait is bounded (clock64 budget); on expiry the error word is set and the CTA drains and frees its
 // tensor memory.  Writes O (bf16) and the natural-log row log-sum-exp, which the backward kernels of flash_attn.cu use.
@@ -32,14 +33,16 @@ struct Args {
     int* err;
 };
 
+constexpr float LAG = 8.f;            // how far, as a power of two, a row's weights may run ahead of the maximum they are measured in
+
 template <int D>
 struct __align__(1024) Smem {
     uint8_t q[BM * D * 2];
     uint8_t k[2][BN * D * 2];
     uint8_t v[2][BN * D * 2];
-    uint8_t p[BM * BN * 2];
-    uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], o_full[2], p_ready;
-    float mx[2][SPLIT][BM], ls[SPLIT][BM];
+    uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done[2];
+    float mx[2][2][2][BM];            // [parity of the group's tile][group][half of the columns]
+    float ls[2][2][BM], ms[2][BM];    // sums and maxima at the end
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -52,7 +55,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     Smem<D>& sm = *reinterpret_cast<Smem<D>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int DK = D / 64;                              // 64-element blocks along the head dimension
     constexpr uint32_t TMEM_COLS = 512;
-    constexpr uint32_t O_COL = 2 * BN;                      // partial outputs behind the two score buffers
+    constexpr uint32_t O_COL = 2 * BN;                      // the groups' outputs behind the two score buffers
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qb = gridDim.x - 1 - blockIdx.x;              // long (late) query tiles first
     const int h = blockIdx.y, b = blockIdx.z;
@@ -73,9 +76,9 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int s = 0; s < 2; ++s) {
             mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1);
             mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1);
-            mbar_init(&sm.s_full[s], 1); mbar_init(&sm.o_full[s], 1);
+            mbar_init(&sm.s_full[s], 1); mbar_init(&sm.pv_done[s], 1);
+            mbar_init(&sm.p_ready[s], 8);
         }
-        mbar_init(&sm.p_ready, 4 * SPLIT);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -133,152 +136,154 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             };
             if (ok) ok = issue_s(0);
             for (int j = 0; ok && j < n_it; ++j) {
-                if (j + 1 < n_it) { ok = issue_s(j + 1); if (!ok) break; }
                 const int s = j & 1;
+                if (j + 1 < n_it) {
+                    // the other score buffer holds P_{j-1}: its product has to complete
+                    if (j > 0 && !mbar_wait_suspend(&sm.pv_done[s ^ 1], ((j - 1) >> 1) & 1, abort_flag, err, 0x2400)) break;
+                    ok = issue_s(j + 1);
+                    if (!ok) break;
+                }
                 if (!mbar_wait_suspend(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x2200 | s)) break;
-                if (!mbar_wait_suspend(&sm.p_ready, j & 1, abort_flag, err, 0x2300)) break;
+                if (!mbar_wait_suspend(&sm.p_ready[s], (j >> 1) & 1, abort_flag, err, 0x2300 | s)) break;
                 tc_fence_after();
-                const uint32_t pl = desc_lo<false>(s32(sm.p)), vl = desc_lo<true>(s32(sm.v[s]));
+                const uint32_t vl = desc_lo<true>(s32(sm.v[s]));
 #pragma unroll
                 for (int kk = 0; kk < BN / UMMA_K; ++kk) {
-                    const uint32_t aoff = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4;
+                    // every half of the columns left its 32 columns of P at its beginning
                     const uint32_t boff = ((kk / 4) * (DK * 8192) + (kk % 4) * 2048) >> 4;
-                    umma_lo(tmem_base + O_COL + s * D, pl + aoff, vl + boff, idesc_o, kk > 0 ? 1u : 0u, issue);
+                    umma_ta(tmem_base + O_COL + s * D, tmem_base + s * BN + kk / 4 * 64 + kk % 4 * 8, vl + boff, idesc_o, (j > 1 || kk > 0) ? 1u : 0u, issue);
                 }
                 umma_commit_if(&sm.v_empty[s], issue);
-                umma_commit_if(&sm.o_full[s], issue);
+                umma_commit_if(&sm.pv_done[s], issue);
             }
         }
     } else if (warp >= 4) {
-        // 4*SPLIT softmax warps: the SPLIT warps with the same (warp & 3) own the 32 query rows of that TMEM lane
-        // quarter and split the score / output columns between them
-        const int qd = warp & 3;
-        const int part = (warp - 4) >> 2;
+        const int qd = warp & 3, quarter = (warp - 4) >> 2, grp = quarter >> 1, part = quarter & 1;
         const int r = qd * 32 + lane;                         // query row inside the tile
         const int qi = a.q_offset + q0 + r;                   // absolute position of this query
         const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
-        const float sc = a.scale * LOG2E;
-        constexpr int CW = BN / SPLIT;                        // score columns of this thread
-        constexpr int OW = D / SPLIT;                         // output columns of this thread
+        const uint32_t s_addr = lane_addr + grp * BN + part * 64, o_addr = lane_addr + O_COL + grp * D + part * (D / 2);
+        const float sc = a.scale * LOG2E, lag = LAG / sc;
+        float m = -INFINITY, l = 0.f;
+        bool ok = true;                                       // after a wait that ran out only the barriers are kept up with
+        for (int j = grp; j < n_it; j += 2) {
+            const int k = j >> 1;
+            const int tile_key0 = (nb_lo + j) * BN;
+            if (ok) ok = mbar_wait_suspend(&sm.s_full[grp], k & 1, abort_flag, err, 0x3100 | grp);
+            if (!ok) {
+                asm volatile("bar.sync %0, 64;" :: "r"(1 + grp * 4 + qd) : "memory");
+                continue;
+            }
+            tc_fence_after();
+            uint32_t v[64];
+            tmem_ld64(s_addr, v);
+            tmem_ld_wait();
+            const bool need_mask = (tile_key0 + BN - 1 > a.q_offset + q0) || (tile_key0 + BN > a.Tk) ||
+                                   (a.window > 0 && tile_key0 <= a.q_offset + q0 + BM - 1 - a.window);
+            if (need_mask) {
+                const int key0 = tile_key0 + part * 64;
+                const int hi = min(qi, a.Tk - 1) - key0, lo = a.window > 0 ? qi - a.window - key0 : -1;      // visible: lo < c <= hi
+#pragma unroll
+                for (int c = 0; c < 64; ++c)
+                    if (c > hi || c <= lo) v[c] = 0xff800000u;                                               // -inf
+            }
+            float mx4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                mx4[e] = fmaxf(__uint_as_float(v[e]), __uint_as_float(v[e + 4]));
+#pragma unroll
+                for (int c = 8; c < 64; c += 8) mx4[e] = max3(mx4[e], __uint_as_float(v[c + e]), __uint_as_float(v[c + e + 4]));
+            }
+            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            sm.mx[k & 1][grp][part][r] = mx;
+            asm volatile("bar.sync %0, 64;" :: "r"(1 + grp * 4 + qd) : "memory");
+            mx = fmaxf(mx, sm.mx[k & 1][grp][part ^ 1][r]);
+            // both halves of a row see the same numbers and decide alike
+            const bool grow = mx > m + lag;                   // also the first visible key of the row (m = -inf)
+            const bool scaled = grow && m != -INFINITY;
+            const float corr = scaled ? exp2f((m - mx) * sc) : 1.f;
+            if (grow) m = mx;
+            l *= corr;
+            if (__any_sync(0xffffffffu, scaled)) {            // k > 0; the scores of tile j were issued behind the last product of this group
+                ok = mbar_wait_suspend(&sm.pv_done[grp], (k - 1) & 1, abort_flag, err, 0x3200 | grp);
+                if (!ok) continue;
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < D / 2; c += 16) {
+                    uint32_t o[16];
+                    tmem_ld16(o_addr + c, o);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                    tmem_st16(o_addr + c, o);
+                }
+            }
+            const float nm = m == -INFINITY ? 0.f : -m * sc;
+            const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(nm, nm);
+            float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < 64; c += 32) {
+                uint32_t p[16];
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float2 x01 = __ffma2_rn(make_float2(__uint_as_float(v[c + i]), __uint_as_float(v[c + i + 1])), sc2, nm2);
+                    const float2 x23 = __ffma2_rn(make_float2(__uint_as_float(v[c + i + 2]), __uint_as_float(v[c + i + 3])), sc2, nm2);
+                    const float p0 = exp2f(x01.x), p1 = exp2f(x01.y), p2 = exp2f(x23.x), p3 = exp2f(x23.y);
+                    sum0 = __fadd2_rn(sum0, make_float2(p0, p1));
+                    sum1 = __fadd2_rn(sum1, make_float2(p2, p3));
+                    p[i >> 1] = pack_bf16(p0, p1);
+                    p[(i >> 1) + 1] = pack_bf16(p2, p3);
+                }
+                tmem_st16(s_addr + (c >> 1), p);              // over scores that are in registers
+            }
+            l += (sum0.x + sum0.y) + (sum1.x + sum1.y);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.p_ready[grp]);
+        }
+        // join the groups: every warp takes a quarter of the columns of both outputs
+        sm.ls[grp][part][r] = l;
+        if (part == 0) sm.ms[grp][r] = m;
+        asm volatile("bar.sync 9, 512;" ::: "memory");        // behind it at most the last product of each group is outstanding
+        float w[2], mm = fmaxf(sm.ms[0][r], sm.ms[1][r]);
+        l = 0.f;
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const float mg = sm.ms[g][r];
+            w[g] = mg == -INFINITY ? 0.f : exp2f((mg - mm) * sc);
+            l += w[g] * (sm.ls[g][0][r] + sm.ls[g][1][r]);
+        }
+        constexpr int OW = D / 4;
         float o[OW];
 #pragma unroll
         for (int i = 0; i < OW; ++i) o[i] = 0.f;
-        float m = -INFINITY, l = 0.f, corr_prev = 1.f;
-        // CW keys = CW * 2 bytes inside the 128-byte row of key block (part * CW) / 64
-        uint8_t* prow = sm.p + ((part * CW) >> 6) * (BM * 128) + (r >> 3) * 1024 + (r & 7) * 128;
-        const int ch0 = ((part * CW) & 63) >> 3;
-        bool alive = n_it > 0;
-        for (int j = 0; alive && j < n_it; ++j) {
-            const int s = j & 1;
-            const int tile_key0 = (nb_lo + j) * BN;
-            const int key0 = tile_key0 + part * CW;           // first key of this thread's columns
-            if (!mbar_wait_suspend(&sm.s_full[s], (j >> 1) & 1, abort_flag, err, 0x3100 | s)) { alive = false; break; }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            if (g >= n_it) break;
+            const int last = n_it - 1 - ((n_it - 1 - g) & 1);                    // the group's last tile
+            if (!mbar_wait_suspend(&sm.pv_done[g], (last >> 1) & 1, abort_flag, err, 0x3300 | g)) break;
             tc_fence_after();
-            const bool need_mask = (tile_key0 + BN - 1 > a.q_offset + q0) || (tile_key0 + BN > a.Tk) ||
-                                   (a.window > 0 && tile_key0 <= a.q_offset + q0 + BM - 1 - a.window);
-            // pass 1: row maximum, 16 columns at a time (keeps the live register set small)
-            float mx4[4] = {m, -INFINITY, -INFINITY, -INFINITY};
+            uint32_t x[OW];
+            tmem_ld<OW>(lane_addr + O_COL + g * D + quarter * OW, x);
+            tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < CW; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + s * BN + part * CW + c, v);
-                tmem_ld_wait();
-                if (need_mask) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int key = key0 + c + i;
-                        const bool vis = key <= qi && key < a.Tk && (a.window <= 0 || key > qi - a.window);
-                        if (!vis) v[i] = 0xff800000u;         // -inf
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e)                              // 3-input max: two scores per instruction
-                    mx4[e] = max3(max3(mx4[e], __uint_as_float(v[e]), __uint_as_float(v[e + 4])), __uint_as_float(v[e + 8]),
-                                  __uint_as_float(v[e + 12]));
-            }
-            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            // row maximum over the SPLIT parts (buffers alternate so that a fast thread cannot overwrite a value a slow
-            // one still has to read)
-            sm.mx[s][part][r] = mx;
-            asm volatile("bar.sync %0, %1;" :: "r"(1 + qd), "n"(32 * SPLIT) : "memory");
-#pragma unroll
-            for (int q2 = 0; q2 < SPLIT; ++q2) mx = fmaxf(mx, sm.mx[s][q2][r]);
-            const float corr = (m == -INFINITY) ? 1.f : exp2f((m - mx) * sc);
-            const float msc = (mx == -INFINITY) ? 0.f : mx * sc;
-            m = mx;
-            // the P buffer and the partial output of the previous tile are free once P_{j-1} V_{j-1} has completed
-            if (j > 0 && !mbar_wait_suspend(&sm.o_full[s ^ 1], ((j - 1) >> 1) & 1, abort_flag, err, 0x3200 | s)) { alive = false; break; }
-            // pass 2: p = exp2(s * sc - m * sc), row sum, bf16 pack, swizzled 16-byte stores
-            float ps4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int c = 0; c < CW; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + s * BN + part * CW + c, v);
-                tmem_ld_wait();
-                if (need_mask) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int key = key0 + c + i;
-                        const bool vis = key <= qi && key < a.Tk && (a.window <= 0 || key > qi - a.window);
-                        if (!vis) v[i] = 0xff800000u;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i += 4) {
-                    const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(-msc, -msc);
-                    const float2 x01 = __ffma2_rn(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), sc2, nm2);
-                    const float2 x23 = __ffma2_rn(make_float2(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), sc2, nm2);
-                    const float p0 = exp2f(x01.x), p1 = exp2f(x01.y), p2 = exp2f(x23.x), p3 = exp2f(x23.y);
-                    const float2 s01 = __fadd2_rn(make_float2(ps4[0], ps4[1]), make_float2(p0, p1));
-                    const float2 s23 = __fadd2_rn(make_float2(ps4[2], ps4[3]), make_float2(p2, p3));
-                    ps4[0] = s01.x; ps4[1] = s01.y; ps4[2] = s23.x; ps4[3] = s23.y;
-                    v[i >> 1] = pack_bf16(p0, p1);
-                    v[(i >> 1) + 1] = pack_bf16(p2, p3);
-                }
-                const int ch = ch0 + (c >> 3);
-                *reinterpret_cast<uint4*>(prow + ((ch ^ (r & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
-                *reinterpret_cast<uint4*>(prow + (((ch + 1) ^ (r & 7)) << 4)) = make_uint4(v[4], v[5], v[6], v[7]);
-            }
-            l = l * corr + ((ps4[0] + ps4[1]) + (ps4[2] + ps4[3]));
-            // hand P_j to the MMA warp
-            tc_fence_before();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready);
-            // fold the previous tile's partial output while the tensor core runs P_j V_j
-            if (j > 0) {
-                tc_fence_after();
-                fold_o<OW>(o, lane_addr + O_COL + (s ^ 1) * D + part * OW, corr_prev);
-            }
-            corr_prev = corr;
+            for (int i = 0; i < OW; ++i) o[i] += w[g] * __uint_as_float(x[i]);
         }
-        if (alive && n_it > 0) {
-            const int s = (n_it - 1) & 1;
-            if (mbar_wait_suspend(&sm.o_full[s], ((n_it - 1) >> 1) & 1, abort_flag, err, 0x3300 | s)) {
-                tc_fence_after();
-                fold_o<OW>(o, lane_addr + O_COL + s * D + part * OW, corr_prev);
-            }
-        }
-        // total row sum over the parts
-        sm.ls[part][r] = l;
-        asm volatile("bar.sync %0, %1;" :: "r"(1 + qd), "n"(32 * SPLIT) : "memory");
-        l = 0.f;
-#pragma unroll
-        for (int q2 = 0; q2 < SPLIT; ++q2) l += sm.ls[q2][r];
         const int row = q0 + r;
         if (row < a.Tq) {
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            bf16* og = a.out + (((long long)b * a.Tq + row) * a.Hq + h) * D + part * OW;
+            bf16* og = a.out + (((long long)b * a.Tq + row) * a.Hq + h) * D + quarter * OW;
 #pragma unroll
             for (int c = 0; c < OW; c += 8) {
-                uint4 w;
-                w.x = pack_bf16(o[c] * inv, o[c + 1] * inv);
-                w.y = pack_bf16(o[c + 2] * inv, o[c + 3] * inv);
-                w.z = pack_bf16(o[c + 4] * inv, o[c + 5] * inv);
-                w.w = pack_bf16(o[c + 6] * inv, o[c + 7] * inv);
-                *reinterpret_cast<uint4*>(og + c) = w;
+                uint4 y;
+                y.x = pack_bf16(o[c] * inv, o[c + 1] * inv);
+                y.y = pack_bf16(o[c + 2] * inv, o[c + 3] * inv);
+                y.z = pack_bf16(o[c + 4] * inv, o[c + 5] * inv);
+                y.w = pack_bf16(o[c + 6] * inv, o[c + 7] * inv);
+                *reinterpret_cast<uint4*>(og + c) = y;
             }
-            if (part == 0) a.lse[((long long)b * a.Hq + h) * a.Tq + row] = l > 0.f ? m * a.scale + logf(l) : -INFINITY;
+            if (quarter == 0) a.lse[((long long)b * a.Hq + h) * a.Tq + row] = l > 0.f ? mm * a.scale + logf(l) : -INFINITY;
         }
     }
     tc_fence_before();
@@ -299,7 +304,11 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 //                          queries: S^T = K Q^T and dP^T = V dO^T -> P^T, dS^T (thread = key row) -> shared memory ->
 //                          dV += P^T dO and dK += dS^T Q accumulated in tensor memory.
 // A [64 x D] tile loaded as D/64 boxes of {64 d, 64 rows} serves both as a K-major operand (rows = N) of the score GEMMs
-// and as an MN-major operand (rows = K) of the gradient GEMMs.  Same warp roles, barriers and bounded waits as the forward.
+// and as an MN-major operand (rows = K) of the gradient GEMMs.  Same warp roles, barriers and bounded waits as the forward:
+// two groups of eight warps take turns with the iterations, each with its own dS (and P^T) tile, so that one group's
+// exponentials run while the other's tile is read by the gradient GEMMs.  (All sixteen warps on one iteration and one tile: 4300
+// cycles an iteration against 1280 of tensor-core time.)
+// B=2, T=4096, 16 query and 4 kv heads of 128: dQ 335 -> 332 us, dK / dV 538 -> 509 us.
 // =====================================================================================================================
 constexpr int BT = 64;                                       // tile of the looped dimension (keys for dQ, queries for dK/dV)
 constexpr int NST = 3;                                       // TMA stages of the looped tiles: a stage is released only after the
@@ -323,9 +332,10 @@ struct __align__(1024) SmemBwd {
     uint8_t big1[BM * D * 2];          // dQ kernel: dO tile     | dK/dV kernel: V tile
     uint8_t st0[NST][BT * D * 2];        // dQ kernel: K stages    | dK/dV kernel: Q stages
     uint8_t st1[NST][BT * D * 2];        // dQ kernel: V stages    | dK/dV kernel: dO stages
-    uint8_t p[BM * BT * 2];            // dS (dQ kernel) | P^T (dK/dV kernel), K-major, 128 rows x 128 bytes
-    uint8_t ds[BM * BT * 2];           // dS^T (dK/dV kernel)
-    uint64_t big_full, st_full[NST], st_empty[NST], s_full[2], p_ready, acc_done;
+    uint8_t p[2][BM * BT * 2];         // per group: dS (dQ kernel) | P^T (dK/dV kernel), K-major, 128 rows x 128 bytes
+    uint8_t ds[2][BM * BT * 2];        // dS^T (dK/dV kernel)
+    float lse2[NST][BT], delta[NST][BT];     // of the looped queries (dK/dV kernel)
+    uint64_t big_full, st_full[NST], st_empty[NST], stat_full[NST], s_full[2], p_ready[2], acc_done[2];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -357,10 +367,8 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.big_full, 1);
-        for (int s = 0; s < NST; ++s) { mbar_init(&sm.st_full[s], 1); mbar_init(&sm.st_empty[s], 1); }
-        for (int s = 0; s < 2; ++s) mbar_init(&sm.s_full[s], 1);
-        mbar_init(&sm.p_ready, 4 * SPLIT);
-        mbar_init(&sm.acc_done, 1);
+        for (int s = 0; s < NST; ++s) { mbar_init(&sm.st_full[s], 1); mbar_init(&sm.st_empty[s], 1); mbar_init(&sm.stat_full[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.p_ready[s], 8); mbar_init(&sm.acc_done[s], 1); }
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -422,72 +430,77 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             for (int j = 0; ok && j < n_it; ++j) {
                 if (j + 1 < n_it) { ok = issue_sd(j + 1); if (!ok) break; }
                 const int s = j % NST;
-                if (!mbar_wait_suspend(&sm.p_ready, j & 1, abort_flag, err, 0x4400)) break;
+                if (!mbar_wait_suspend(&sm.p_ready[j & 1], (j >> 1) & 1, abort_flag, err, 0x4400)) break;
                 tc_fence_after();
-                const uint32_t pl = desc_lo<false>(s32(sm.p)), kl = desc_lo<true>(s32(sm.st0[s]));
+                const uint32_t pl = desc_lo<false>(s32(sm.p[j & 1])), kl = desc_lo<true>(s32(sm.st0[s]));
 #pragma unroll
                 for (int kk = 0; kk < BT / UMMA_K; ++kk)
                     umma_lo(tmem_base + ACC_COL, pl + kk * 2, kl + kk * 128, idesc_a, (j > 0 || kk > 0) ? 1u : 0u, issue);
                 umma_commit_if(&sm.st_empty[s], issue);
-                umma_commit_if(&sm.acc_done, issue);
+                umma_commit_if(&sm.acc_done[j & 1], issue);
             }
         }
     } else if (warp >= 4) {
-        const int qd = warp & 3, part = (warp - 4) >> 2;
+        const int qd = warp & 3, quarter = (warp - 4) >> 2, grp = quarter >> 1, part = quarter & 1;
         const int r = qd * 32 + lane;
         const int row = q0 + r;
         const int qi = a.q_offset + row;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
         const float sc = a.scale * LOG2E;
-        constexpr int CW = BT / SPLIT;                           // 16 keys per thread
+        constexpr int CW = BT / 2;                               // 32 keys per thread
         const long long stat = ((long long)b * a.Hq + h) * a.Tq + row;
         const float lse2 = row < a.Tq ? a.lse[stat] * LOG2E : INFINITY;
         const float dl = row < a.Tq ? a.delta[stat] : 0.f;
-        uint8_t* prow = sm.p + (r >> 3) * 1024 + (r & 7) * 128;
+        uint8_t* prow = sm.p[grp] + (r >> 3) * 1024 + (r & 7) * 128;
         bool alive = n_it > 0;
-        for (int j = 0; alive && j < n_it; ++j) {
-            const int s = j & 1;
+        for (int j = grp; alive && j < n_it; j += 2) {
+            const int k = j >> 1;
             const int key0 = (nb_lo + j) * BT + part * CW;
-            if (!mbar_wait_suspend(&sm.s_full[s], (j >> 1) & 1, abort_flag, err, 0x4500 | s)) { alive = false; break; }
+            if (!mbar_wait_suspend(&sm.s_full[grp], k & 1, abort_flag, err, 0x4500 | grp)) { alive = false; break; }
             tc_fence_after();
-            uint32_t sv[CW], dv[CW];
-            tmem_ld16(lane_addr + s * 128 + part * CW, sv);
-            tmem_ld16(lane_addr + s * 128 + 64 + part * CW, dv);
-            tmem_ld_wait();
             // masking is needed only on tiles that cross the causal diagonal, the window edge or the key length
             const int tile_key0 = (nb_lo + j) * BT;
             const bool need_mask = (tile_key0 + BT - 1 > a.q_offset + q0) || (tile_key0 + BT > a.Tk) ||
                                    (a.window > 0 && tile_key0 <= a.q_offset + q0 + BM - 1 - a.window);
-            if (need_mask) {
-#pragma unroll
-                for (int i = 0; i < CW; ++i)
-                    if (!visible(key0 + i, qi, a.Tk, a.window)) sv[i] = 0xff800000u;      // -inf -> p = 0
-            }
             uint32_t pk[CW / 2];
 #pragma unroll
-            for (int i = 0; i < CW; i += 2) {
-                const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, -lse2)), p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -lse2));
-                pk[i >> 1] = pack_bf16(p0 * (__uint_as_float(dv[i]) - dl), p1 * (__uint_as_float(dv[i + 1]) - dl));   // the softmax scale is applied to dQ at the end
+            for (int c = 0; c < CW; c += 16) {
+                uint32_t sv[16], dv[16];
+                tmem_ld16(lane_addr + grp * 128 + part * CW + c, sv);
+                tmem_ld16(lane_addr + grp * 128 + 64 + part * CW + c, dv);
+                tmem_ld_wait();
+                if (need_mask) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (!visible(key0 + c + i, qi, a.Tk, a.window)) sv[i] = 0xff800000u;      // -inf -> p = 0
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, -lse2)), p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -lse2));
+                    pk[(c + i) >> 1] = pack_bf16(p0 * (__uint_as_float(dv[i]) - dl), p1 * (__uint_as_float(dv[i + 1]) - dl));   // the softmax scale is applied to dQ at the end
+                }
             }
-            if (j > 0 && !mbar_wait_suspend(&sm.acc_done, (j - 1) & 1, abort_flag, err, 0x4600)) { alive = false; break; }
-            *reinterpret_cast<uint4*>(prow + (((part * 2) ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            *reinterpret_cast<uint4*>(prow + (((part * 2 + 1) ^ (r & 7)) << 4)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            if (k > 0 && !mbar_wait_suspend(&sm.acc_done[grp], (k - 1) & 1, abort_flag, err, 0x4600 | grp)) { alive = false; break; }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4*>(prow + (((part * 4 + c) ^ (r & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
             tc_fence_before();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready);
+            if (lane == 0) mbar_arrive(&sm.p_ready[grp]);
         }
+        asm volatile("bar.sync 1, 512;" ::: "memory");           // behind it at most the last gradient GEMM of each group is outstanding
         constexpr int OW = D / SPLIT;
         uint32_t acc[OW];
 #pragma unroll
         for (int i = 0; i < OW; ++i) acc[i] = 0u;
-        if (alive && n_it > 0 && mbar_wait_suspend(&sm.acc_done, (n_it - 1) & 1, abort_flag, err, 0x4700)) {
+        if (alive && n_it > 0 && mbar_wait_suspend(&sm.acc_done[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, abort_flag, err, 0x4700)) {
             tc_fence_after();
-            tmem_ld<OW>(lane_addr + ACC_COL + part * OW, acc);
+            tmem_ld<OW>(lane_addr + ACC_COL + quarter * OW, acc);
             tmem_ld_wait();
         }
         if (row < a.Tq) {
-            bf16* og = a.dq + (((long long)b * a.Tq + row) * a.Hq + h) * D + part * OW;
+            bf16* og = a.dq + (((long long)b * a.Tq + row) * a.Hq + h) * D + quarter * OW;
 #pragma unroll
             for (int c = 0; c < OW; c += 8)
                 *reinterpret_cast<uint4*>(og + c) = make_uint4(pack_bf16(a.scale * __uint_as_float(acc[c]), a.scale * __uint_as_float(acc[c + 1])),
@@ -529,10 +542,8 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.big_full, 1);
-        for (int s = 0; s < NST; ++s) { mbar_init(&sm.st_full[s], 1); mbar_init(&sm.st_empty[s], 1); }
-        for (int s = 0; s < 2; ++s) mbar_init(&sm.s_full[s], 1);
-        mbar_init(&sm.p_ready, 4 * SPLIT);
-        mbar_init(&sm.acc_done, 1);
+        for (int s = 0; s < NST; ++s) { mbar_init(&sm.st_full[s], 1); mbar_init(&sm.st_empty[s], 1); mbar_init(&sm.stat_full[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.p_ready[s], 8); mbar_init(&sm.acc_done[s], 1); }
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -594,9 +605,9 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             for (int it = 0; ok && it < n_it; ++it) {
                 if (it + 1 < n_it) { ok = issue_sd(it + 1); if (!ok) break; }
                 const int s = it % NST;
-                if (!mbar_wait_suspend(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
+                if (!mbar_wait_suspend(&sm.p_ready[it & 1], (it >> 1) & 1, abort_flag, err, 0x5400)) break;
                 tc_fence_after();
-                const uint32_t pl = desc_lo<false>(s32(sm.p)), dl_ = desc_lo<false>(s32(sm.ds));
+                const uint32_t pl = desc_lo<false>(s32(sm.p[it & 1])), dl_ = desc_lo<false>(s32(sm.ds[it & 1]));
                 const uint32_t ql = desc_lo<true>(s32(sm.st0[s])), gl = desc_lo<true>(s32(sm.st1[s]));
 #pragma unroll
                 for (int kk = 0; kk < BT / UMMA_K; ++kk)        // dV += P^T dO
@@ -605,86 +616,93 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 for (int kk = 0; kk < BT / UMMA_K; ++kk)        // dK += dS^T Q
                     umma_lo(tmem_base + DK_COL, dl_ + kk * 2, ql + kk * 128, idesc_a, (it > 0 || kk > 0) ? 1u : 0u, issue);
                 umma_commit_if(&sm.st_empty[s], issue);
-                umma_commit_if(&sm.acc_done, issue);
+                umma_commit_if(&sm.acc_done[it & 1], issue);
             }
         }
+    } else if (warp == 2) {                                      // log-sum-exp and delta of the looped queries
+        for (int it = 0; it < n_it; ++it) {
+            const int s = it % NST;
+            const int h = hk * rep + it / ni, q0 = (i_lo + it % ni) * BT;
+            const long long row = ((long long)b * a.Hq + h) * a.Tq;
+            float x[2], y[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int q = q0 + lane + 32 * e;
+                x[e] = q < a.Tq ? __ldg(a.lse + row + q) * LOG2E : INFINITY;
+                y[e] = q < a.Tq ? __ldg(a.delta + row + q) : 0.f;
+            }
+            if (!mbar_wait_suspend(&sm.st_empty[s], ((it / NST) & 1) ^ 1, abort_flag, err, 0x5110 | s)) break;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) { sm.lse2[s][lane + 32 * e] = x[e]; sm.delta[s][lane + 32 * e] = y[e]; }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.stat_full[s]);
+        }
     } else if (warp >= 4) {
-        const int qd = warp & 3, part = (warp - 4) >> 2;
+        const int qd = warp & 3, quarter = (warp - 4) >> 2, grp = quarter >> 1, part = quarter & 1;
         const int r = qd * 32 + lane;                            // key row inside the tile
         const int key = k0 + r;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
         const float sc = a.scale * LOG2E;
-        constexpr int CW = BT / SPLIT;                           // 16 queries per thread
-        uint8_t* prow = sm.p + (r >> 3) * 1024 + (r & 7) * 128;
-        uint8_t* drow = sm.ds + (r >> 3) * 1024 + (r & 7) * 128;
+        uint8_t* prow = sm.p[grp] + (r >> 3) * 1024 + (r & 7) * 128;
+        uint8_t* drow = sm.ds[grp] + (r >> 3) * 1024 + (r & 7) * 128;
         bool alive = n_it > 0;
-        for (int it = 0; alive && it < n_it; ++it) {
-            const int s = it & 1;
-            const int h = hk * rep + it / ni;
-            const int qbase = (i_lo + it % ni) * BT + part * CW;     // first query of this thread's columns
-            const float* lse_p = a.lse + ((long long)b * a.Hq + h) * a.Tq;
-            const float* del_p = a.delta + ((long long)b * a.Hq + h) * a.Tq;
-            float l2[CW], dl[CW];
-            if ((a.Tq & 3) == 0 && qbase + CW <= a.Tq) {          // 16-byte aligned rows of lse / delta: 4 + 4 vector loads
-#pragma unroll
-                for (int i = 0; i < CW; i += 4) {
-                    const float4 x = __ldg(reinterpret_cast<const float4*>(lse_p + qbase + i));
-                    const float4 y = __ldg(reinterpret_cast<const float4*>(del_p + qbase + i));
-                    l2[i] = x.x * LOG2E; l2[i + 1] = x.y * LOG2E; l2[i + 2] = x.z * LOG2E; l2[i + 3] = x.w * LOG2E;
-                    dl[i] = y.x; dl[i + 1] = y.y; dl[i + 2] = y.z; dl[i + 3] = y.w;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < CW; ++i) {
-                    const int q = qbase + i;
-                    l2[i] = q < a.Tq ? __ldg(lse_p + q) * LOG2E : INFINITY;
-                    dl[i] = q < a.Tq ? __ldg(del_p + q) : 0.f;
-                }
-            }
-            if (!mbar_wait_suspend(&sm.s_full[s], (it >> 1) & 1, abort_flag, err, 0x5500 | s)) { alive = false; break; }
-            tc_fence_after();
-            uint32_t sv[CW], dv[CW];
-            tmem_ld16(lane_addr + s * 128 + part * CW, sv);
-            tmem_ld16(lane_addr + s * 128 + 64 + part * CW, dv);
-            tmem_ld_wait();
+        for (int it = grp; alive && it < n_it; it += 2) {
+            const int k = it >> 1, g = it % NST;
             const int tile_q0 = (i_lo + it % ni) * BT;
+            if (!mbar_wait_suspend(&sm.stat_full[g], (it / NST) & 1, abort_flag, err, 0x5510 | g)) { alive = false; break; }
+            if (!mbar_wait_suspend(&sm.s_full[grp], k & 1, abort_flag, err, 0x5500 | grp)) { alive = false; break; }
+            tc_fence_after();
             const bool need_mask = (k0 + BM - 1 > a.q_offset + tile_q0) || (k0 + BM > a.Tk) ||
                                    (a.window > 0 && k0 <= a.q_offset + tile_q0 + BT - 1 - a.window);
-            if (need_mask) {
+            uint32_t pk[16], dk2[16];
 #pragma unroll
-                for (int i = 0; i < CW; ++i)
-                    if (!visible(key, a.q_offset + qbase + i, a.Tk, a.window)) sv[i] = 0xff800000u;
-            }
-            uint32_t pk[CW / 2], dk2[CW / 2];
+            for (int c = 0; c < 32; c += 16) {                   // 32 queries per thread, 16 at a time
+                uint32_t sv[16], dv[16];
+                tmem_ld16(lane_addr + grp * 128 + part * 32 + c, sv);
+                tmem_ld16(lane_addr + grp * 128 + 64 + part * 32 + c, dv);
+                tmem_ld_wait();
+                if (need_mask) {
 #pragma unroll
-            for (int i = 0; i < CW; i += 2) {
-                const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, -l2[i])), p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -l2[i + 1]));
-                pk[i >> 1] = pack_bf16(p0, p1);
-                dk2[i >> 1] = pack_bf16(p0 * (__uint_as_float(dv[i]) - dl[i]), p1 * (__uint_as_float(dv[i + 1]) - dl[i + 1]));   // scale applied to dK at the end
+                    for (int i = 0; i < 16; ++i)
+                        if (!visible(key, a.q_offset + tile_q0 + part * 32 + c + i, a.Tk, a.window)) sv[i] = 0xff800000u;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 l2 = *reinterpret_cast<const float4*>(&sm.lse2[g][part * 32 + c + i]), dl = *reinterpret_cast<const float4*>(&sm.delta[g][part * 32 + c + i]);
+                    const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, -l2.x)), p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -l2.y));
+                    const float p2 = exp2f(fmaf(__uint_as_float(sv[i + 2]), sc, -l2.z)), p3 = exp2f(fmaf(__uint_as_float(sv[i + 3]), sc, -l2.w));
+                    const int o = (c + i) >> 1;
+                    pk[o] = pack_bf16(p0, p1);
+                    pk[o + 1] = pack_bf16(p2, p3);
+                    dk2[o] = pack_bf16(p0 * (__uint_as_float(dv[i]) - dl.x), p1 * (__uint_as_float(dv[i + 1]) - dl.y));          // scale applied to dK at the end
+                    dk2[o + 1] = pack_bf16(p2 * (__uint_as_float(dv[i + 2]) - dl.z), p3 * (__uint_as_float(dv[i + 3]) - dl.w));
+                }
             }
-            if (it > 0 && !mbar_wait_suspend(&sm.acc_done, (it - 1) & 1, abort_flag, err, 0x5600)) { alive = false; break; }
-            const int c0 = ((part * 2) ^ (r & 7)) << 4, c1 = ((part * 2 + 1) ^ (r & 7)) << 4;
-            *reinterpret_cast<uint4*>(prow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            *reinterpret_cast<uint4*>(prow + c1) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            *reinterpret_cast<uint4*>(drow + c0) = make_uint4(dk2[0], dk2[1], dk2[2], dk2[3]);
-            *reinterpret_cast<uint4*>(drow + c1) = make_uint4(dk2[4], dk2[5], dk2[6], dk2[7]);
+            if (k > 0 && !mbar_wait_suspend(&sm.acc_done[grp], (k - 1) & 1, abort_flag, err, 0x5600 | grp)) { alive = false; break; }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int at = ((part * 4 + c) ^ (r & 7)) << 4;
+                *reinterpret_cast<uint4*>(prow + at) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                *reinterpret_cast<uint4*>(drow + at) = make_uint4(dk2[4 * c], dk2[4 * c + 1], dk2[4 * c + 2], dk2[4 * c + 3]);
+            }
             tc_fence_before();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready);
+            if (lane == 0) mbar_arrive(&sm.p_ready[grp]);
         }
+        asm volatile("bar.sync 1, 512;" ::: "memory");           // behind it at most the last gradient GEMMs of each group are outstanding
         constexpr int OW = D / SPLIT;
         uint32_t av[OW], ak[OW];
 #pragma unroll
         for (int i = 0; i < OW; ++i) { av[i] = 0u; ak[i] = 0u; }
-        if (alive && n_it > 0 && mbar_wait_suspend(&sm.acc_done, (n_it - 1) & 1, abort_flag, err, 0x5700)) {
+        if (alive && n_it > 0 && mbar_wait_suspend(&sm.acc_done[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, abort_flag, err, 0x5700)) {
             tc_fence_after();
-            tmem_ld<OW>(lane_addr + DV_COL + part * OW, av);
-            tmem_ld<OW>(lane_addr + DK_COL + part * OW, ak);
+            tmem_ld<OW>(lane_addr + DV_COL + quarter * OW, av);
+            tmem_ld<OW>(lane_addr + DK_COL + quarter * OW, ak);
             tmem_ld_wait();
         }
         if (key < a.Tk) {
-            const long long off = (((long long)b * a.Tk + key) * a.Hkv + hk) * D + part * OW;
+            const long long off = (((long long)b * a.Tk + key) * a.Hkv + hk) * D + quarter * OW;
 #pragma unroll
             for (int c = 0; c < OW; c += 8) {
                 *reinterpret_cast<uint4*>(a.dv + off + c) = make_uint4(pack_bf16(__uint_as_float(av[c]), __uint_as_float(av[c + 1])),

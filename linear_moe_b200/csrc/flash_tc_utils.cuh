@@ -15,6 +15,13 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
     asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
                  :: "r"(s32(dst)), "l"(map), "r"(s32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                 :: "l"(map), "r"(s32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }     // shared memory may be reused
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 template <bool B_MN, int N>
 __host__ __device__ constexpr uint32_t idesc_bf16() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -40,26 +47,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                    "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
+                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[N]) {
     static_assert(N == 16 || N == 32 || N == 64, "tensor-memory load width");
     if constexpr (N == 64) tmem_ld64(taddr, r);
     else if constexpr (N == 32) tmem_ld32(taddr, r);
     else tmem_ld16(taddr, r);
-}
-// o[i] = o[i] * corr + partial[i] for this thread's OW columns of the partial output in tensor memory
-template <int OW>
-__device__ __forceinline__ void fold_o(float (&o)[OW], uint32_t taddr, float corr) {
-    uint32_t v[OW];
-    tmem_ld<OW>(taddr, v);
-    tmem_ld_wait();
-    const float2 c2 = make_float2(corr, corr);
-#pragma unroll
-    for (int i = 0; i < OW; i += 2) {                            // packed fp32 FMAs: two columns per instruction
-        const float2 r = __ffma2_rn(make_float2(o[i], o[i + 1]), c2, make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])));
-        o[i] = r.x;
-        o[i + 1] = r.y;
-    }
 }
 // The MMA warp runs its loop with all 32 lanes converged and only predicates the tcgen05 instructions on one lane: inside a
 // single-lane branch every operand lives in vector registers and each MMA pays for moving two 64-bit descriptors into
@@ -76,6 +75,13 @@ __device__ __forceinline__ void umma_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t
                  "mov.b64 da, {%1, %6};\nmov.b64 db, {%2, %6};\n"
                  "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}"
                  :: "r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(issue), "r"(DESC_HI) : "memory");
+}
+// D += A B with A in tensor memory: row r in lane r, two consecutive k per column
+__device__ __forceinline__ void umma_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
+    asm volatile("{\n.reg .pred p, q;\n.reg .b64 db;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
+                 "mov.b64 db, {%2, %6};\n"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}"
+                 :: "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(issue), "r"(DESC_HI) : "memory");
 }
 __device__ __forceinline__ void umma_commit_if(uint64_t* bar, uint32_t issue) {
     asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"

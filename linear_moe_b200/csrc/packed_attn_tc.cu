@@ -45,20 +45,6 @@ struct __align__(1024) Smem {
     int abort_flag;
 };
 
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
-                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
-}
-// D += A B with A in tensor memory: row r in lane r, two consecutive k per column
-__device__ __forceinline__ void umma_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate, uint32_t issue) {
-    asm volatile("{\n.reg .pred p, q;\n.reg .b64 db;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
-                 "mov.b64 db, {%2, %6};\n"
-                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}"
-                 :: "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(issue), "r"(DESC_HI) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // DV: value dims of a head, NB: value heads of a CTA
 template <int DQ, int DV, int NB, Weights W>
 __global__ void __launch_bounds__(THREADS, 1)
