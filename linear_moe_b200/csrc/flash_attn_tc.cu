@@ -296,24 +296,22 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 
 // =====================================================================================================================
-// Backward on tcgen05, two kernels that recompute the scores (7 GEMMs per tile pair instead of 5, no atomics):
-//   fa_bwd_dq_tc_kernel    one CTA = 128 queries of one head; loops over tiles of 64 keys:
-//                          S = Q K^T and dP = dO V^T into tensor memory -> dS = P (dP - delta) scale (softmax warps,
-//                          thread = query row) -> shared memory -> dQ += dS K accumulated in tensor memory.
-//   fa_bwd_dkv_tc_kernel   one CTA = 128 keys of one KV head; loops over the query heads of the group and tiles of 64
-//                          queries: S^T = K Q^T and dP^T = V dO^T -> P^T, dS^T (thread = key row) -> shared memory ->
+// Backward on tcgen05, two kernels that recompute the scores (7 GEMMs per tile pair instead of 5, no atomics), on tiles of
+// 128 queries x 128 keys:
+//   fa_bwd_dq_tc_kernel    one CTA = 128 queries of one head, looping over the key tiles:
+//                          S = Q K^T and dP = dO V^T into tensor memory -> dS = P (dP - delta) (softmax warps, thread = query row) ->
+//                          shared memory -> dQ += dS K accumulated in tensor memory.
+//   fa_bwd_dkv_tc_kernel   one CTA = 128 keys of one KV head, looping over the query heads of the group and their query
+//                          tiles: S^T = K Q^T and dP^T = V dO^T -> P^T, dS^T (thread = key row) -> shared memory ->
 //                          dV += P^T dO and dK += dS^T Q accumulated in tensor memory.
-// A [64 x D] tile loaded as D/64 boxes of {64 d, 64 rows} serves both as a K-major operand (rows = N) of the score GEMMs
-// and as an MN-major operand (rows = K) of the gradient GEMMs.  Same warp roles, barriers and bounded waits as the forward:
-// two groups of eight warps take turns with the iterations, each with its own dS (and P^T) tile, so that one group's
-// exponentials run while the other's tile is read by the gradient GEMMs.  (All sixteen warps on one iteration and one tile: 4300
-// cycles an iteration against 1280 of tensor-core time.)
-// B=2, T=4096, 16 query and 4 kv heads of 128: dQ 335 -> 332 us, dK / dV 538 -> 509 us.
+// A tile of 128 rows loaded as D/64 boxes of {64 d, 128 rows} serves both as a K-major operand (rows = N) of the score GEMMs
+// and as an MN-major operand (rows = K) of the gradient GEMMs.  Same warp roles and bounded waits as the forward; all sixteen softmax
+// warps share a tile, four per 32 rows with 32 columns each.  The order of the products keeps the tensor core busy while
+// the warps work: a score GEMM is issued as soon as its scores have been read, ahead of the gradient GEMM of the tile before.
+// Issuing a product costs about 70 cycles whatever its width, so the 64-wide tiles that stood here first (24 instructions per
+// 128 x 64 scores, now 32 per 128 x 128) were bound by the issuing warp: 2650 - 2790 cycles per 128 x 64.
+// B=2, T=4096, 16 query and 4 kv heads of 128: dk / dv 514 -> 397 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125).
 // =====================================================================================================================
-constexpr int BT = 64;                                       // tile of the looped dimension (keys for dQ, queries for dK/dV)
-constexpr int NST = 3;                                       // TMA stages of the looped tiles: a stage is released only after the
-                                                             // gradient MMAs of its iteration, so two stages would expose the load latency
-
 struct BwdArgs {
     const float* lse;     // [B, Hq, Tq] natural-log sum-exp from the forward
     const float* delta;   // [B, Hq, Tq] rowsum(dO * O)
@@ -326,32 +324,84 @@ struct BwdArgs {
     int* err;
 };
 
-template <int D>
-struct __align__(1024) SmemBwd {
-    uint8_t big0[BM * D * 2];          // dQ kernel: Q tile      | dK/dV kernel: K tile
-    uint8_t big1[BM * D * 2];          // dQ kernel: dO tile     | dK/dV kernel: V tile
-    uint8_t st0[NST][BT * D * 2];        // dQ kernel: K stages    | dK/dV kernel: Q stages
-    uint8_t st1[NST][BT * D * 2];        // dQ kernel: V stages    | dK/dV kernel: dO stages
-    uint8_t p[2][BM * BT * 2];         // per group: dS (dQ kernel) | P^T (dK/dV kernel), K-major, 128 rows x 128 bytes
-    uint8_t ds[2][BM * BT * 2];        // dS^T (dK/dV kernel)
-    float lse2[NST][BT], delta[NST][BT];     // of the looped queries (dK/dV kernel)
-    uint64_t big_full, st_full[NST], st_empty[NST], stat_full[NST], s_full[2], p_ready[2], acc_done[2];
-    uint32_t tmem_base;
-    int abort_flag;
-};
+constexpr int BLK = BM * 128;                                // one 64-column block of a 128-row tile
 
 __device__ __forceinline__ bool visible(int key, int qi, int Tk, int window) {
     return key <= qi && key < Tk && (window <= 0 || key > qi - window);
 }
+template <int D>
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int h, int row, int b) {
+#pragma unroll
+    for (int kb = 0; kb < D / 64; ++kb) tma_load_4d(dst + kb * BLK, map, bar, kb * 64, h, row, b);
+}
+// [128 x 128] = A B^T over D, both tiles K-major
+template <int D>
+__device__ __forceinline__ void score_product(uint32_t tmem_d, const uint8_t* A, const uint8_t* B, uint32_t issue) {
+    const uint32_t al = desc_lo<false>(s32(A)), bl = desc_lo<false>(s32(B));
+#pragma unroll
+    for (int kk = 0; kk < D / UMMA_K; ++kk) {
+        const uint32_t off = ((kk / 4) * BLK + (kk % 4) * 32) >> 4;
+        umma_lo(tmem_d, al + off, bl + off, idesc_bf16<false, 128>(), kk > 0 ? 1u : 0u, issue);
+    }
+}
+// [128 x D] (+)= A B over 128: A a K-major [128 x 128] tile, B's rows are K
+template <int D>
+__device__ __forceinline__ void grad_product(uint32_t tmem_d, const uint8_t* A, const uint8_t* B, bool add, uint32_t issue) {
+    const uint32_t al = desc_lo<false>(s32(A)), bl = ((s32(B) >> 4) & 0x3FFFu) | ((uint32_t)(BLK >> 4) << 16);
+#pragma unroll
+    for (int kk = 0; kk < 128 / UMMA_K; ++kk)
+        umma_lo(tmem_d, al + (((kk / 4) * BLK + (kk % 4) * 32) >> 4), bl + ((kk * 2048) >> 4), idesc_bf16<true, D>(), (add || kk > 0) ? 1u : 0u, issue);
+}
+// this thread's 32 columns (64 bytes) of row r of a [128 x 128] tile
+__device__ __forceinline__ void store_columns(uint8_t* tile, int r, int part, const uint32_t (&v)[16]) {
+    uint8_t* row = tile + (part >> 1) * BLK + r * 128;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(row + ((((part & 1) * 4 + c) ^ (r & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+__device__ __forceinline__ void hand_over(uint64_t* bar) {
+    tc_fence_before();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+// a thread's part of an accumulator row, times `scale`, to memory
+template <int OW>
+__device__ __forceinline__ void write_row(bf16* out, uint32_t taddr, float scale, bool valid, bool empty) {
+    uint32_t v[OW];
+    tmem_ld<OW>(taddr, v);
+    tmem_ld_wait();
+    if (!valid) return;
+#pragma unroll
+    for (int c = 0; c < OW; c += 8) {
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = empty ? 0.f : scale * __uint_as_float(v[c + e]);
+        *reinterpret_cast<uint4*>(out + c) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+    }
+}
+
+// With 128-wide heads the tiles fill the shared memory: it has to start on a 1024-byte boundary (there is no static one), which the
+// kernels check before anything else.
+template <int D>
+struct __align__(1024) SmemDq {
+    uint8_t q[BM * D * 2], g[BM * D * 2], k[2][BM * D * 2], v[2][BM * D * 2], ds[BM * BM * 2];
+    uint64_t qg_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], dp_full, ds_ready, dq_done;
+    uint32_t tmem_base;
+    int abort_flag;
+};
 
 template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdArgs a) {
     extern __shared__ uint8_t smem_raw[];
-    SmemBwd<D>& sm = *reinterpret_cast<SmemBwd<D>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int DK = D / 64;
-    constexpr uint32_t TMEM_COLS = 512, ACC_COL = 256;
+    SmemDq<D>& sm = *reinterpret_cast<SmemDq<D>*>(smem_raw);
+    if ((s32(smem_raw) & 1023u) != 0) {
+        if (threadIdx.x == 0) atomicCAS(a.err, 0, 0x4001);
+        return;
+    }
+    constexpr uint32_t TMEM_COLS = 512, DP = 256, DQ = 384;                  // two buffers of scores in front
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qb = gridDim.x - 1 - blockIdx.x;
     const int h = blockIdx.y, b = blockIdx.z;
@@ -362,13 +412,17 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int last_q = min(a.Tq, q0 + BM) - 1;
     const int k_hi = min(a.Tk, a.q_offset + last_q + 1);
     const int k_lo = a.window > 0 ? max(0, a.q_offset + q0 - a.window + 1) : 0;
-    const int nb_lo = k_lo / BT, nb_hi = (k_hi + BT - 1) / BT;
+    const int nb_lo = k_lo / BN, nb_hi = (k_hi + BN - 1) / BN;
     const int n_it = max(nb_hi - nb_lo, 0);
 
     if (threadIdx.x == 0) {
-        mbar_init(&sm.big_full, 1);
-        for (int s = 0; s < NST; ++s) { mbar_init(&sm.st_full[s], 1); mbar_init(&sm.st_empty[s], 1); mbar_init(&sm.stat_full[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.p_ready[s], 8); mbar_init(&sm.acc_done[s], 1); }
+        mbar_init(&sm.qg_full, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1);
+            mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1);
+            mbar_init(&sm.s_full[s], 1);
+        }
+        mbar_init(&sm.dp_full, 1); mbar_init(&sm.ds_ready, 4 * SPLIT); mbar_init(&sm.dq_done, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -383,131 +437,107 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
-            mbar_expect_tx(&sm.big_full, 2 * BM * D * 2);
-#pragma unroll
-            for (int kb = 0; kb < DK; ++kb) {
-                tma_load_4d(sm.big0 + kb * BM * 128, &tmQ, &sm.big_full, kb * 64, h, q0, b);
-                tma_load_4d(sm.big1 + kb * BM * 128, &tmG, &sm.big_full, kb * 64, h, q0, b);
-            }
+            mbar_expect_tx(&sm.qg_full, 2 * BM * D * 2);
+            load_tile<D>(sm.q, &tmQ, &sm.qg_full, h, q0, b);
+            load_tile<D>(sm.g, &tmG, &sm.qg_full, h, q0, b);
             for (int j = 0; j < n_it; ++j) {
-                const int s = j % NST;
-                const int key0 = (nb_lo + j) * BT;
-                if (!mbar_wait_suspend(&sm.st_empty[s], ((j / NST) & 1) ^ 1, abort_flag, err, 0x4100 | s)) break;
-                mbar_expect_tx(&sm.st_full[s], 2 * BT * D * 2);
-#pragma unroll
-                for (int kb = 0; kb < DK; ++kb) {
-                    tma_load_4d(sm.st0[s] + kb * 8192, &tmK, &sm.st_full[s], kb * 64, hk, key0, b);
-                    tma_load_4d(sm.st1[s] + kb * 8192, &tmV, &sm.st_full[s], kb * 64, hk, key0, b);
-                }
+                const int s = j & 1, key0 = (nb_lo + j) * BN;
+                const uint32_t ph = ((j >> 1) & 1) ^ 1;
+                if (!mbar_wait_suspend(&sm.k_empty[s], ph, abort_flag, err, 0x4100 | s)) break;
+                mbar_expect_tx(&sm.k_full[s], BM * D * 2);
+                load_tile<D>(sm.k[s], &tmK, &sm.k_full[s], hk, key0, b);
+                if (!mbar_wait_suspend(&sm.v_empty[s], ph, abort_flag, err, 0x4110 | s)) break;
+                mbar_expect_tx(&sm.v_full[s], BM * D * 2);
+                load_tile<D>(sm.v[s], &tmV, &sm.v_full[s], hk, key0, b);
             }
         }
     } else if (warp == 1) {
         if (n_it > 0) {
             const uint32_t issue = lane == 0 ? 1u : 0u;
-            constexpr uint32_t idesc_s = idesc_bf16<false, BT>();       // [128 q] x [64 keys], both K-major
-            constexpr uint32_t idesc_a = idesc_bf16<true, D>();         // dQ += dS K: B = K tile read MN-major
-            bool ok = mbar_wait_suspend(&sm.big_full, 0, abort_flag, err, 0x4200);
-            auto issue_sd = [&](int j) -> bool {
-                const int s = j & 1, g = j % NST;                    // tensor-memory buffer, shared-memory stage
-                if (!mbar_wait_suspend(&sm.st_full[g], (j / NST) & 1, abort_flag, err, 0x4300 | g)) return false;
+            bool ok = mbar_wait_suspend(&sm.qg_full, 0, abort_flag, err, 0x4200);
+            auto scores = [&](int j) -> bool {
+                const int s = j & 1;
+                if (!mbar_wait_suspend(&sm.k_full[s], (j >> 1) & 1, abort_flag, err, 0x4300 | s)) return false;
                 tc_fence_after();
-                const uint32_t ql = desc_lo<false>(s32(sm.big0)), gl = desc_lo<false>(s32(sm.big1));
-                const uint32_t kl = desc_lo<false>(s32(sm.st0[g])), vl = desc_lo<false>(s32(sm.st1[g]));
-#pragma unroll
-                for (int kk = 0; kk < D / UMMA_K; ++kk) {
-                    const uint32_t ao = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4, bo = ((kk / 4) * 8192 + (kk % 4) * 32) >> 4;
-                    umma_lo(tmem_base + s * 128, ql + ao, kl + bo, idesc_s, kk > 0 ? 1u : 0u, issue);
-                }
-#pragma unroll
-                for (int kk = 0; kk < D / UMMA_K; ++kk) {
-                    const uint32_t ao = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4, bo = ((kk / 4) * 8192 + (kk % 4) * 32) >> 4;
-                    umma_lo(tmem_base + s * 128 + 64, gl + ao, vl + bo, idesc_s, kk > 0 ? 1u : 0u, issue);
-                }
+                score_product<D>(tmem_base + s * 128, sm.q, sm.k[s], issue);
                 umma_commit_if(&sm.s_full[s], issue);
                 return true;
             };
-            if (ok) ok = issue_sd(0);
-            for (int j = 0; ok && j < n_it; ++j) {
-                if (j + 1 < n_it) { ok = issue_sd(j + 1); if (!ok) break; }
-                const int s = j % NST;
-                if (!mbar_wait_suspend(&sm.p_ready[j & 1], (j >> 1) & 1, abort_flag, err, 0x4400)) break;
+            auto dprobs = [&](int j) -> bool {
+                const int s = j & 1;
+                if (!mbar_wait_suspend(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x4310 | s)) return false;
                 tc_fence_after();
-                const uint32_t pl = desc_lo<false>(s32(sm.p[j & 1])), kl = desc_lo<true>(s32(sm.st0[s]));
-#pragma unroll
-                for (int kk = 0; kk < BT / UMMA_K; ++kk)
-                    umma_lo(tmem_base + ACC_COL, pl + kk * 2, kl + kk * 128, idesc_a, (j > 0 || kk > 0) ? 1u : 0u, issue);
-                umma_commit_if(&sm.st_empty[s], issue);
-                umma_commit_if(&sm.acc_done[j & 1], issue);
+                score_product<D>(tmem_base + DP, sm.g, sm.v[s], issue);
+                umma_commit_if(&sm.v_empty[s], issue);
+                umma_commit_if(&sm.dp_full, issue);
+                return true;
+            };
+            if (ok) ok = scores(0) && dprobs(0);
+            if (ok && n_it > 1) ok = scores(1);
+            for (int j = 0; ok && j < n_it; ++j) {
+                const int s = j & 1;
+                if (!mbar_wait_suspend(&sm.ds_ready, j & 1, abort_flag, err, 0x4400)) break;
+                if (j + 1 < n_it && !dprobs(j + 1)) break;
+                tc_fence_after();
+                grad_product<D>(tmem_base + DQ, sm.ds, sm.k[s], j > 0, issue);
+                umma_commit_if(&sm.k_empty[s], issue);
+                umma_commit_if(&sm.dq_done, issue);
+                if (j + 2 < n_it) ok = scores(j + 2);
             }
         }
     } else if (warp >= 4) {
-        const int qd = warp & 3, quarter = (warp - 4) >> 2, grp = quarter >> 1, part = quarter & 1;
+        const int qd = warp & 3, part = (warp - 4) >> 2;
         const int r = qd * 32 + lane;
         const int row = q0 + r;
         const int qi = a.q_offset + row;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
         const float sc = a.scale * LOG2E;
-        constexpr int CW = BT / 2;                               // 32 keys per thread
         const long long stat = ((long long)b * a.Hq + h) * a.Tq + row;
         const float lse2 = row < a.Tq ? a.lse[stat] * LOG2E : INFINITY;
         const float dl = row < a.Tq ? a.delta[stat] : 0.f;
-        uint8_t* prow = sm.p[grp] + (r >> 3) * 1024 + (r & 7) * 128;
         bool alive = n_it > 0;
-        for (int j = grp; alive && j < n_it; j += 2) {
-            const int k = j >> 1;
-            const int key0 = (nb_lo + j) * BT + part * CW;
-            if (!mbar_wait_suspend(&sm.s_full[grp], k & 1, abort_flag, err, 0x4500 | grp)) { alive = false; break; }
-            tc_fence_after();
+        for (int j = 0; alive && j < n_it; ++j) {
+            const int s = j & 1;
+            const int tile_key0 = (nb_lo + j) * BN, key0 = tile_key0 + part * 32;
             // masking is needed only on tiles that cross the causal diagonal, the window edge or the key length
-            const int tile_key0 = (nb_lo + j) * BT;
-            const bool need_mask = (tile_key0 + BT - 1 > a.q_offset + q0) || (tile_key0 + BT > a.Tk) ||
+            const bool need_mask = (tile_key0 + BN - 1 > a.q_offset + q0) || (tile_key0 + BN > a.Tk) ||
                                    (a.window > 0 && tile_key0 <= a.q_offset + q0 + BM - 1 - a.window);
-            uint32_t pk[CW / 2];
+            if (!mbar_wait_suspend(&sm.s_full[s], (j >> 1) & 1, abort_flag, err, 0x4500 | s)) { alive = false; break; }
+            tc_fence_after();
+            float p[32];
 #pragma unroll
-            for (int c = 0; c < CW; c += 16) {
-                uint32_t sv[16], dv[16];
-                tmem_ld16(lane_addr + grp * 128 + part * CW + c, sv);
-                tmem_ld16(lane_addr + grp * 128 + 64 + part * CW + c, dv);
+            for (int c = 0; c < 32; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(lane_addr + s * 128 + part * 32 + c, v);
                 tmem_ld_wait();
                 if (need_mask) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
-                        if (!visible(key0 + c + i, qi, a.Tk, a.window)) sv[i] = 0xff800000u;      // -inf -> p = 0
+                        if (!visible(key0 + c + i, qi, a.Tk, a.window)) v[i] = 0xff800000u;      // -inf -> p = 0
                 }
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, -lse2)), p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -lse2));
-                    pk[(c + i) >> 1] = pack_bf16(p0 * (__uint_as_float(dv[i]) - dl), p1 * (__uint_as_float(dv[i + 1]) - dl));   // the softmax scale is applied to dQ at the end
-                }
+                for (int i = 0; i < 16; ++i) p[c + i] = exp2f(fmaf(__uint_as_float(v[i]), sc, -lse2));
             }
-            if (k > 0 && !mbar_wait_suspend(&sm.acc_done[grp], (k - 1) & 1, abort_flag, err, 0x4600 | grp)) { alive = false; break; }
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                *reinterpret_cast<uint4*>(prow + (((part * 4 + c) ^ (r & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-            tc_fence_before();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready[grp]);
-        }
-        asm volatile("bar.sync 1, 512;" ::: "memory");           // behind it at most the last gradient GEMM of each group is outstanding
-        constexpr int OW = D / SPLIT;
-        uint32_t acc[OW];
-#pragma unroll
-        for (int i = 0; i < OW; ++i) acc[i] = 0u;
-        if (alive && n_it > 0 && mbar_wait_suspend(&sm.acc_done[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, abort_flag, err, 0x4700)) {
+            if (!mbar_wait_suspend(&sm.dp_full, j & 1, abort_flag, err, 0x4510)) { alive = false; break; }
             tc_fence_after();
-            tmem_ld<OW>(lane_addr + ACC_COL + quarter * OW, acc);
-            tmem_ld_wait();
-        }
-        if (row < a.Tq) {
-            bf16* og = a.dq + (((long long)b * a.Tq + row) * a.Hq + h) * D + quarter * OW;
+            uint32_t pk[16];
 #pragma unroll
-            for (int c = 0; c < OW; c += 8)
-                *reinterpret_cast<uint4*>(og + c) = make_uint4(pack_bf16(a.scale * __uint_as_float(acc[c]), a.scale * __uint_as_float(acc[c + 1])),
-                                                               pack_bf16(a.scale * __uint_as_float(acc[c + 2]), a.scale * __uint_as_float(acc[c + 3])),
-                                                               pack_bf16(a.scale * __uint_as_float(acc[c + 4]), a.scale * __uint_as_float(acc[c + 5])),
-                                                               pack_bf16(a.scale * __uint_as_float(acc[c + 6]), a.scale * __uint_as_float(acc[c + 7])));
+            for (int c = 0; c < 32; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(lane_addr + DP + part * 32 + c, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i += 2)                                                // the softmax scale is applied to dQ at the end
+                    pk[(c + i) >> 1] = pack_bf16(p[c + i] * (__uint_as_float(v[i]) - dl), p[c + i + 1] * (__uint_as_float(v[i + 1]) - dl));
+            }
+            if (j > 0 && !mbar_wait_suspend(&sm.dq_done, (j - 1) & 1, abort_flag, err, 0x4600)) { alive = false; break; }
+            store_columns(sm.ds, r, part, pk);
+            hand_over(&sm.ds_ready);
         }
+        if (alive) alive = mbar_wait_suspend(&sm.dq_done, (n_it - 1) & 1, abort_flag, err, 0x4700);
+        tc_fence_after();
+        constexpr int OW = D / SPLIT;
+        write_row<OW>(a.dq + (((long long)b * a.Tq + row) * a.Hq + h) * D + part * OW, lane_addr + DQ + part * OW, a.scale, row < a.Tq, !alive);
     }
     tc_fence_before();
     __syncthreads();
@@ -519,31 +549,46 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
 
 template <int D>
+struct __align__(1024) SmemDkv {
+    uint8_t k[BM * D * 2], v[BM * D * 2], q[2][BM * D * 2], g[BM * D * 2], p[BM * BM * 2], ds[BM * BM * 2];
+    float lse2[2][BM], delta[2][BM];                                         // of the looped queries
+    uint64_t kv_full, q_full[2], q_empty[2], stat_full[2], g_full, g_empty, s_full, dp_full, p_ready, ds_ready, dv_done, dk_done;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdArgs a) {
     extern __shared__ uint8_t smem_raw[];
-    SmemBwd<D>& sm = *reinterpret_cast<SmemBwd<D>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int DK = D / 64;
-    constexpr uint32_t TMEM_COLS = 512, DV_COL = 256, DK_COL = 256 + D;
+    SmemDkv<D>& sm = *reinterpret_cast<SmemDkv<D>*>(smem_raw);
+    if ((s32(smem_raw) & 1023u) != 0) {
+        if (threadIdx.x == 0) atomicCAS(a.err, 0, 0x5001);
+        return;
+    }
+    constexpr uint32_t TMEM_COLS = 512, ST = 0, DP = 128, DV = 256, DKC = 384;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kb_tile = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
     const int rep = a.Hq / a.Hkv;
     const int k0 = kb_tile * BM;
     volatile int* abort_flag = &sm.abort_flag;
     int* err = a.err;
-    // query tiles (of 64) that can see a key of this tile: q >= k0 - q_offset, and with a window q < k0 + 127 + window - q_offset
-    const int i_lo = max(0, k0 - a.q_offset) / BT;
+    // query tiles that can see a key of this tile: q >= k0 - q_offset, and with a window q < k0 + 127 + window - q_offset
+    const int i_lo = max(0, k0 - a.q_offset) / BM;
     int q_end = a.Tq;
     if (a.window > 0) q_end = min(a.Tq, max(0, k0 + BM - 1 + a.window - a.q_offset));
-    const int i_hi = (q_end + BT - 1) / BT;
+    const int i_hi = (q_end + BM - 1) / BM;
     const int ni = max(i_hi - i_lo, 0);
     const int n_it = ni * rep;
 
     if (threadIdx.x == 0) {
-        mbar_init(&sm.big_full, 1);
-        for (int s = 0; s < NST; ++s) { mbar_init(&sm.st_full[s], 1); mbar_init(&sm.st_empty[s], 1); mbar_init(&sm.stat_full[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.p_ready[s], 8); mbar_init(&sm.acc_done[s], 1); }
+        mbar_init(&sm.kv_full, 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(&sm.q_full[s], 1); mbar_init(&sm.q_empty[s], 1); mbar_init(&sm.stat_full[s], 1); }
+        mbar_init(&sm.g_full, 1); mbar_init(&sm.g_empty, 1);
+        mbar_init(&sm.s_full, 1); mbar_init(&sm.dp_full, 1);
+        mbar_init(&sm.p_ready, 4 * SPLIT); mbar_init(&sm.ds_ready, 4 * SPLIT);
+        mbar_init(&sm.dv_done, 1); mbar_init(&sm.dk_done, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -558,163 +603,138 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
-            mbar_expect_tx(&sm.big_full, 2 * BM * D * 2);
-#pragma unroll
-            for (int kb = 0; kb < DK; ++kb) {
-                tma_load_4d(sm.big0 + kb * BM * 128, &tmK, &sm.big_full, kb * 64, hk, k0, b);
-                tma_load_4d(sm.big1 + kb * BM * 128, &tmV, &sm.big_full, kb * 64, hk, k0, b);
-            }
+            mbar_expect_tx(&sm.kv_full, 2 * BM * D * 2);
+            load_tile<D>(sm.k, &tmK, &sm.kv_full, hk, k0, b);
+            load_tile<D>(sm.v, &tmV, &sm.kv_full, hk, k0, b);
             for (int it = 0; it < n_it; ++it) {
-                const int s = it % NST;
-                const int h = hk * rep + it / ni, q0 = (i_lo + it % ni) * BT;
-                if (!mbar_wait_suspend(&sm.st_empty[s], ((it / NST) & 1) ^ 1, abort_flag, err, 0x5100 | s)) break;
-                mbar_expect_tx(&sm.st_full[s], 2 * BT * D * 2);
-#pragma unroll
-                for (int kb = 0; kb < DK; ++kb) {
-                    tma_load_4d(sm.st0[s] + kb * 8192, &tmQ, &sm.st_full[s], kb * 64, h, q0, b);
-                    tma_load_4d(sm.st1[s] + kb * 8192, &tmG, &sm.st_full[s], kb * 64, h, q0, b);
-                }
+                const int s = it & 1;
+                const int h = hk * rep + it / ni, q0 = (i_lo + it % ni) * BM;
+                if (!mbar_wait_suspend(&sm.q_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, err, 0x5100 | s)) break;
+                mbar_expect_tx(&sm.q_full[s], BM * D * 2);
+                load_tile<D>(sm.q[s], &tmQ, &sm.q_full[s], h, q0, b);
+                if (!mbar_wait_suspend(&sm.g_empty, (it & 1) ^ 1, abort_flag, err, 0x5120)) break;
+                mbar_expect_tx(&sm.g_full, BM * D * 2);
+                load_tile<D>(sm.g, &tmG, &sm.g_full, h, q0, b);
             }
         }
     } else if (warp == 1) {
         if (n_it > 0) {
             const uint32_t issue = lane == 0 ? 1u : 0u;
-            constexpr uint32_t idesc_s = idesc_bf16<false, BT>();       // [128 keys] x [64 queries], both K-major
-            constexpr uint32_t idesc_a = idesc_bf16<true, D>();         // B = dO / Q tile read MN-major
-            bool ok = mbar_wait_suspend(&sm.big_full, 0, abort_flag, err, 0x5200);
-            auto issue_sd = [&](int it) -> bool {
-                const int s = it & 1, g = it % NST;                  // tensor-memory buffer, shared-memory stage
-                if (!mbar_wait_suspend(&sm.st_full[g], (it / NST) & 1, abort_flag, err, 0x5300 | g)) return false;
+            bool ok = mbar_wait_suspend(&sm.kv_full, 0, abort_flag, err, 0x5200);
+            auto scores = [&](int it) -> bool {
+                if (!mbar_wait_suspend(&sm.q_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5300 | (it & 1))) return false;
                 tc_fence_after();
-                const uint32_t kl = desc_lo<false>(s32(sm.big0)), vl = desc_lo<false>(s32(sm.big1));
-                const uint32_t ql = desc_lo<false>(s32(sm.st0[g])), gl = desc_lo<false>(s32(sm.st1[g]));
-#pragma unroll
-                for (int kk = 0; kk < D / UMMA_K; ++kk) {
-                    const uint32_t ao = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4, bo = ((kk / 4) * 8192 + (kk % 4) * 32) >> 4;
-                    umma_lo(tmem_base + s * 128, kl + ao, ql + bo, idesc_s, kk > 0 ? 1u : 0u, issue);
-                }
-#pragma unroll
-                for (int kk = 0; kk < D / UMMA_K; ++kk) {
-                    const uint32_t ao = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4, bo = ((kk / 4) * 8192 + (kk % 4) * 32) >> 4;
-                    umma_lo(tmem_base + s * 128 + 64, vl + ao, gl + bo, idesc_s, kk > 0 ? 1u : 0u, issue);
-                }
-                umma_commit_if(&sm.s_full[s], issue);
+                score_product<D>(tmem_base + ST, sm.k, sm.q[it & 1], issue);
+                umma_commit_if(&sm.s_full, issue);
                 return true;
             };
-            if (ok) ok = issue_sd(0);
-            for (int it = 0; ok && it < n_it; ++it) {
-                if (it + 1 < n_it) { ok = issue_sd(it + 1); if (!ok) break; }
-                const int s = it % NST;
-                if (!mbar_wait_suspend(&sm.p_ready[it & 1], (it >> 1) & 1, abort_flag, err, 0x5400)) break;
+            auto dprobs = [&](int it) -> bool {
+                if (!mbar_wait_suspend(&sm.g_full, it & 1, abort_flag, err, 0x5310)) return false;
                 tc_fence_after();
-                const uint32_t pl = desc_lo<false>(s32(sm.p[it & 1])), dl_ = desc_lo<false>(s32(sm.ds[it & 1]));
-                const uint32_t ql = desc_lo<true>(s32(sm.st0[s])), gl = desc_lo<true>(s32(sm.st1[s]));
-#pragma unroll
-                for (int kk = 0; kk < BT / UMMA_K; ++kk)        // dV += P^T dO
-                    umma_lo(tmem_base + DV_COL, pl + kk * 2, gl + kk * 128, idesc_a, (it > 0 || kk > 0) ? 1u : 0u, issue);
-#pragma unroll
-                for (int kk = 0; kk < BT / UMMA_K; ++kk)        // dK += dS^T Q
-                    umma_lo(tmem_base + DK_COL, dl_ + kk * 2, ql + kk * 128, idesc_a, (it > 0 || kk > 0) ? 1u : 0u, issue);
-                umma_commit_if(&sm.st_empty[s], issue);
-                umma_commit_if(&sm.acc_done[it & 1], issue);
+                score_product<D>(tmem_base + DP, sm.v, sm.g, issue);
+                umma_commit_if(&sm.dp_full, issue);
+                return true;
+            };
+            if (ok) ok = scores(0) && dprobs(0);
+            for (int it = 0; ok && it < n_it; ++it) {
+                if (!mbar_wait_suspend(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
+                if (it + 1 < n_it && !scores(it + 1)) break;
+                tc_fence_after();
+                grad_product<D>(tmem_base + DV, sm.p, sm.g, it > 0, issue);                  // dV += P^T dO
+                umma_commit_if(&sm.g_empty, issue);
+                umma_commit_if(&sm.dv_done, issue);
+                if (!mbar_wait_suspend(&sm.ds_ready, it & 1, abort_flag, err, 0x5410)) break;
+                tc_fence_after();
+                grad_product<D>(tmem_base + DKC, sm.ds, sm.q[it & 1], it > 0, issue);        // dK += dS^T Q
+                umma_commit_if(&sm.q_empty[it & 1], issue);
+                umma_commit_if(&sm.dk_done, issue);
+                if (it + 1 < n_it) ok = dprobs(it + 1);
             }
         }
     } else if (warp == 2) {                                      // log-sum-exp and delta of the looped queries
         for (int it = 0; it < n_it; ++it) {
-            const int s = it % NST;
-            const int h = hk * rep + it / ni, q0 = (i_lo + it % ni) * BT;
+            const int s = it & 1;
+            const int h = hk * rep + it / ni, q0 = (i_lo + it % ni) * BM;
             const long long row = ((long long)b * a.Hq + h) * a.Tq;
-            float x[2], y[2];
+            float x[4], y[4];
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
+            for (int e = 0; e < 4; ++e) {
                 const int q = q0 + lane + 32 * e;
                 x[e] = q < a.Tq ? __ldg(a.lse + row + q) * LOG2E : INFINITY;
                 y[e] = q < a.Tq ? __ldg(a.delta + row + q) : 0.f;
             }
-            if (!mbar_wait_suspend(&sm.st_empty[s], ((it / NST) & 1) ^ 1, abort_flag, err, 0x5110 | s)) break;
+            if (!mbar_wait_suspend(&sm.q_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, err, 0x5110 | s)) break;
 #pragma unroll
-            for (int e = 0; e < 2; ++e) { sm.lse2[s][lane + 32 * e] = x[e]; sm.delta[s][lane + 32 * e] = y[e]; }
+            for (int e = 0; e < 4; ++e) { sm.lse2[s][lane + 32 * e] = x[e]; sm.delta[s][lane + 32 * e] = y[e]; }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.stat_full[s]);
         }
     } else if (warp >= 4) {
-        const int qd = warp & 3, quarter = (warp - 4) >> 2, grp = quarter >> 1, part = quarter & 1;
+        const int qd = warp & 3, part = (warp - 4) >> 2;
         const int r = qd * 32 + lane;                            // key row inside the tile
         const int key = k0 + r;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
         const float sc = a.scale * LOG2E;
-        uint8_t* prow = sm.p[grp] + (r >> 3) * 1024 + (r & 7) * 128;
-        uint8_t* drow = sm.ds[grp] + (r >> 3) * 1024 + (r & 7) * 128;
         bool alive = n_it > 0;
-        for (int it = grp; alive && it < n_it; it += 2) {
-            const int k = it >> 1, g = it % NST;
-            const int tile_q0 = (i_lo + it % ni) * BT;
-            if (!mbar_wait_suspend(&sm.stat_full[g], (it / NST) & 1, abort_flag, err, 0x5510 | g)) { alive = false; break; }
-            if (!mbar_wait_suspend(&sm.s_full[grp], k & 1, abort_flag, err, 0x5500 | grp)) { alive = false; break; }
-            tc_fence_after();
+        for (int it = 0; alive && it < n_it; ++it) {
+            const int s = it & 1;
+            const int tile_q0 = (i_lo + it % ni) * BM;
             const bool need_mask = (k0 + BM - 1 > a.q_offset + tile_q0) || (k0 + BM > a.Tk) ||
-                                   (a.window > 0 && k0 <= a.q_offset + tile_q0 + BT - 1 - a.window);
-            uint32_t pk[16], dk2[16];
+                                   (a.window > 0 && k0 <= a.q_offset + tile_q0 + BM - 1 - a.window);
+            if (!mbar_wait_suspend(&sm.stat_full[s], (it >> 1) & 1, abort_flag, err, 0x5510 | s)) { alive = false; break; }
+            if (!mbar_wait_suspend(&sm.s_full, it & 1, abort_flag, err, 0x5500)) { alive = false; break; }
+            tc_fence_after();
+            float p[32];
+            uint32_t pk[16];
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {                   // 32 queries per thread, 16 at a time
-                uint32_t sv[16], dv[16];
-                tmem_ld16(lane_addr + grp * 128 + part * 32 + c, sv);
-                tmem_ld16(lane_addr + grp * 128 + 64 + part * 32 + c, dv);
+            for (int c = 0; c < 32; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(lane_addr + ST + part * 32 + c, v);
                 tmem_ld_wait();
                 if (need_mask) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
-                        if (!visible(key, a.q_offset + tile_q0 + part * 32 + c + i, a.Tk, a.window)) sv[i] = 0xff800000u;
+                        if (!visible(key, a.q_offset + tile_q0 + part * 32 + c + i, a.Tk, a.window)) v[i] = 0xff800000u;
                 }
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) {
-                    const float4 l2 = *reinterpret_cast<const float4*>(&sm.lse2[g][part * 32 + c + i]), dl = *reinterpret_cast<const float4*>(&sm.delta[g][part * 32 + c + i]);
-                    const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), sc, -l2.x)), p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), sc, -l2.y));
-                    const float p2 = exp2f(fmaf(__uint_as_float(sv[i + 2]), sc, -l2.z)), p3 = exp2f(fmaf(__uint_as_float(sv[i + 3]), sc, -l2.w));
-                    const int o = (c + i) >> 1;
-                    pk[o] = pack_bf16(p0, p1);
-                    pk[o + 1] = pack_bf16(p2, p3);
-                    dk2[o] = pack_bf16(p0 * (__uint_as_float(dv[i]) - dl.x), p1 * (__uint_as_float(dv[i + 1]) - dl.y));          // scale applied to dK at the end
-                    dk2[o + 1] = pack_bf16(p2 * (__uint_as_float(dv[i + 2]) - dl.z), p3 * (__uint_as_float(dv[i + 3]) - dl.w));
+                    const float4 l2 = *reinterpret_cast<const float4*>(&sm.lse2[s][part * 32 + c + i]);
+                    p[c + i] = exp2f(fmaf(__uint_as_float(v[i]), sc, -l2.x));
+                    p[c + i + 1] = exp2f(fmaf(__uint_as_float(v[i + 1]), sc, -l2.y));
+                    p[c + i + 2] = exp2f(fmaf(__uint_as_float(v[i + 2]), sc, -l2.z));
+                    p[c + i + 3] = exp2f(fmaf(__uint_as_float(v[i + 3]), sc, -l2.w));
+                    pk[(c + i) >> 1] = pack_bf16(p[c + i], p[c + i + 1]);
+                    pk[((c + i) >> 1) + 1] = pack_bf16(p[c + i + 2], p[c + i + 3]);
                 }
             }
-            if (k > 0 && !mbar_wait_suspend(&sm.acc_done[grp], (k - 1) & 1, abort_flag, err, 0x5600 | grp)) { alive = false; break; }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int at = ((part * 4 + c) ^ (r & 7)) << 4;
-                *reinterpret_cast<uint4*>(prow + at) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-                *reinterpret_cast<uint4*>(drow + at) = make_uint4(dk2[4 * c], dk2[4 * c + 1], dk2[4 * c + 2], dk2[4 * c + 3]);
-            }
-            tc_fence_before();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready[grp]);
-        }
-        asm volatile("bar.sync 1, 512;" ::: "memory");           // behind it at most the last gradient GEMMs of each group are outstanding
-        constexpr int OW = D / SPLIT;
-        uint32_t av[OW], ak[OW];
-#pragma unroll
-        for (int i = 0; i < OW; ++i) { av[i] = 0u; ak[i] = 0u; }
-        if (alive && n_it > 0 && mbar_wait_suspend(&sm.acc_done[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, abort_flag, err, 0x5700)) {
+            if (it > 0 && !mbar_wait_suspend(&sm.dv_done, (it - 1) & 1, abort_flag, err, 0x5600)) { alive = false; break; }
+            store_columns(sm.p, r, part, pk);
+            hand_over(&sm.p_ready);
+            if (!mbar_wait_suspend(&sm.dp_full, it & 1, abort_flag, err, 0x5520)) { alive = false; break; }
             tc_fence_after();
-            tmem_ld<OW>(lane_addr + DV_COL + quarter * OW, av);
-            tmem_ld<OW>(lane_addr + DK_COL + quarter * OW, ak);
-            tmem_ld_wait();
-        }
-        if (key < a.Tk) {
-            const long long off = (((long long)b * a.Tk + key) * a.Hkv + hk) * D + quarter * OW;
 #pragma unroll
-            for (int c = 0; c < OW; c += 8) {
-                *reinterpret_cast<uint4*>(a.dv + off + c) = make_uint4(pack_bf16(__uint_as_float(av[c]), __uint_as_float(av[c + 1])),
-                                                                       pack_bf16(__uint_as_float(av[c + 2]), __uint_as_float(av[c + 3])),
-                                                                       pack_bf16(__uint_as_float(av[c + 4]), __uint_as_float(av[c + 5])),
-                                                                       pack_bf16(__uint_as_float(av[c + 6]), __uint_as_float(av[c + 7])));
-                *reinterpret_cast<uint4*>(a.dk + off + c) = make_uint4(pack_bf16(a.scale * __uint_as_float(ak[c]), a.scale * __uint_as_float(ak[c + 1])),
-                                                                       pack_bf16(a.scale * __uint_as_float(ak[c + 2]), a.scale * __uint_as_float(ak[c + 3])),
-                                                                       pack_bf16(a.scale * __uint_as_float(ak[c + 4]), a.scale * __uint_as_float(ak[c + 5])),
-                                                                       pack_bf16(a.scale * __uint_as_float(ak[c + 6]), a.scale * __uint_as_float(ak[c + 7])));
+            for (int c = 0; c < 32; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(lane_addr + DP + part * 32 + c, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {                                              // scale applied to dK at the end
+                    const float4 dl = *reinterpret_cast<const float4*>(&sm.delta[s][part * 32 + c + i]);
+                    pk[(c + i) >> 1] = pack_bf16(p[c + i] * (__uint_as_float(v[i]) - dl.x), p[c + i + 1] * (__uint_as_float(v[i + 1]) - dl.y));
+                    pk[((c + i) >> 1) + 1] = pack_bf16(p[c + i + 2] * (__uint_as_float(v[i + 2]) - dl.z), p[c + i + 3] * (__uint_as_float(v[i + 3]) - dl.w));
+                }
             }
+            if (it > 0 && !mbar_wait_suspend(&sm.dk_done, (it - 1) & 1, abort_flag, err, 0x5610)) { alive = false; break; }
+            store_columns(sm.ds, r, part, pk);
+            hand_over(&sm.ds_ready);
         }
+        if (alive) alive = mbar_wait_suspend(&sm.dv_done, (n_it - 1) & 1, abort_flag, err, 0x5700) &&
+                           mbar_wait_suspend(&sm.dk_done, (n_it - 1) & 1, abort_flag, err, 0x5710);
+        tc_fence_after();
+        constexpr int OW = D / SPLIT;
+        const long long off = (((long long)b * a.Tk + key) * a.Hkv + hk) * D + part * OW;
+        write_row<OW>(a.dv + off, lane_addr + DV + part * OW, 1.f, key < a.Tk, !alive);
+        write_row<OW>(a.dk + off, lane_addr + DKC + part * OW, a.scale, key < a.Tk, !alive);
     }
     tc_fence_before();
     __syncthreads();
@@ -774,16 +794,16 @@ LMOE_API int lmoe_flash_attn_fwd_tc(const void* q, const long long* qs, const vo
 }
 
 template <int D>
-static int launch_bwd_tc(const CUtensorMap& q128, const CUtensorMap& g128, const CUtensorMap& k64, const CUtensorMap& v64,
-                         const CUtensorMap& q64, const CUtensorMap& g64, const CUtensorMap& k128, const CUtensorMap& v128,
-                         const BwdArgs& a, const bf16* o, const bf16* d_o, float* delta, cudaStream_t st) {
+static int launch_bwd_tc(const CUtensorMap& q, const CUtensorMap& g, const CUtensorMap& k, const CUtensorMap& v, const BwdArgs& a, const bf16* o,
+                         const bf16* d_o, float* delta, cudaStream_t st) {
     const long long rows = (long long)a.B * a.Tq * a.Hq;
     fa_delta_tc_kernel<D><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(o, d_o, delta, a.B, a.Tq, a.Hq);
-    const size_t smem = sizeof(SmemBwd<D>) + 1024;
-    cudaFuncSetAttribute(fa_bwd_dq_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(fa_bwd_dkv_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    fa_bwd_dq_tc_kernel<D><<<dim3((a.Tq + BM - 1) / BM, a.Hq, a.B), THREADS, smem, st>>>(q128, g128, k64, v64, a);
-    fa_bwd_dkv_tc_kernel<D><<<dim3((a.Tk + BM - 1) / BM, a.Hkv, a.B), THREADS, smem, st>>>(q64, g64, k128, v128, a);
+    int rc = (int)cudaFuncSetAttribute(fa_bwd_dq_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemDq<D>));
+    if (rc) return rc;
+    rc = (int)cudaFuncSetAttribute(fa_bwd_dkv_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemDkv<D>));
+    if (rc) return rc;
+    fa_bwd_dq_tc_kernel<D><<<dim3((a.Tq + BM - 1) / BM, a.Hq, a.B), THREADS, sizeof(SmemDq<D>), st>>>(q, g, k, v, a);
+    fa_bwd_dkv_tc_kernel<D><<<dim3((a.Tk + BM - 1) / BM, a.Hkv, a.B), THREADS, sizeof(SmemDkv<D>), st>>>(q, g, k, v, a);
     return (int)cudaGetLastError();
 }
 
@@ -794,18 +814,14 @@ LMOE_API int lmoe_flash_attn_bwd_tc(const void* q, const long long* qs, const vo
     BwdArgs a = *ap;
     a.delta = delta;
     const long long gs[3] = {(long long)a.Tq * a.Hq * D, (long long)a.Hq * D, (long long)D};
-    CUtensorMap q128, g128, k64, v64, q64, g64, k128, v128;
+    CUtensorMap mq, mg, mk, mv;
     int rc = 0;
-    rc |= make_map_4d(&q128, q, a.B, a.Tq, a.Hq, D, qs[0], qs[1], qs[2], BM);
-    rc |= make_map_4d(&g128, d_o, a.B, a.Tq, a.Hq, D, gs[0], gs[1], gs[2], BM);
-    rc |= make_map_4d(&k64, k, a.B, a.Tk, a.Hkv, D, ks[0], ks[1], ks[2], BT);
-    rc |= make_map_4d(&v64, v, a.B, a.Tk, a.Hkv, D, vs[0], vs[1], vs[2], BT);
-    rc |= make_map_4d(&q64, q, a.B, a.Tq, a.Hq, D, qs[0], qs[1], qs[2], BT);
-    rc |= make_map_4d(&g64, d_o, a.B, a.Tq, a.Hq, D, gs[0], gs[1], gs[2], BT);
-    rc |= make_map_4d(&k128, k, a.B, a.Tk, a.Hkv, D, ks[0], ks[1], ks[2], BM);
-    rc |= make_map_4d(&v128, v, a.B, a.Tk, a.Hkv, D, vs[0], vs[1], vs[2], BM);
+    rc |= make_map_4d(&mq, q, a.B, a.Tq, a.Hq, D, qs[0], qs[1], qs[2], BM);
+    rc |= make_map_4d(&mg, d_o, a.B, a.Tq, a.Hq, D, gs[0], gs[1], gs[2], BM);
+    rc |= make_map_4d(&mk, k, a.B, a.Tk, a.Hkv, D, ks[0], ks[1], ks[2], BM);
+    rc |= make_map_4d(&mv, v, a.B, a.Tk, a.Hkv, D, vs[0], vs[1], vs[2], BM);
     if (rc) return -11;
-    if (D == 128) return launch_bwd_tc<128>(q128, g128, k64, v64, q64, g64, k128, v128, a, (const bf16*)o, (const bf16*)d_o, delta, st);
-    if (D == 64) return launch_bwd_tc<64>(q128, g128, k64, v64, q64, g64, k128, v128, a, (const bf16*)o, (const bf16*)d_o, delta, st);
+    if (D == 128) return launch_bwd_tc<128>(mq, mg, mk, mv, a, (const bf16*)o, (const bf16*)d_o, delta, st);
+    if (D == 64) return launch_bwd_tc<64>(mq, mg, mk, mv, a, (const bf16*)o, (const bf16*)d_o, delta, st);
     return -1;
 }

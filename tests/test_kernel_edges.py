@@ -1,0 +1,57 @@
+"""Kernels at the edges of their tiles: one row more or less than a tile, the shortest inputs, views that only just qualify.
+
+Tolerances: bf16 rounds to a relative error of at most u = 2^-9.  A result passes through at most four rounded tiles after its inputs
+(an output) or eight (a gradient), each a sum of terms of the size of the result, so the relative Frobenius error is below 4u and 8u;
+twice that leaves room for sums whose terms cancel."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from linear_moe_b200 import ops
+from linear_moe_b200.ops import cuda as K
+from linear_moe_b200.ref import lsm as RL
+from linear_moe_b200.ref import ops as R
+
+U = 2.0 ** -9
+OUT, GRAD = 8 * U, 16 * U
+
+
+def rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-12)).item()
+
+
+def run(f, ins, gout):
+    ins = [t.detach().clone().requires_grad_(True) for t in ins]
+    out = f(*ins)
+    out = out if isinstance(out, tuple) else (out,)
+    torch.autograd.backward(out[: len(gout)], gout)
+    return list(out), [t.grad for t in ins]
+
+
+def rand(*shape, scale=0.5):
+    return (scale * torch.randn(*shape, device="cuda")).bfloat16()
+
+
+def check(got, want, names):
+    for name, a, b, tol in zip(names, got[0] + got[1], want[0] + want[1], [OUT] * len(got[0]) + [GRAD] * len(got[1])):
+        assert rel(a, b) < tol, (name, rel(a, b), tol)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Tq,Tk,window", [(1, 1, None), (127, 127, None), (128, 128, None), (129, 129, None), (255, 383, None), (257, 257, 128),
+                                          (300, 300, 1), (513, 513, 129)])
+def test_attention_tile_edges(D, Tq, Tk, window):
+    from linear_moe_b200.ops import flash, gemm
+    torch.manual_seed(0)
+    q, kv, go = rand(2, Tq, 4, D, scale=1), rand(2, Tk, 2, 2 * D, scale=1), rand(2, Tq, 4, D, scale=1)
+    k, v = kv.split(D, dim=-1)
+    assert flash.supported(q, k, v, True, window)
+    got = run(lambda q, k, v: flash.FlashAttention.apply(q, k, v, D ** -0.5, Tk - Tq, window), [q, k, v], [go])
+    gemm.check_error()
+    want = run(lambda q, k, v: R.softmax_attention(q, k, v, D ** -0.5, True, Tk - Tq, window), [t.float() for t in (q, k, v)], [go.float()])
+    if max(Tk if window is None else window, 1) == 1:           # one key each: dq and dk are exactly zero
+        for a, b in zip(got[1][:2], want[1][:2]):
+            assert a.abs().max() < 16 * U and b.abs().max() < 1e-4
+        got, want = (got[0], got[1][2:]), (want[0], want[1][2:])
+    check(got, want, ["o"] + ["dq", "dk", "dv"][-len(got[1]):])
