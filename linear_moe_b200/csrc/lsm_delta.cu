@@ -20,6 +20,7 @@
 // Reference counterpart: fla.ops.gated_delta_rule / delta_rule chunk kernels called by
 // sequence_modeling/gated_deltanet/gated_deltanet.py:99-116 and deltanet/deltanet.py:127-130.
 #include "mma_utils.cuh"
+#include "tcgen05_utils.cuh"
 
 namespace lmoe {
 namespace dr {
@@ -43,12 +44,17 @@ struct Args {
     float* dS0;                        // backward out: [BH, dk, dv]
     long long os_b, os_t, os_h, gs_b, gs_t, gs_h;
     int N, dv, T, H;
+    int ldw, lda;                      // row strides of W, Qd, Kd and of A in memory: LDK and LDC of Cfg, or dk and C
+    int* err;                          // error word of the bounded waits
 };
 
 // Both walks are chains over the chunks, bound by the latency of a step: two products with a barrier behind each.  Eight warps
 // share a step's tiles, everything that does not depend on the state is taken off the chain (the outputs by four warps beside
 // the other four's pseudo values; Qd^T dO ahead of the barrier), and the next chunk's tiles arrive during the step.
-// 2 x 4096 tokens, 16 heads of 128 (64 chunks, 128 CTAs): forward 169 -> 142 us, without outputs 107, reverse 150 -> 140.
+// The tile kernel writes its tiles with the padded rows they have in shared memory, so that a tile is one bulk copy of one thread: as 16-byte
+// copies of all threads the issue alone took 2000 of a step's 4100 cycles.  Dense tiles (built with torch ops) take that way still.
+// 2 x 4096 tokens, 16 heads of 128 (64 chunks, 128 CTAs): forward 142 -> 128 us, without outputs 107 -> 95, reverse 140 -> 116
+// (with four warps and everything on the chain: 169 and 150).
 template <int DK> struct Cfg {
     static constexpr int LDK = DK + 8;
     static constexpr int LDC = C + 8;
@@ -60,10 +66,30 @@ template <int DK> struct Cfg {
     static constexpr size_t smem(bool out) { return (size_t)(2 * (out ? FULL : QD) + DK * LDV + 2 * C * LDV) * 2; }      // + state, Vn, O
 };
 
+__device__ __forceinline__ void bulk_copy(bf16* dst, const bf16* src, int elements, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(smem_u32(dst)), "l"(src), "r"(elements * 2), "r"(smem_u32(bar)) : "memory");
+}
+template <int DK> __device__ __forceinline__ bool padded(const Args& a) { return a.ldw == Cfg<DK>::LDK && a.lda == Cfg<DK>::LDC; }
+
 template <int DK, bool FULL>
-__device__ __forceinline__ void issue_chunk(bf16* st, const Args& a, const bf16* x, long long xs_t, int x_rows, long long bh, int n) {
+__device__ __forceinline__ void issue_chunk(bf16* st, const Args& a, const bf16* x, long long xs_t, int x_rows, long long bh, int n, uint64_t* bar) {
     using F = Cfg<DK>;
     const long long cn = bh * a.N + n;
+    if (padded<DK>(a)) {
+        if (threadIdx.x == 0) {
+            constexpr int TILE = C * F::LDK, TA = C * F::LDC;
+            tc::mbar_expect_tx(bar, (FULL ? 3 * TILE + TA : 2 * TILE) * 2);
+            bulk_copy(st, a.W + cn * TILE, TILE, bar);
+            bulk_copy(st + TILE, a.Kd + cn * TILE, TILE, bar);
+            if (FULL) {
+                bulk_copy(st + F::QD, a.Qd + cn * TILE, TILE, bar);
+                bulk_copy(st + F::AQ, a.A + cn * TA, TA, bar);
+            }
+        }
+        load_tile_async<C, DVS, F::LDV>(st + 2 * C * F::LDK, x + (long long)n * C * xs_t, xs_t, x_rows - n * C);
+        return;
+    }
     load_tile_async<C, DK, F::LDK>(st, a.W + cn * C * DK, DK, C);
     load_tile_async<C, DK, F::LDK>(st + C * F::LDK, a.Kd + cn * C * DK, DK, C);
     load_tile_async<C, DVS, F::LDV>(st + 2 * C * F::LDK, x + (long long)n * C * xs_t, xs_t, x_rows - n * C);
@@ -71,6 +97,22 @@ __device__ __forceinline__ void issue_chunk(bf16* st, const Args& a, const bf16*
         load_tile_async<C, DK, F::LDK>(st + F::QD, a.Qd + cn * C * DK, DK, C);
         load_tile_async<C, C, F::LDC>(st + F::AQ, a.A + cn * C * C, C, C);
     }
+}
+
+__device__ __forceinline__ void init_stages(uint64_t* full, int* aborted) {
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&full[0], 1);
+        tc::mbar_init(&full[1], 1);
+        *aborted = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+}
+// Barrier of the block behind the arrival of the i-th step's tiles; false for all threads if they did not come.
+template <int DK>
+__device__ __forceinline__ bool stage_ready(const Args& a, uint64_t* full, int* aborted, int i) {
+    const bool ok = !padded<DK>(a) || tc::mbar_wait(&full[i & 1], (i >> 1) & 1, aborted, a.err, 0x6b00 | (i & 1));
+    return __syncthreads_and(ok);
 }
 
 // write a [rows x DVS] bf16 tile held in shared memory (row stride LDV) to global rows of stride `gld`
@@ -125,13 +167,16 @@ __global__ void __launch_bounds__(NT) delta_scan_fwd_kernel(Args a) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int s_m0 = DK == 128 ? 16 * w : 16 * (w & 3), s_n0 = DK == 128 ? 0 : 16 * (w >> 2);
     const int m0 = 16 * (w & 3), v_n0 = OUT ? 0 : 16 * (w >> 2);
+    __shared__ uint64_t full[2];
+    __shared__ int aborted;
     const bool outs = OUT && w >= 4;                 // these warps make O = Qd S + A Vn while the others make Vn = U - W S
     const bf16* u = a.U + (bh * a.N) * C * a.dv + col0;
     bf16* og = OUT ? a.O + (bh / a.H) * a.os_b + (bh % a.H) * a.os_h + col0 : nullptr;
 
     float S[F::SN][4];
     load_state<F::SN>(S, a.S0 == nullptr ? nullptr : a.S0 + bh * DK * a.dv, a.dv, col0, Sb, F::LDV, s_m0, s_n0);
-    if (a.N > 0) issue_chunk<DK, OUT>(stage, a, u, a.dv, a.N * C, bh, 0);
+    init_stages(full, &aborted);
+    if (a.N > 0) issue_chunk<DK, OUT>(stage, a, u, a.dv, a.N * C, bh, 0, &full[0]);
     cp_async_commit();
     for (int n = 0; n < a.N; ++n) {
         const bf16* Wt = stage + (n & 1) * STAGE;
@@ -140,8 +185,8 @@ __global__ void __launch_bounds__(NT) delta_scan_fwd_kernel(Args a) {
         const bf16* Qt = Wt + F::QD;
         const bf16* At = Wt + F::AQ;
         cp_async_wait<0>();
-        __syncthreads();                                           // tiles of chunk n and Sb visible; chunk n - 1 is done with its stage
-        if (n + 1 < a.N) issue_chunk<DK, OUT>(stage + ((n + 1) & 1) * STAGE, a, u, a.dv, a.N * C, bh, n + 1);
+        if (!stage_ready<DK>(a, full, &aborted, n)) break;         // tiles of chunk n and Sb visible; chunk n - 1 is done with its stage
+        if (n + 1 < a.N) issue_chunk<DK, OUT>(stage + ((n + 1) & 1) * STAGE, a, u, a.dv, a.N * C, bh, n + 1, &full[(n + 1) & 1]);
         cp_async_commit();
         const float gamma = a.gamma[bh * a.N + n];
         if (a.Vn != nullptr) store_rows<F::LDV>(Sb, a.Sn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
@@ -200,10 +245,13 @@ __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
     const int s_m0 = DK == 128 ? 16 * w : 16 * (w & 3), s_n0 = DK == 128 ? 0 : 16 * (w >> 2);
     const int m0 = 16 * (w & 3), v_n0 = 16 * (w >> 2);
     const bf16* dO = a.dO + (bh / a.H) * a.gs_b + (bh % a.H) * a.gs_h + col0;
+    __shared__ uint64_t full[2];
+    __shared__ int aborted;
 
     float S[F::SN][4];
     load_state<F::SN>(S, a.dSfinal == nullptr ? nullptr : a.dSfinal + bh * DK * a.dv, a.dv, col0, Sb, F::LDV, s_m0, s_n0);
-    if (a.N > 0) issue_chunk<DK, true>(stage, a, dO, a.gs_t, a.T, bh, a.N - 1);
+    init_stages(full, &aborted);
+    if (a.N > 0) issue_chunk<DK, true>(stage, a, dO, a.gs_t, a.T, bh, a.N - 1, &full[0]);
     cp_async_commit();
     for (int i = 0; i < a.N; ++i) {
         const int n = a.N - 1 - i;
@@ -213,8 +261,8 @@ __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
         const bf16* Qt = Wt + F::QD;
         const bf16* At = Wt + F::AQ;
         cp_async_wait<0>();
-        __syncthreads();
-        if (n > 0) issue_chunk<DK, true>(stage + ((i + 1) & 1) * STAGE, a, dO, a.gs_t, a.T, bh, n - 1);
+        if (!stage_ready<DK>(a, full, &aborted, i)) break;
+        if (n > 0) issue_chunk<DK, true>(stage + ((i + 1) & 1) * STAGE, a, dO, a.gs_t, a.T, bh, n - 1, &full[(i + 1) & 1]);
         cp_async_commit();
         const float gamma = a.gamma[bh * a.N + n];
         store_rows<F::LDV>(Sb, a.dSn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
@@ -261,7 +309,7 @@ struct PrepArgs {
     long long qs_b, qs_t, qs_h, ks_b, ks_t, ks_h, vs_b, vs_t, vs_h;
     const float* beta;                 // [B,T,H]
     const float* g;                    // [B,T,H] log decay, or null
-    bf16 *W, *U, *Qd, *Kd, *A;         // outputs, [BH, N, C, D] / [BH, N, C, C]
+    bf16 *W, *U, *Qd, *Kd, *A;         // outputs: U [BH, N, C, D]; W, Qd, Kd with rows of D + 8, A with rows of C + 8 (as the scans stage them)
     float* gamma;                      // [BH, N]
     int B, T, H, N;
     float scale;
@@ -392,7 +440,7 @@ __global__ void __launch_bounds__(NTP, 3) delta_prep_fwd_kernel(PrepArgs a) {
             warp_gemm<4, D, false, false>(kk, Ks, LD, m0, Ks, LD, nc);
             warp_gemm<4, D, false, false>(qk, Qs, LD, m0, Ks, LD, nc);
         }
-        bf16* Ag = a.A + cn * C * C;
+        bf16* Ag = a.A + cn * C * LDC;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -405,7 +453,7 @@ __global__ void __launch_bounds__(NTP, 3) delta_prep_fwd_kernel(PrepArgs a) {
                                                                           i > j + 1 ? be * d1 * kk[nt][2 * hh + 1] : 0.f);
                 const float a0 = i >= j ? a.scale * d0 * qk[nt][2 * hh] : 0.f;
                 const float a1 = i >= j + 1 ? a.scale * d1 * qk[nt][2 * hh + 1] : 0.f;
-                *reinterpret_cast<__nv_bfloat162*>(Ag + i * C + j) = __floats2bfloat162_rn(a0, a1);
+                *reinterpret_cast<__nv_bfloat162*>(Ag + i * LDC + j) = __floats2bfloat162_rn(a0, a1);
             }
     }
     cp_async_wait<0>();
@@ -428,8 +476,8 @@ __global__ void __launch_bounds__(NTP, 3) delta_prep_fwd_kernel(PrepArgs a) {
         }
         o1.store(Qs + i * LD + c);
         o2.store(Vs + i * LD + c);
-        o3.store(a.Qd + (cn * C + i) * D + c);
-        o4.store(a.Kd + (cn * C + i) * D + c);
+        o3.store(a.Qd + (cn * C + i) * LD + c);
+        o4.store(a.Kd + (cn * C + i) * LD + c);
     }
     if (threadIdx.x == 0) a.gamma[cn] = __expf(btot);
     unit_lower_inverse(F);
@@ -457,15 +505,16 @@ __global__ void __launch_bounds__(NTP, 3) delta_prep_fwd_kernel(PrepArgs a) {
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
         const bf16* X = which == 0 ? Qs : Vs;
-        bf16* Y = (which == 0 ? a.W : a.U) + cn * C * D + half * (D / 2);
+        const int ld = which == 0 ? LD : D;
+        bf16* Y = (which == 0 ? a.W : a.U) + cn * C * ld + half * (D / 2);
         float acc[NH][4];
         zero_acc<NH>(acc);
         for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<NH, 16, false, true>(acc, Tb + k0, LDC, m0, X + k0 * LD, LD, half * (D / 2));
         const int r = m0 + (l >> 2), cc = (l & 3) * 2;
 #pragma unroll
         for (int nt = 0; nt < NH; ++nt) {
-            *reinterpret_cast<__nv_bfloat162*>(Y + r * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
-            *reinterpret_cast<__nv_bfloat162*>(Y + (r + 8) * D + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
+            *reinterpret_cast<__nv_bfloat162*>(Y + r * ld + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
+            *reinterpret_cast<__nv_bfloat162*>(Y + (r + 8) * ld + cc + nt * 8) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
         }
     }
 }
@@ -821,7 +870,8 @@ using namespace lmoe;
 // dir 0: forward, dir 1: backward.  dk in {64, 128}; dv a multiple of 32.  Grid = (dv / 32, B*H).
 LMOE_API int lmoe_delta_scan(int dir, int dk, int BH, const dr::Args* ap, cudaStream_t st) {
     const dr::Args a = *ap;
-    if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0 || a.H <= 0) return -1;
+    if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0 || a.H <= 0 || a.err == nullptr) return -1;
+    if (!(a.ldw == dk && a.lda == dr::C) && !(a.ldw == dk + 8 && a.lda == dr::C + 8)) return -1;
     dim3 grid(a.dv / dr::DVS, BH);
     const bool out = dir != 0 || a.O != nullptr;
 #define LMOE_DR_LAUNCH(KERNEL, DK)                                                                                     \

@@ -1364,7 +1364,7 @@ class _DeltaArgs(ctypes.Structure):
     _fields_ = ([(n, ctypes.c_void_p) for n in ("W", "U", "Qd", "Kd", "A", "gamma", "S0", "dO", "dSfinal", "O", "Vn", "Sn",
                                                  "Sfinal", "dVn", "dSn", "dS0")] +
                 [(n, ctypes.c_longlong) for n in ("os_b", "os_t", "os_h", "gs_b", "gs_t", "gs_h")] +
-                [(n, ctypes.c_int) for n in ("N", "dv", "T", "H")])
+                [(n, ctypes.c_int) for n in ("N", "dv", "T", "H", "ldw", "lda")] + [("err", ctypes.c_void_p)])
 
 
 def _delta_prepare(q, k, v, beta, g, scale, C=64):
@@ -1423,8 +1423,12 @@ def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64, inverse=None):
     N = (T + C - 1) // C
     q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
     bf, dev = torch.bfloat16, q.device
-    W, U, Qd, Kd = (torch.empty(B, H, N, C, D, dtype=bf, device=dev) for _ in range(4))
-    A = torch.empty(B, H, N, C, C, dtype=bf, device=dev)
+    # rows of W, Qd, Kd and A as the scan kernels keep them in shared memory: eight more elements than the tile has columns
+    def padded(n):
+        r = C * (n + 8)
+        return torch.empty_strided((B, H, N, C, n), (H * N * r, N * r, r, n + 8, 1), dtype=bf, device=dev)
+    W, Qd, Kd, A = padded(D), padded(D), padded(D), padded(C)
+    U = torch.empty(B, H, N, C, D, dtype=bf, device=dev)
     gamma = torch.empty(B, H, N, dtype=torch.float32, device=dev)
     bt = beta.float().contiguous()
     gt = None if g is None else g.float().contiguous()
@@ -1452,6 +1456,7 @@ def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, out=None, keep=True):
     ``out``: a bf16 ``[B,T,H,dv]`` buffer (unit stride along ``dv``) for ``O``, or ``None`` where nobody needs it.  Returns ``Vn``
     ``[B,H,N,C,dv]`` bf16 and the state entering every chunk ``Sn`` ``[B,H,N,dk,dv]`` bf16 (both ``None`` without ``keep``)
     and the final state in fp32."""
+    from . import gemm
     B, H, N, C, dk = W.shape
     dv = U.shape[-1]
     dev = W.device
@@ -1469,7 +1474,8 @@ def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, out=None, keep=True):
     if out is not None:
         a.O, a.T = out.data_ptr(), out.shape[1]
         a.os_b, a.os_t, a.os_h = out.stride(0), out.stride(1), out.stride(2)
-    a.N, a.dv, a.H = N, dv, H
+    a.N, a.dv, a.H, a.ldw, a.lda = N, dv, H, W.stride(3), A.stride(3)
+    a.err = gemm._err(dev).data_ptr()
     _check(lib().lmoe_delta_scan(_i32(0), _i32(dk), _i32(B * H), ctypes.byref(a), _st()), "delta_scan_fwd")
     return Vn, Sn, Sf
 
@@ -1478,6 +1484,7 @@ def _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf):
     """``delta_scan_bwd_kernel``: the reverse recurrence ``dVn = A^T dO + Kd dS'``, ``dS = gamma dS' + Qd^T dO - W^T dVn`` for ``dO``
     ``[B,T,H,dv]`` (:func:`_inner_contig`).  Returns ``dVn`` ``[B,H,N,C,dv]``, the gradient of the state leaving every chunk
     ``dSn`` ``[B,H,N,dk,dv]`` (bf16) and the gradient of the initial state (fp32)."""
+    from . import gemm
     B, H, N, C, dk = W.shape
     dv = dO.shape[-1]
     dev = W.device
@@ -1492,7 +1499,8 @@ def _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf):
     a.dO, a.dSfinal = dO.data_ptr(), 0 if dsf is None else dsf.data_ptr()
     a.gs_b, a.gs_t, a.gs_h = dO.stride(0), dO.stride(1), dO.stride(2)
     a.dVn, a.dSn, a.dS0 = dVn.data_ptr(), dSn.data_ptr(), dS0.data_ptr()
-    a.N, a.dv, a.T, a.H = N, dv, dO.shape[1], H
+    a.N, a.dv, a.T, a.H, a.ldw, a.lda = N, dv, dO.shape[1], H, W.stride(3), A.stride(3)
+    a.err = gemm._err(dev).data_ptr()
     _check(lib().lmoe_delta_scan(_i32(1), _i32(dk), _i32(B * H), ctypes.byref(a), _st()), "delta_scan_bwd")
     return dVn, dSn, dS0
 

@@ -55,3 +55,39 @@ def test_attention_tile_edges(D, Tq, Tk, window):
             assert a.abs().max() < 16 * U and b.abs().max() < 1e-4
         got, want = (got[0], got[1][2:]), (want[0], want[1][2:])
     check(got, want, ["o"] + ["dq", "dk", "dv"][-len(got[1]):])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [1, 15, 63, 64, 65, 200])
+def test_delta_rule_chunk_edges(D, T):
+    torch.manual_seed(0)
+    B, H = 2, 3
+    q, k, v = rand(B, T, H, 3 * D).split(D, dim=-1)
+    k = torch.nn.functional.normalize(k.float(), dim=-1).bfloat16()
+    beta, g = torch.rand(B, T, H, device="cuda"), torch.nn.functional.logsigmoid(torch.randn(B, T, H, device="cuda") + 2)
+    S0 = 0.2 * torch.randn(B, H, D, D, device="cuda")
+    go, gS = rand(B, T, H, D, scale=1), 0.05 * torch.randn(B, H, D, D, device="cuda")
+    ins = [q, k, v, beta, g, S0]
+    got = run(lambda q, k, v, beta, g, S: ops.lsm_delta(q, k, v, beta, g, None, S, 64), ins, [go, gS])
+    want = run(lambda q, k, v, beta, g, S: RL.recurrent_lsm(q, k, v, beta=beta, g=g, initial_state=S), [t.float() for t in ins], [go.float(), gS])
+    check(got, want, ["o", "S", "dq", "dk", "dv", "dbeta", "dg", "dS0"])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [1, 64, 130, 320])
+def test_delta_scans_of_padded_and_dense_tiles(D, T):
+    """The tile kernel's padded rows (one bulk copy per tile) and dense tiles (copies by all threads) give the same bits."""
+    torch.manual_seed(0)
+    B, H = 1, 3
+    q, v = rand(B, T, H, D), rand(B, T, H, D)
+    k = torch.nn.functional.normalize(torch.randn(B, T, H, D, device="cuda"), dim=-1).bfloat16()
+    tiles = K._delta_prepare_kernel(q, k, v, torch.rand(B, T, H, device="cuda"), None, D ** -0.5)
+    assert tiles[0].stride(3) == D + 8
+    dense = [t.contiguous() for t in tiles]
+    go, outs = rand(B, T, H, D, scale=1), []
+    for W, U_, Qd, Kd, A, gamma in (tiles, dense):
+        o = torch.empty(B, T, H, D, dtype=torch.bfloat16, device="cuda")
+        outs.append([o, *K._delta_scan_fwd(W, U_, Qd, Kd, A, gamma, None, o), *K._delta_scan_fwd(W, U_, Qd, Kd, A, gamma, None),
+                     *K._delta_scan_bwd(W, Qd, Kd, A, gamma, go, None)])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
