@@ -15,13 +15,19 @@
 //   dk = e^{b_m - b_j} . [ (scale dO V^T . mask)^T q~ + V (diag(e^{b_C - b_m}) dS)^T ]
 //   dv = (scale q~ k~^T . mask)^T dO + k~ (diag(e^{b_C - b_m}) dS)
 //   dS <- diag(e^{b_m}) [ diag(e^{b_C - b_m}) dS + scale q~^T dO ]
-// The gate gradient is d g = reverse-cumsum_t (q . dq - k . dk) per channel, taken by the caller.
+// The gate gradient is d g = reverse-cumsum_t (q . dq - k . dk) per channel (the kernels at the end of this file).
+//
+// 512 threads, one CTA per SM: a warp owns 16 rows of every product and a quarter of its columns (of the state: half or a quarter).  For the
+// gates a thread owns two channels and VCH / GR consecutive tokens: running sums stay in registers, the GR groups of tokens meet in one
+// small table, and the next chunk's gates and tiles are on their way while this one is worked on.  (With eight warps, single buffers and a
+// 64-step running sum in 128 threads the chunks were bound by latency.)  8 x 2048 tokens, 8 heads of 128: outputs 135 -> 97 us, dq
+// 138 -> 102, dk / dv 187 -> 141, group summaries 82 and 71 -> 43 and 41.
 #include "mma_utils.cuh"
 
 namespace lmoe {
 
 constexpr int VCH = 64;
-constexpr int VTHREADS = 256;
+constexpr int VTHREADS = 512;
 
 struct GlaArgs {
     const bf16 *q, *k, *v, *d_o;
@@ -36,45 +42,76 @@ struct GlaArgs {
 };
 
 template <int D> struct VCfg {
-    static constexpr int LD = D + 8;
-    static constexpr int PLD = VCH + 8;
-    static constexpr int S_RB = D / 16;
-    static constexpr int S_NT = D * D / 1024;
-    static constexpr int O_NT = D / 16;
+    static constexpr int LD = D + 8, PLD = VCH + 8, TILE = VCH * LD;
+    static constexpr int S_RB = D / 16, S_CB = 16 / S_RB, S_NT = D / (8 * S_CB);      // the state: row blocks, column blocks, n-tiles per warp
+    static constexpr int O_NT = D / 32;                                               // n-tiles of a [VCH x D] product per warp
+    static constexpr int PAIRS = D / 2, GR = VTHREADS / PAIRS, RPG = VCH / GR;        // gates: channel pairs, groups of tokens, tokens per group
 };
 
-// Load the chunk's gates, turn them into inclusive cumulative sums b[i][d] in shared memory (fp32, [VCH][D]).
+// A thread's place for the gates: channels 2 * pair and 2 * pair + 1 of tokens grp * RPG ..
+template <int D> struct Place {
+    int pair, grp, row0;
+    __device__ __forceinline__ Place() : pair(threadIdx.x % VCfg<D>::PAIRS), grp(threadIdx.x / VCfg<D>::PAIRS) { row0 = grp * VCfg<D>::RPG; }
+};
 template <int D>
-__device__ __forceinline__ void load_cumsum(const GlaArgs& a, int b, int h, int c, float* bt) {
-    const float* g = a.gk + (((int64_t)b * a.T + (int64_t)c * VCH) * a.H + h) * D;
-    const int valid = a.T - c * VCH;
-    for (int i = threadIdx.x; i < VCH * (D / 4); i += blockDim.x) {
-        int r = i / (D / 4), cc = (i % (D / 4)) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < valid) v = *reinterpret_cast<const float4*>(g + (int64_t)r * a.H * D + cc);
-        *reinterpret_cast<float4*>(bt + r * D + cc) = v;
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        float s = 0.f;
-#pragma unroll 8
-        for (int r = 0; r < VCH; ++r) { s += bt[r * D + d]; bt[r * D + d] = s; }
-    }
-    __syncthreads();
+__device__ __forceinline__ void load_gates(const GlaArgs& a, int b, int h, int c, const Place<D>& at, float2 (&g)[VCfg<D>::RPG]) {
+    const float* p = a.gk + (((int64_t)b * a.T + (int64_t)c * VCH + at.row0) * a.H + h) * D + 2 * at.pair;
+    const int valid = a.T - c * VCH - at.row0;
+#pragma unroll
+    for (int i = 0; i < VCfg<D>::RPG; ++i)
+        g[i] = i < valid ? __ldg(reinterpret_cast<const float2*>(p + (int64_t)i * a.H * D)) : make_float2(0.f, 0.f);
 }
-
-// tile[r][d] *= exp(sign * (bt[r][d] - ref[d])) * mul, ref[d] = bt[ref_row][d] (ref_row < 0: ref = 0)
-template <int D, int LD>
-__device__ __forceinline__ void rescale_tile(bf16* tile, const float* bt, int ref_row, float sign, float mul) {
-    for (int i = threadIdx.x; i < VCH * (D / 2); i += blockDim.x) {
-        int r = i / (D / 2), d = (i % (D / 2)) * 2;
-        float r0 = ref_row >= 0 ? bt[ref_row * D + d] : 0.f, r1 = ref_row >= 0 ? bt[ref_row * D + d + 1] : 0.f;
-        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(tile + r * LD + d);
-        float2 x = __bfloat1622float2(*p);
-        x.x *= __expf(sign * (bt[r * D + d] - r0)) * mul;
-        x.y *= __expf(sign * (bt[r * D + d + 1] - r1)) * mul;
-        *p = __floats2bfloat162_rn(x.x, x.y);
+template <int D>
+__device__ __forceinline__ void save_group_sum(float* sums, const Place<D>& at, const float2 (&g)[VCfg<D>::RPG]) {
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VCfg<D>::RPG; ++i) { s.x += g[i].x; s.y += g[i].y; }
+    *reinterpret_cast<float2*>(sums + at.grp * D + 2 * at.pair) = s;
+}
+// of groups lo .. hi - 1, this thread's channels
+template <int D>
+__device__ __forceinline__ float2 groups_sum(const float* sums, const Place<D>& at, int lo, int hi) {
+    float2 s = make_float2(0.f, 0.f);
+    for (int j = lo; j < hi; ++j) {
+        const float2 x = *reinterpret_cast<const float2*>(sums + j * D + 2 * at.pair);
+        s.x += x.x; s.y += x.y;
     }
+    return s;
+}
+// g[i] <- b_i - b_m (m: the chunk's middle token), from the gates of the chunk
+template <int D>
+__device__ __forceinline__ void about_middle(float2 (&g)[VCfg<D>::RPG], const float* sums, const Place<D>& at) {
+    constexpr int GR = VCfg<D>::GR, RPG = VCfg<D>::RPG;
+    if (at.grp < GR / 2) {
+        float2 s = groups_sum<D>(sums, at, at.grp + 1, GR / 2);
+#pragma unroll
+        for (int i = RPG - 1; i >= 0; --i) {
+            const float2 x = g[i];
+            g[i] = make_float2(-s.x, -s.y);
+            s.x += x.x; s.y += x.y;
+        }
+    } else {
+        float2 s = groups_sum<D>(sums, at, GR / 2, at.grp);
+#pragma unroll
+        for (int i = 0; i < RPG; ++i) { s.x += g[i].x; s.y += g[i].y; g[i] = s; }
+    }
+}
+// tab[0][d] = e^{b_m}, tab[1][d] = e^{b_C - b_m}
+template <int D>
+__device__ __forceinline__ void half_decays(float* tab, const float* sums) {
+    constexpr int GR = VCfg<D>::GR;
+    if (threadIdx.x < 2 * D) {
+        const int d = threadIdx.x % D, half = threadIdx.x / D;
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < GR / 2; ++j) s += sums[(half * (GR / 2) + j) * D + d];
+        tab[half * D + d] = __expf(s);
+    }
+}
+__device__ __forceinline__ void mul2(bf16* p, float fx, float fy) {
+    __nv_bfloat162* x = reinterpret_cast<__nv_bfloat162*>(p);
+    const float2 v = __bfloat1622float2(*x);
+    *x = __floats2bfloat162_rn(v.x * fx, v.y * fy);
 }
 
 template <int NT>
@@ -82,13 +119,12 @@ __device__ __forceinline__ void rowscale_acc(float (&acc)[NT][4], float f0, floa
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) { acc[nt][0] *= f0; acc[nt][1] *= f0; acc[nt][2] *= f1; acc[nt][3] *= f1; }
 }
-
 // mask only (no decay): keep (row >= col) if LOWER else (row <= col); multiply by scale; store bf16
 template <int LOWER>
-__device__ __forceinline__ void mask_store_plain(const float (&acc)[4][4], bf16* P, int pld, int m0, int n0, float scale) {
+__device__ __forceinline__ void mask_store_plain(const float (&acc)[2][4], bf16* P, int pld, int m0, int n0, float scale) {
     const int l = threadIdx.x & 31;
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             int r = m0 + (l >> 2) + 8 * hh, c = n0 + nt * 8 + (l & 3) * 2;
@@ -97,14 +133,39 @@ __device__ __forceinline__ void mask_store_plain(const float (&acc)[4][4], bf16*
                 __floats2bfloat162_rn(k0 ? acc[nt][2 * hh] * scale : 0.f, k1 ? acc[nt][2 * hh + 1] * scale : 0.f);
         }
 }
-
+// this warp's [16 x D / 4] block of a tile to global rows
 template <int D, int LD>
-__device__ __forceinline__ void vstore_tile(const bf16* smem, bf16* gmem, int64_t row_stride, int valid_rows) {
-    constexpr int VPR = D / 8;
-    for (int i = threadIdx.x; i < VCH * VPR; i += blockDim.x) {
-        int r = i / VPR, c = (i % VPR) * 8;
-        if (r < valid_rows)
-            *reinterpret_cast<uint4*>(gmem + (int64_t)r * row_stride + c) = *reinterpret_cast<const uint4*>(smem + r * LD + c);
+__device__ __forceinline__ void store_block(const bf16* tile, int m0, int n0, bf16* g, int64_t row_stride, int valid) {
+    constexpr int VPR = D / 32;
+    const int l = threadIdx.x & 31;
+#pragma unroll
+    for (int i = l; i < 16 * VPR; i += 32) {
+        const int r = m0 + i / VPR, c = n0 + (i % VPR) * 8;
+        if (r < valid) *reinterpret_cast<uint4*>(g + (int64_t)r * row_stride + c) = *reinterpret_cast<const uint4*>(tile + r * LD + c);
+    }
+}
+// Write diag(f) * S (registers, rows r and r + 8) as bf16 into Sb.
+template <int D>
+__device__ __forceinline__ void store_state_scaled(const float (&acc)[VCfg<D>::S_NT][4], bf16* Sb, int s_m0, int s_n0, float f0, float f1) {
+    using C = VCfg<D>;
+    const int l = threadIdx.x & 31;
+    const int r = s_m0 + (l >> 2), c = s_n0 + (l & 3) * 2;
+#pragma unroll
+    for (int nt = 0; nt < C::S_NT; ++nt) {
+        *reinterpret_cast<__nv_bfloat162*>(Sb + r * C::LD + c + nt * 8) = __floats2bfloat162_rn(acc[nt][0] * f0, acc[nt][1] * f0);
+        *reinterpret_cast<__nv_bfloat162*>(Sb + (r + 8) * C::LD + c + nt * 8) = __floats2bfloat162_rn(acc[nt][2] * f1, acc[nt][3] * f1);
+    }
+}
+template <int D>
+__device__ __forceinline__ void load_state_regs(const float* src, float (&acc)[VCfg<D>::S_NT][4], int s_m0, int s_n0) {
+    using C = VCfg<D>;
+    const int l = threadIdx.x & 31;
+    const int r = s_m0 + (l >> 2), cc = s_n0 + (l & 3) * 2;
+#pragma unroll
+    for (int nt = 0; nt < C::S_NT; ++nt) {
+        float2 x = *reinterpret_cast<const float2*>(src + (int64_t)r * D + cc + nt * 8);
+        float2 y = *reinterpret_cast<const float2*>(src + (int64_t)(r + 8) * D + cc + nt * 8);
+        acc[nt][0] = x.x; acc[nt][1] = x.y; acc[nt][2] = y.x; acc[nt][3] = y.y;
     }
 }
 
@@ -113,44 +174,69 @@ __device__ __forceinline__ void vstore_tile(const bf16* smem, bf16* gmem, int64_
 //                      REV = 1: dS <- diag(e^{b_C}) dS + (Q e^{b} scale)^T dO (descending chunks)
 // ---------------------------------------------------------------------------------------------
 template <int D, int REV>
-__global__ void __launch_bounds__(VTHREADS) gla_state_scan_kernel(GlaArgs a) {
+__global__ void __launch_bounds__(VTHREADS, 1) gla_state_scan_kernel(GlaArgs a) {
     using C = VCfg<D>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* Xs = reinterpret_cast<bf16*>(smem_raw);
-    bf16* Ys = Xs + VCH * C::LD;
-    float* bt = reinterpret_cast<float*>(Ys + VCH * C::LD);        // [VCH][D]
+    bf16* Xs = reinterpret_cast<bf16*>(smem_raw);                  // [2][VCH][LD]
+    bf16* Ys = Xs + 2 * C::TILE;                                   // [2][VCH][LD]
+    float* sums = reinterpret_cast<float*>(Ys + 2 * C::TILE);      // [2][GR][D]
     const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int nchunks = (a.T + VCH - 1) / VCH;
-    const int c_lo = grp * a.cpg, c_hi = min(nchunks, c_lo + a.cpg);
+    const int c_lo = grp * a.cpg, c_hi = min(nchunks, c_lo + a.cpg), n = c_hi - c_lo;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int s_m0 = 16 * (w % C::S_RB), s_n0 = (w / C::S_RB) * (C::S_NT * 8);
+    const int r = s_m0 + (l >> 2);
+    const Place<D> at;
     const bf16* xg = REV ? a.q + b * a.qs_b + h * a.qs_h : a.k + b * a.ks_b + h * a.ks_h;
     const int64_t xs_t = REV ? a.qs_t : a.ks_t;
     const bf16* yg = REV ? a.d_o + ((int64_t)b * a.T * a.H + h) * D : a.v + b * a.vs_b + h * a.vs_h;
     const int64_t ys_t = REV ? (int64_t)a.H * D : a.vs_t;
+    auto chunk_at = [&](int i) { return REV ? c_hi - 1 - i : c_lo + i; };
+    auto issue = [&](int i) {
+        const int c = chunk_at(i);
+        load_tile_async<VCH, D, C::LD>(Xs + (i & 1) * C::TILE, xg + (int64_t)c * VCH * xs_t, xs_t, a.T - c * VCH);
+        load_tile_async<VCH, D, C::LD>(Ys + (i & 1) * C::TILE, yg + (int64_t)c * VCH * ys_t, ys_t, a.T - c * VCH);
+    };
     float acc[C::S_NT][4];
     zero_acc<C::S_NT>(acc);
-    float gs0 = 0.f, gs1 = 0.f;                                    // running group decay of rows r, r+8 (threads with l&3 == 0, s_n0 == 0)
-    for (int i = 0; i < c_hi - c_lo; ++i) {
-        const int c = REV ? c_hi - 1 - i : c_lo + i;
-        load_tile_async<VCH, D, C::LD>(Xs, xg + (int64_t)c * VCH * xs_t, xs_t, a.T - c * VCH);
-        load_tile_async<VCH, D, C::LD>(Ys, yg + (int64_t)c * VCH * ys_t, ys_t, a.T - c * VCH);
-        cp_async_commit();
-        load_cumsum<D>(a, b, h, c, bt);
+    float gs0 = 0.f, gs1 = 0.f;                                    // running group decay of rows r, r + 8
+    float2 g[C::RPG];
+    if (n > 0) { issue(0); load_gates<D>(a, b, h, chunk_at(0), at, g); save_group_sum<D>(sums, at, g); }
+    cp_async_commit();
+    for (int i = 0; i < n; ++i) {
+        bf16 *X = Xs + (i & 1) * C::TILE, *Y = Ys + (i & 1) * C::TILE;
+        float* sm = sums + (i & 1) * C::GR * D;
         cp_async_wait<0>();
-        __syncthreads();
-        if (REV) rescale_tile<D, C::LD>(Xs, bt, -1, 1.f, a.scale);             // q e^{b} scale
-        else rescale_tile<D, C::LD>(Xs, bt, VCH - 1, -1.f, 1.f);               // k e^{b_C - b}
-        __syncthreads();
-        const int r = s_m0 + (l >> 2);
-        const float t0 = bt[(VCH - 1) * D + r], t1 = bt[(VCH - 1) * D + r + 8];
+        __syncthreads();                                           // tiles and group sums of this chunk visible; the other stage is free
+        if (i + 1 < n) issue(i + 1);
+        cp_async_commit();
+        if (REV) {                                                 // q e^{b} scale
+            float2 s = groups_sum<D>(sm, at, 0, at.grp);
+#pragma unroll
+            for (int e = 0; e < C::RPG; ++e) {
+                s.x += g[e].x; s.y += g[e].y;
+                mul2(X + (at.row0 + e) * C::LD + 2 * at.pair, __expf(s.x) * a.scale, __expf(s.y) * a.scale);
+            }
+        } else {                                                   // k e^{b_C - b}
+            float2 s = groups_sum<D>(sm, at, at.grp + 1, C::GR);
+#pragma unroll
+            for (int e = C::RPG - 1; e >= 0; --e) {
+                mul2(X + (at.row0 + e) * C::LD + 2 * at.pair, __expf(s.x), __expf(s.y));
+                s.x += g[e].x; s.y += g[e].y;
+            }
+        }
+        if (i + 1 < n) load_gates<D>(a, b, h, chunk_at(i + 1), at, g);
+        float t0 = 0.f, t1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < C::GR; ++j) { t0 += sm[j * D + r]; t1 += sm[j * D + r + 8]; }
         rowscale_acc<C::S_NT>(acc, __expf(t0), __expf(t1));
         gs0 += t0; gs1 += t1;
-        warp_gemm<C::S_NT, VCH, true, true>(acc, Xs, C::LD, s_m0, Ys, C::LD, s_n0);
         __syncthreads();
+        warp_gemm<C::S_NT, VCH, true, true>(acc, X, C::LD, s_m0, Y, C::LD, s_n0);
+        if (i + 1 < n) save_group_sum<D>(sums + ((i + 1) & 1) * C::GR * D, at, g);
     }
     float* out = a.states + ((int64_t)bh * a.G + grp) * D * D;
-    const int r = s_m0 + (l >> 2), cc = s_n0 + (l & 3) * 2;
+    const int cc = s_n0 + (l & 3) * 2;
 #pragma unroll
     for (int nt = 0; nt < C::S_NT; ++nt) {
         *reinterpret_cast<float2*>(out + (int64_t)r * D + cc + nt * 8) = make_float2(acc[nt][0], acc[nt][1]);
@@ -195,53 +281,25 @@ __global__ void gla_combine_kernel(float* __restrict__ states, const float* __re
     if (final_out != nullptr) final_out[(int64_t)bh * DD + e] = carry;
 }
 
-// Write diag(e^{f[row]}) * S (registers) as bf16 into Sb.
-template <int D>
-__device__ __forceinline__ void store_state_scaled(const float (&acc)[VCfg<D>::S_NT][4], bf16* Sb, int s_m0, int s_n0, float f0, float f1) {
-    using C = VCfg<D>;
-    const int l = threadIdx.x & 31;
-    const int r = s_m0 + (l >> 2), c = s_n0 + (l & 3) * 2;
-#pragma unroll
-    for (int nt = 0; nt < C::S_NT; ++nt) {
-        *reinterpret_cast<__nv_bfloat162*>(Sb + r * C::LD + c + nt * 8) = __floats2bfloat162_rn(acc[nt][0] * f0, acc[nt][1] * f0);
-        *reinterpret_cast<__nv_bfloat162*>(Sb + (r + 8) * C::LD + c + nt * 8) = __floats2bfloat162_rn(acc[nt][2] * f1, acc[nt][3] * f1);
-    }
-}
-
-template <int D>
-__device__ __forceinline__ void load_state_regs(const float* src, float (&acc)[VCfg<D>::S_NT][4], int s_m0, int s_n0) {
-    using C = VCfg<D>;
-    const int l = threadIdx.x & 31;
-    const int r = s_m0 + (l >> 2), cc = s_n0 + (l & 3) * 2;
-#pragma unroll
-    for (int nt = 0; nt < C::S_NT; ++nt) {
-        float2 x = *reinterpret_cast<const float2*>(src + (int64_t)r * D + cc + nt * 8);
-        float2 y = *reinterpret_cast<const float2*>(src + (int64_t)(r + 8) * D + cc + nt * 8);
-        acc[nt][0] = x.x; acc[nt][1] = x.y; acc[nt][2] = y.x; acc[nt][3] = y.y;
-    }
-}
-
 // ---------------------------------------------------------------------------------------------
 // 3a. forward output (MODE 0) / backward dq (MODE 1): forward sweep carrying S.
 // ---------------------------------------------------------------------------------------------
 template <int D, int MODE>
-__global__ void __launch_bounds__(VTHREADS) gla_fwd_sweep_kernel(GlaArgs a) {
+__global__ void __launch_bounds__(VTHREADS, 1) gla_fwd_sweep_kernel(GlaArgs a) {
     using C = VCfg<D>;
-    constexpr int MID = VCH / 2 - 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* Tq = reinterpret_cast<bf16*>(smem_raw);                  // q (mode 0) | dO (mode 1)
-    bf16* Tk = Tq + VCH * C::LD;
-    bf16* Tv = Tk + VCH * C::LD;
-    bf16* Sb = Tv + VCH * C::LD;
+    bf16* tiles = reinterpret_cast<bf16*>(smem_raw);               // [2] x { q (mode 0) | dO (mode 1), k, v }
+    bf16* Sb = tiles + 6 * C::TILE;
     bf16* P = Sb + D * C::LD;
-    float* bt = reinterpret_cast<float*>(P + VCH * C::PLD);
+    float* sums = reinterpret_cast<float*>(P + VCH * C::PLD);      // [2][GR][D]
+    float* tabs = sums + 2 * C::GR * D;                            // [2][2][D]
     const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int nchunks = (a.T + VCH - 1) / VCH;
     const int c_lo = grp * a.cpg, c_hi = min(nchunks, c_lo + a.cpg);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int s_m0 = 16 * (w % C::S_RB), s_n0 = (w / C::S_RB) * (C::S_NT * 8);
-    const int o_m0 = 16 * (w & 3), o_n0 = (w >> 2) * (D / 2);
-    const int a_m0 = 16 * (w & 3), a_n0 = (w >> 2) * 32;
+    const int s_m0 = 16 * (w % C::S_RB), s_n0 = (w / C::S_RB) * (C::S_NT * 8), sr = s_m0 + (l >> 2);
+    const int m0 = 16 * (w & 3), o_n0 = (w >> 2) * (D / 4), a_n0 = (w >> 2) * 16;
+    const Place<D> at;
     const bf16* qg = MODE == 0 ? a.q + b * a.qs_b + h * a.qs_h : a.d_o + ((int64_t)b * a.T * a.H + h) * D;
     const int64_t qst = MODE == 0 ? a.qs_t : (int64_t)a.H * D;
     const bf16* kg = a.k + b * a.ks_b + h * a.ks_h;
@@ -249,55 +307,79 @@ __global__ void __launch_bounds__(VTHREADS) gla_fwd_sweep_kernel(GlaArgs a) {
     bf16* og; int64_t ost;
     if (MODE == 0) { og = a.o + ((int64_t)b * a.T * a.H + h) * D; ost = (int64_t)a.H * D; }
     else { og = a.dq + b * a.dqs_b + h * a.dqs_h; ost = a.dqs_t; }
+    auto issue = [&](int c) {
+        const int valid = a.T - c * VCH;
+        bf16* t = tiles + ((c - c_lo) & 1) * 3 * C::TILE;
+        load_tile_async<VCH, D, C::LD>(t, qg + (int64_t)c * VCH * qst, qst, valid);
+        load_tile_async<VCH, D, C::LD>(t + C::TILE, kg + (int64_t)c * VCH * a.ks_t, a.ks_t, valid);
+        load_tile_async<VCH, D, C::LD>(t + 2 * C::TILE, vg + (int64_t)c * VCH * a.vs_t, a.vs_t, valid);
+    };
     float acc_s[C::S_NT][4];
     load_state_regs<D>(a.states + ((int64_t)bh * a.G + grp) * D * D, acc_s, s_m0, s_n0);
+    float2 g[C::RPG], up[MODE == 1 ? C::RPG : 1];                  // up: e^{b_i - b_m} for dq's epilogue
+    if (c_lo < c_hi) { issue(c_lo); load_gates<D>(a, b, h, c_lo, at, g); save_group_sum<D>(sums, at, g); }
+    cp_async_commit();
+    __syncthreads();
+    if (c_lo < c_hi) half_decays<D>(tabs, sums);
     for (int c = c_lo; c < c_hi; ++c) {
-        const int valid = a.T - c * VCH;
-        load_tile_async<VCH, D, C::LD>(Tq, qg + (int64_t)c * VCH * qst, qst, valid);
-        load_tile_async<VCH, D, C::LD>(Tk, kg + (int64_t)c * VCH * a.ks_t, a.ks_t, valid);
-        load_tile_async<VCH, D, C::LD>(Tv, vg + (int64_t)c * VCH * a.vs_t, a.vs_t, valid);
-        cp_async_commit();
-        load_cumsum<D>(a, b, h, c, bt);
+        const int s = (c - c_lo) & 1, valid = a.T - c * VCH;
+        bf16 *Tq = tiles + s * 3 * C::TILE, *Tk = Tq + C::TILE, *Tv = Tk + C::TILE;
+        const float *sm = sums + s * C::GR * D, *tab = tabs + s * 2 * D;
+        float *sm_next = sums + (s ^ 1) * C::GR * D, *tab_next = tabs + (s ^ 1) * 2 * D;
         cp_async_wait<0>();
-        __syncthreads();
-        if (MODE == 0) rescale_tile<D, C::LD>(Tq, bt, MID, 1.f, 1.f);          // q~ ; in mode 1 the tile is dO (unscaled)
-        rescale_tile<D, C::LD>(Tk, bt, MID, -1.f, 1.f);                        // k~
-        {
-            const int r = s_m0 + (l >> 2);
-            store_state_scaled<D>(acc_s, Sb, s_m0, s_n0, __expf(bt[MID * D + r]), __expf(bt[MID * D + r + 8]));
+        __syncthreads();                                            // tiles and tables of this chunk visible; the other stage is free
+        if (c + 1 < c_hi) issue(c + 1);
+        cp_async_commit();
+        about_middle<D>(g, sm, at);
+#pragma unroll
+        for (int i = 0; i < C::RPG; ++i) {
+            const int o = (at.row0 + i) * C::LD + 2 * at.pair;
+            if (MODE == 0) mul2(Tq + o, __expf(g[i].x), __expf(g[i].y));            // q~ (in mode 1 the tile is dO, unscaled)
+            else up[i] = make_float2(__expf(g[i].x), __expf(g[i].y));
+            mul2(Tk + o, __expf(-g[i].x), __expf(-g[i].y));                         // k~
         }
+        const float em0 = tab[sr], em1 = tab[sr + 8], ee0 = tab[D + sr], ee1 = tab[D + sr + 8];
+        rowscale_acc<C::S_NT>(acc_s, em0, em1);                                     // e^{b_m} S
+        store_state_scaled<D>(acc_s, Sb, s_m0, s_n0, 1.f, 1.f);
+        if (c + 1 < c_hi) load_gates<D>(a, b, h, c + 1, at, g);
         __syncthreads();
-        float acc_o[C::O_NT][4], acc_a[4][4];
+        float acc_o[C::O_NT][4];
         zero_acc<C::O_NT>(acc_o);
-        zero_acc<4>(acc_a);
-        if (MODE == 0) {
-            warp_gemm<C::O_NT, D, false, true>(acc_o, Tq, C::LD, o_m0, Sb, C::LD, o_n0);          // q~ (e^{b_m} S)
-            warp_gemm<4, D, false, false>(acc_a, Tq, C::LD, a_m0, Tk, C::LD, a_n0);               // q~ k~^T
-        } else {
-            warp_gemm<C::O_NT, D, false, false>(acc_o, Tq, C::LD, o_m0, Sb, C::LD, o_n0);         // dO (e^{b_m} S)^T
-            warp_gemm<4, D, false, false>(acc_a, Tq, C::LD, a_m0, Tv, C::LD, a_n0);               // dO V^T
-        }
-        rowscale_acc<C::O_NT>(acc_o, a.scale, a.scale);
-        mask_store_plain<1>(acc_a, P, C::PLD, a_m0, a_n0, a.scale);
-        __syncthreads();
-        if (MODE == 0) warp_gemm<C::O_NT, VCH, false, true>(acc_o, P, C::PLD, o_m0, Tv, C::LD, o_n0);   // A V
-        else warp_gemm<C::O_NT, VCH, false, true>(acc_o, P, C::PLD, o_m0, Tk, C::LD, o_n0);             // dA k~
-        // state: S <- e^{b_C - b_m} [ e^{b_m} S + k~^T V ]
         {
-            const int r = s_m0 + (l >> 2);
-            const float m0 = bt[MID * D + r], m1 = bt[MID * D + r + 8];
-            const float e0 = bt[(VCH - 1) * D + r], e1 = bt[(VCH - 1) * D + r + 8];
-            rowscale_acc<C::S_NT>(acc_s, __expf(m0), __expf(m1));
-            warp_gemm<C::S_NT, VCH, true, true>(acc_s, Tk, C::LD, s_m0, Tv, C::LD, s_n0);
-            rowscale_acc<C::S_NT>(acc_s, __expf(e0 - m0), __expf(e1 - m1));
+            float acc_a[2][4];
+            zero_acc<2>(acc_a);
+            if (MODE == 0) {
+                warp_gemm<C::O_NT, D, false, true>(acc_o, Tq, C::LD, m0, Sb, C::LD, o_n0);          // q~ (e^{b_m} S)
+                if (a_n0 <= m0) warp_gemm<2, D, false, false>(acc_a, Tq, C::LD, m0, Tk, C::LD, a_n0);     // q~ k~^T
+            } else {
+                warp_gemm<C::O_NT, D, false, false>(acc_o, Tq, C::LD, m0, Sb, C::LD, o_n0);         // dO (e^{b_m} S)^T
+                if (a_n0 <= m0) warp_gemm<2, D, false, false>(acc_a, Tq, C::LD, m0, Tv, C::LD, a_n0);     // dO V^T
+            }
+            rowscale_acc<C::O_NT>(acc_o, a.scale, a.scale);
+            if (a_n0 <= m0) mask_store_plain<1>(acc_a, P, C::PLD, m0, a_n0, a.scale);               // (the blocks above are never read)
         }
-        __syncthreads();                                            // Tq free (its last readers were before the previous barrier's gemms)
-        store_acc_bf16<C::O_NT>(acc_o, Tq, C::LD, o_m0, o_n0);
+        if (c + 1 < c_hi) save_group_sum<D>(sm_next, at, g);
         __syncthreads();
-        if (MODE == 1) rescale_tile<D, C::LD>(Tq, bt, MID, 1.f, 1.f);          // dq = e^{b_i - b_m} . (...)
-        __syncthreads();
-        vstore_tile<D, C::LD>(Tq, og + (int64_t)c * VCH * ost, ost, valid);
-        __syncthreads();
+        if (c + 1 < c_hi) half_decays<D>(tab_next, sm_next);
+        const bf16* X = MODE == 0 ? Tv : Tk;
+        for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<C::O_NT, 16, false, true>(acc_o, P + k0, C::PLD, m0, X + k0 * C::LD, C::LD, o_n0);   // A V | dA k~
+        store_acc_bf16<C::O_NT>(acc_o, Tq, C::LD, m0, o_n0);                        // (nobody reads Tq any more)
+        // state: S <- e^{b_C - b_m} [ e^{b_m} S + k~^T V ]
+        warp_gemm<C::S_NT, VCH, true, true>(acc_s, Tk, C::LD, s_m0, Tv, C::LD, s_n0);
+        rowscale_acc<C::S_NT>(acc_s, ee0, ee1);
+        if (MODE == 0) {
+            __syncwarp();
+            store_block<D, C::LD>(Tq, m0, o_n0, og + (int64_t)c * VCH * ost, ost, valid);
+        } else {
+            __syncthreads();                                        // dq = e^{b_i - b_m} . (...), by the threads that have the factors
+#pragma unroll
+            for (int i = 0; i < C::RPG; ++i) {
+                const int row = at.row0 + i;
+                const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Tq + row * C::LD + 2 * at.pair));
+                if (row < valid)
+                    *reinterpret_cast<__nv_bfloat162*>(og + ((int64_t)c * VCH + row) * ost + 2 * at.pair) = __floats2bfloat162_rn(x.x * up[i].x, x.y * up[i].y);
+            }
+        }
     }
 }
 
@@ -305,25 +387,22 @@ __global__ void __launch_bounds__(VTHREADS) gla_fwd_sweep_kernel(GlaArgs a) {
 // 3b. backward dk, dv: reverse sweep carrying dS.
 // ---------------------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(VTHREADS) gla_bwd_dkv_kernel(GlaArgs a) {
+__global__ void __launch_bounds__(VTHREADS, 1) gla_bwd_dkv_kernel(GlaArgs a) {
     using C = VCfg<D>;
-    constexpr int MID = VCH / 2 - 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* Tq = reinterpret_cast<bf16*>(smem_raw);
-    bf16* Tk = Tq + VCH * C::LD;
-    bf16* Tv = Tk + VCH * C::LD;
-    bf16* Tg = Tv + VCH * C::LD;
-    bf16* Sb = Tg + VCH * C::LD;                                    // diag(e^{b_C - b_m}) dS
+    bf16* tiles = reinterpret_cast<bf16*>(smem_raw);                // [2] x { q, k, v, dO }
+    bf16* Sb = tiles + 8 * C::TILE;                                 // diag(e^{b_C - b_m}) dS
     bf16* P1 = Sb + D * C::LD;
     bf16* P2 = P1 + VCH * C::PLD;
-    float* bt = reinterpret_cast<float*>(P2 + VCH * C::PLD);
+    float* sums = reinterpret_cast<float*>(P2 + VCH * C::PLD);      // [2][GR][D]
+    float* tabs = sums + 2 * C::GR * D;                             // [2][2][D]
     const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int nchunks = (a.T + VCH - 1) / VCH;
     const int c_lo = grp * a.cpg, c_hi = min(nchunks, c_lo + a.cpg);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int s_m0 = 16 * (w % C::S_RB), s_n0 = (w / C::S_RB) * (C::S_NT * 8);
-    const int o_m0 = 16 * (w & 3), o_n0 = (w >> 2) * (D / 2);
-    const int a_m0 = 16 * (w & 3), a_n0 = (w >> 2) * 32;
+    const int s_m0 = 16 * (w % C::S_RB), s_n0 = (w / C::S_RB) * (C::S_NT * 8), sr = s_m0 + (l >> 2);
+    const int m0 = 16 * (w & 3), o_n0 = (w >> 2) * (D / 4), a_n0 = (w >> 2) * 16;
+    const Place<D> at;
     const bf16* qg = a.q + b * a.qs_b + h * a.qs_h;
     const bf16* kg = a.k + b * a.ks_b + h * a.ks_h;
     const bf16* vg = a.v + b * a.vs_b + h * a.vs_h;
@@ -331,61 +410,87 @@ __global__ void __launch_bounds__(VTHREADS) gla_bwd_dkv_kernel(GlaArgs a) {
     const int64_t gst = (int64_t)a.H * D;
     bf16* dkg = a.dk + b * a.dks_b + h * a.dks_h;
     bf16* dvg = a.dv + b * a.dvs_b + h * a.dvs_h;
+    auto issue = [&](int c) {
+        const int valid = a.T - c * VCH;
+        bf16* t = tiles + ((c_hi - 1 - c) & 1) * 4 * C::TILE;
+        load_tile_async<VCH, D, C::LD>(t, qg + (int64_t)c * VCH * a.qs_t, a.qs_t, valid);
+        load_tile_async<VCH, D, C::LD>(t + C::TILE, kg + (int64_t)c * VCH * a.ks_t, a.ks_t, valid);
+        load_tile_async<VCH, D, C::LD>(t + 2 * C::TILE, vg + (int64_t)c * VCH * a.vs_t, a.vs_t, valid);
+        load_tile_async<VCH, D, C::LD>(t + 3 * C::TILE, gg + (int64_t)c * VCH * gst, gst, valid);
+    };
     float acc_s[C::S_NT][4];
     load_state_regs<D>(a.states + ((int64_t)bh * a.G + grp) * D * D, acc_s, s_m0, s_n0);
+    float2 g[C::RPG], dn[C::RPG];                                   // dn: e^{b_m - b_j} for dk's epilogue
+    if (c_lo < c_hi) { issue(c_hi - 1); load_gates<D>(a, b, h, c_hi - 1, at, g); save_group_sum<D>(sums, at, g); }
+    cp_async_commit();
+    __syncthreads();
+    if (c_lo < c_hi) half_decays<D>(tabs, sums);
     for (int c = c_hi - 1; c >= c_lo; --c) {
-        const int valid = a.T - c * VCH;
-        load_tile_async<VCH, D, C::LD>(Tq, qg + (int64_t)c * VCH * a.qs_t, a.qs_t, valid);
-        load_tile_async<VCH, D, C::LD>(Tk, kg + (int64_t)c * VCH * a.ks_t, a.ks_t, valid);
-        load_tile_async<VCH, D, C::LD>(Tv, vg + (int64_t)c * VCH * a.vs_t, a.vs_t, valid);
-        load_tile_async<VCH, D, C::LD>(Tg, gg + (int64_t)c * VCH * gst, gst, valid);
-        cp_async_commit();
-        load_cumsum<D>(a, b, h, c, bt);
+        const int s = (c_hi - 1 - c) & 1, valid = a.T - c * VCH;
+        bf16 *Tq = tiles + s * 4 * C::TILE, *Tk = Tq + C::TILE, *Tv = Tk + C::TILE, *Tg = Tv + C::TILE;
+        const float *sm = sums + s * C::GR * D, *tab = tabs + s * 2 * D;
+        float *sm_next = sums + (s ^ 1) * C::GR * D, *tab_next = tabs + (s ^ 1) * 2 * D;
         cp_async_wait<0>();
         __syncthreads();
-        rescale_tile<D, C::LD>(Tq, bt, MID, 1.f, 1.f);
-        rescale_tile<D, C::LD>(Tk, bt, MID, -1.f, 1.f);
-        const int r = s_m0 + (l >> 2);
-        const float m0 = bt[MID * D + r], m1 = bt[MID * D + r + 8];
-        const float e0 = bt[(VCH - 1) * D + r], e1 = bt[(VCH - 1) * D + r + 8];
-        store_state_scaled<D>(acc_s, Sb, s_m0, s_n0, __expf(e0 - m0), __expf(e1 - m1));
+        if (c > c_lo) issue(c - 1);
+        cp_async_commit();
+        about_middle<D>(g, sm, at);
+#pragma unroll
+        for (int i = 0; i < C::RPG; ++i) {
+            const int o = (at.row0 + i) * C::LD + 2 * at.pair;
+            mul2(Tq + o, __expf(g[i].x), __expf(g[i].y));
+            dn[i] = make_float2(__expf(-g[i].x), __expf(-g[i].y));
+            mul2(Tk + o, dn[i].x, dn[i].y);
+        }
+        const float em0 = tab[sr], em1 = tab[sr + 8], ee0 = tab[D + sr], ee1 = tab[D + sr + 8];
+        store_state_scaled<D>(acc_s, Sb, s_m0, s_n0, ee0, ee1);
         __syncthreads();
-        float acc_dv[C::O_NT][4], acc_dk[C::O_NT][4], acc_a[4][4], acc_b[4][4];
+        float acc_dv[C::O_NT][4], acc_dk[C::O_NT][4];
         zero_acc<C::O_NT>(acc_dv);
         zero_acc<C::O_NT>(acc_dk);
-        zero_acc<4>(acc_a);
-        zero_acc<4>(acc_b);
-        warp_gemm<4, D, false, false>(acc_a, Tk, C::LD, a_m0, Tq, C::LD, a_n0);               // k~ q~^T
-        warp_gemm<4, D, false, false>(acc_b, Tv, C::LD, a_m0, Tg, C::LD, a_n0);               // V dO^T
-        warp_gemm<C::O_NT, D, false, true>(acc_dv, Tk, C::LD, o_m0, Sb, C::LD, o_n0);         // k~ (e^{b_C-b_m} dS)
-        warp_gemm<C::O_NT, D, false, false>(acc_dk, Tv, C::LD, o_m0, Sb, C::LD, o_n0);        // V (e^{b_C-b_m} dS)^T
-        mask_store_plain<0>(acc_a, P1, C::PLD, a_m0, a_n0, a.scale);
-        mask_store_plain<0>(acc_b, P2, C::PLD, a_m0, a_n0, a.scale);
+        if (a_n0 >= m0) {
+            float acc_a[2][4];
+            zero_acc<2>(acc_a);
+            warp_gemm<2, D, false, false>(acc_a, Tk, C::LD, m0, Tq, C::LD, a_n0);             // k~ q~^T
+            mask_store_plain<0>(acc_a, P1, C::PLD, m0, a_n0, a.scale);
+            zero_acc<2>(acc_a);
+            warp_gemm<2, D, false, false>(acc_a, Tv, C::LD, m0, Tg, C::LD, a_n0);             // V dO^T
+            mask_store_plain<0>(acc_a, P2, C::PLD, m0, a_n0, a.scale);
+        }
+        warp_gemm<C::O_NT, D, false, true>(acc_dv, Tk, C::LD, m0, Sb, C::LD, o_n0);           // k~ (e^{b_C-b_m} dS)
+        warp_gemm<C::O_NT, D, false, false>(acc_dk, Tv, C::LD, m0, Sb, C::LD, o_n0);          // V (e^{b_C-b_m} dS)^T
+        if (c > c_lo) { load_gates<D>(a, b, h, c - 1, at, g); save_group_sum<D>(sm_next, at, g); }
         __syncthreads();
-        warp_gemm<C::O_NT, VCH, false, true>(acc_dv, P1, C::PLD, o_m0, Tg, C::LD, o_n0);      // Abar dO
-        warp_gemm<C::O_NT, VCH, false, true>(acc_dk, P2, C::PLD, o_m0, Tq, C::LD, o_n0);      // Bbar q~
+        if (c > c_lo) half_decays<D>(tab_next, sm_next);
+        for (int k0 = m0; k0 < VCH; k0 += 16) {
+            warp_gemm<C::O_NT, 16, false, true>(acc_dv, P1 + k0, C::PLD, m0, Tg + k0 * C::LD, C::LD, o_n0);      // Abar dO
+            warp_gemm<C::O_NT, 16, false, true>(acc_dk, P2 + k0, C::PLD, m0, Tq + k0 * C::LD, C::LD, o_n0);      // Bbar q~
+        }
+        store_acc_bf16<C::O_NT>(acc_dv, Tv, C::LD, m0, o_n0);                                 // (K and V have been read)
+        store_acc_bf16<C::O_NT>(acc_dk, Tk, C::LD, m0, o_n0);
         // dS <- e^{b_m} [ e^{b_C - b_m} dS + scale q~^T dO ]: fold `scale` by scaling around the product
-        rowscale_acc<C::S_NT>(acc_s, __expf(e0 - m0) / a.scale, __expf(e1 - m1) / a.scale);
+        rowscale_acc<C::S_NT>(acc_s, ee0 / a.scale, ee1 / a.scale);
         warp_gemm<C::S_NT, VCH, true, true>(acc_s, Tq, C::LD, s_m0, Tg, C::LD, s_n0);
-        rowscale_acc<C::S_NT>(acc_s, __expf(m0) * a.scale, __expf(m1) * a.scale);
-        __syncthreads();
-        store_acc_bf16<C::O_NT>(acc_dv, Tv, C::LD, o_m0, o_n0);
-        store_acc_bf16<C::O_NT>(acc_dk, Tk, C::LD, o_m0, o_n0);
-        __syncthreads();
-        rescale_tile<D, C::LD>(Tk, bt, MID, -1.f, 1.f);                        // dk = e^{b_m - b_j} . (...)
-        __syncthreads();
-        vstore_tile<D, C::LD>(Tv, dvg + (int64_t)c * VCH * a.dvs_t, a.dvs_t, valid);
-        vstore_tile<D, C::LD>(Tk, dkg + (int64_t)c * VCH * a.dks_t, a.dks_t, valid);
-        __syncthreads();
+        rowscale_acc<C::S_NT>(acc_s, em0 * a.scale, em1 * a.scale);
+        __syncwarp();
+        store_block<D, C::LD>(Tv, m0, o_n0, dvg + (int64_t)c * VCH * a.dvs_t, a.dvs_t, valid);
+        __syncthreads();                                            // dk = e^{b_m - b_j} . (...), by the threads that have the factors
+#pragma unroll
+        for (int i = 0; i < C::RPG; ++i) {
+            const int row = at.row0 + i;
+            const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Tk + row * C::LD + 2 * at.pair));
+            if (row < valid)
+                *reinterpret_cast<__nv_bfloat162*>(dkg + ((int64_t)c * VCH + row) * a.dks_t + 2 * at.pair) = __floats2bfloat162_rn(x.x * dn[i].x, x.y * dn[i].y);
+        }
     }
 }
 
-template <int D> constexpr size_t gla_smem_scan() { return (size_t)2 * VCH * VCfg<D>::LD * 2 + (size_t)VCH * D * 4; }
+template <int D> constexpr size_t gla_smem_scan() { return (size_t)4 * VCfg<D>::TILE * 2 + (size_t)2 * VCfg<D>::GR * D * 4; }
 template <int D> constexpr size_t gla_smem_sweep() {
-    return (size_t)3 * VCH * VCfg<D>::LD * 2 + (size_t)D * VCfg<D>::LD * 2 + (size_t)VCH * VCfg<D>::PLD * 2 + (size_t)VCH * D * 4;
+    return (size_t)6 * VCfg<D>::TILE * 2 + (size_t)D * VCfg<D>::LD * 2 + (size_t)VCH * VCfg<D>::PLD * 2 + (size_t)(2 * VCfg<D>::GR + 4) * D * 4;
 }
 template <int D> constexpr size_t gla_smem_dkv() {
-    return (size_t)4 * VCH * VCfg<D>::LD * 2 + (size_t)D * VCfg<D>::LD * 2 + (size_t)2 * VCH * VCfg<D>::PLD * 2 + (size_t)VCH * D * 4;
+    return (size_t)8 * VCfg<D>::TILE * 2 + (size_t)D * VCfg<D>::LD * 2 + (size_t)2 * VCH * VCfg<D>::PLD * 2 + (size_t)(2 * VCfg<D>::GR + 4) * D * 4;
 }
 
 }  // namespace lmoe

@@ -1214,6 +1214,7 @@ class _LsmVector(torch.autograd.Function):
             _gla_combine(0, states, gdecay, seed, final, B * H, G, D)
         _gla_launch(2, D, a)
         ctx.lasp = lasp
+        ctx.set_materialize_grads(False)                 # no zeros for an output without a gradient (mostly the final state)
         ctx.save_for_backward(q, k, v, gf, states, gdecay, final)
         ctx.scale, ctx.grid, ctx.has_init, ctx.g_dtype = scale, (G, cpg), init is not None, gk.dtype
         return o, final
@@ -1223,7 +1224,7 @@ class _LsmVector(torch.autograd.Function):
         q, k, v, gf, states, gdecay, final = ctx.saved_tensors
         B, T, H, D = q.shape
         G, cpg = ctx.grid
-        d_o = d_o.contiguous().to(q.dtype)
+        d_o = torch.zeros(B, T, H, D, dtype=q.dtype, device=q.device) if d_o is None else d_o.contiguous().to(q.dtype)
         dqkv = torch.empty(B, T, H, 3 * D, dtype=q.dtype, device=q.device)
         dq, dk, dv = dqkv[..., :D], dqkv[..., D:2 * D], dqkv[..., 2 * D:]
         dstates = torch.empty_like(states)

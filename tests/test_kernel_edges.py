@@ -91,3 +91,18 @@ def test_delta_scans_of_padded_and_dense_tiles(D, T):
                      *K._delta_scan_bwd(W, Qd, Kd, A, gamma, go, None)])
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [2, 15, 17, 63, 64, 65, 129, 200])
+def test_vector_decay_chunk_edges(D, T):
+    torch.manual_seed(0)
+    B, H = 2, 3
+    q, k, v = rand(B, T, H, 3 * D).split(D, dim=-1)
+    g = torch.nn.functional.logsigmoid(2 * torch.randn(B, T, H, D, device="cuda")) / 4
+    S0, gS = 0.3 * torch.randn(B, H, D, D, device="cuda"), 0.1 * torch.randn(B, H, D, D, device="cuda")
+    go = rand(B, T, H, D, scale=1)
+    ins = [q, k, v, g, S0]
+    got = run(lambda q, k, v, g, S: ops.lsm_vector(q, k, v, g, None, S, None, 64), ins, [go, gS])
+    want = run(lambda q, k, v, g, S: RL.recurrent_lsm(q, k, v, gk=g, initial_state=S), [t.float() for t in ins], [go.float(), gS])
+    check(got, want, ["o", "S", "dq", "dk", "dv", "dg", "dS0"])
