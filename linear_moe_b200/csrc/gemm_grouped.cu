@@ -46,7 +46,14 @@ struct Params {
     int out_f32;              // pair kernel: C is fp32 (weight gradients straight into the fp32 accumulators)
     int accumulate;           // with out_f32: C += result instead of C = result
     const float* row_scale;   // mode 1, bf16 output: C = (row_scale[row] * relu(result))^2 (null: C = result)
+    // pair kernel, mode 1: what becomes of the result in the epilogue.  Passes of their own over [rows, 2 f] took 67 us (SwiGLU) and 118 us (its
+    // gradient) for 8192 tokens x 8 of 64 experts of 896; the epilogues run beside the next tile's products.
+    int epilogue;             // EPI_*
+    int bn;                   // columns of N per tile: BN, or BN / 2 where a tile holds as many gate and up columns
+    bf16* act;                // EPI_SWIGLU: silu(gate) * up [rows, N], beside C = [gate | up] [rows, 2 N]
+    const bf16* pre;          // EPI_DSWIGLU: [gate | up] [rows, 2 N]; C is their gradient
 };
+enum { EPI_NONE, EPI_SWIGLU, EPI_DSWIGLU };
 
 // the squared-relu epilogue on a thread's 32 columns of one row
 __device__ __forceinline__ void relu2(uint32_t (&v)[32], float scale) {
@@ -57,6 +64,12 @@ __device__ __forceinline__ void relu2(uint32_t (&v)[32], float scale) {
     }
 }
 
+
+// Where a role stands in the list of experts: tiles come in ascending order, so the search goes on from the last one.  (From the first
+// expert every time, 64 experts cost each role a chain of up to 64 loads per tile.)
+struct Cursor {
+    int e = 0, base = 0;
+};
 
 // One output tile of the (possibly grouped) problem.
 struct Tile {
@@ -69,8 +82,8 @@ struct Tile {
 };
 
 // `bm` = rows of one output tile: 128 for one CTA, 256 for a CTA pair
-__device__ __forceinline__ bool decode_tile(const Params& p, int t, Tile& o, const int bm = BM) {
-    const int tiles_n = (p.N + BN - 1) / BN;
+__device__ __forceinline__ bool decode_tile(const Params& p, int t, Tile& o, Cursor& cur, const int bm = BM) {
+    const int bn = p.bn, tiles_n = (p.N + bn - 1) / bn;
     if (p.mode == 0) {
         const int tiles_m = (p.M + bm - 1) / bm;
         if (t >= tiles_m * tiles_n) return false;
@@ -82,25 +95,24 @@ __device__ __forceinline__ bool decode_tile(const Params& p, int t, Tile& o, con
         return true;
     }
     if (p.mode == 1) {
-        int base = 0;
-        for (int e = 0; e < p.num_groups; ++e) {
-            const int r0 = p.offs[e], r1 = p.offs[e + 1];
+        for (; cur.e < p.num_groups; ++cur.e) {
+            const int e = cur.e, r0 = p.offs[e], r1 = p.offs[e + 1];
             const int tm_e = (r1 - r0) / bm;
             const int n_e = tm_e * tiles_n;
-            if (t < base + n_e) {
-                const int lt = t - base;
+            if (t < cur.base + n_e) {
+                const int lt = t - cur.base;
                 const int tm = lt % tm_e, tn = lt / tm_e;
                 o.a_row = r0 + tm * bm;
                 o.a_k0 = 0;
-                // B map: K-major -> rows [e*N + tn*BN), k from 0.  MN-major -> mn column tn*BN, k rows from e*K
-                o.b_row = tn * BN;
+                // B map: K-major -> rows [e*N + tn*bn), k from 0.  MN-major -> mn column tn*bn, k rows from e*K
+                o.b_row = tn * bn;
                 o.b_k0 = e * p.b_group_rows;              // used as a row offset (K-major: added to b_row) or k offset (MN-major)
                 o.kblocks = (p.K + BK - 1) / BK;
-                o.c_off = (long long)(r0 + tm * bm) * p.ldc + (long long)tn * BN;
-                o.rows_valid = bm; o.cols_valid = p.N - tn * BN;
+                o.c_off = (long long)(r0 + tm * bm) * p.ldc + (long long)tn * bn;
+                o.rows_valid = bm; o.cols_valid = p.N - tn * bn;
                 return true;
             }
-            base += n_e;
+            cur.base += n_e;
         }
         return false;
     }
@@ -147,7 +159,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (lane == 0) {
             int it = 0;
             Tile t;
-            for (int tile = blockIdx.x; !*abort_flag && decode_tile(p, tile, t); tile += gridDim.x) {
+            Cursor cur;
+            for (int tile = blockIdx.x; !*abort_flag && decode_tile(p, tile, t, cur); tile += gridDim.x) {
                 for (int kb = 0; kb < t.kblocks; ++kb, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
@@ -179,7 +192,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             constexpr uint32_t idesc = make_idesc<A_MN, B_MN, BM, BN>();
             int it = 0, lt = 0;
             Tile t;
-            for (int tile = blockIdx.x; !*abort_flag && decode_tile(p, tile, t); tile += gridDim.x, ++lt) {
+            Cursor cur;
+            for (int tile = blockIdx.x; !*abort_flag && decode_tile(p, tile, t, cur); tile += gridDim.x, ++lt) {
                 const int buf = lt & 1;
                 const uint32_t aph = (lt >> 1) & 1;
                 if (!mbar_wait(&sm.tmem_empty[buf], aph ^ 1, abort_flag, err, 0x200 | buf)) break;
@@ -208,7 +222,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const int q = warp & 3;
         int lt = 0;
         Tile t;
-        for (int tile = blockIdx.x; decode_tile(p, tile, t); tile += gridDim.x, ++lt) {
+        Cursor cur;
+        for (int tile = blockIdx.x; decode_tile(p, tile, t, cur); tile += gridDim.x, ++lt) {
             const int buf = lt & 1;
             const uint32_t aph = (lt >> 1) & 1;
             if (!mbar_wait(&sm.tmem_full[buf], aph, abort_flag, err, 0x400 | buf)) break;
@@ -282,6 +297,31 @@ struct __align__(1024) SmemPair {
     int abort_flag;
 };
 
+// A row's 32 numbers as bf16 into half `hc` of the warp's staging buffer (32 rows x 128 bytes, 16-byte chunks xor-swizzled) ...
+__device__ __forceinline__ void stage32(uint8_t* stg, int lane, int hc, const uint32_t (&v)[32], bool zero) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        uint4 o = make_uint4(0, 0, 0, 0);
+        if (!zero) {
+            o.x = pack_bf16(__uint_as_float(v[g * 8 + 0]), __uint_as_float(v[g * 8 + 1]));
+            o.y = pack_bf16(__uint_as_float(v[g * 8 + 2]), __uint_as_float(v[g * 8 + 3]));
+            o.z = pack_bf16(__uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5]));
+            o.w = pack_bf16(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7]));
+        }
+        *reinterpret_cast<uint4*>(stg + lane * 128 + (((hc * 4 + g) ^ (lane & 7)) << 4)) = o;
+    }
+}
+// ... and from there to memory: 8 lanes write one row's 128 contiguous bytes, whole lines, 4 rows per instruction
+__device__ __forceinline__ void unstage64(const uint8_t* stg, int lane, bf16* dst, long long ld, int cols_valid, int rows_valid = 32) {
+    const int chunk = lane & 7;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+        const int rr = it * 4 + (lane >> 3);
+        const uint4 o = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((chunk ^ (rr & 7)) << 4));
+        if (rr < rows_valid && chunk * 8 + 8 <= cols_valid) *reinterpret_cast<uint4*>(dst + rr * ld + chunk * 8) = o;
+    }
+}
+
 template <bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, bf16* __restrict__ C, Params p) {
@@ -309,12 +349,14 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = sm.tmem_base;
     const int half = (int)rank * 128;                        // this CTA's rows of A (M) and of B (N) inside the pair tile
+    const int b_half = p.epilogue == EPI_SWIGLU ? (int)rank * p.N : half;          // (128 gate columns and the up columns that go with them)
 
     if (warp == 0) {
         if (lane == 0) {
             int it = 0;
             Tile t;
-            for (int tile = pair; !*abort_flag && decode_tile(p, tile, t, 256); tile += num_pairs) {
+            Cursor cur;
+            for (int tile = pair; !*abort_flag && decode_tile(p, tile, t, cur, 256); tile += num_pairs) {
                 for (int kb = 0; kb < t.kblocks; ++kb, ++it) {
                     const int s = it % P_STAGES;
                     const uint32_t ph = (it / P_STAGES) & 1;
@@ -334,7 +376,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                         tma_load_2d_pair(sb, &tmB, fl, (p.mode == 1 ? 0 : t.b_k0) + kb * BK, brow);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) tma_load_2d_pair(sb + j * 8192, &tmB, fl, t.b_row + half + j * 64, t.b_k0 + kb * BK);
+                        for (int j = 0; j < 2; ++j) tma_load_2d_pair(sb + j * 8192, &tmB, fl, t.b_row + b_half + j * 64, t.b_k0 + kb * BK);
                     }
                 }
             }
@@ -346,7 +388,8 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                                        ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             int it = 0, lt = 0;
             Tile t;
-            for (int tile = pair; !*abort_flag && decode_tile(p, tile, t, 256); tile += num_pairs, ++lt) {
+            Cursor cur;
+            for (int tile = pair; !*abort_flag && decode_tile(p, tile, t, cur, 256); tile += num_pairs, ++lt) {
                 const int buf = lt & 1;
                 const uint32_t aph = (lt >> 1) & 1;
                 if (!mbar_wait(&sm.tmem_empty[buf], aph ^ 1, abort_flag, err, 0x6200 | buf)) break;
@@ -375,7 +418,8 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         const int q = warp & 3;
         int lt = 0;
         Tile t;
-        for (int tile = pair; decode_tile(p, tile, t, 256); tile += num_pairs, ++lt) {
+        Cursor cur;
+        for (int tile = pair; decode_tile(p, tile, t, cur, 256); tile += num_pairs, ++lt) {
             const int buf = lt & 1;
             const uint32_t aph = (lt >> 1) & 1;
             if (!mbar_wait(&sm.tmem_full[buf], aph, abort_flag, err, 0x6400 | buf)) break;
@@ -413,6 +457,67 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                     }
                     __syncwarp();
                 }
+            } else if (p.epilogue == EPI_SWIGLU) {
+                // columns 0 .. 127: gate, 128 .. 255: up.  64 of each through the staging buffer, then the activation
+#pragma unroll 1
+                for (int c = 0; c < 128; c += 64) {
+                    const bool more = c + 64 <= t.cols_valid;
+#pragma unroll 1
+                    for (int what = 0; what < 3; ++what) {
+#pragma unroll
+                        for (int hc = 0; hc < 2; ++hc) {
+                            uint32_t v[32], u[32];
+                            tmem_ld32(taddr + c + hc * 32 + (what == 1 ? 128 : 0), v);
+                            if (what == 2) tmem_ld32(taddr + 128 + c + hc * 32, u);
+                            tmem_ld_wait();
+                            if (what == 2) {
+#pragma unroll
+                                for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(silu_f(__uint_as_float(v[e])) * __uint_as_float(u[e]));
+                            }
+                            stage32(stg, lane, hc, v, false);
+                        }
+                        __syncwarp();
+                        bf16* dst = what == 2 ? p.act + (long long)(t.a_row + r0) * p.N + t.b_row + c
+                                              : C + t.c_off + (long long)r0 * p.ldc + c + (what == 1 ? p.N : 0);
+                        unstage64(stg, lane, dst, what == 2 ? p.N : p.ldc, t.cols_valid - c);
+                        __syncwarp();
+                    }
+                    if (!more) break;
+                }
+            } else if (p.epilogue == EPI_DSWIGLU) {
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 64) {
+#pragma unroll
+                    for (int hc = 0; hc < 2; ++hc) {
+                        uint32_t v[32];
+                        tmem_ld32(taddr + c + hc * 32, v);
+                        tmem_ld_wait();
+                        stage32(stg, lane, hc, v, false);
+                    }
+                    __syncwarp();
+                    const int chunk = lane & 7, col = c + chunk * 8;
+                    if (col + 8 <= t.cols_valid) {                   // eight lanes per row: its gate and up values come in whole lines
+                        const long long at = (long long)(t.a_row + r0 + (lane >> 3)) * (2 * p.N) + t.b_row + col;
+                        Vec<bf16> gt[8], up[8];
+#pragma unroll
+                        for (int it = 0; it < 8; ++it) { gt[it].load(p.pre + at + (long long)it * 8 * p.N); up[it].load(p.pre + at + (long long)it * 8 * p.N + p.N); }
+#pragma unroll
+                        for (int it = 0; it < 8; ++it) {
+                            const int rr = it * 4 + (lane >> 3);
+                            Vec<bf16> d, dg, du;
+                            d.raw = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((chunk ^ (rr & 7)) << 4));
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                const float gv = gt[it].get(e), dv = d.get(e);
+                                dg.set(e, dv * up[it].get(e) * dsilu_f(gv));
+                                du.set(e, dv * silu_f(gv));
+                            }
+                            dg.store(C + at + (long long)it * 8 * p.N);
+                            du.store(C + at + (long long)it * 8 * p.N + p.N);
+                        }
+                    }
+                    __syncwarp();
+                }
             } else
 #pragma unroll 1
             for (int c = 0; c < BN; c += 64) {
@@ -422,30 +527,10 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                     tmem_ld32(taddr + c + hc * 32, v);
                     tmem_ld_wait();
                     if (p.row_scale != nullptr) relu2(v, scale);
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        uint4 o;
-                        if (zero) o = make_uint4(0, 0, 0, 0);
-                        else {
-                            o.x = pack_bf16(__uint_as_float(v[g * 8 + 0]), __uint_as_float(v[g * 8 + 1]));
-                            o.y = pack_bf16(__uint_as_float(v[g * 8 + 2]), __uint_as_float(v[g * 8 + 3]));
-                            o.z = pack_bf16(__uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5]));
-                            o.w = pack_bf16(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7]));
-                        }
-                        *reinterpret_cast<uint4*>(stg + lane * 128 + (((hc * 4 + g) ^ (lane & 7)) << 4)) = o;
-                    }
+                    stage32(stg, lane, hc, v, zero);
                 }
                 __syncwarp();
-                // 8 lanes write one row's 128 contiguous bytes: whole lines, 4 rows per instruction
-                const int chunk = lane & 7;
-                const int col = c + chunk * 8;
-#pragma unroll
-                for (int it = 0; it < 8; ++it) {
-                    const int rr = it * 4 + (lane >> 3);
-                    const uint4 o = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((chunk ^ (rr & 7)) << 4));
-                    if (r0 + rr < t.rows_valid && col + 8 <= t.cols_valid)
-                        *reinterpret_cast<uint4*>(C + t.c_off + (long long)(r0 + rr) * p.ldc + col) = o;
-                }
+                unstage64(stg, lane, C + t.c_off + (long long)r0 * p.ldc + c, p.ldc, t.cols_valid - c, t.rows_valid - r0);
                 __syncwarp();
             }
             tc_fence_before();
@@ -484,7 +569,7 @@ using namespace lmoe::gg;
 static int gemm_grouped_impl(const void* A, int a_rows, int a_cols, int lda, int a_mn, const void* B, int b_rows, int b_cols,
                              int ldb, int b_mn, void* C, int ldc, int mode, int M, int N, int K, int num_groups,
                              const int* offs, long long c_group_stride, int* err, int num_sms, int pairs, int out_f32, int accumulate,
-                             const float* row_scale, cudaStream_t st) {
+                             const float* row_scale, cudaStream_t st, int epilogue = EPI_NONE, void* act = nullptr, const void* pre = nullptr) {
     if (lda % 8 || ldb % 8 || ldc % 8 || a_cols % 8 || b_cols % 8 || N % 8) return -1;
     CUtensorMap ma, mb;
     int rc = make_map(&ma, A, (uint64_t)a_rows, (uint64_t)a_cols, (uint64_t)lda, a_mn ? 64 : BM);
@@ -495,6 +580,8 @@ static int gemm_grouped_impl(const void* A, int a_rows, int a_cols, int lda, int
     p.mode = mode; p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.num_groups = num_groups; p.offs = offs;
     p.c_group_stride = c_group_stride; p.b_group_rows = b_mn ? K : N; p.err = err;
     p.out_f32 = out_f32; p.accumulate = accumulate; p.row_scale = row_scale;
+    p.epilogue = epilogue; p.bn = epilogue == EPI_SWIGLU ? BN / 2 : BN; p.act = (bf16*)act; p.pre = (const bf16*)pre;
+    if (epilogue != EPI_NONE && (!pairs || mode != 1 || a_mn || out_f32 || (epilogue == EPI_SWIGLU && !b_mn))) return -4;
     if (out_f32 && !pairs) return -3;
     if (pairs) {
         if (!a_mn && !b_mn) return launch_pair<false, false>(ma, mb, (bf16*)C, p, num_sms, st);
@@ -524,4 +611,18 @@ LMOE_API int lmoe_gemm_grouped_relu2(const void* A, int a_rows, int lda, const v
     if (row_scale == nullptr) return -1;
     return gemm_grouped_impl(A, a_rows, K, lda, 0, W, num_groups * N, K, ldb, 0, C, ldc, 1, 0, N, K, num_groups, offs, 0, err, num_sms, pairs,
                              0, 0, row_scale, st);
+}
+
+// Expert MLPs with the activation in the epilogue (CTA pairs; offsets multiples of 256, f a multiple of 8).
+// pre [rows, 2 f] = x[rows_e, h] W1[e] for W1 [num_groups, h, 2 f] = [gate | up], act [rows, f] = silu(gate) * up.
+LMOE_API int lmoe_gemm_grouped_swiglu(const void* x, int rows, int h, const void* W1, void* pre, void* act, int f, int num_groups, const int* offs,
+                                      int* err, int num_sms, cudaStream_t st) {
+    return gemm_grouped_impl(x, rows, h, h, 0, W1, num_groups * h, 2 * f, 2 * f, 1, pre, 2 * f, 1, 0, f, h, num_groups, offs, 0, err, num_sms, 1, 0, 0,
+                             nullptr, st, EPI_SWIGLU, act, nullptr);
+}
+// d_pre [rows, 2 f] from dy [rows, h] and W2 [num_groups, f, h]: the gradient of act = dy[rows_e] W2[e]^T goes through the activation at `pre`.
+LMOE_API int lmoe_gemm_grouped_dswiglu(const void* dy, int rows, int h, const void* W2, const void* pre, void* d_pre, int f, int num_groups,
+                                       const int* offs, int* err, int num_sms, cudaStream_t st) {
+    return gemm_grouped_impl(dy, rows, h, h, 0, W2, num_groups * f, h, h, 0, d_pre, 2 * f, 1, 0, f, h, num_groups, offs, 0, err, num_sms, 1, 0, 0,
+                             nullptr, st, EPI_DSWIGLU, nullptr, pre);
 }

@@ -255,17 +255,71 @@ class GroupedLinear(torch.autograd.Function):
         dx = torch.empty_like(x) if ctx.dx_out is None else ctx.dx_out.buf[: x.shape[0]]
         assert dx.shape == x.shape and dx.is_contiguous()
         _gg(dy, False, w.view(E * Kd, N), False, dx, 1, 0, Kd, N, E, offs, 0)              # dy @ w[e]^T
-        mg = getattr(w, "main_grad", None)
-        if PAIRS and mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and mg.shape == w.shape:
-            # weight gradient straight into the fp32 accumulator (first write after zero_grad overwrites, later ones add)
-            fresh = getattr(w, "_main_grad_fresh", False)
-            _gg(x, True, dy, True, mg, 2, Kd, N, 0, E, offs, Kd * N, accumulate=not fresh)
-            w._main_grad_fresh = False
-            w._direct_wgrad = True
-            return dx, None, None, None, None
-        dw = torch.empty_like(w)
-        _gg(x, True, dy, True, dw, 2, Kd, N, 0, E, offs, Kd * N)                           # x_e^T @ dy_e
-        return dx, dw, None, None, None
+        return dx, _grouped_wgrad(w, x, dy, offs), None, None, None
+
+
+def _grouped_wgrad(w, x, dy, offs):
+    """``x_e^T @ dy_e`` for ``w [E, K, N]``: into the fp32 accumulator of the parameter where it has one (first write after
+    zero_grad overwrites, later ones add; returns None), else a tensor."""
+    E, Kd, N = w.shape
+    mg = getattr(w, "main_grad", None)
+    if PAIRS and mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and mg.shape == w.shape:
+        fresh = getattr(w, "_main_grad_fresh", False)
+        _gg(x, True, dy, True, mg, 2, Kd, N, 0, E, offs, Kd * N, accumulate=not fresh)
+        w._main_grad_fresh = False
+        w._direct_wgrad = True
+        return None
+    dw = torch.empty_like(w)
+    _gg(x, True, dy, True, dw, 2, Kd, N, 0, E, offs, Kd * N)
+    return dw
+
+
+class _ExpertMLP(torch.autograd.Function):
+    """``swiglu(x w1[e]) w2[e]`` over a padded expert-sorted buffer (``w1 [E, h, 2f]`` = [gate | up], ``w2 [E, f, h]``): the activation
+    and its gradient are epilogues of the grouped GEMMs.  ``out`` / ``dx_out`` as in :class:`GroupedLinear`."""
+
+    @staticmethod
+    def forward(ctx, x, w1, w2, offs, out, dx_out):
+        from . import cuda as K
+        E, h, f2 = w1.shape
+        rows, f = x.shape[0], f2 // 2
+        pre = torch.empty(rows, f2, dtype=torch.bfloat16, device=x.device)
+        act = torch.empty(rows, f, dtype=torch.bfloat16, device=x.device)
+        i = ctypes.c_int
+        K._check(K.lib().lmoe_gemm_grouped_swiglu(K._p(x), i(rows), i(h), K._p(w1), K._p(pre), K._p(act), i(f), i(E), K._p(offs),
+                                                  K._p(_err(x.device)), i(K.NUM_SMS), K._st()), "gemm_grouped_swiglu")
+        y = torch.empty(rows, h, dtype=torch.bfloat16, device=x.device) if out is None else out.buf[:rows]
+        assert y.shape == (rows, h) and y.is_contiguous()
+        _gg(act, False, w2.view(E * f, h), True, y, 1, 0, h, f, E, offs, 0)
+        ctx.save_for_backward(x, w1, w2, offs, pre, act)
+        ctx.dx_out = dx_out
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        from . import cuda as K
+        x, w1, w2, offs, pre, act = ctx.saved_tensors
+        E, h, f2 = w1.shape
+        rows, f = x.shape[0], f2 // 2
+        dy = dy.contiguous()
+        d_pre = torch.empty_like(pre)
+        i = ctypes.c_int
+        K._check(K.lib().lmoe_gemm_grouped_dswiglu(K._p(dy), i(rows), i(h), K._p(w2), K._p(pre), K._p(d_pre), i(f), i(E), K._p(offs),
+                                                   K._p(_err(x.device)), i(K.NUM_SMS), K._st()), "gemm_grouped_dswiglu")
+        dw2 = _grouped_wgrad(w2, act, dy, offs)
+        dx = torch.empty_like(x) if ctx.dx_out is None else ctx.dx_out.buf[:rows]
+        assert dx.shape == x.shape and dx.is_contiguous()
+        _gg(d_pre, False, w1.view(E * h, f2), False, dx, 1, 0, h, f2, E, offs, 0)
+        return dx, _grouped_wgrad(w1, x, d_pre, offs), dw2, None, None, None
+
+
+def expert_mlp(x, w1, w2, offs, out=None, dx_out=None):
+    """Two grouped linears with SwiGLU between them; every offset a multiple of :data:`ROW_ALIGN`."""
+    if PAIRS and x.is_contiguous() and w1.is_contiguous() and w2.is_contiguous() and w1.shape[2] == 2 * w2.shape[1]:
+        return _ExpertMLP.apply(x, w1, w2, offs, out, dx_out)
+    from . import cuda as K
+    act = K.swiglu(GroupedLinear.apply(x, w1, offs, None, dx_out))
+    return GroupedLinear.apply(act, w2, offs, out, None)
 
 
 def supports_grouped(x, w1, w2) -> bool:
@@ -276,9 +330,8 @@ def supports_grouped(x, w1, w2) -> bool:
 
 def grouped_mlp(x_sorted: torch.Tensor, tokens_per_expert: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
     """Expert-sorted tokens ``[T, h]`` through per-expert SwiGLU MLPs (``w1 [E,h,2f]``, ``w2 [E,f,h]``).  Tokens are
-    scattered into a 128-row-padded buffer (index arithmetic on the device only), run through two grouped GEMMs with the
-    SwiGLU kernel in between, and gathered back."""
-    from . import cuda as K
+    scattered into a padded buffer (index arithmetic on the device only), run through two grouped GEMMs with SwiGLU in the
+    first one's epilogue, and gathered back."""
     E = w1.shape[0]
     T, h = x_sorted.shape
     counts = tokens_per_expert.to(torch.int64)
@@ -288,7 +341,5 @@ def grouped_mlp(x_sorted: torch.Tensor, tokens_per_expert: torch.Tensor, w1: tor
     dest = offs[:-1].to(torch.int64)[eid] + (torch.arange(T, device=x_sorted.device) - start[eid])
     Tp = (T + E * (ROW_ALIGN - 1) + ROW_ALIGN - 1) // ROW_ALIGN * ROW_ALIGN
     xp = torch.zeros(Tp, h, dtype=x_sorted.dtype, device=x_sorted.device).index_copy(0, dest, x_sorted)
-    y1 = GroupedLinear.apply(xp, w1, offs)
-    act = K.swiglu(y1)
-    y2 = GroupedLinear.apply(act, w2, offs)
+    y2 = expert_mlp(xp, w1, w2, offs)
     return y2.index_select(0, dest)

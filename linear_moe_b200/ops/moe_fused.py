@@ -53,13 +53,10 @@ class _Combine(torch.autograd.Function):
 
 def fused_moe(h: torch.Tensor, probs: torch.Tensor, idx: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, ws) -> torch.Tensor:
     """``h [T, hid]`` bf16, ``probs/idx [T, k]``, local expert weights ``w1 [El, hid, 2f]``, ``w2 [El, f, hid]``."""
-    from . import cuda as K
     route = ws.route(idx)
     xr = _Dispatch.apply(h, ws, route)
     # between ranks, the second GEMM writes its result, and the first GEMM's backward its input gradient, straight into
     # the buffer the peers pull from (no copy into it)
     res = ws.result_holder()
-    y1 = gemm.GroupedLinear.apply(xr, w1, route.offs, None, res)
-    act = K.swiglu(y1)
-    y2 = gemm.GroupedLinear.apply(act, w2, route.offs, res, None)
+    y2 = gemm.expert_mlp(xr, w1, w2, route.offs, res, res)
     return _Combine.apply(y2, probs, ws, route)

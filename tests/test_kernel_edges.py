@@ -106,3 +106,26 @@ def test_vector_decay_chunk_edges(D, T):
     got = run(lambda q, k, v, g, S: ops.lsm_vector(q, k, v, g, None, S, None, 64), ins, [go, gS])
     want = run(lambda q, k, v, g, S: RL.recurrent_lsm(q, k, v, gk=g, initial_state=S), [t.float() for t in ins], [go.float(), gS])
     check(got, want, ["o", "S", "dq", "dk", "dv", "dg", "dS0"])
+
+
+@pytest.mark.parametrize("h,f", [(128, 8), (200, 120), (256, 136), (512, 264)])
+@pytest.mark.parametrize("counts", [[512, 0, 256], [0, 0, 768], [256, 1024, 0]])
+def test_expert_mlp_epilogues(h, f, counts):
+    """The activation and its gradient as epilogues of the grouped products: widths that end inside a tile, experts without rows."""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    E, rows = len(counts), sum(counts)
+    offs = torch.tensor([0] + counts, device="cuda").cumsum(0).int()
+    assert all(c % gemm.ROW_ALIGN == 0 for c in counts)
+    x, w1, w2, go = rand(rows, h, scale=1), rand(E, h, 2 * f, scale=h ** -0.5), rand(E, f, h, scale=f ** -0.5), rand(rows, h, scale=1)
+
+    def plain(x, w1, w2):
+        ys = []
+        for e, xe in enumerate(x.split(counts)):
+            gate, up = (xe @ w1[e]).chunk(2, dim=-1)
+            ys.append((torch.nn.functional.silu(gate) * up) @ w2[e])
+        return torch.cat(ys)
+    got = run(lambda x, w1, w2: gemm.expert_mlp(x, w1, w2, offs), [x, w1, w2], [go])
+    gemm.check_error()
+    want = run(plain, [t.float() for t in (x, w1, w2)], [go.float()])
+    check(got, want, ["y", "dx", "dw1", "dw2"])
