@@ -25,25 +25,13 @@
 //   S  <- e^{b_C} S + (K .* e^{b_C - b_j})^T V                 (D x D)
 // Tensor-core work uses mma.sync m16n8k16 on ldmatrix fragments; the fp32 state lives in registers
 // across the whole group, with a bf16 copy in shared memory as the B operand of Q S.
+#include "lsm_scalar.cuh"
 #include "mma_utils.cuh"
 
 namespace lmoe {
 
 constexpr int CH = 64;             // chunk length
 constexpr int NTHREADS = 256;
-
-struct LsmArgs {
-    const bf16 *q, *k, *v, *d_o;   // d_o: contiguous [B,T,H,D] (backward only)
-    int64_t qs_b, qs_t, qs_h, ks_b, ks_t, ks_h, vs_b, vs_t, vs_h;
-    bf16 *o, *dq, *dk, *dv;        // outputs (o contiguous; dq/dk/dv with the strides below)
-    int64_t dqs_b, dqs_t, dqs_h, dks_b, dks_t, dks_h, dvs_b, dvs_t, dvs_h;
-    const float* g;                // gmode 1: [H]; gmode 2: [B,T,H]
-    int gmode;
-    float scale;
-    int B, T, H, G, cpg;           // G groups of cpg chunks
-    float* states;                 // [B,H,G,D,D]
-    float* gdecay;                 // [B,H,G] total log decay per group (gmode 2)
-};
 
 template <int D> struct Cfg {
     static constexpr int LD = D + 8;               // padded row stride of D-wide tiles
@@ -481,6 +469,7 @@ LMOE_API int lmoe_lsm_scalar_launch(int which, int D, const LsmArgs* ap, cudaStr
         if (rc) return rc;                                     \
         KERNEL<<<grid, NTHREADS, SMEM, st>>>(a);               \
     } while (0)
+    if (a.chunk != 64) return D == 128 && a.chunk == 128 ? lst::launch(which, a, st) : -2;
     if (D == 128) {
         if (which == 0) LAUNCH((state_scan_kernel<128, 0>), smem_scan<128>());
         else if (which == 1) LAUNCH((state_scan_kernel<128, 1>), smem_scan<128>());

@@ -939,7 +939,7 @@ class _LsmArgs(ctypes.Structure):
                 [(n, ctypes.c_int64) for n in ("dqs_b", "dqs_t", "dqs_h", "dks_b", "dks_t", "dks_h", "dvs_b", "dvs_t", "dvs_h")] +
                 [("g", ctypes.c_void_p), ("gmode", ctypes.c_int), ("scale", ctypes.c_float)] +
                 [(n, ctypes.c_int) for n in ("B", "T", "H", "G", "cpg")] +
-                [("states", ctypes.c_void_p), ("gdecay", ctypes.c_void_p)])
+                [("states", ctypes.c_void_p), ("gdecay", ctypes.c_void_p), ("err", ctypes.c_void_p), ("chunk", ctypes.c_int)])
 
 
 def _inner_contig(t):
@@ -957,7 +957,43 @@ def lsm_groups(B, H, T):
     return G, cpg
 
 
-def _lsm_args(q, k, v, g, gmode, scale, B, T, H, G, cpg, states, gdecay, d_o=None, o=None, dq=None, dk=None, dv=None):
+def _scalar_chunk(B, T, H, D, g):
+    """Tokens per chunk: 128 (tensor-core kernels, csrc/lsm_scalar_tc.cu) or 64 (csrc/lsm_scalar.cu).
+
+    128 for 128-wide heads from eight chunks per SM on.  Forward and backward of 16 heads take 375 us in chunks of 64 and 212 in chunks
+    of 128 there (9472 tokens); 604 and 305 at 16384, 193 and 123 at 4096, 78 and 72 at 1024, 47 and 61 at 128.  Below the line the
+    gain is 2 % of a model's training step at most, and a change of rounding costs more than that: where a head decays within a few
+    tokens, single elements of a model's embedding gradient move by more than the tensor's root mean square between any two
+    roundings (both forms are equally far from 64-bit results).  Where decays are trained it stays at 64 as well: their gradient is
+    a sum over all later tokens of differences of bf16 products, in which the rounding of another chunking shows as 3 - 4 %."""
+    return 128 if D == 128 and B * H * T >= 8 * 128 * num_sms() and not (g is not None and g.requires_grad) else 64
+
+
+def _scalar_groups(B, H, T, chunk):
+    """``(groups, 64-token chunks per group)`` of the scalar-decay kernels.  In chunks of 128 tokens: the number of groups with
+    the fewest chunks in a row over all waves (one CTA per SM; a group costs about a chunk beside its own)."""
+    if chunk != 128:
+        return lsm_groups(B, H, T)
+    n, sms, BH = (T + 127) // 128, num_sms(), max(B * H, 1)
+    best = None
+    for want in range(1, max(1, min(n, 4 * sms // BH)) + 1):
+        cpg = -(-n // want)
+        G = -(-n // cpg)
+        cost = -(-BH * G // sms) * (cpg + 1)
+        if best is None or cost < best[0]:
+            best = (cost, G, cpg)
+    return best[1], 2 * best[2]
+
+
+def _tma_view(t):
+    """As :func:`_inner_contig`, for kernels that read through tensor maps: no repeated (stride zero) dimensions either."""
+    if any(s <= 0 for s, n in zip(t.stride(), t.shape) if n > 1):
+        return t.contiguous()
+    return _inner_contig(t)
+
+
+def _lsm_args(q, k, v, g, gmode, scale, B, T, H, G, cpg, states, gdecay, chunk, d_o=None, o=None, dq=None, dk=None, dv=None):
+    from . import gemm
     a = _LsmArgs()
     a.q, a.k, a.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
     a.d_o = 0 if d_o is None else d_o.data_ptr()
@@ -974,6 +1010,7 @@ def _lsm_args(q, k, v, g, gmode, scale, B, T, H, G, cpg, states, gdecay, d_o=Non
     a.B, a.T, a.H, a.G, a.cpg = B, T, H, G, cpg
     a.states = states.data_ptr()
     a.gdecay = 0 if gdecay is None else gdecay.data_ptr()
+    a.err, a.chunk = gemm._err(q.device).data_ptr(), chunk
     return a
 
 
@@ -995,16 +1032,18 @@ class _LsmScalar(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, scale, init):
         B, T, H, D = q.shape
-        q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
+        chunk = _scalar_chunk(B, T, H, D, g)
+        fix = _tma_view if chunk == 128 else _inner_contig
+        q, k, v = fix(q), fix(k), fix(v)
         gmode = 0 if g is None else (1 if g.dim() == 1 else 2)
         gf = None if g is None else g.float().contiguous()
-        G, cpg = lsm_groups(B, H, T)
+        G, cpg = _scalar_groups(B, H, T, chunk)
         states = torch.empty(B, H, G, D, D, dtype=torch.float32, device=q.device)
         gdecay = torch.empty(B, H, G, dtype=torch.float32, device=q.device) if gmode == 2 else None
         o = torch.empty(B, T, H, D, dtype=q.dtype, device=q.device)
         final = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device)
         seed = None if init is None else init.float().contiguous()
-        a = _lsm_args(q, k, v, gf, gmode, scale, B, T, H, G, cpg, states, gdecay, o=o)
+        a = _lsm_args(q, k, v, gf, gmode, scale, B, T, H, G, cpg, states, gdecay, chunk, o=o)
         _lsm_launch(0, D, a)
         lasp = _LASP_CTX if init is None else None
         if lasp is not None:       # sequence split over ranks: exchange fused into the combine kernel
@@ -1014,8 +1053,9 @@ class _LsmScalar(torch.autograd.Function):
             _lsm_combine(0, states, gdecay, gf if gmode == 1 else None, seed, final, B * H, H, G, cpg, T, D)
         _lsm_launch(2, D, a)
         ctx.lasp = lasp
+        ctx.set_materialize_grads(False)                 # no zeros for an output without a gradient (mostly the final state)
         ctx.save_for_backward(q, k, v, gf, states, gdecay, final)
-        ctx.scale, ctx.gmode, ctx.grid, ctx.has_init = scale, gmode, (G, cpg), init is not None
+        ctx.scale, ctx.gmode, ctx.grid, ctx.has_init = scale, gmode, (G, cpg, chunk), init is not None
         ctx.g_dtype = None if g is None else g.dtype
         return o, final
 
@@ -1023,8 +1063,8 @@ class _LsmScalar(torch.autograd.Function):
     def backward(ctx, d_o, dfinal):
         q, k, v, gf, states, gdecay, final = ctx.saved_tensors
         B, T, H, D = q.shape
-        G, cpg = ctx.grid
-        d_o = d_o.contiguous()
+        G, cpg, chunk = ctx.grid
+        d_o = torch.zeros(B, T, H, D, dtype=q.dtype, device=q.device) if d_o is None else d_o.contiguous()
         if d_o.dtype != q.dtype:
             d_o = d_o.to(q.dtype)
         # dq | dk | dv are written straight into one [B,T,H,3D] buffer: when q,k,v were views of a fused
@@ -1034,10 +1074,10 @@ class _LsmScalar(torch.autograd.Function):
         dstates = torch.empty_like(states)
         dinit = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device) if ctx.has_init else None
         # forward-direction sweep: dq (entering states of every group are still in `states`)
-        a = _lsm_args(q, k, v, gf, ctx.gmode, ctx.scale, B, T, H, G, cpg, states, gdecay, d_o=d_o, dq=dq)
+        a = _lsm_args(q, k, v, gf, ctx.gmode, ctx.scale, B, T, H, G, cpg, states, gdecay, chunk, d_o=d_o, dq=dq)
         _lsm_launch(3, D, a)
         # reverse-direction: group summaries of dS, suffix combine, dk/dv sweep
-        a2 = _lsm_args(q, k, v, gf, ctx.gmode, ctx.scale, B, T, H, G, cpg, dstates, None, d_o=d_o, dk=dk, dv=dv)
+        a2 = _lsm_args(q, k, v, gf, ctx.gmode, ctx.scale, B, T, H, G, cpg, dstates, None, chunk, d_o=d_o, dk=dk, dv=dv)
         _lsm_launch(1, D, a2)
         seed = None if dfinal is None else dfinal.float().contiguous()
         if ctx.lasp is not None:

@@ -1,0 +1,29 @@
+"""Rules that pick a kernel variant, over all that they accept (no GPU needed)."""
+import torch
+
+from linear_moe_b200.ops import cuda as K
+
+
+def test_scalar_decay_chunk_rule(monkeypatch):
+    monkeypatch.setattr(K, "num_sms", lambda: 148)
+    g, line = torch.zeros(2, 8, 3), 8 * 128 * 148
+    assert K._scalar_chunk(1, line, 1, 128, None) == K._scalar_chunk(4, -(-line // 16), 4, 128, g) == 128
+    assert K._scalar_chunk(1, line - 1, 1, 128, None) == K._scalar_chunk(1, line, 1, 64, None) == 64
+    assert K._scalar_chunk(1, line, 1, 128, g.clone().requires_grad_(True)) == 64
+    for chunk in (64, 128):                                     # every token in exactly one group, no group empty
+        for BH in (1, 3, 16, 148, 1000):
+            for T in list(range(1, 400)) + [4096, 16384, 100003]:
+                G, cpg = K._scalar_groups(1, BH, T, chunk)
+                assert cpg * 64 % chunk == 0 and (G - 1) * cpg * 64 < T <= G * cpg * 64
+
+
+def test_tensor_map_views():
+    """Views that tensor maps cannot describe (repeated rows, strided columns, odd strides) are copied, the others stay."""
+    x = torch.zeros(2, 5, 3, 128, dtype=torch.bfloat16)
+    wide = torch.zeros(2, 5, 3, 3 * 128, dtype=torch.bfloat16)
+    for t in (x, wide[..., 128:256], x.transpose(1, 2).contiguous().transpose(1, 2), x[:, :, :1], x[:1], x[:, :1].expand(-1, 1, -1, -1)):
+        assert K._tma_view(t) is t
+    odd = torch.zeros(2, 5, 3, 129, dtype=torch.bfloat16)[..., :128]
+    for t in (x[:, :, :1].expand(-1, -1, 3, -1), x[:1].expand(2, -1, -1, -1), x.transpose(2, 3), odd):
+        c = K._tma_view(t)
+        assert c.is_contiguous() and torch.equal(c, t)

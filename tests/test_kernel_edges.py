@@ -129,3 +129,39 @@ def test_expert_mlp_epilogues(h, f, counts):
     gemm.check_error()
     want = run(plain, [t.float() for t in (x, w1, w2)], [go.float()])
     check(got, want, ["y", "dx", "dw1", "dw2"])
+
+
+@pytest.mark.parametrize("T", [2, 127, 128, 129, 400])
+@pytest.mark.parametrize("decay", ["none", "head", "token"])
+@pytest.mark.parametrize("layout", ["fused", "heads first", "shared keys"])
+def test_scalar_decay_wide_chunks(T, decay, layout, monkeypatch):
+    """128-wide heads in chunks of 128 tokens (decays that are not trained), over the strides that callers come with."""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    B, H, D = 2, 3, 128
+    g = {"none": None, "head": -torch.tensor([0.002, 0.1, 1.5], device="cuda"), "token": -0.3 * torch.rand(B, T, H, device="cuda")}[decay]
+    q, k, v = rand(B, T, H, 3 * D).split(D, dim=-1)
+    if layout == "heads first":
+        q, k, v = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v))
+    elif layout == "shared keys":
+        k, v = k[:, :, :1].expand(-1, -1, H, -1), v[:, :1, :1].expand(-1, T, H, -1)
+    S0, gS = 0.3 * torch.randn(B, H, D, D, device="cuda"), 0.1 * torch.randn(B, H, D, D, device="cuda")
+    go = rand(B, T, H, D, scale=1)
+    monkeypatch.setattr(K, "_scalar_chunk", lambda *a: 128)       # the rule takes longer inputs only
+
+    def kernel(q, k, v, S):
+        return ops.lsm_scalar(q, k, v, g, None, S, 64)
+
+    def ref(q, k, v, S):
+        gt = None if g is None else (g.expand(B, T, H) if g.dim() == 1 else g)
+        return RL.recurrent_lsm(q, k, v, g=gt, initial_state=S)
+    got, want = [], []
+    for f, ins, res in ((kernel, (q, k, v, S0), got), (ref, [t.float() for t in (q, k, v, S0)], want)):
+        ins = [t.detach().requires_grad_(True) for t in ins]
+        out = f(*ins)
+        res += [list(out), list(torch.autograd.grad(out, ins, [go.to(out[0].dtype), gS]))]
+    gemm.check_error()
+    check(got, want, ["o", "S", "dq", "dk", "dv", "dS0"])
+    with torch.no_grad():
+        o, S = kernel(q, k, v, S0)
+    assert torch.equal(o, got[0][0]) and torch.equal(S, got[0][1])
