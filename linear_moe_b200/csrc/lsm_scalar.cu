@@ -499,3 +499,13 @@ LMOE_API int lmoe_lsm_scalar_combine(int rev, float* states, const float* gdecay
     else combine_kernel<0><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
     return (int)cudaGetLastError();
 }
+
+// Summaries, combine and outputs of a forward call: the three launches behind one host call.  gconst: the constant log decays [H] of
+// gmode 1, else null; seed: the initial state or null.
+LMOE_API int lmoe_lsm_scalar_forward(int D, const LsmArgs* ap, const float* gconst, const float* seed, float* final_out, cudaStream_t st) {
+    int rc = lmoe_lsm_scalar_launch(0, D, ap, st);
+    if (rc) return rc;
+    rc = lmoe_lsm_scalar_combine(0, ap->states, ap->gdecay, gconst, seed, final_out, ap->B * ap->H, ap->H, ap->G, ap->cpg, ap->T, D, st);
+    if (rc) return rc;
+    return lmoe_lsm_scalar_launch(2, D, ap, st);
+}

@@ -534,6 +534,15 @@ LMOE_API int lmoe_gla_combine(int rev, float* states, const float* gdecay, const
     return (int)cudaGetLastError();
 }
 
+// Summaries, combine and outputs of a forward call: the three launches behind one host call.
+LMOE_API int lmoe_gla_forward(int D, const GlaArgs* ap, const float* seed, float* final_out, cudaStream_t st) {
+    int rc = lmoe_gla_launch(0, D, ap, st);
+    if (rc) return rc;
+    rc = lmoe_gla_combine(0, ap->states, ap->gdecay, seed, final_out, ap->B * ap->H, ap->G, D, st);
+    if (rc) return rc;
+    return lmoe_gla_launch(2, D, ap, st);
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Gradient of the vector log-gates: dg[b,t,h,d] = sum_{i >= t} (q . dq - k . dk)[b,i,h,d]  (reverse cumulative sum
 // over time per channel).  Two launches over segments of 256 tokens: per-segment channel sums, then every segment

@@ -71,6 +71,10 @@ def _p(t: Optional[torch.Tensor]):
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
 _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
@@ -994,24 +998,12 @@ def _tma_view(t):
 
 def _lsm_args(q, k, v, g, gmode, scale, B, T, H, G, cpg, states, gdecay, chunk, d_o=None, o=None, dq=None, dk=None, dv=None):
     from . import gemm
-    a = _LsmArgs()
-    a.q, a.k, a.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    a.d_o = 0 if d_o is None else d_o.data_ptr()
-    a.qs_b, a.qs_t, a.qs_h = q.stride(0), q.stride(1), q.stride(2)
-    a.ks_b, a.ks_t, a.ks_h = k.stride(0), k.stride(1), k.stride(2)
-    a.vs_b, a.vs_t, a.vs_h = v.stride(0), v.stride(1), v.stride(2)
-    a.o = 0 if o is None else o.data_ptr()
-    for name, t in (("dq", dq), ("dk", dk), ("dv", dv)):
-        setattr(a, name, 0 if t is None else t.data_ptr())
-        if t is not None:
-            setattr(a, name + "s_b", t.stride(0)), setattr(a, name + "s_t", t.stride(1)), setattr(a, name + "s_h", t.stride(2))
-    a.g = 0 if g is None else g.data_ptr()
-    a.gmode, a.scale = gmode, float(scale)
-    a.B, a.T, a.H, a.G, a.cpg = B, T, H, G, cpg
-    a.states = states.data_ptr()
-    a.gdecay = 0 if gdecay is None else gdecay.data_ptr()
-    a.err, a.chunk = gemm._err(q.device).data_ptr(), chunk
-    return a
+    grads = []
+    for t in (dq, dk, dv):
+        grads += (0, 0, 0) if t is None else t.stride()[:3]
+    return _LsmArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(d_o), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
+                    _ptr(o), _ptr(dq), _ptr(dk), _ptr(dv), *grads, _ptr(g), gmode, float(scale), B, T, H, G, cpg,
+                    states.data_ptr(), _ptr(gdecay), gemm._err(q.device).data_ptr(), chunk)
 
 
 def _lsm_launch(which, D, args):
@@ -1026,36 +1018,51 @@ def _lsm_combine(rev, states, gdecay, gconst, seed, final_out, BH, H, G, cpg, T,
 _LASP_CTX = None          # set by parallel.fused_comm.lasp2_scalar while a sequence-parallel call is running
 
 
+def _plain_call() -> bool:
+    """Is this call outside everything that looks into an autograd function (gradients, forward-mode AD, functional transforms,
+    tracing)?  Then its forward pass is called directly: a prompt of 777 tokens, 8 heads of 64, whose kernels take 13 us, took
+    70 us with the function's bookkeeping, argument structs filled field by field and three host calls, and takes 40 without."""
+    return not (torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None)
+
+
+def _scalar_forward(q, k, v, g, scale, init):
+    """Returns the output, the final state and what the backward pass needs: (tensors, gmode, (groups, chunks, tokens of a
+    chunk), exchange)."""
+    B, T, H, D = q.shape
+    chunk = _scalar_chunk(B, T, H, D, g)
+    fix = _tma_view if chunk == 128 else _inner_contig
+    q, k, v = fix(q), fix(k), fix(v)
+    gmode = 0 if g is None else (1 if g.dim() == 1 else 2)
+    gf = None if g is None else g.float().contiguous()
+    G, cpg = _scalar_groups(B, H, T, chunk)
+    f32, dev = torch.float32, q.device
+    states = torch.empty(B, H, G, D, D, dtype=f32, device=dev)
+    gdecay = torch.empty(B, H, G, dtype=f32, device=dev) if gmode == 2 else None
+    o = torch.empty(B, T, H, D, dtype=q.dtype, device=dev)
+    final = torch.empty(B, H, D, D, dtype=f32, device=dev)
+    a = _lsm_args(q, k, v, gf, gmode, scale, B, T, H, G, cpg, states, gdecay, chunk, o=o)
+    lasp = _LASP_CTX if init is None else None
+    if lasp is not None:       # sequence split over ranks: exchange fused into the combine kernel
+        _lsm_launch(0, D, a)
+        lasp.combine(0, states, gf if gmode == 1 else None, final, B * H, H, G, cpg, T, D,
+                     gdecay=gdecay, dmode=1 if gmode == 2 else 0)
+        _lsm_launch(2, D, a)
+    else:
+        seed = None if init is None else init.float().contiguous()
+        _check(lib().lmoe_lsm_scalar_forward(D, ctypes.byref(a), _p(gf if gmode == 1 else None), _p(seed), _p(final), _st()), "lsm_scalar", 3)
+    return o, final, ((q, k, v, gf, states, gdecay, final), gmode, (G, cpg, chunk), lasp)
+
+
 class _LsmScalar(torch.autograd.Function):
     """o, S_T = scalar-decay linear attention.  q,k,v bf16 [B,T,H,D]; g None | [H] | [B,T,H] fp32."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, scale, init):
-        B, T, H, D = q.shape
-        chunk = _scalar_chunk(B, T, H, D, g)
-        fix = _tma_view if chunk == 128 else _inner_contig
-        q, k, v = fix(q), fix(k), fix(v)
-        gmode = 0 if g is None else (1 if g.dim() == 1 else 2)
-        gf = None if g is None else g.float().contiguous()
-        G, cpg = _scalar_groups(B, H, T, chunk)
-        states = torch.empty(B, H, G, D, D, dtype=torch.float32, device=q.device)
-        gdecay = torch.empty(B, H, G, dtype=torch.float32, device=q.device) if gmode == 2 else None
-        o = torch.empty(B, T, H, D, dtype=q.dtype, device=q.device)
-        final = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device)
-        seed = None if init is None else init.float().contiguous()
-        a = _lsm_args(q, k, v, gf, gmode, scale, B, T, H, G, cpg, states, gdecay, chunk, o=o)
-        _lsm_launch(0, D, a)
-        lasp = _LASP_CTX if init is None else None
-        if lasp is not None:       # sequence split over ranks: exchange fused into the combine kernel
-            lasp.combine(0, states, gf if gmode == 1 else None, final, B * H, H, G, cpg, T, D,
-                         gdecay=gdecay, dmode=1 if gmode == 2 else 0)
-        else:
-            _lsm_combine(0, states, gdecay, gf if gmode == 1 else None, seed, final, B * H, H, G, cpg, T, D)
-        _lsm_launch(2, D, a)
-        ctx.lasp = lasp
+        o, final, (saved, ctx.gmode, ctx.grid, ctx.lasp) = _scalar_forward(q, k, v, g, scale, init)
         ctx.set_materialize_grads(False)                 # no zeros for an output without a gradient (mostly the final state)
-        ctx.save_for_backward(q, k, v, gf, states, gdecay, final)
-        ctx.scale, ctx.gmode, ctx.grid, ctx.has_init = scale, gmode, (G, cpg, chunk), init is not None
+        ctx.save_for_backward(*saved)
+        ctx.scale, ctx.has_init = scale, init is not None
         ctx.g_dtype = None if g is None else g.dtype
         return o, final
 
@@ -1168,6 +1175,8 @@ def lsm_scalar(q, k, v, g, scale, initial_state, chunk_size):
     if q.shape[1] == 1 and _LASP_CTX is None and not (torch.is_grad_enabled() and
                                                       any(t.requires_grad for t in (q, k, v) if t is not None)):
         return _lsm_step(q, k, v, g, None, scale, initial_state)
+    if _plain_call():
+        return _scalar_forward(q, k, v, g, scale, initial_state)[:2]
     base = _fused_base(q, k, v)
     if base is not None:
         return _LsmScalarFused.apply(base, g, scale, initial_state)
@@ -1204,22 +1213,12 @@ class _GlaArgs(ctypes.Structure):
 
 
 def _gla_args(q, k, v, gk, scale, B, T, H, G, cpg, states, gdecay, d_o=None, o=None, dq=None, dk=None, dv=None):
-    a = _GlaArgs()
-    a.q, a.k, a.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    a.d_o = 0 if d_o is None else d_o.data_ptr()
-    a.qs_b, a.qs_t, a.qs_h = q.stride(0), q.stride(1), q.stride(2)
-    a.ks_b, a.ks_t, a.ks_h = k.stride(0), k.stride(1), k.stride(2)
-    a.vs_b, a.vs_t, a.vs_h = v.stride(0), v.stride(1), v.stride(2)
-    a.o = 0 if o is None else o.data_ptr()
-    for name, t in (("dq", dq), ("dk", dk), ("dv", dv)):
-        setattr(a, name, 0 if t is None else t.data_ptr())
-        if t is not None:
-            setattr(a, name + "s_b", t.stride(0)), setattr(a, name + "s_t", t.stride(1)), setattr(a, name + "s_h", t.stride(2))
-    a.gk, a.scale = gk.data_ptr(), float(scale)
-    a.B, a.T, a.H, a.G, a.cpg = B, T, H, G, cpg
-    a.states = states.data_ptr()
-    a.gdecay = 0 if gdecay is None else gdecay.data_ptr()
-    return a
+    grads = []
+    for t in (dq, dk, dv):
+        grads += (0, 0, 0) if t is None else t.stride()[:3]
+    return _GlaArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(d_o), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
+                    _ptr(o), _ptr(dq), _ptr(dk), _ptr(dv), *grads, gk.data_ptr(), float(scale), B, T, H, G, cpg,
+                    states.data_ptr(), _ptr(gdecay))
 
 
 def _gla_launch(which, D, args):
@@ -1231,32 +1230,38 @@ def _gla_combine(rev, states, gdecay, seed, final_out, BH, G, D):
                                   _st()), "gla_combine")
 
 
+def _vector_forward(q, k, v, gk, scale, init):
+    """Returns the output, the final state and what the backward pass needs: (tensors, (groups, chunks), exchange)."""
+    B, T, H, D = q.shape
+    q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
+    gf = gk.float().contiguous()
+    G, cpg = lsm_groups(B, H, T)
+    f32, dev = torch.float32, q.device
+    states = torch.empty(B, H, G, D, D, dtype=f32, device=dev)
+    gdecay = torch.empty(B, H, G, D, dtype=f32, device=dev)
+    o = torch.empty(B, T, H, D, dtype=q.dtype, device=dev)
+    final = torch.empty(B, H, D, D, dtype=f32, device=dev)
+    a = _gla_args(q, k, v, gf, scale, B, T, H, G, cpg, states, gdecay, o=o)
+    lasp = _LASP_CTX if init is None else None
+    if lasp is not None:       # sequence split over ranks: exchange fused into the combine kernel
+        _gla_launch(0, D, a)
+        lasp.combine(0, states, None, final, B * H, H, G, cpg, T, D, gdecay=gdecay, dmode=2)
+        _gla_launch(2, D, a)
+    else:
+        seed = None if init is None else init.float().contiguous()
+        _check(lib().lmoe_gla_forward(D, ctypes.byref(a), _p(seed), _p(final), _st()), "gla", 3)
+    return o, final, ((q, k, v, gf, states, gdecay, final), (G, cpg), lasp)
+
+
 class _LsmVector(torch.autograd.Function):
     """o, S_T = linear attention with a log decay per key channel.  q,k,v bf16 [B,T,H,D]; gk [B,T,H,D]."""
 
     @staticmethod
     def forward(ctx, q, k, v, gk, scale, init):
-        B, T, H, D = q.shape
-        q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
-        gf = gk.float().contiguous()
-        G, cpg = lsm_groups(B, H, T)
-        states = torch.empty(B, H, G, D, D, dtype=torch.float32, device=q.device)
-        gdecay = torch.empty(B, H, G, D, dtype=torch.float32, device=q.device)
-        o = torch.empty(B, T, H, D, dtype=q.dtype, device=q.device)
-        final = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device)
-        seed = None if init is None else init.float().contiguous()
-        a = _gla_args(q, k, v, gf, scale, B, T, H, G, cpg, states, gdecay, o=o)
-        _gla_launch(0, D, a)
-        lasp = _LASP_CTX if init is None else None
-        if lasp is not None:       # sequence split over ranks: exchange fused into the combine kernel
-            lasp.combine(0, states, None, final, B * H, H, G, cpg, T, D, gdecay=gdecay, dmode=2)
-        else:
-            _gla_combine(0, states, gdecay, seed, final, B * H, G, D)
-        _gla_launch(2, D, a)
-        ctx.lasp = lasp
+        o, final, (saved, ctx.grid, ctx.lasp) = _vector_forward(q, k, v, gk, scale, init)
         ctx.set_materialize_grads(False)                 # no zeros for an output without a gradient (mostly the final state)
-        ctx.save_for_backward(q, k, v, gf, states, gdecay, final)
-        ctx.scale, ctx.grid, ctx.has_init, ctx.g_dtype = scale, (G, cpg), init is not None, gk.dtype
+        ctx.save_for_backward(*saved)
+        ctx.scale, ctx.has_init, ctx.g_dtype = scale, init is not None, gk.dtype
         return o, final
 
     @staticmethod
@@ -1384,6 +1389,8 @@ def lsm_vector(q, k, v, gk, scale, initial_state, bonus, chunk_size):
         return _lsm_vector_bonus(q, k, v, gk, scale, initial_state, bonus, chunk_size)
     if q.shape[1] == 1 and not (torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v, gk))):
         return _lsm_step(q, k, v, None, gk, scale, initial_state)
+    if _plain_call():
+        return _vector_forward(q, k, v, gk, scale, initial_state)[:2]
     base = _fused_base(q, k, v)
     if base is not None:
         return _LsmVectorFused.apply(base, gk, scale, initial_state)
@@ -1473,15 +1480,9 @@ def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64, inverse=None):
     gamma = torch.empty(B, H, N, dtype=torch.float32, device=dev)
     bt = beta.float().contiguous()
     gt = None if g is None else g.float().contiguous()
-    a = _DeltaPrepArgs()
-    a.q, a.k, a.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    a.qs_b, a.qs_t, a.qs_h = q.stride(0), q.stride(1), q.stride(2)
-    a.ks_b, a.ks_t, a.ks_h = k.stride(0), k.stride(1), k.stride(2)
-    a.vs_b, a.vs_t, a.vs_h = v.stride(0), v.stride(1), v.stride(2)
-    a.beta, a.g = bt.data_ptr(), 0 if gt is None else gt.data_ptr()
-    a.W, a.U, a.Qd, a.Kd, a.A, a.gamma = (t.data_ptr() for t in (W, U, Qd, Kd, A, gamma))
-    a.B, a.T, a.H, a.N, a.scale = B, T, H, N, float(scale)
-    a.Tinv = 0 if inverse is None else inverse.data_ptr()
+    a = _DeltaPrepArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3], bt.data_ptr(), _ptr(gt),
+                       W.data_ptr(), U.data_ptr(), Qd.data_ptr(), Kd.data_ptr(), A.data_ptr(), gamma.data_ptr(), B, T, H, N, float(scale),
+                       _ptr(inverse))
     _check(lib().lmoe_delta_prepare(_i32(D), ctypes.byref(a), _st()), "delta_prepare")
     return W, U, Qd, Kd, A, gamma
 
@@ -1506,17 +1507,10 @@ def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, out=None, keep=True):
     Sn = torch.empty(B, H, N, dk, dv, dtype=bf, device=dev) if keep else None
     Sf = torch.empty(B, H, dk, dv, dtype=torch.float32, device=dev)
     s0 = None if S0 is None else S0.float().contiguous()
-    a = _DeltaArgs()
-    a.W, a.U, a.Qd, a.Kd, a.A, a.gamma = (t.data_ptr() for t in (W, U, Qd, Kd, A, gamma))
-    a.S0 = 0 if s0 is None else s0.data_ptr()
-    a.Sfinal = Sf.data_ptr()
-    if keep:
-        a.Vn, a.Sn = Vn.data_ptr(), Sn.data_ptr()
-    if out is not None:
-        a.O, a.T = out.data_ptr(), out.shape[1]
-        a.os_b, a.os_t, a.os_h = out.stride(0), out.stride(1), out.stride(2)
-    a.N, a.dv, a.H, a.ldw, a.lda = N, dv, H, W.stride(3), A.stride(3)
-    a.err = gemm._err(dev).data_ptr()
+    o_strides, T = ((0, 0, 0), 0) if out is None else (out.stride()[:3], out.shape[1])
+    a = _DeltaArgs(W.data_ptr(), U.data_ptr(), Qd.data_ptr(), Kd.data_ptr(), A.data_ptr(), gamma.data_ptr(), _ptr(s0), 0, 0, _ptr(out),
+                   _ptr(Vn), _ptr(Sn), Sf.data_ptr(), 0, 0, 0, *o_strides, 0, 0, 0, N, dv, T, H, W.stride(3), A.stride(3),
+                   gemm._err(dev).data_ptr())
     _check(lib().lmoe_delta_scan(_i32(0), _i32(dk), _i32(B * H), ctypes.byref(a), _st()), "delta_scan_fwd")
     return Vn, Sn, Sf
 
@@ -1611,6 +1605,11 @@ def _delta_prepare_bwd_kernel(q, k, v, beta, g, scale, Sn, dSn, Vn, dVn, dO, Tin
     return dq, dk, dv, dbeta, dg
 
 
+def _delta_tile_kernels(q, k, v) -> bool:
+    return (q.dtype == k.dtype == v.dtype == torch.bfloat16 and v.shape[-1] == q.shape[-1]
+            and os.environ.get("LMOE_DELTA_PREP_KERNEL", "1") != "0")
+
+
 class _DeltaRuleScan(torch.autograd.Function):
     """(Gated) delta rule on the kernels of ``csrc/lsm_delta.cu``.  Forward: the chunk-parallel WY / UT tile kernel, then the
     scan kernel.  Only the inputs are kept.  Backward (bf16, equal key / value widths): tiles and forward scan again, the
@@ -1622,8 +1621,7 @@ class _DeltaRuleScan(torch.autograd.Function):
         B, T, H, dk = q.shape
         scale = dk ** -0.5 if scale is None else scale
         with torch.no_grad(), _tf32():
-            ctx.kernel_tiles = (q.dtype == k.dtype == v.dtype == torch.bfloat16 and v.shape[-1] == dk
-                                and os.environ.get("LMOE_DELTA_PREP_KERNEL", "1") != "0")
+            ctx.kernel_tiles = _delta_tile_kernels(q, k, v)
             if ctx.kernel_tiles:
                 tiles = _delta_prepare_kernel(q, k, v, beta, g, scale)
             else:
@@ -1721,6 +1719,9 @@ def lsm_delta(q, k, v, beta, g, scale, initial_state, chunk_size):
             and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, beta, g)))):
         return _lsm_delta_step(q, k, v, beta, g, D ** -0.5 if scale is None else scale, initial_state)
     if q.is_cuda and D in (64, 128) and k.shape[-1] == D and v.shape[-1] % 32 == 0 and os.environ.get("LMOE_DELTA_KERNEL", "1") != "0":
+        if _plain_call() and _delta_tile_kernels(q, k, v):
+            o = torch.empty(*q.shape[:3], D, dtype=q.dtype, device=q.device)
+            return o, _delta_scan_fwd(*_delta_prepare_kernel(q, k, v, beta, g, D ** -0.5 if scale is None else scale), initial_state, o, keep=False)[2]
         return _DeltaRuleScan.apply(q, k, v, beta, g, initial_state, scale, chunk_size)
     return _DeltaRuleTorch.apply(q, k, v, beta, g, initial_state, scale, chunk_size)
 

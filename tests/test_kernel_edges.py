@@ -165,3 +165,30 @@ def test_scalar_decay_wide_chunks(T, decay, layout, monkeypatch):
     with torch.no_grad():
         o, S = kernel(q, k, v, S0)
     assert torch.equal(o, got[0][0]) and torch.equal(S, got[0][1])
+
+
+@pytest.mark.parametrize("kind,D", [("scalar", 64), ("scalar", 128), ("vector", 64), ("vector", 128), ("delta", 128)])
+@pytest.mark.parametrize("T", [2, 200])
+def test_forward_in_one_host_call(kind, D, T):
+    """Without gradients the forward pass goes past the autograd function: same bits, and not inside a transform."""
+    torch.manual_seed(0)
+    B, H = 2, 3
+    q, k, v = rand(B, T, H, 3 * D).split(D, dim=-1)
+    g = -0.3 * torch.rand((B, T, H, D) if kind == "vector" else (B, T, H), device="cuda")
+    S0 = 0.3 * torch.randn(B, H, D, D, device="cuda")
+    f = {"scalar": lambda q: ops.lsm_scalar(q, k, v, g, None, S0, 64), "vector": lambda q: ops.lsm_vector(q, k, v, g, None, S0, None, 64),
+         "delta": lambda q: ops.lsm_delta(q, k, v, -g, g, None, S0, 64)}[kind]
+    want = f(q.detach().requires_grad_(True))
+    with torch.no_grad():
+        assert K._plain_call()
+        got = f(q)
+        with torch.autograd.forward_ad.dual_level():
+            assert not K._plain_call()
+        torch.func.vmap(lambda x: (x, assert_not_plain())[0])(torch.zeros(2))
+        torch.jit.trace(lambda x: (x + 1, assert_not_plain())[0], torch.zeros(2), check_trace=False)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert not K._plain_call()
+
+
+def assert_not_plain():
+    assert not K._plain_call()
