@@ -48,13 +48,13 @@ struct Args {
     int* err;                          // error word of the bounded waits
 };
 
-// Both walks are chains over the chunks, bound by the latency of a step: two products with a barrier behind each.  Eight warps
-// share a step's tiles, everything that does not depend on the state is taken off the chain (the outputs by four warps beside
-// the other four's pseudo values; Qd^T dO ahead of the barrier), and the next chunk's tiles arrive during the step.
-// The tile kernel writes its tiles with the padded rows they have in shared memory, so that a tile is one bulk copy of one thread: as 16-byte
-// copies of all threads the issue alone took 2000 of a step's 4100 cycles.  Dense tiles (built with torch ops) take that way still.
-// 2 x 4096 tokens, 16 heads of 128 (64 chunks, 128 CTAs): forward 142 -> 128 us, without outputs 107 -> 95, reverse 140 -> 116
-// (with four warps and everything on the chain: 169 and 150).
+// Both walks are chains over the chunks, bound by the latency of a step: two products with a barrier behind each.  Eight warps share the
+// products and a ninth brings the tiles, up to two chunks ahead.  The tile kernel writes them with the padded rows they have in shared memory, so
+// that a tile is one bulk copy; dense tiles (built with torch ops) and U or dO come 16 bytes at a time.  (As 16-byte copies of all threads the issue alone took 2000
+// of a step's 4100 cycles, and 400 as bulk copies of one of the working threads; with the outputs in four warps of their own the others
+// waited 600 cycles for the longest of them.)
+// 2 x 4096 tokens, 16 heads of 128 (64 chunks, 128 CTAs): forward 98 us, without outputs 83, reverse 96
+// (with four warps and everything on the chain: 169, 169 and 150).
 template <int DK> struct Cfg {
     static constexpr int LDK = DK + 8;
     static constexpr int LDC = C + 8;
@@ -63,57 +63,84 @@ template <int DK> struct Cfg {
     // a stage (bf16 elements): W, Kd: C x LDK; X (U or dO): C x LDV; Qd: C x LDK; A: C x LDC (the last two not where no output is wanted)
     static constexpr int QD = 2 * C * LDK + C * LDV, AQ = QD + C * LDK;
     static constexpr int FULL = AQ + C * LDC;
-    static constexpr size_t smem(bool out) { return (size_t)(2 * (out ? FULL : QD) + DK * LDV + 2 * C * LDV) * 2; }      // + state, Vn, O
+    // Stages: three where one CTA fills an SM's shared memory anyway, else two, and a second CTA fits.
+    static __host__ __device__ constexpr int stages(bool out) { return DK == 128 && out ? 3 : 2; }
+    static __host__ __device__ constexpr size_t smem(bool out) {                          // + two states, Vn, O
+        return (size_t)(stages(out) * (out ? FULL : QD) + 2 * DK * LDV + (out ? 2 : 1) * C * LDV) * 2;
+    }
 };
 
 __device__ __forceinline__ void bulk_copy(bf16* dst, const bf16* src, int elements, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(smem_u32(dst)), "l"(src), "r"(elements * 2), "r"(smem_u32(bar)) : "memory");
 }
-template <int DK> __device__ __forceinline__ bool padded(const Args& a) { return a.ldw == Cfg<DK>::LDK && a.lda == Cfg<DK>::LDC; }
-
-template <int DK, bool FULL>
-__device__ __forceinline__ void issue_chunk(bf16* st, const Args& a, const bf16* x, long long xs_t, int x_rows, long long bh, int n, uint64_t* bar) {
-    using F = Cfg<DK>;
-    const long long cn = bh * a.N + n;
-    if (padded<DK>(a)) {
-        if (threadIdx.x == 0) {
-            constexpr int TILE = C * F::LDK, TA = C * F::LDC;
-            tc::mbar_expect_tx(bar, (FULL ? 3 * TILE + TA : 2 * TILE) * 2);
-            bulk_copy(st, a.W + cn * TILE, TILE, bar);
-            bulk_copy(st + TILE, a.Kd + cn * TILE, TILE, bar);
-            if (FULL) {
-                bulk_copy(st + F::QD, a.Qd + cn * TILE, TILE, bar);
-                bulk_copy(st + F::AQ, a.A + cn * TA, TA, bar);
-            }
-        }
-        load_tile_async<C, DVS, F::LDV>(st + 2 * C * F::LDK, x + (long long)n * C * xs_t, xs_t, x_rows - n * C);
-        return;
-    }
-    load_tile_async<C, DK, F::LDK>(st, a.W + cn * C * DK, DK, C);
-    load_tile_async<C, DK, F::LDK>(st + C * F::LDK, a.Kd + cn * C * DK, DK, C);
-    load_tile_async<C, DVS, F::LDV>(st + 2 * C * F::LDK, x + (long long)n * C * xs_t, xs_t, x_rows - n * C);
-    if (FULL) {
-        load_tile_async<C, DK, F::LDK>(st + F::QD, a.Qd + cn * C * DK, DK, C);
-        load_tile_async<C, C, F::LDC>(st + F::AQ, a.A + cn * C * C, C, C);
+// a tile of C rows in shared memory (row stride LD) by one warp: one bulk copy by lane `which` if memory has the same rows, else 16 bytes per
+// copy; rows from `rows` on become zeros
+template <int COLS, int LD>
+__device__ __forceinline__ void warp_tile(bf16* dst, const bf16* src, long long ld_src, int rows, int lane) {
+#pragma unroll 8
+    for (int i = lane; i < C * (COLS / 8); i += 32) {
+        const int r = i / (COLS / 8), c = (i % (COLS / 8)) * 8;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     :: "r"(smem_u32(dst + r * LD + c)), "l"(src + (r < rows ? r : 0) * ld_src + c), "r"(r < rows ? 16 : 0) : "memory");
     }
 }
+template <int COLS, int LD>
+__device__ __forceinline__ void produce_tile(bf16* dst, const bf16* src, int ld_src, int lane, int which, uint64_t* bar) {
+    if (ld_src != LD) warp_tile<COLS, LD>(dst, src, ld_src, C, lane);
+    else if (lane == which) bulk_copy(dst, src, C * LD, bar);
+}
 
-__device__ __forceinline__ void init_stages(uint64_t* full, int* aborted) {
+struct Pipe {
+    uint64_t full[3], empty[3];
+    int aborted;
+};
+template <int STAGES>
+__device__ __forceinline__ void init_pipe(Pipe& p) {
     if (threadIdx.x == 0) {
-        tc::mbar_init(&full[0], 1);
-        tc::mbar_init(&full[1], 1);
-        *aborted = 0;
+        for (int s = 0; s < STAGES; ++s) { tc::mbar_init(&p.full[s], 33); tc::mbar_init(&p.empty[s], NT / 32); }
+        p.aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
 }
-// Barrier of the block behind the arrival of the i-th step's tiles; false for all threads if they did not come.
-template <int DK>
-__device__ __forceinline__ bool stage_ready(const Args& a, uint64_t* full, int* aborted, int i) {
-    const bool ok = !padded<DK>(a) || tc::mbar_wait(&full[i & 1], (i >> 1) & 1, aborted, a.err, 0x6b00 | (i & 1));
-    return __syncthreads_and(ok);
+// The producer warp: the tiles of the steps in order, each as soon as its stage is free.  x: U or dO; rows past x_rows are zeros.
+template <int DK, bool FULL, int STAGES, bool REV>
+__device__ __forceinline__ void produce(bf16* stage, const Args& a, Pipe& p, const bf16* x, long long xs_t, int x_rows, long long bh) {
+    using F = Cfg<DK>;
+    constexpr int STAGE = FULL ? F::FULL : F::QD;
+    const int lane = threadIdx.x & 31;
+    for (int i = 0; i < a.N; ++i) {
+        const int n = REV ? a.N - 1 - i : i, s = i % STAGES;
+        if (!tc::mbar_wait(&p.empty[s], ((i / STAGES) & 1) ^ 1, &p.aborted, a.err, 0x6c00 | s)) break;
+        const long long cn = bh * a.N + n;
+        bf16* st = stage + s * STAGE;
+        bf16* xt = st + 2 * C * F::LDK;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // what was written and read here comes before the copies
+        if (lane == 0) {
+            constexpr int TILE = C * F::LDK, TA = C * F::LDC;
+            tc::mbar_expect_tx(&p.full[s], ((a.ldw == F::LDK ? (FULL ? 3 : 2) * TILE : 0) + (FULL && a.lda == F::LDC ? TA : 0)) * 2);
+        }
+        __syncwarp();
+        produce_tile<DK, F::LDK>(st, a.W + cn * C * a.ldw, a.ldw, lane, 0, &p.full[s]);
+        produce_tile<DK, F::LDK>(st + C * F::LDK, a.Kd + cn * C * a.ldw, a.ldw, lane, 1, &p.full[s]);
+        if (FULL) {
+            produce_tile<DK, F::LDK>(st + F::QD, a.Qd + cn * C * a.ldw, a.ldw, lane, 2, &p.full[s]);
+            produce_tile<C, F::LDC>(st + F::AQ, a.A + cn * C * a.lda, a.lda, lane, 3, &p.full[s]);
+        }
+        warp_tile<DVS, F::LDV>(xt, x + (long long)n * C * xs_t, xs_t, x_rows - n * C, lane);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(&p.full[s])) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
+// Barrier of the NT threads that multiply; false for all of them if it is for one.
+__device__ __forceinline__ bool all_of(bool ok) {
+    int r;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 q, %1, 0;\nbarrier.cta.red.and.pred p, 1, %2, q;\nselp.b32 %0, 1, 0, p;\n}"
+                 : "=r"(r) : "r"((int)ok), "n"(NT) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void sync_workers() { asm volatile("barrier.cta.sync 1, %0;" :: "n"(NT) : "memory"); }
 
 // write a [rows x DVS] bf16 tile held in shared memory (row stride LDV) to global rows of stride `gld`
 template <int LDV>
@@ -153,118 +180,111 @@ __device__ __forceinline__ void save_state(const float (&S)[SN][4], float* dst, 
 }
 
 // OUT: the outputs O are wanted (the forward pass); without: Vn and the entering states only (what the backward pass rebuilds).
+// Eight warps multiply: 16 x 16 of Vn = U - W S each, a barrier, their part of the next state and 16 x 16 of O = Qd S + A Vn, which the next
+// step does not wait for any longer than for the state (two copies of the state, so that Qd S may still read the old one).
 template <int DK, bool OUT>
-__global__ void __launch_bounds__(NT) delta_scan_fwd_kernel(Args a) {
+__global__ void __launch_bounds__(NT + 32, DK == 128 && OUT ? 1 : 2) delta_scan_fwd_kernel(Args a) {
     using F = Cfg<DK>;
-    constexpr int STAGE = OUT ? F::FULL : F::QD, VN = OUT ? 4 : 2;   // VN: n-tiles of Vn per warp (four warps or all eight)
+    constexpr int STAGES = F::stages(OUT), STAGE = OUT ? F::FULL : F::QD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ Pipe pipe;
     bf16* stage = reinterpret_cast<bf16*>(smem_raw);
-    bf16* Sb = stage + 2 * STAGE;                    // [DK][LDV]
-    bf16* Vb = Sb + DK * F::LDV;                     // [C][LDV]  Vn of the chunk
+    bf16* Sb = stage + STAGES * STAGE;               // [2][DK][LDV]
+    bf16* Vb = Sb + 2 * DK * F::LDV;                 // [C][LDV]  Vn of the chunk
     bf16* Ob = Vb + C * F::LDV;                      // [C][LDV]  output staging
     const int col0 = blockIdx.x * DVS;
     const long long bh = blockIdx.y;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int s_m0 = DK == 128 ? 16 * w : 16 * (w & 3), s_n0 = DK == 128 ? 0 : 16 * (w >> 2);
-    const int m0 = 16 * (w & 3), v_n0 = OUT ? 0 : 16 * (w >> 2);
-    __shared__ uint64_t full[2];
-    __shared__ int aborted;
-    const bool outs = OUT && w >= 4;                 // these warps make O = Qd S + A Vn while the others make Vn = U - W S
-    const bf16* u = a.U + (bh * a.N) * C * a.dv + col0;
+    const int m0 = 16 * (w & 3), v_n0 = 16 * (w >> 2);
+    init_pipe<STAGES>(pipe);
+    if (w == NT / 32) {
+        produce<DK, OUT, STAGES, false>(stage, a, pipe, a.U + (bh * a.N) * C * a.dv + col0, a.dv, a.N * C, bh);
+        return;
+    }
     bf16* og = OUT ? a.O + (bh / a.H) * a.os_b + (bh % a.H) * a.os_h + col0 : nullptr;
-
     float S[F::SN][4];
     load_state<F::SN>(S, a.S0 == nullptr ? nullptr : a.S0 + bh * DK * a.dv, a.dv, col0, Sb, F::LDV, s_m0, s_n0);
-    init_stages(full, &aborted);
-    if (a.N > 0) issue_chunk<DK, OUT>(stage, a, u, a.dv, a.N * C, bh, 0, &full[0]);
-    cp_async_commit();
     for (int n = 0; n < a.N; ++n) {
-        const bf16* Wt = stage + (n & 1) * STAGE;
+        const float gamma = a.gamma[bh * a.N + n];
+        const bf16* Wt = stage + (n % STAGES) * STAGE;
         const bf16* Kt = Wt + C * F::LDK;
         const bf16* Ut = Wt + 2 * C * F::LDK;
         const bf16* Qt = Wt + F::QD;
         const bf16* At = Wt + F::AQ;
-        cp_async_wait<0>();
-        if (!stage_ready<DK>(a, full, &aborted, n)) break;         // tiles of chunk n and Sb visible; chunk n - 1 is done with its stage
-        if (n + 1 < a.N) issue_chunk<DK, OUT>(stage + ((n + 1) & 1) * STAGE, a, u, a.dv, a.N * C, bh, n + 1, &full[(n + 1) & 1]);
-        cp_async_commit();
-        const float gamma = a.gamma[bh * a.N + n];
-        if (a.Vn != nullptr) store_rows<F::LDV>(Sb, a.Sn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
-        float acc[VN][4];
-        zero_acc<VN>(acc);
-        if (!outs) {
-            warp_gemm<VN, DK, false, true>(acc, Wt, F::LDK, m0, Sb, F::LDV, v_n0);
-            const int r = m0 + (l >> 2);
+        const bf16* So = Sb + (n & 1) * DK * F::LDV;
+        const bool ok = tc::mbar_wait(&pipe.full[n % STAGES], (n / STAGES) & 1, &pipe.aborted, a.err, 0x6b00 | (n % STAGES));
+        if (!all_of(ok)) break;                                    // the state in front of the chunk is complete, Vb free
+        if (a.Vn != nullptr) store_rows<F::LDV>(So, a.Sn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
+        float acc[2][4];
+        zero_acc<2>(acc);
+        warp_gemm<2, DK, false, true>(acc, Wt, F::LDK, m0, So, F::LDV, v_n0);
+        const int r0 = m0 + (l >> 2);
 #pragma unroll
-            for (int nt = 0; nt < VN; ++nt) {
-                const int c = v_n0 + nt * 8 + (l & 3) * 2;
-                const __nv_bfloat162 u0 = *reinterpret_cast<const __nv_bfloat162*>(Ut + r * F::LDV + c);
-                const __nv_bfloat162 u1 = *reinterpret_cast<const __nv_bfloat162*>(Ut + (r + 8) * F::LDV + c);
-                acc[nt][0] = __bfloat162float(u0.x) - acc[nt][0]; acc[nt][1] = __bfloat162float(u0.y) - acc[nt][1];
-                acc[nt][2] = __bfloat162float(u1.x) - acc[nt][2]; acc[nt][3] = __bfloat162float(u1.y) - acc[nt][3];
-            }
-            store_acc_bf16<VN>(acc, Vb, F::LDV, m0, v_n0);
-        } else {
-            warp_gemm<VN, DK, false, true>(acc, Qt, F::LDK, m0, Sb, F::LDV, 0);
+        for (int nt = 0; nt < 2; ++nt) {
+            const int c = v_n0 + nt * 8 + (l & 3) * 2;
+            const __nv_bfloat162 u0 = *reinterpret_cast<const __nv_bfloat162*>(Ut + r0 * F::LDV + c);
+            const __nv_bfloat162 u1 = *reinterpret_cast<const __nv_bfloat162*>(Ut + (r0 + 8) * F::LDV + c);
+            acc[nt][0] = __bfloat162float(u0.x) - acc[nt][0]; acc[nt][1] = __bfloat162float(u0.y) - acc[nt][1];
+            acc[nt][2] = __bfloat162float(u1.x) - acc[nt][2]; acc[nt][3] = __bfloat162float(u1.y) - acc[nt][3];
         }
-        __syncthreads();                                           // Vb complete; every read of Sb done
+        store_acc_bf16<2>(acc, Vb, F::LDV, m0, v_n0);
+        sync_workers();                                            // Vb complete
         // S <- gamma S + Kd^T Vn
 #pragma unroll
         for (int nt = 0; nt < F::SN; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) S[nt][e] *= gamma;
         warp_gemm<F::SN, C, true, true>(S, Kt, F::LDK, s_m0, Vb, F::LDV, s_n0);
-        store_acc_bf16<F::SN>(S, Sb, F::LDV, s_m0, s_n0);
+        store_acc_bf16<F::SN>(S, Sb + ((n + 1) & 1) * DK * F::LDV, F::LDV, s_m0, s_n0);
         if (a.Vn != nullptr) store_rows<F::LDV>(Vb, a.Vn + ((bh * a.N + n) * C) * a.dv + col0, C, a.dv);
-        if (outs) {
-            for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<VN, 16, false, true>(acc, At + k0, F::LDC, m0, Vb + k0 * F::LDV, F::LDV, 0);
-            store_acc_bf16<VN>(acc, Ob, F::LDV, m0, 0);
+        if (OUT) {
+            zero_acc<2>(acc);
+            warp_gemm<2, DK, false, true>(acc, Qt, F::LDK, m0, So, F::LDV, v_n0);
+            for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<2, 16, false, true>(acc, At + k0, F::LDC, m0, Vb + k0 * F::LDV, F::LDV, v_n0);
+            store_acc_bf16<2>(acc, Ob, F::LDV, m0, v_n0);
             __syncwarp();
-            for (int i = l; i < 16 * (DVS / 8); i += 32) {         // the warp's own 16 rows
-                const int r = m0 + i / (DVS / 8), c = (i % (DVS / 8)) * 8, t = n * C + r;
-                if (t < a.T) *reinterpret_cast<uint4*>(og + (long long)t * a.os_t + c) = *reinterpret_cast<const uint4*>(Ob + r * F::LDV + c);
-            }
-            __syncwarp();
+            const int r = m0 + (l >> 1), c = v_n0 + (l & 1) * 8, t = n * C + r;       // the warp's own 16 x 16
+            if (t < a.T) *reinterpret_cast<uint4*>(og + (long long)t * a.os_t + c) = *reinterpret_cast<const uint4*>(Ob + r * F::LDV + c);
         }
+        __syncwarp();
+        if (l == 0) tc::mbar_arrive(&pipe.empty[n % STAGES]);
     }
     save_state<F::SN>(S, a.Sfinal + bh * DK * a.dv, a.dv, col0, s_m0, s_n0);
 }
 
 // Reverse walk: dS' enters from the right (gradient of the state leaving the chunk).
 template <int DK>
-__global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
+__global__ void __launch_bounds__(NT + 32, 1) delta_scan_bwd_kernel(Args a) {
     using F = Cfg<DK>;
-    constexpr int STAGE = F::FULL;
+    constexpr int STAGES = F::stages(true), STAGE = F::FULL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ Pipe pipe;
     bf16* stage = reinterpret_cast<bf16*>(smem_raw);
-    bf16* Sb = stage + 2 * STAGE;                    // [DK][LDV]  bf16 copy of dS'
+    bf16* Sb = stage + STAGES * STAGE;                    // [DK][LDV]  bf16 copy of dS'
     bf16* Vb = Sb + DK * F::LDV;                     // [C][LDV]   dVn of the chunk
     const int col0 = blockIdx.x * DVS;
     const long long bh = blockIdx.y;
     const int w = threadIdx.x >> 5;
     const int s_m0 = DK == 128 ? 16 * w : 16 * (w & 3), s_n0 = DK == 128 ? 0 : 16 * (w >> 2);
     const int m0 = 16 * (w & 3), v_n0 = 16 * (w >> 2);
-    const bf16* dO = a.dO + (bh / a.H) * a.gs_b + (bh % a.H) * a.gs_h + col0;
-    __shared__ uint64_t full[2];
-    __shared__ int aborted;
-
+    init_pipe<STAGES>(pipe);
+    if (w == NT / 32) {
+        produce<DK, true, STAGES, true>(stage, a, pipe, a.dO + (bh / a.H) * a.gs_b + (bh % a.H) * a.gs_h + col0, a.gs_t, a.T, bh);
+        return;
+    }
     float S[F::SN][4];
     load_state<F::SN>(S, a.dSfinal == nullptr ? nullptr : a.dSfinal + bh * DK * a.dv, a.dv, col0, Sb, F::LDV, s_m0, s_n0);
-    init_stages(full, &aborted);
-    if (a.N > 0) issue_chunk<DK, true>(stage, a, dO, a.gs_t, a.T, bh, a.N - 1, &full[0]);
-    cp_async_commit();
     for (int i = 0; i < a.N; ++i) {
         const int n = a.N - 1 - i;
-        const bf16* Wt = stage + (i & 1) * STAGE;
+        const float gamma = a.gamma[bh * a.N + n];
+        const bf16* Wt = stage + (i % STAGES) * STAGE;
         const bf16* Kt = Wt + C * F::LDK;
         const bf16* Gt = Wt + 2 * C * F::LDK;         // dO slice
         const bf16* Qt = Wt + F::QD;
         const bf16* At = Wt + F::AQ;
-        cp_async_wait<0>();
-        if (!stage_ready<DK>(a, full, &aborted, i)) break;
-        if (n > 0) issue_chunk<DK, true>(stage + ((i + 1) & 1) * STAGE, a, dO, a.gs_t, a.T, bh, n - 1, &full[(i + 1) & 1]);
-        cp_async_commit();
-        const float gamma = a.gamma[bh * a.N + n];
+        const bool ok = tc::mbar_wait(&pipe.full[i % STAGES], (i / STAGES) & 1, &pipe.aborted, a.err, 0x6b10 | (i % STAGES));
+        if (!all_of(ok)) break;                                    // the gradient behind the chunk is complete, Vb free
         store_rows<F::LDV>(Sb, a.dSn + ((bh * a.N + n) * DK) * a.dv + col0, DK, a.dv);
         // dVn = A^T dO + Kd dS'
         float acc[2][4];
@@ -278,7 +298,7 @@ __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) S[nt][e] *= gamma;
         warp_gemm<F::SN, C, true, true>(S, Qt, F::LDK, s_m0, Gt, F::LDV, s_n0);
-        __syncthreads();                                           // Vb complete; reads of Sb done
+        sync_workers();                                            // Vb complete; reads of Sb done
         float t[F::SN][4];
         zero_acc<F::SN>(t);
         warp_gemm<F::SN, C, true, true>(t, Wt, F::LDK, s_m0, Vb, F::LDV, s_n0);
@@ -288,6 +308,8 @@ __global__ void __launch_bounds__(NT) delta_scan_bwd_kernel(Args a) {
             for (int e = 0; e < 4; ++e) S[nt][e] -= t[nt][e];
         store_acc_bf16<F::SN>(S, Sb, F::LDV, s_m0, s_n0);
         store_rows<F::LDV>(Vb, a.dVn + ((bh * a.N + n) * C) * a.dv + col0, C, a.dv);
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) tc::mbar_arrive(&pipe.empty[i % STAGES]);
     }
     save_state<F::SN>(S, a.dS0 + bh * DK * a.dv, a.dv, col0, s_m0, s_n0);
 }
@@ -879,7 +901,7 @@ LMOE_API int lmoe_delta_scan(int dir, int dk, int BH, const dr::Args* ap, cudaSt
         auto kernel = KERNEL;                                                                                          \
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dr::Cfg<DK>::smem(out)); \
         if (e != cudaSuccess) return (int)e;                                                                           \
-        kernel<<<grid, dr::NT, dr::Cfg<DK>::smem(out), st>>>(a);                                                       \
+        kernel<<<grid, dr::NT + 32, dr::Cfg<DK>::smem(out), st>>>(a);                                                      \
     } while (0)
     if (dir != 0) { if (dk == 128) LMOE_DR_LAUNCH(dr::delta_scan_bwd_kernel<128>, 128); else LMOE_DR_LAUNCH(dr::delta_scan_bwd_kernel<64>, 64); }
     else if (out) { if (dk == 128) LMOE_DR_LAUNCH((dr::delta_scan_fwd_kernel<128, true>), 128); else LMOE_DR_LAUNCH((dr::delta_scan_fwd_kernel<64, true>), 64); }
