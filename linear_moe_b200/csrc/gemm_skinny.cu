@@ -1,14 +1,16 @@
 // y[M, N] = x[M, K] W[N, K]^T for M <= 16: the linears of one-token decode steps.
 //
 // With a handful of rows the product is bound by reading W once (2 N K bytes); a 256 x 256 tensor-core tile would spend
-// its time on rows that do not exist.  Here a CTA owns 16 rows of W and its eight warps split K.  Every lane streams
-// 16-byte pieces of two W rows and of one x row straight from global memory into mma.sync.m16n8k16 fragments: the sum
-// over k does not care about the order of k, so the eight consecutive elements a lane loads are used as the k slots
-// that lane owns in two MMA steps (the same assignment for the W and the x fragment), and no shared-memory staging or
-// transposition is needed.  The eight partial tiles are added through shared memory.  No atomics: results are
-// deterministic.  The kernel is launched with programmatic stream serialization: its first eight steps of W are in
-// flight before it waits for the kernel that produces x, so consecutive linears of a decode step keep HBM busy across
-// the kernel boundaries (the small kernels in between call griddepcontrol.launch_dependents at their start).
+// its time on rows that do not exist.  Here a CTA owns 16 rows of W at a time and its eight warps split K.  Every lane brings
+// 16-byte pieces of two W rows into slots of shared memory of its own and from there, with one x row, into mma.sync.m16n8k16
+// fragments: the sum over k does not care about the order of k, so the eight consecutive elements a lane loads are used as the
+// k slots that lane owns in two MMA steps (the same assignment for the W and the x fragment), and nothing is transposed or
+// exchanged.  The eight partial tiles are added through shared memory.  No atomics: results are deterministic.
+// Two CTAs per SM walk the row blocks with 64 KB of copies in flight each, over the ends of row blocks too.  (One CTA per row block,
+// its loads in registers, drained the memory system at every block's end: W of 128256 x 2048 96 us, now 91, 16384 x 2048 16.4, now
+// 13.5.)  The kernel is launched with programmatic stream serialization: its first eight steps of W are in flight before it waits
+// for the kernel that produces x, so consecutive linears of a decode step keep HBM busy across the kernel boundaries (the small
+// kernels in between call griddepcontrol.launch_dependents at their start).
 #include <cstdlib>
 
 #include "common.cuh"
@@ -17,7 +19,10 @@
 namespace lmoe {
 namespace sk {
 
-__device__ __forceinline__ uint4 ld_stream(const bf16* p) { return __ldcs(reinterpret_cast<const uint4*>(p)); }
+// 16 bytes of global memory to shared memory, zeros where `ok` is false
+__device__ __forceinline__ void copy16(uint32_t dst, const bf16* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
 
 __device__ __forceinline__ uint32_t sk_cluster_rank() {
     uint32_t r;
@@ -45,18 +50,20 @@ __device__ __forceinline__ void put(void* y, long long i, float v) {
     else reinterpret_cast<float*>(y)[i] += v;
 }
 
-template <int NTILES, int KS, int OUT>
-__global__ void __launch_bounds__(256) gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ W,
-                                                          long long ldw, void* y, long long ldy, int M, int N, int K) {
-    __shared__ float red[8][NTILES][32][4];
-    __shared__ float cred[KS][NTILES][32][4];
+// A CTA, or a cluster of KS that split K, takes row blocks blockIdx.x / KS, + gridDim.x / KS, ...  A lane's pieces of W go through PF slots of
+// shared memory that only this lane writes and reads, so nothing but its own copies is waited for, and the next steps' copies stay
+// in flight over the reduction and the store of a row block.
+// ONE: a lane's piece of x (K / KS at most PF steps) stays in registers.
+constexpr int PF = 8, STEP = 256;                                        // slots; elements of K per step of the eight warps
+template <int NTILES, int KS, int OUT, bool ONE>
+__global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long long ldx, const bf16* W,
+                                                             long long ldw, void* y, long long ldy, int M, int N, int K) {
+    extern __shared__ __align__(16) uint4 slots[];                       // [PF][2][256]
+    __shared__ float red[2][8][NTILES][32][4];
+    __shared__ float cred[2][KS][NTILES][32][4];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int g = l >> 2, q = l & 3;
     const uint32_t crank = KS > 1 ? sk_cluster_rank() : 0;
-    const int row_lo = (blockIdx.x / KS) * 16 + g, row_hi = row_lo + 8;
-    const bool lo_ok = row_lo < N, hi_ok = row_hi < N;
-    const bf16* w_lo = W + (long long)(lo_ok ? row_lo : 0) * ldw + q * 8;
-    const bf16* w_hi = W + (long long)(hi_ok ? row_hi : 0) * ldw + q * 8;
     const bf16* xr[NTILES];
     bool x_ok[NTILES];
 #pragma unroll
@@ -64,100 +71,138 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const bf16* __restrict
         x_ok[t] = g + 8 * t < M;
         xr[t] = x + (long long)(x_ok[t] ? g + 8 * t : 0) * ldx + q * 8;
     }
-    float acc[NTILES][4];
-#pragma unroll
-    for (int t = 0; t < NTILES; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
     const uint4 zero = make_uint4(0, 0, 0, 0);
     const int kslice = K / KS;                                           // a multiple of 32 (checked by the launcher)
     const int k_beg = (int)crank * kslice + w * 32, k_end = (int)(crank + 1) * kslice;
-    // The weights do not depend on the kernel before this one: the first PF steps of W are requested before waiting for
+    const int steps = (kslice + STEP - 1) / STEP, blocks = (N + 15) / 16, stride = gridDim.x / KS;
+    const uint32_t my = (uint32_t)__cvta_generic_to_shared(slots) + threadIdx.x * 16;
+    int c_block = blockIdx.x / KS, c_k = k_beg, c_step = 0;              // the next step to copy
+    auto copy = [&](int slot) {
+        const int r = c_block * 16 + g;
+        const bool in = c_block < blocks && c_k < k_end, lo = in && r < N, hi = in && r + 8 < N;
+        copy16(my + slot * 8192, W + (lo ? (long long)r * ldw + c_k + q * 8 : 0), lo);
+        copy16(my + slot * 8192 + 4096, W + (hi ? (long long)(r + 8) * ldw + c_k + q * 8 : 0), hi);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        c_k += STEP;
+        if (++c_step == steps) {
+            c_step = 0;
+            c_k = k_beg;
+            c_block += stride;
+        }
+    };
+    // The weights do not depend on the kernel before this one: the first steps of W are requested before waiting for
     // it (programmatic dependent launch), so the weight stream of one linear overlaps the tail of whatever produced x.
-    constexpr int PF = 8;
-    uint4 pa_lo[PF], pa_hi[PF];
 #pragma unroll
-    for (int i = 0; i < PF; ++i) {
-        const int k0 = k_beg + i * 256;
-        pa_lo[i] = (lo_ok && k0 < k_end) ? ld_stream(w_lo + k0) : zero;
-        pa_hi[i] = (hi_ok && k0 < k_end) ? ld_stream(w_hi + k0) : zero;
-    }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     // the next kernel may start its own prefetch
-    asm volatile("griddepcontrol.wait;" ::: "memory");                  // x is complete and visible from here on
+    for (int i = 0; i < PF; ++i) copy(i);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     // the next kernel may start its own copies
+    // x is complete and visible from here on.  (No pointer of this kernel is __restrict__: loads through those may move ahead of the wait.)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint4 xk[ONE ? NTILES : 1][PF];
+    if (ONE) {
 #pragma unroll
-    for (int i = 0; i < PF; ++i) {
-        const int k0 = k_beg + i * 256;
-        if (k0 < k_end) {
-            const uint32_t f1[4] = {pa_lo[i].x, pa_hi[i].x, pa_lo[i].y, pa_hi[i].y};
-            const uint32_t f2[4] = {pa_lo[i].z, pa_hi[i].z, pa_lo[i].w, pa_hi[i].w};
+        for (int i = 0; i < PF; ++i)
 #pragma unroll
             for (int t = 0; t < NTILES; ++t) {
-                const uint4 b = x_ok[t] ? *reinterpret_cast<const uint4*>(xr[t] + k0) : zero;
-                mma16816(acc[t], f1, b.x, b.y);
-                mma16816(acc[t], f2, b.z, b.w);
+                const int k = k_beg + i * STEP;
+                xk[ONE ? t : 0][i] = x_ok[t] && k < k_end ? *reinterpret_cast<const uint4*>(xr[t] + k) : zero;
             }
-        }
     }
+    int slot = 0, buf = 0;
+    for (int block = blockIdx.x / KS; block < blocks; block += stride, buf ^= 1) {
+        const int row_lo = block * 16 + g, row_hi = row_lo + 8;
+        const bool lo_ok = row_lo < N, hi_ok = row_hi < N;
+        float acc[NTILES][4];
+#pragma unroll
+        for (int t = 0; t < NTILES; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+        auto use = [&](const uint4 (&b)[NTILES]) {
+            asm volatile("cp.async.wait_group %0;" :: "n"(PF - 1) : "memory");
+            const uint4 a_lo = slots[slot * 512 + threadIdx.x], a_hi = slots[slot * 512 + 256 + threadIdx.x];
+            const uint32_t f1[4] = {a_lo.x, a_hi.x, a_lo.y, a_hi.y};
+            const uint32_t f2[4] = {a_lo.z, a_hi.z, a_lo.w, a_hi.w};
+#pragma unroll
+            for (int t = 0; t < NTILES; ++t) {
+                mma16816(acc[t], f1, b[t].x, b[t].y);
+                mma16816(acc[t], f2, b[t].z, b[t].w);
+            }
+            copy(slot);                                                  // behind the use of what the slot held
+            slot = (slot + 1) % PF;
+        };
+        if (ONE) {
+#pragma unroll
+            for (int i = 0; i < PF; ++i)
+                if (i < steps) {
+                    uint4 b[NTILES];
+#pragma unroll
+                    for (int t = 0; t < NTILES; ++t) b[t] = xk[ONE ? t : 0][i];
+                    use(b);
+                }
+        } else {
 #pragma unroll 4
-    for (int k0 = k_beg + PF * 256; k0 < k_end; k0 += 256) {
-        const uint4 a_lo = lo_ok ? ld_stream(w_lo + k0) : zero;
-        const uint4 a_hi = hi_ok ? ld_stream(w_hi + k0) : zero;
-        const uint32_t f1[4] = {a_lo.x, a_hi.x, a_lo.y, a_hi.y};
-        const uint32_t f2[4] = {a_lo.z, a_hi.z, a_lo.w, a_hi.w};
+            for (int i = 0; i < steps; ++i) {
+                const int k = k_beg + i * STEP;
+                uint4 b[NTILES];
 #pragma unroll
-        for (int t = 0; t < NTILES; ++t) {
-            const uint4 b = x_ok[t] ? *reinterpret_cast<const uint4*>(xr[t] + k0) : zero;
-            mma16816(acc[t], f1, b.x, b.y);
-            mma16816(acc[t], f2, b.z, b.w);
+                for (int t = 0; t < NTILES; ++t) b[t] = x_ok[t] && k < k_end ? *reinterpret_cast<const uint4*>(xr[t] + k) : zero;
+                use(b);
+            }
         }
-    }
 #pragma unroll
-    for (int t = 0; t < NTILES; ++t)
+        for (int t = 0; t < NTILES; ++t)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) red[w][t][l][e] = acc[t][e];
-    __syncthreads();
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
-    if (w < NTILES) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[e] += red[i][w][l][e];
-    }
-    if (KS > 1) {
-        // the CTA's partial tile goes to slot `crank` of the first CTA; it adds the slots in rank order (deterministic)
+            for (int e = 0; e < 4; ++e) red[buf][w][t][l][e] = acc[t][e];
+        __syncthreads();
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
         if (w < NTILES) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) st_cluster_f32(&cred[crank][w][l][e], 0, s[e]);
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[e] += red[buf][i][w][l][e];
         }
-        sk_cluster_sync();
-        if (crank != 0) return;
+        if (KS > 1) {
+            // the CTA's partial tile goes to slot `crank` of the first CTA; it adds the slots in rank order (deterministic)
+            if (w < NTILES) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) st_cluster_f32(&cred[buf][crank][w][l][e], 0, s[e]);
+            }
+            sk_cluster_sync();
+            if (crank != 0) continue;
+            if (w < NTILES) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    s[e] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < KS; ++i) s[e] += cred[buf][i][w][l][e];
+                }
+            }
+        }
         if (w < NTILES) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s[e] = 0.f;
-#pragma unroll
-                for (int i = 0; i < KS; ++i) s[e] += cred[i][w][l][e];
+            const int n0 = 8 * w + 2 * q;                                   // batch rows n0, n0 + 1
+            if (n0 < M) {
+                if (lo_ok) put<OUT>(y, (long long)n0 * ldy + row_lo, s[0]);
+                if (hi_ok) put<OUT>(y, (long long)n0 * ldy + row_hi, s[2]);
+            }
+            if (n0 + 1 < M) {
+                if (lo_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_lo, s[1]);
+                if (hi_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_hi, s[3]);
             }
         }
     }
-    if (w < NTILES) {
-        const int n0 = 8 * w + 2 * q;                                   // batch rows n0, n0 + 1
-        if (n0 < M) {
-            if (lo_ok) put<OUT>(y, (long long)n0 * ldy + row_lo, s[0]);
-            if (hi_ok) put<OUT>(y, (long long)n0 * ldy + row_hi, s[2]);
-        }
-        if (n0 + 1 < M) {
-            if (lo_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_lo, s[1]);
-            if (hi_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_hi, s[3]);
-        }
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 template <int NTILES, int KS, int OUT>
 static int launch_skinny(const bf16* x, long long ldx, const bf16* W, long long ldw, void* y, long long ldy, int M, int N, int K,
-                         cudaStream_t st) {
-    const int blocks = ((N + 15) / 16) * KS;
+                         int sms, cudaStream_t st) {
+    const int row_blocks = (N + 15) / 16, blocks = min(row_blocks, 2 * sms / KS) * KS;       // two CTAs per SM
+    constexpr int SMEM = PF * 8192;
+    const bool one = K / KS <= PF * STEP;
+    const auto kernel = one ? gemm_skinny_kernel<NTILES, KS, OUT, true> : gemm_skinny_kernel<NTILES, KS, OUT, false>;
+    const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     int na = 0;
@@ -178,23 +223,24 @@ static int launch_skinny(const bf16* x, long long ldx, const bf16* W, long long 
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NTILES, KS, OUT>, x, ldx, W, ldw, y, ldy, M, N, K);
+    return (int)cudaLaunchKernelEx(&cfg, kernel, x, ldx, W, ldw, y, ldy, M, N, K);
 }
 
 template <int OUT>
 static int dispatch(const bf16* x, long long ldx, const bf16* W, long long ldw, void* y, long long ldy, int M, int N, int K,
                     cudaStream_t st) {
-    // few row blocks: four CTAs of a cluster split K so that the whole GPU streams W
+    // few row blocks: the four CTAs of a cluster split K so that the whole GPU streams W.  Clusters walk the row blocks too: as 512 CTAs in two waves
+    // W of 2048 x 2048 and 2048 x 8192 cost a decode step of four layers 6 us of 318 more than with the copies of both rounds in flight at once.
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
     }
     const bool split = (N + 15) / 16 < 2 * sms && K % 128 == 0;
-    if (M <= 8) return split ? launch_skinny<1, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, st)
-                             : launch_skinny<1, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, st);
-    return split ? launch_skinny<2, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, st)
-                 : launch_skinny<2, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, st);
+    if (M <= 8) return split ? launch_skinny<1, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st)
+                             : launch_skinny<1, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st);
+    return split ? launch_skinny<2, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st)
+                 : launch_skinny<2, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st);
 }
 
 }  // namespace sk

@@ -192,3 +192,18 @@ def test_forward_in_one_host_call(kind, D, T):
 
 def assert_not_plain():
     assert not K._plain_call()
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,k", [(1, 32), (17, 2048), (130, 2080), (5000, 2048), (5000, 2304), (4752, 96), (300, 8192), (300, 8320), (20000, 288)])
+def test_weight_streaming_edges(M, N, k):
+    """Row blocks walked by two CTAs per SM or split over a cluster; x held in registers or not; K that ends inside a step."""
+    torch.manual_seed(0)
+    x, w = rand(M, k + 8, scale=1)[:, :k], rand(N, k, scale=k ** -0.5)
+    assert K._skinny_ok(x, w)
+    y = K.linear_skinny(x, w)
+    assert rel(y, x.double() @ w.double().t()) < OUT
+    acc = torch.randn(M, N, device="cuda")
+    want = acc.double() + x.double() @ w.double().t()
+    K._skinny_f32(x, w, acc, True)
+    assert rel(acc, want) < 1e-5                                # fp32 sums of exact products: sqrt(K) 2^-24, K up to 8320
