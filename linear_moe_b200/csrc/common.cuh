@@ -102,6 +102,28 @@ __device__ __forceinline__ void store4(bf16* y, float4 v) {
 // this one is still running; that kernel waits for this one's completion before it reads anything this one writes.
 // Without such a dependent in the stream the instruction does nothing.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// What a kernel launched with launch_early does ahead of its first access to memory: waits until the kernel before it has completed.
+// Such a kernel's pointers are not __restrict__: the compiler may move loads through const __restrict__ pointers ahead of the wait.
+// Ahead of pdl_trigger, so that whatever starts early behind it still finds everything older than this kernel complete.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A launch that may start while the kernel before it in the stream is running, if that one calls pdl_trigger.  The small kernels between the
+// weight-streaming products of a decode step go out this way: their blocks are in place when the product ends.
+template <typename T> struct launch_arg { using type = T; };
+template <typename... P>
+inline int launch_early(void (*kernel)(P...), int64_t blocks, int threads, cudaStream_t st, typename launch_arg<P>::type... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    return (int)cudaGetLastError();
+}
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }

@@ -22,13 +22,14 @@ static inline int pick_threads(int nvec) {
 // RMSNorm forward: r = x (+ res); y = r * rsqrt(mean(r^2) + eps) * w.  One block per row.
 // ---------------------------------------------------------------------------------------------
 template <typename T, int MAXV>
-__global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ w,
-                                    T* __restrict__ y, T* __restrict__ res_out, float* __restrict__ rstd_out,
+__global__ void rms_norm_fwd_kernel(const T* x, const T* res, const T* w,
+                                    T* y, T* res_out, float* rstd_out,
                                     int N, float eps) {
     __shared__ float red[32];
     constexpr int VN = Vec<T>::N;
     const int64_t row = blockIdx.x;
     const int nvec = N / VN;
+    pdl_wait();
     pdl_trigger();
     const T* xr = x + row * N;
     Vec<T> v[MAXV];
@@ -182,9 +183,10 @@ template <> struct Quad<float> {
 };
 
 template <typename T, int DMAX>
-__global__ void head_norm_gate_fwd_kernel(const T* __restrict__ o, const T* __restrict__ w, const T* __restrict__ gate,
-                                          T* __restrict__ y, float* __restrict__ rstd_out, int64_t rows, int D,
+__global__ void head_norm_gate_fwd_kernel(const T* o, const T* w, const T* gate,
+                                          T* y, float* rstd_out, int64_t rows, int D,
                                           float eps, int do_norm) {
+    pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
     constexpr int PER = DMAX / 128;
@@ -361,7 +363,8 @@ __global__ void gated_rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __r
 // SwiGLU: y[r, c] = silu(x[r, c]) * x[r, F + c]
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void swiglu_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int F) {
+__global__ void swiglu_fwd_kernel(const T* x, T* y, int64_t rows, int F) {
+    pdl_wait();
     pdl_trigger();
     constexpr int VN = Vec<T>::N;
     const int64_t nvec = rows * (F / VN);
@@ -963,13 +966,13 @@ LMOE_API int lmoe_rms_norm_fwd(const void* x, const void* res, const void* w, vo
         int threads = pick_threads(nvec);
         if (nvec > threads * 8) return -2;
         if (nvec <= threads * 1)
-            rms_norm_fwd_kernel<T, 1><<<rows, threads, 0, st>>>((const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
+            return launch_early(rms_norm_fwd_kernel<T, 1>, rows, threads, st, (const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
         else if (nvec <= threads * 2)
-            rms_norm_fwd_kernel<T, 2><<<rows, threads, 0, st>>>((const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
+            return launch_early(rms_norm_fwd_kernel<T, 2>, rows, threads, st, (const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
         else if (nvec <= threads * 4)
-            rms_norm_fwd_kernel<T, 4><<<rows, threads, 0, st>>>((const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
+            return launch_early(rms_norm_fwd_kernel<T, 4>, rows, threads, st, (const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
         else
-            rms_norm_fwd_kernel<T, 8><<<rows, threads, 0, st>>>((const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
+            return launch_early(rms_norm_fwd_kernel<T, 8>, rows, threads, st, (const T*)x, (const T*)res, (const T*)w, (T*)y, (T*)res_out, rstd, N, eps);
     })
     return (int)cudaGetLastError();
 }
@@ -1006,9 +1009,9 @@ LMOE_API int lmoe_head_norm_gate_fwd(const void* o, const void* w, const void* g
     int64_t need = (rows + wpb - 1) / wpb;
     int blocks = (int)(need < 148 * 8 ? need : 148 * 8);
     DISPATCH_T(dtype, {
-        if (D <= 128) head_norm_gate_fwd_kernel<T, 128><<<blocks, wpb * 32, 0, st>>>((const T*)o, (const T*)w, (const T*)gate, (T*)y, rstd, rows, D, eps, do_norm);
-        else if (D <= 256) head_norm_gate_fwd_kernel<T, 256><<<blocks, wpb * 32, 0, st>>>((const T*)o, (const T*)w, (const T*)gate, (T*)y, rstd, rows, D, eps, do_norm);
-        else head_norm_gate_fwd_kernel<T, 512><<<blocks, wpb * 32, 0, st>>>((const T*)o, (const T*)w, (const T*)gate, (T*)y, rstd, rows, D, eps, do_norm);
+        if (D <= 128) return launch_early(head_norm_gate_fwd_kernel<T, 128>, blocks, wpb * 32, st, (const T*)o, (const T*)w, (const T*)gate, (T*)y, rstd, rows, D, eps, do_norm);
+        else if (D <= 256) return launch_early(head_norm_gate_fwd_kernel<T, 256>, blocks, wpb * 32, st, (const T*)o, (const T*)w, (const T*)gate, (T*)y, rstd, rows, D, eps, do_norm);
+        else return launch_early(head_norm_gate_fwd_kernel<T, 512>, blocks, wpb * 32, st, (const T*)o, (const T*)w, (const T*)gate, (T*)y, rstd, rows, D, eps, do_norm);
     })
     return (int)cudaGetLastError();
 }
@@ -1054,7 +1057,7 @@ LMOE_API int lmoe_gated_rms_norm_bwd(const void* dy, const void* x, const void* 
 LMOE_API int lmoe_swiglu_fwd(const void* x, void* y, int64_t rows, int F, int dtype, cudaStream_t st) {
     DISPATCH_T(dtype, {
         if (F % Vec<T>::N != 0) return -1;
-        swiglu_fwd_kernel<T><<<grid_for(rows * (F / Vec<T>::N), 256), 256, 0, st>>>((const T*)x, (T*)y, rows, F);
+        return launch_early(swiglu_fwd_kernel<T>, grid_for(rows * (F / Vec<T>::N), 256), 256, st, (const T*)x, (T*)y, rows, F);
     })
     return (int)cudaGetLastError();
 }

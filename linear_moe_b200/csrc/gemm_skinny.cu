@@ -41,8 +41,10 @@ __device__ __forceinline__ void st_cluster_f32(float* p, uint32_t rank, float v)
 
 // NTILES 1: M <= 8, 2: M <= 16.  KS: CTAs of a cluster that split K between them (for matrices with few rows, so that
 // every SM streams a piece of W); their partial tiles meet in the shared memory of the cluster's first CTA.
-// OUT: bf16 result, fp32 result, or fp32 added to what y holds (the residual stream of a decode step).
-enum { OUT_BF16 = 0, OUT_F32 = 1, OUT_F32_ADD = 2 };
+// OUT: bf16 result, fp32 result, fp32 added to what y holds (the residual stream of a decode step), or bf16 silu(gate) * up
+// for W = [gate | up] [2 N, K], where a CTA's 16 rows of W are eight of gate and the eight of up that go with them.
+enum { OUT_BF16 = 0, OUT_F32 = 1, OUT_F32_ADD = 2, OUT_SWIGLU = 3 };
+template <int OUT> constexpr int ROWS = OUT == OUT_SWIGLU ? 8 : 16;      // columns of y per row block
 template <int OUT>
 __device__ __forceinline__ void put(void* y, long long i, float v) {
     if (OUT == OUT_BF16) reinterpret_cast<bf16*>(y)[i] = __float2bfloat16(v);
@@ -55,6 +57,8 @@ __device__ __forceinline__ void put(void* y, long long i, float v) {
 // in flight over the reduction and the store of a row block.
 // ONE: a lane's piece of x (K / KS at most PF steps) stays in registers.
 constexpr int PF = 8, STEP = 256;                                        // slots; elements of K per step of the eight warps
+__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16(v)); }
+
 template <int NTILES, int KS, int OUT, bool ONE>
 __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long long ldx, const bf16* W,
                                                              long long ldw, void* y, long long ldy, int M, int N, int K) {
@@ -74,14 +78,14 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long
     const uint4 zero = make_uint4(0, 0, 0, 0);
     const int kslice = K / KS;                                           // a multiple of 32 (checked by the launcher)
     const int k_beg = (int)crank * kslice + w * 32, k_end = (int)(crank + 1) * kslice;
-    const int steps = (kslice + STEP - 1) / STEP, blocks = (N + 15) / 16, stride = gridDim.x / KS;
+    const int steps = (kslice + STEP - 1) / STEP, blocks = (N + ROWS<OUT> - 1) / ROWS<OUT>, stride = gridDim.x / KS;
     const uint32_t my = (uint32_t)__cvta_generic_to_shared(slots) + threadIdx.x * 16;
     int c_block = blockIdx.x / KS, c_k = k_beg, c_step = 0;              // the next step to copy
     auto copy = [&](int slot) {
-        const int r = c_block * 16 + g;
-        const bool in = c_block < blocks && c_k < k_end, lo = in && r < N, hi = in && r + 8 < N;
+        const int r = c_block * ROWS<OUT> + g, r_hi = OUT == OUT_SWIGLU ? r + N : r + 8;
+        const bool in = c_block < blocks && c_k < k_end, lo = in && r < N, hi = in && (OUT == OUT_SWIGLU ? r : r_hi) < N;
         copy16(my + slot * 8192, W + (lo ? (long long)r * ldw + c_k + q * 8 : 0), lo);
-        copy16(my + slot * 8192 + 4096, W + (hi ? (long long)(r + 8) * ldw + c_k + q * 8 : 0), hi);
+        copy16(my + slot * 8192 + 4096, W + (hi ? (long long)r_hi * ldw + c_k + q * 8 : 0), hi);
         asm volatile("cp.async.commit_group;" ::: "memory");
         c_k += STEP;
         if (++c_step == steps) {
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long
     }
     int slot = 0, buf = 0;
     for (int block = blockIdx.x / KS; block < blocks; block += stride, buf ^= 1) {
-        const int row_lo = block * 16 + g, row_hi = row_lo + 8;
+        const int row_lo = block * ROWS<OUT> + g, row_hi = row_lo + 8;
         const bool lo_ok = row_lo < N, hi_ok = row_hi < N;
         float acc[NTILES][4];
 #pragma unroll
@@ -177,6 +181,11 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long
         }
         if (w < NTILES) {
             const int n0 = 8 * w + 2 * q;                                   // batch rows n0, n0 + 1
+            if (OUT == OUT_SWIGLU) {                                        // of gate and up in bf16, as where they pass through memory
+                if (lo_ok && n0 < M) put<OUT_BF16>(y, (long long)n0 * ldy + row_lo, silu_f(bf16_round(s[0])) * bf16_round(s[2]));
+                if (lo_ok && n0 + 1 < M) put<OUT_BF16>(y, (long long)(n0 + 1) * ldy + row_lo, silu_f(bf16_round(s[1])) * bf16_round(s[3]));
+                continue;
+            }
             if (n0 < M) {
                 if (lo_ok) put<OUT>(y, (long long)n0 * ldy + row_lo, s[0]);
                 if (hi_ok) put<OUT>(y, (long long)n0 * ldy + row_hi, s[2]);
@@ -193,7 +202,7 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long
 template <int NTILES, int KS, int OUT>
 static int launch_skinny(const bf16* x, long long ldx, const bf16* W, long long ldw, void* y, long long ldy, int M, int N, int K,
                          int sms, cudaStream_t st) {
-    const int row_blocks = (N + 15) / 16, blocks = min(row_blocks, 2 * sms / KS) * KS;       // two CTAs per SM
+    const int row_blocks = (N + ROWS<OUT> - 1) / ROWS<OUT>, blocks = min(row_blocks, 2 * sms / KS) * KS;       // two CTAs per SM
     constexpr int SMEM = PF * 8192;
     const bool one = K / KS <= PF * STEP;
     const auto kernel = one ? gemm_skinny_kernel<NTILES, KS, OUT, true> : gemm_skinny_kernel<NTILES, KS, OUT, false>;
@@ -236,7 +245,7 @@ static int dispatch(const bf16* x, long long ldx, const bf16* W, long long ldw, 
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
     }
-    const bool split = (N + 15) / 16 < 2 * sms && K % 128 == 0;
+    const bool split = (N + ROWS<OUT> - 1) / ROWS<OUT> < 2 * sms && K % 128 == 0;
     if (M <= 8) return split ? launch_skinny<1, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st)
                              : launch_skinny<1, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st);
     return split ? launch_skinny<2, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st)
@@ -267,4 +276,12 @@ LMOE_API int lmoe_gemm_skinny_f32(const void* x, long long ldx, const void* W, l
     if (!skinny_shape_ok(x, ldx, W, ldw, M, N, K)) return -1;
     return accumulate ? sk::dispatch<sk::OUT_F32_ADD>((const bf16*)x, ldx, (const bf16*)W, ldw, y, ldy, M, N, K, st)
                       : sk::dispatch<sk::OUT_F32>((const bf16*)x, ldx, (const bf16*)W, ldw, y, ldy, M, N, K, st);
+}
+
+// y [M, F] = silu(gate) * up for [gate | up] = x W^T, W [2 F, K]; the bits of lmoe_gemm_skinny followed by the SwiGLU kernel.
+LMOE_API int lmoe_gemm_skinny_swiglu(const void* x, long long ldx, const void* W, long long ldw, void* y, long long ldy, int M, int F,
+                                     int K, cudaStream_t st) {
+    using namespace lmoe;
+    if (!skinny_shape_ok(x, ldx, W, ldw, M, F, K)) return -1;
+    return sk::dispatch<sk::OUT_SWIGLU>((const bf16*)x, ldx, (const bf16*)W, ldw, y, ldy, M, F, K, st);
 }

@@ -15,18 +15,20 @@ namespace {
 
 template <int D>
 __global__ void __launch_bounds__(4 * D)
-lsm_scalar_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                       const __nv_bfloat16* __restrict__ v, long long qs_b, long long qs_h, long long ks_b, long long ks_h,
-                       long long vs_b, long long vs_h, const float* __restrict__ g, const float* __restrict__ gk,
-                       const float* __restrict__ s_in, float* __restrict__ s_out, __nv_bfloat16* __restrict__ o, int H,
+lsm_scalar_step_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k,
+                       const __nv_bfloat16* v, long long qs_b, long long qs_h, long long ks_b, long long ks_h,
+                       long long vs_b, long long vs_h, const float* g, long long gs_b, const float* gk,
+                       const float* s_in, float* s_out, __nv_bfloat16* o, int H,
                        float scale) {
     __shared__ float qs[D], ks[D], dec[D], part[4][D];
     const int bh = blockIdx.x, b = bh / H, h = bh % H;
     const int j = threadIdx.x % D, r = threadIdx.x / D;
+    pdl_wait();
+    pdl_trigger();
     if (threadIdx.x < D) {
         qs[threadIdx.x] = __bfloat162float(q[b * qs_b + h * qs_h + threadIdx.x]) * scale;
         ks[threadIdx.x] = __bfloat162float(k[b * ks_b + h * ks_h + threadIdx.x]);
-        dec[threadIdx.x] = (g == nullptr ? 1.f : __expf(g[bh])) * (gk == nullptr ? 1.f : __expf(gk[(long long)bh * D + threadIdx.x]));
+        dec[threadIdx.x] = (g == nullptr ? 1.f : __expf(g[b * gs_b + h])) * (gk == nullptr ? 1.f : __expf(gk[(long long)bh * D + threadIdx.x]));
     }
     const float vj = __bfloat162float(v[b * vs_b + h * vs_h + j]);
     __syncthreads();
@@ -55,14 +57,16 @@ lsm_scalar_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
 // and written once.
 template <int D>
 __global__ void __launch_bounds__(4 * D)
-lsm_delta_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                      const __nv_bfloat16* __restrict__ v, long long qs_b, long long qs_h, long long ks_b, long long ks_h,
-                      long long vs_b, long long vs_h, const float* __restrict__ g, const float* __restrict__ beta,
-                      const float* __restrict__ s_in, float* __restrict__ s_out, __nv_bfloat16* __restrict__ o, int H,
+lsm_delta_step_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k,
+                      const __nv_bfloat16* v, long long qs_b, long long qs_h, long long ks_b, long long ks_h,
+                      long long vs_b, long long vs_h, const float* g, const float* beta,
+                      const float* s_in, float* s_out, __nv_bfloat16* o, int H,
                       float scale) {
     __shared__ float qs[D], ks[D], part[4][D];
     const int bh = blockIdx.x, b = bh / H, h = bh % H;
     const int j = threadIdx.x % D, r = threadIdx.x / D;
+    pdl_wait();
+    pdl_trigger();
     if (threadIdx.x < D) {
         qs[threadIdx.x] = __bfloat162float(q[b * qs_b + h * qs_h + threadIdx.x]) * scale;
         ks[threadIdx.x] = __bfloat162float(k[b * ks_b + h * ks_h + threadIdx.x]);
@@ -100,24 +104,22 @@ lsm_delta_step_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* 
 }  // namespace
 }  // namespace lmoe
 
-// q, k, v: bf16, one token per (batch, head), element strides over batch and head, contiguous over D.  g: [B*H] log
-// decay of this token or null; gk: [B*H, D] log decay per key channel or null.  s_in: [B*H, D, D] fp32 or null (zero
+// q, k, v: bf16, one token per (batch, head), element strides over batch and head, contiguous over D.  g: [B, H] log
+// decay of this token (batch stride gs_b, zero for one decay per head) or null; gk: [B*H, D] log decay per key channel or null.  s_in: [B*H, D, D] fp32 or null (zero
 // state); s_out is a different buffer.  o: [B*H, D] bf16.
 LMOE_API int lmoe_lsm_scalar_step(const void* q, const void* k, const void* v, long long qs_b, long long qs_h, long long ks_b,
-                                  long long ks_h, long long vs_b, long long vs_h, const float* g, const float* gk,
+                                  long long ks_h, long long vs_b, long long vs_h, const float* g, long long gs_b, const float* gk,
                                   const float* s_in, float* s_out, void* o, int B, int H, int D, float scale,
                                   cudaStream_t st) {
     using namespace lmoe;
     const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)k, *vv = (const __nv_bfloat16*)v;
     if (D == 128)
-        lsm_scalar_step_kernel<128><<<B * H, 512, 0, st>>>(qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, gk, s_in, s_out,
+        return launch_early(lsm_scalar_step_kernel<128>, B * H, 512, st, qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, gs_b, gk, s_in, s_out,
                                                           (__nv_bfloat16*)o, H, scale);
-    else if (D == 64)
-        lsm_scalar_step_kernel<64><<<B * H, 256, 0, st>>>(qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, gk, s_in, s_out,
+    if (D == 64)
+        return launch_early(lsm_scalar_step_kernel<64>, B * H, 256, st, qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, gs_b, gk, s_in, s_out,
                                                          (__nv_bfloat16*)o, H, scale);
-    else
-        return -1;
-    return (int)cudaGetLastError();
+    return -1;
 }
 
 // Delta-rule step; beta: [B*H]; g: [B*H] log decay or null (plain DeltaNet).  Other arguments as above.
@@ -128,12 +130,10 @@ LMOE_API int lmoe_lsm_delta_step(const void* q, const void* k, const void* v, lo
     using namespace lmoe;
     const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)k, *vv = (const __nv_bfloat16*)v;
     if (D == 128)
-        lsm_delta_step_kernel<128><<<B * H, 512, 0, st>>>(qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, beta, s_in, s_out,
+        return launch_early(lsm_delta_step_kernel<128>, B * H, 512, st, qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, beta, s_in, s_out,
                                                          (__nv_bfloat16*)o, H, scale);
-    else if (D == 64)
-        lsm_delta_step_kernel<64><<<B * H, 256, 0, st>>>(qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, beta, s_in, s_out,
+    if (D == 64)
+        return launch_early(lsm_delta_step_kernel<64>, B * H, 256, st, qq, kk, vv, qs_b, qs_h, ks_b, ks_h, vs_b, vs_h, g, beta, s_in, s_out,
                                                         (__nv_bfloat16*)o, H, scale);
-    else
-        return -1;
-    return (int)cudaGetLastError();
+    return -1;
 }

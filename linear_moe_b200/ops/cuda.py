@@ -222,6 +222,18 @@ def linear_skinny(x, weight):
     return y
 
 
+def linear_skinny_swiglu(x, weight):
+    """``silu(gate) * up`` of ``[gate | up] = x W^T`` for up to 16 rows, in one launch."""
+    x2 = _rows(x)
+    M, K = x2.shape
+    N = weight.shape[0] // 2
+    y = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=x.device)
+    ll = ctypes.c_longlong
+    _check(lib().lmoe_gemm_skinny_swiglu(_p(x2), ll(x2.stride(0)), _p(weight), ll(weight.stride(0)), _p(y), ll(N), _i32(M), _i32(N),
+                                         _i32(K), _st()), "gemm_skinny_swiglu")
+    return y
+
+
 def _skinny_f32(x, weight, y, accumulate: bool):
     ll = ctypes.c_longlong
     _check(lib().lmoe_gemm_skinny_f32(_p(x), ll(x.stride(0)), _p(weight), ll(weight.stride(0)), _p(y), ll(y.stride(0)), _i32(x.shape[0]),
@@ -343,7 +355,7 @@ def mlp_swiglu(x, w1, w2):
     """SwiGLU MLP ``fc2(swiglu(fc1(x)))`` without biases; the fully fused form when the shapes allow it."""
     from . import fp8, gemm
     if _skinny_ok(x, w1):
-        return linear(swiglu(linear(x, w1)), w2)
+        return linear(linear_skinny_swiglu(x, w1) if w1.shape[0] % 16 == 0 else swiglu(linear(x, w1)), w2)
     if (not fp8.enabled() and x.dtype == w1.dtype == w2.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and x.numel() > 0
             and gemm.dense_ok(w1, w2) and w1.shape[0] % 128 == 0 and w2.shape[0] % 8 == 0 and w2.shape[1] * 2 == w1.shape[0]
             and os.environ.get("LMOE_FUSED_MLP", "1") != "0"):
@@ -356,7 +368,7 @@ def linear_swiglu(x, weight):
     else go through :func:`linear` followed by the SwiGLU kernel."""
     from . import fp8, gemm
     if _skinny_ok(x, weight):
-        return swiglu(linear(x, weight))
+        return linear_skinny_swiglu(x, weight) if weight.shape[0] % 16 == 0 else swiglu(linear(x, weight))
     if (not (fp8.enabled() and fp8.supported(x, weight)) and weight.dtype == x.dtype == torch.bfloat16 and weight.dim() == 2
             and x.shape[-1] % 8 == 0 and x.numel() > 0 and gemm.dense_ok(weight) and weight.shape[0] % 16 == 0
             and os.environ.get("LMOE_FUSED_SWIGLU", "1") != "0"):
@@ -1188,17 +1200,18 @@ def _lsm_step(q, k, v, g, gk, scale, initial_state):
     g: None | [H] | [B,1,H]; gk: None | [B,1,H,D]."""
     B, _, H, D = q.shape
     q, k, v = (t if t.stride(-1) == 1 else t.contiguous() for t in (q, k, v))
-    gf = None
+    gf, g_stride = None, 0                                    # a constant decay per head is read with a batch stride of zero
     if g is not None:
-        gf = (g.float().expand(B, H) if g.dim() == 1 else g.float().reshape(B, H)).contiguous()
+        gf, g_stride = (g.float().expand(H), 0) if g.dim() == 1 else (g.float().reshape(B, H), H)
+        gf = gf.contiguous()
     gkf = None if gk is None else gk.float().reshape(B, H, D).contiguous()
     s_in = None if initial_state is None else initial_state.float().contiguous()
     s_out = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device)
     o = torch.empty(B, 1, H, D, dtype=q.dtype, device=q.device)
     ll = ctypes.c_longlong
     _check(lib().lmoe_lsm_scalar_step(_p(q), _p(k), _p(v), ll(q.stride(0)), ll(q.stride(2)), ll(k.stride(0)), ll(k.stride(2)),
-                                      ll(v.stride(0)), ll(v.stride(2)), _p(gf), _p(gkf), _p(s_in), _p(s_out), _p(o), ctypes.c_int(B),
-                                      ctypes.c_int(H), ctypes.c_int(D), ctypes.c_float(scale), _st()), "lsm_scalar_step")
+                                      ll(v.stride(0)), ll(v.stride(2)), _p(gf), ll(g_stride), _p(gkf), _p(s_in), _p(s_out), _p(o),
+                                      ctypes.c_int(B), ctypes.c_int(H), ctypes.c_int(D), ctypes.c_float(scale), _st()), "lsm_scalar_step")
     return o, s_out
 
 

@@ -207,3 +207,37 @@ def test_weight_streaming_edges(M, N, k):
     want = acc.double() + x.double() @ w.double().t()
     K._skinny_f32(x, w, acc, True)
     assert rel(acc, want) < 1e-5                                # fp32 sums of exact products: sqrt(K) 2^-24, K up to 8320
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("F,K_", [(8, 32), (24, 2048), (2504, 2048), (2400, 4096), (5000, 96)])
+def test_weight_streaming_swiglu(M, F, K_):
+    """The activation in the weight-streaming product gives the bits of the two launches it replaces."""
+    torch.manual_seed(0)
+    x, w = rand(M, K_, scale=1), rand(2 * F, K_, scale=2 * K_ ** -0.5)
+    assert torch.equal(K.linear_skinny_swiglu(x, w), K.swiglu(K.linear_skinny(x, w)))
+
+
+def test_early_launches_wait():
+    """Chains of kernels that may start while the one before them runs: every link reads what the one before has written."""
+    torch.manual_seed(0)
+    n, h, H, D = 8, 1024, 8, 128
+    w = [rand(h, h, scale=h ** -0.5) for _ in range(8)]
+    gain, S0 = torch.ones(h, device="cuda").bfloat16(), torch.randn(n, H, D, D, device="cuda")
+    wide = [torch.cat([m, m]) for m in w]
+    x = rand(n, h, scale=1)
+
+    def chain(pause):
+        y, S = x, S0
+        with torch.no_grad():
+            for m, m2 in zip(w, wide):
+                y = K.linear_skinny(y, m); pause()
+                y = K.rms_norm(y, gain); pause()
+                o, S = K.lsm_scalar(*(y.view(n, 1, H, D),) * 3, None, 0.05, S, 64); pause()
+                y = K.head_norm_gate(o, gain[:D], y.view(n, 1, H, D), 1e-6, True).reshape(n, h); pause()
+                y = K.linear_skinny_swiglu(y, m2); pause()
+        return y, S
+    want = chain(torch.cuda.synchronize)
+    for _ in range(20):
+        for a, b in zip(chain(lambda: None), want):
+            assert torch.equal(a, b)
