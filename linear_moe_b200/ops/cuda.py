@@ -1476,6 +1476,18 @@ class _DeltaPrepArgs(ctypes.Structure):
                 [(n, ctypes.c_int) for n in ("B", "T", "H", "N")] + [("scale", ctypes.c_float), ("Tinv", ctypes.c_void_p)])
 
 
+def _padded_tiles(B, H, N, C, widths, device):
+    """bf16 ``[B,H,N,C,n]`` tiles, one per width, with rows as the scan kernels keep them in shared memory: eight more elements than
+    the tile has columns.  One allocation holds all rows to their ends: a scan fetches a tile as one copy of ``C (n + 8)`` elements."""
+    flat = torch.empty(B * H * N * C * (sum(widths) + 8 * len(widths)), dtype=torch.bfloat16, device=device)
+    tiles, at = [], 0
+    for n in widths:
+        r = C * (n + 8)
+        tiles.append(flat.as_strided((B, H, N, C, n), (H * N * r, N * r, r, n + 8, 1), at))
+        at += B * H * N * r
+    return tiles
+
+
 def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64, inverse=None):
     """The tiles of :func:`_delta_prepare` from one chunk-parallel kernel (``delta_prep_fwd_kernel``, csrc/lsm_delta.cu):
     K K^T, the triangular inverse (in fp32, by blocks), W, U, Q K^T and the decay-scaled copies of Q, K.
@@ -1484,11 +1496,7 @@ def _delta_prepare_kernel(q, k, v, beta, g, scale, C=64, inverse=None):
     N = (T + C - 1) // C
     q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
     bf, dev = torch.bfloat16, q.device
-    # rows of W, Qd, Kd and A as the scan kernels keep them in shared memory: eight more elements than the tile has columns
-    def padded(n):
-        r = C * (n + 8)
-        return torch.empty_strided((B, H, N, C, n), (H * N * r, N * r, r, n + 8, 1), dtype=bf, device=dev)
-    W, Qd, Kd, A = padded(D), padded(D), padded(D), padded(C)
+    W, Qd, Kd, A = _padded_tiles(B, H, N, C, (D, D, D, C), dev)
     U = torch.empty(B, H, N, C, D, dtype=bf, device=dev)
     gamma = torch.empty(B, H, N, dtype=torch.float32, device=dev)
     bt = beta.float().contiguous()

@@ -27,3 +27,15 @@ def test_tensor_map_views():
     for t in (x[:, :, :1].expand(-1, -1, 3, -1), x[:1].expand(2, -1, -1, -1), x.transpose(2, 3), odd):
         c = K._tma_view(t)
         assert c.is_contiguous() and torch.equal(c, t)
+
+
+def test_padded_tiles_own_their_rows():
+    """A scan fetches a tile of C rows of n + 8 elements as one copy: every such row, the last one's end included, is in the tile's
+    storage and in no other tile, and starts where 16-byte copies may."""
+    for B, H, N, C, widths in ((1, 1, 1, 64, (128, 128, 128, 64)), (2, 3, 5, 64, (64, 64, 64, 64))):
+        end = 0
+        for t, n in zip(K._padded_tiles(B, H, N, C, widths, "cpu"), widths):
+            assert t.shape == (B, H, N, C, n) and t.stride() == (H * N * C * (n + 8), N * C * (n + 8), C * (n + 8), n + 8, 1)
+            assert t.storage_offset() >= end and t.storage_offset() % 8 == 0
+            end = t.storage_offset() + B * H * N * C * (n + 8)
+            assert end * t.element_size() <= t.untyped_storage().nbytes()
