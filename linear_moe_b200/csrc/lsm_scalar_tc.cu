@@ -306,7 +306,7 @@ lsm_state_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
 struct __align__(1024) SmemSweep {
     uint8_t t0[2][TILE], t1[2][TILE], t2[2][TILE], sb[TILE];
     float lb[2][CT], tab[2][CT];                    // sums of the log decays; column factors e^{b of the block's last - b_j}
-    uint64_t full[2], empty[2], tab_full[2], tab_empty[2], sb_ready, c1, p_ready, c2, o_full, o_ready;
+    uint64_t full[2], empty[2], tab_full[2], tab_empty[2], sb_ready, c1, p_ready, c2, o_full, o_ready[2];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -330,8 +330,8 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
     volatile int* abort_flag = &sm.abort_flag;
     int* err = a.err;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); mbar_init(&sm.tab_full[s], 1); mbar_init(&sm.tab_empty[s], WARPS); }
-        mbar_init(&sm.sb_ready, WARPS); mbar_init(&sm.p_ready, WARPS); mbar_init(&sm.o_ready, WARPS);
+        for (int s = 0; s < 2; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); mbar_init(&sm.tab_full[s], 1); mbar_init(&sm.tab_empty[s], WARPS); mbar_init(&sm.o_ready[s], WARPS); }
+        mbar_init(&sm.sb_ready, WARPS); mbar_init(&sm.p_ready, WARPS);
         mbar_init(&sm.c1, 1); mbar_init(&sm.c2, 1); mbar_init(&sm.o_full, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -391,7 +391,7 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
         if (ok && n > 1) ok = tables(1);
         for (int i = 0; ok && i < n; ++i) {
             const int s = i & 1;
-            ok = mbar_wait_suspend(&sm.o_ready, i & 1, abort_flag, err, 0x8310);
+            ok = mbar_wait_suspend(&sm.o_ready[s], (i >> 1) & 1, abort_flag, err, 0x8310 | s);
             if (!ok) break;
             if (lane == 0) {
                 tma_store(&tmO, sm.t0[s], h, (c_lo + i) * CT, b);
@@ -462,7 +462,7 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
             }
             fence_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.o_ready);
+            if (lane == 0) mbar_arrive(&sm.o_ready[s]);
         }
     }
     tc_fence_before();
@@ -479,7 +479,7 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
 struct __align__(1024) SmemDkv {
     uint8_t q[2][TILE], g[2][TILE], k[TILE], v[TILE], db[TILE];
     float lb[2][CT], tab[2][CT];                    // sums of the log decays; column factors e^{b_i - b of the block's first}
-    uint64_t qg_full[2], qg_empty[2], k_full, k_empty, v_full, v_empty, tab_full[2], tab_empty[2], db_ready, c1, p_ready, p1_done, acc_full, o_ready;
+    uint64_t qg_full[2], qg_empty[2], k_full, k_empty, v_full, v_empty, tab_full[2], tab_empty[2], db_ready, c1, p_ready, p1_done, acc_full, o_ready[2];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -501,9 +501,9 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     volatile int* abort_flag = &sm.abort_flag;
     int* err = a.err;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; ++s) { mbar_init(&sm.qg_full[s], 1); mbar_init(&sm.qg_empty[s], 1); mbar_init(&sm.tab_full[s], 1); mbar_init(&sm.tab_empty[s], WARPS); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&sm.qg_full[s], 1); mbar_init(&sm.qg_empty[s], 1); mbar_init(&sm.tab_full[s], 1); mbar_init(&sm.tab_empty[s], WARPS); mbar_init(&sm.o_ready[s], WARPS); }
         mbar_init(&sm.k_full, 1); mbar_init(&sm.k_empty, 1); mbar_init(&sm.v_full, 1); mbar_init(&sm.v_empty, 1);
-        mbar_init(&sm.db_ready, WARPS); mbar_init(&sm.p_ready, WARPS); mbar_init(&sm.o_ready, WARPS);
+        mbar_init(&sm.db_ready, WARPS); mbar_init(&sm.p_ready, WARPS);
         mbar_init(&sm.c1, 1); mbar_init(&sm.p1_done, 1); mbar_init(&sm.acc_full, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -583,7 +583,7 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         if (ok && n > 1) ok = tables(1);
         for (int i = 0; ok && i < n; ++i) {
             const int s = i & 1;
-            ok = mbar_wait_suspend(&sm.o_ready, i & 1, abort_flag, err, 0x9310);
+            ok = mbar_wait_suspend(&sm.o_ready[s], (i >> 1) & 1, abort_flag, err, 0x9310 | s);
             if (!ok) break;
             if (lane == 0) {
                 tma_store(&tmDV, sm.g[s], h, (c_last - i) * CT, b);
@@ -667,7 +667,7 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             publish_state();                                                                    // the next chunk's products may start
             fence_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.o_ready);
+            if (lane == 0) mbar_arrive(&sm.o_ready[s]);
         }
     }
     tc_fence_before();

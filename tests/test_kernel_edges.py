@@ -167,6 +167,27 @@ def test_scalar_decay_wide_chunks(T, decay, layout, monkeypatch):
     assert torch.equal(o, got[0][0]) and torch.equal(S, got[0][1])
 
 
+@pytest.mark.parametrize("chunks", [1, 2, 3, 4, 5, 7])
+@pytest.mark.parametrize("decay", ["head", "token"])
+def test_scalar_decay_wide_chunks_in_long_groups(chunks, decay, monkeypatch):
+    """A group that walks `chunks` chunks of 128 tokens and a shorter one behind it with a ragged tail: stages, barrier phases and output
+    buffers are used again, the state and the running decays go from chunk to chunk and from group to group."""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    B, H, D, T = 2, 2, 128, 128 * (2 * chunks - 1) - 37 if chunks > 1 else 200
+    G = -(-T // (128 * chunks))
+    g = -torch.tensor([0.002, 0.1], device="cuda") if decay == "head" else -0.1 * torch.rand(B, T, H, device="cuda")
+    monkeypatch.setattr(K, "_scalar_chunk", lambda *a: 128)
+    monkeypatch.setattr(K, "_scalar_groups", lambda *a: (G, 2 * chunks))
+    x = rand(B, T, H, 3 * D)
+    S0, gS = 0.3 * torch.randn(B, H, D, D, device="cuda"), 0.1 * torch.randn(B, H, D, D, device="cuda")
+    go = rand(B, T, H, D, scale=1)
+    got = run(lambda x, S: ops.lsm_scalar(*x.split(D, dim=-1), g, None, S, 64), [x, S0], [go, gS])
+    gemm.check_error()
+    want = run(lambda x, S: RL.recurrent_lsm(*x.split(D, dim=-1), g=g.expand(B, T, H), initial_state=S), [x.float(), S0], [go.float(), gS])
+    check(got, want, ["o", "S", "dqkv", "dS0"])
+
+
 @pytest.mark.parametrize("kind,D", [("scalar", 64), ("scalar", 128), ("vector", 64), ("vector", 128), ("delta", 128)])
 @pytest.mark.parametrize("T", [2, 200])
 def test_forward_in_one_host_call(kind, D, T):
