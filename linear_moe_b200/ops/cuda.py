@@ -1074,7 +1074,7 @@ class _LsmScalar(torch.autograd.Function):
         o, final, (saved, ctx.gmode, ctx.grid, ctx.lasp) = _scalar_forward(q, k, v, g, scale, init)
         ctx.set_materialize_grads(False)                 # no zeros for an output without a gradient (mostly the final state)
         ctx.save_for_backward(*saved)
-        ctx.scale, ctx.has_init = scale, init is not None
+        ctx.scale, ctx.has_init, ctx.g_input = scale, init is not None, 3
         ctx.g_dtype = None if g is None else g.dtype
         return o, final
 
@@ -1101,7 +1101,7 @@ class _LsmScalar(torch.autograd.Function):
         seed = None if dfinal is None else dfinal.float().contiguous()
         if ctx.lasp is not None:
             # the gradient of the state that leaves this rank arrives from the ranks after it; the decay gradient needs it
-            need_r = ctx.gmode == 2 or (ctx.gmode == 1 and len(ctx.needs_input_grad) > 3 and ctx.needs_input_grad[3])
+            need_r = ctx.gmode == 2 or (ctx.gmode == 1 and ctx.needs_input_grad[ctx.g_input])
             r_out = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device) if need_r else None
             ctx.lasp.combine(1, dstates, gf if ctx.gmode == 1 else None, None, B * H, H, G, cpg, T, D,
                              gdecay=gdecay, dmode=1 if ctx.gmode == 2 else 0, r_out=r_out)
@@ -1118,7 +1118,7 @@ class _LsmScalar(torch.autograd.Function):
             if dfinal is not None:
                 dg = dg + (final * dfinal.float()).sum((-1, -2))[:, None, :]
             dg = dg.to(ctx.g_dtype)
-        elif ctx.gmode == 1 and len(ctx.needs_input_grad) > 3 and ctx.needs_input_grad[3]:
+        elif ctx.gmode == 1 and ctx.needs_input_grad[ctx.g_input]:
             s = (q.float() * dq.float()).sum(-1) - (k.float() * dk.float()).sum(-1)
             dgt = s.flip(1).cumsum(1).flip(1)
             if dfinal is not None:
@@ -1155,7 +1155,9 @@ class _LsmScalarFused(torch.autograd.Function):
     def forward(ctx, qkv, g, scale, init):
         D = qkv.shape[-1] // 3
         q, k, v = qkv[..., :D], qkv[..., D:2 * D], qkv[..., 2 * D:]
-        return _LsmScalar.forward(ctx, q, k, v, g, scale, init)
+        out = _LsmScalar.forward(ctx, q, k, v, g, scale, init)
+        ctx.g_input = 1                                  # where the decays stand among this function's arguments
+        return out
 
     @staticmethod
     def backward(ctx, d_o, dfinal):

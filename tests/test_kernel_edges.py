@@ -188,6 +188,30 @@ def test_scalar_decay_wide_chunks_in_long_groups(chunks, decay, monkeypatch):
     check(got, want, ["o", "S", "dqkv", "dS0"])
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("init", [True, False])
+def test_trained_constant_decays(D, fused, init):
+    """A log decay per head gets its gradient from one fused projection as well as from three tensors, with a trained initial state and
+    without.  Its gradient is a sum over all tokens of differences of two gradients of GRAD each, here of the result's size."""
+    torch.manual_seed(0)
+    B, T, H = 2, 100, 3
+    x, go = rand(B, T, H, 3 * D), rand(B, T, H, D, scale=1)
+    g, S0 = -torch.tensor([0.02, 0.1, 0.4], device="cuda"), 0.3 * torch.randn(B, H, D, D, device="cuda")
+
+    def kernel(x, g, *S):
+        q, k, v = x.split(D, dim=-1)
+        if not fused:
+            q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        return ops.lsm_scalar(q, k, v, g, None, *S)[0]
+
+    def ref(x, g, *S):
+        return RL.recurrent_lsm(*x.split(D, dim=-1), g=g.expand(B, T, H), initial_state=S[0] if S else None)[0]
+    ins = [x, g] + [S0] * init
+    got, want = run(kernel, ins, [go]), run(ref, [t.float() for t in ins], [go.float()])
+    check(([], got[1]), ([], want[1]), ["dqkv", "dg", "dS0"][:len(ins)])
+
+
 @pytest.mark.parametrize("kind,D", [("scalar", 64), ("scalar", 128), ("vector", 64), ("vector", 128), ("delta", 128)])
 @pytest.mark.parametrize("T", [2, 200])
 def test_forward_in_one_host_call(kind, D, T):
