@@ -973,20 +973,24 @@ def lsm_groups(B, H, T):
     return G, cpg
 
 
-def _scalar_chunk(B, T, H, D, g):
+def _scalar_chunk(B, T, H, D):
     """Tokens per chunk: 128 (tensor-core kernels, csrc/lsm_scalar_tc.cu) or 64 (csrc/lsm_scalar.cu).
 
     128 for 128-wide heads from eight chunks per SM on.  Forward and backward of 16 heads take 375 us in chunks of 64 and 212 in chunks
-    of 128 there (9472 tokens); 604 and 305 at 16384, 193 and 123 at 4096, 78 and 72 at 1024, 47 and 61 at 128.  Below the line the
-    gain is 2 % of a model's training step at most, and a change of rounding costs more than that: where a head decays within a few
-    tokens, single elements of a model's embedding gradient move by more than the tensor's root mean square between any two
-    roundings (both forms are equally far from 64-bit results).  Where decays are trained it stays at 64 as well: their gradient is
-    a sum over all later tokens of differences of bf16 products, in which the rounding of another chunking shows as 3 - 4 %.
+    of 128 there (9472 tokens); 604 and 305 at 16384, 193 and 123 at 4096, 78 and 72 at 1024, 47 and 61 at 128.  So the times cross at
+    about one chunk per SM; that the line stands above it is not a matter of speed or error, only of no result below it having been
+    measured in a whole model yet.
+
+    By shapes alone: a training pass and an evaluation of the same tokens have the same bits.  Trained decays need no exception.  Against 64
+    bits, over 200 - 16384 tokens of 16 heads (geometric means of ten seeds), chunks of 64 are off by 0.0025 - 0.0030 (output) and 0.0025 - 0.0032
+    (input gradients), chunks of 128 by 0.0024 - 0.0028 and 0.0024 - 0.0028; the gradient of a decay per token by 0.0095 / 0.0142 / 0.029 /
+    0.063 / 0.079 (200, 512, 2000, 9600, 16384 tokens) and 0.0085 / 0.0130 / 0.025 / 0.055 / 0.071; that of a decay per head, one
+    sum over all tokens, by 0.008 - 0.21 and 0.007 - 0.24, either form ahead by up to a factor of four from seed to seed.
 
     Short sequences of many heads stay at 64 too: up to 192 tokens the chunks of 128 are mostly empty or few.  Forward pass of 170000
     rows, 64 / 128: 16 - 64 tokens 0.85 - 0.87 (256 x 64 tokens of 16 heads 941 and 1098 us), 96 and 128 tokens 0.95, 192 tokens 0.98; 224 tokens
     1.09, 384 tokens 1.23; forward and backward: 0.86, 1.0, 1.04, 1.18, 1.33."""
-    return 128 if D == 128 and T > 192 and B * H * T >= 8 * 128 * num_sms() and not (g is not None and g.requires_grad) else 64
+    return 128 if D == 128 and T > 192 and B * H * T >= 8 * 128 * num_sms() else 64
 
 
 def _scalar_groups(B, H, T, chunk):
@@ -1046,7 +1050,7 @@ def _scalar_forward(q, k, v, g, scale, init):
     """Returns the output, the final state and what the backward pass needs: (tensors, gmode, (groups, chunks, tokens of a
     chunk), exchange)."""
     B, T, H, D = q.shape
-    chunk = _scalar_chunk(B, T, H, D, g)
+    chunk = _scalar_chunk(B, T, H, D)
     fix = _tma_view if chunk == 128 else _inner_contig
     q, k, v = fix(q), fix(k), fix(v)
     gmode = 0 if g is None else (1 if g.dim() == 1 else 2)

@@ -6,13 +6,12 @@ from linear_moe_b200.ops import cuda as K
 
 def test_scalar_decay_chunk_rule(monkeypatch):
     monkeypatch.setattr(K, "num_sms", lambda: 148)
-    g, line = torch.zeros(2, 8, 3), 8 * 128 * 148
-    assert K._scalar_chunk(1, line, 1, 128, None) == K._scalar_chunk(4, -(-line // 16), 4, 128, g) == 128
-    assert K._scalar_chunk(1, line - 1, 1, 128, None) == K._scalar_chunk(1, line, 1, 64, None) == 64
-    assert K._scalar_chunk(1, line, 1, 128, g.clone().requires_grad_(True)) == 64
+    line = 8 * 128 * 148
+    assert K._scalar_chunk(1, line, 1, 128) == K._scalar_chunk(4, -(-line // 16), 4, 128) == 128
+    assert K._scalar_chunk(1, line - 1, 1, 128) == K._scalar_chunk(1, line, 1, 64) == 64
     for T in (1, 16, 64, 128, 192):                             # short sequences, however many heads
-        assert K._scalar_chunk(256, T, 1000, 128, None) == 64
-    assert K._scalar_chunk(256, 193, 1000, 128, None) == 128
+        assert K._scalar_chunk(256, T, 1000, 128) == 64
+    assert K._scalar_chunk(256, 193, 1000, 128) == 128
     for chunk in (64, 128):                                     # every token in exactly one group, no group empty
         for BH in (1, 3, 16, 148, 1000):
             for T in list(range(1, 400)) + [4096, 16384, 100003]:

@@ -212,6 +212,56 @@ def test_trained_constant_decays(D, fused, init):
     check(([], got[1]), ([], want[1]), ["dqkv", "dg", "dS0"][:len(ins)])
 
 
+@pytest.mark.parametrize("decay", ["head", "token"])
+@pytest.mark.parametrize("B,T,H", [(1, 9500, 16), (3, 200, 256), (1, 38001, 4)])
+def test_scalar_decay_above_the_line(B, T, H, decay):
+    """The wide chunks as the rule takes them, over several waves of groups, with trained decays: outputs and gradients against the chunked
+    recurrence in 64 bits, and the same bits in training and in evaluation.  A log decay's gradient at t is the sum over i >= t of
+    q_i . dq_i - k_i . dk_i, whose products carry independent relative errors of GRAD at most: a random walk of that step."""
+    torch.manual_seed(0)
+    D = 128
+    assert K._scalar_chunk(B, T, H, D) == 128
+    x, go = rand(B, T, H, 3 * D), rand(B, T, H, D, scale=1)
+    a = torch.linspace(-4, 0, H, device="cuda")
+    a = (a if decay == "head" else a + torch.randn(B, T, H, device="cuda")).requires_grad_(True)
+    x1 = x.clone().requires_grad_(True)
+
+    def f(x, a):
+        q, k, v = x.split(D, dim=-1)
+        return ops.lsm_scalar(q, k, v, -torch.exp(a), None, None, 64)
+    o, S = f(x1, a)
+    dx, da = torch.autograd.grad(o, [x1, a], go)
+    with torch.no_grad():
+        o2, S2 = f(x, a)
+    assert torch.equal(o, o2) and torch.equal(S, S2)
+    for h in range(0, H, max(1, H // 4)):                       # four heads: the recurrence in 64 bits is slow
+        xs = x[:, :, h].double().requires_grad_(True)
+        ah = (a[h] if decay == "head" else a[..., h]).detach().double().requires_grad_(True)
+        g = -torch.exp(ah)
+        q, k, v = xs.split(D, dim=-1)
+        want, state = chunked64(q * D ** -0.5, k, v, g.expand(B, T))
+        dxs, dah = torch.autograd.grad(want, [xs, ah], go[:, :, h].double())
+        assert rel(o[:, :, h], want) < OUT and rel(S[:, h], state) < OUT and rel(dx[:, :, h], dxs) < GRAD
+        dq, dk, _ = dxs.split(D, dim=-1)
+        step = ((q * dq).square() + (k * dk).square()).sum(-1).detach()                               # [B, T]
+        if decay == "token":
+            walk = step.flip(1).cumsum(1).flip(1).sqrt()
+        else:                                                   # the term of token i is in the sums of tokens 0 .. i
+            walk = (step * torch.arange(1, T + 1, device="cuda").double().square()).sum().sqrt()
+        assert (da[..., h] - dah).norm() < GRAD * (walk * g.detach()).norm()
+
+
+def chunked64(q, k, v, g, C=100):
+    """The scalar-decay recurrence for one head [B, T, D], decays [B, T], C tokens at a time."""
+    S, out = q.new_zeros(q.shape[0], q.shape[-1], v.shape[-1]), []
+    for t in range(0, q.shape[1], C):
+        Q, K_, V, b = q[:, t:t + C], k[:, t:t + C], v[:, t:t + C], g[:, t:t + C].cumsum(1)
+        decays = (b[:, :, None] - b[:, None, :]).tril().exp().tril()
+        out.append(((Q @ K_.mT) * decays) @ V + b.exp()[..., None] * (Q @ S))
+        S = b[:, -1].exp()[:, None, None] * S + (K_ * (b[:, -1:] - b).exp()[..., None]).mT @ V
+    return torch.cat(out, 1), S
+
+
 @pytest.mark.parametrize("kind,D", [("scalar", 64), ("scalar", 128), ("vector", 64), ("vector", 128), ("delta", 128)])
 @pytest.mark.parametrize("T", [2, 200])
 def test_forward_in_one_host_call(kind, D, T):
