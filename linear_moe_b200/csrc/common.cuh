@@ -107,6 +107,13 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // Ahead of pdl_trigger, so that whatever starts early behind it still finds everything older than this kernel complete.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// SMs of the current device.
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return n;
+}
+
 // A launch that may start while the kernel before it in the stream is running, if that one calls pdl_trigger.  The small kernels between the
 // weight-streaming products of a decode step go out this way: their blocks are in place when the product ends.
 template <typename T> struct launch_arg { using type = T; };

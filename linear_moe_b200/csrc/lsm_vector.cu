@@ -17,7 +17,7 @@
 //   dS <- diag(e^{b_m}) [ diag(e^{b_C - b_m}) dS + scale q~^T dO ]
 // The gate gradient is d g = reverse-cumsum_t (q . dq - k . dk) per channel (the kernels at the end of this file).
 //
-// 512 threads, one CTA per SM: a warp owns 16 rows of every product and a quarter of its columns (of the state: half or a quarter).  For the
+// 512 threads, one CTA per SM (two where 64-wide heads have more CTAs than SMs): a warp owns 16 rows of every product and a quarter of its columns (of the state: half or a quarter).  For the
 // gates a thread owns two channels and VCH / GR consecutive tokens: running sums stay in registers, the GR groups of tokens meet in one
 // small table, and the next chunk's gates and tiles are on their way while this one is worked on.  (With eight warps, single buffers and a
 // 64-step running sum in 128 threads the chunks were bound by latency.)  8 x 2048 tokens, 8 heads of 128: outputs 135 -> 97 us, dq
@@ -173,8 +173,8 @@ __device__ __forceinline__ void load_state_regs(const float* src, float (&acc)[V
 // 1. group summaries.  REV = 0: S <- diag(e^{b_C}) S + (K e^{b_C - b})^T V (ascending chunks)
 //                      REV = 1: dS <- diag(e^{b_C}) dS + (Q e^{b} scale)^T dO (descending chunks)
 // ---------------------------------------------------------------------------------------------
-template <int D, int REV>
-__global__ void __launch_bounds__(VTHREADS, 1) gla_state_scan_kernel(GlaArgs a) {
+template <int D, int REV, int CTAS>
+__global__ void __launch_bounds__(VTHREADS, CTAS) gla_state_scan_kernel(GlaArgs a) {
     using C = VCfg<D>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* Xs = reinterpret_cast<bf16*>(smem_raw);                  // [2][VCH][LD]
@@ -284,8 +284,8 @@ __global__ void gla_combine_kernel(float* __restrict__ states, const float* __re
 // ---------------------------------------------------------------------------------------------
 // 3a. forward output (MODE 0) / backward dq (MODE 1): forward sweep carrying S.
 // ---------------------------------------------------------------------------------------------
-template <int D, int MODE>
-__global__ void __launch_bounds__(VTHREADS, 1) gla_fwd_sweep_kernel(GlaArgs a) {
+template <int D, int MODE, int CTAS>
+__global__ void __launch_bounds__(VTHREADS, CTAS) gla_fwd_sweep_kernel(GlaArgs a) {
     using C = VCfg<D>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* tiles = reinterpret_cast<bf16*>(smem_raw);               // [2] x { q (mode 0) | dO (mode 1), k, v }
@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(VTHREADS, 1) gla_fwd_sweep_kernel(GlaArgs a) {
 // ---------------------------------------------------------------------------------------------
 // 3b. backward dk, dv: reverse sweep carrying dS.
 // ---------------------------------------------------------------------------------------------
-template <int D>
-__global__ void __launch_bounds__(VTHREADS, 1) gla_bwd_dkv_kernel(GlaArgs a) {
+template <int D, int CTAS>
+__global__ void __launch_bounds__(VTHREADS, CTAS) gla_bwd_dkv_kernel(GlaArgs a) {
     using C = VCfg<D>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* tiles = reinterpret_cast<bf16*>(smem_raw);                // [2] x { q, k, v, dO }
@@ -497,9 +497,8 @@ template <int D> constexpr size_t gla_smem_dkv() {
 
 using namespace lmoe;
 
-// which: 0 forward state scan, 1 reverse state scan, 2 forward output, 3 backward dq, 4 backward dk/dv
-LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t st) {
-    const GlaArgs a = *ap;
+template <int D, int CTAS>
+static int gla_launch(int which, const GlaArgs& a, cudaStream_t st) {
     dim3 grid(a.G, a.B * a.H);
 #define GLAUNCH(KERNEL, SMEM)                                                                              \
     do {                                                                                                   \
@@ -507,23 +506,24 @@ LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t s
         if (rc) return rc;                                                                                 \
         KERNEL<<<grid, VTHREADS, SMEM, st>>>(a);                                                           \
     } while (0)
-    if (D == 128) {
-        if (which == 0) GLAUNCH((gla_state_scan_kernel<128, 0>), gla_smem_scan<128>());
-        else if (which == 1) GLAUNCH((gla_state_scan_kernel<128, 1>), gla_smem_scan<128>());
-        else if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<128, 0>), gla_smem_sweep<128>());
-        else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<128, 1>), gla_smem_sweep<128>());
-        else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<128>), gla_smem_dkv<128>());
-        else return -1;
-    } else if (D == 64) {
-        if (which == 0) GLAUNCH((gla_state_scan_kernel<64, 0>), gla_smem_scan<64>());
-        else if (which == 1) GLAUNCH((gla_state_scan_kernel<64, 1>), gla_smem_scan<64>());
-        else if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<64, 0>), gla_smem_sweep<64>());
-        else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<64, 1>), gla_smem_sweep<64>());
-        else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<64>), gla_smem_dkv<64>());
-        else return -1;
-    } else return -2;
+    if (which == 0) GLAUNCH((gla_state_scan_kernel<D, 0, CTAS>), gla_smem_scan<D>());
+    else if (which == 1) GLAUNCH((gla_state_scan_kernel<D, 1, CTAS>), gla_smem_scan<D>());
+    else if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<D, 0, CTAS>), gla_smem_sweep<D>());
+    else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<D, 1, CTAS>), gla_smem_sweep<D>());
+    else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<D, CTAS>), gla_smem_dkv<D>());
+    else return -1;
 #undef GLAUNCH
     return (int)cudaGetLastError();
+}
+
+// which: 0 forward state scan, 1 reverse state scan, 2 forward output, 3 backward dq, 4 backward dk/dv
+LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t st) {
+    if (D == 128) return gla_launch<128, 1>(which, *ap, st);
+    if (D != 64) return -2;
+    // 64-wide heads, more CTAs than SMs: two per SM with 64 registers a thread overlap each other's steps.  Outputs, one and two per SM:
+    // 64 x 256 tokens of 16 heads 216 and 185 us, 64 x 128 144 and 123, 32 x 64 56 and 50; where every CTA has an SM to itself the
+    // registers are worth more (8 x 2048 of 8 heads, 128 CTAs: 81 and 91).
+    return (long long)ap->G * ap->B * ap->H > sm_count() ? gla_launch<64, 2>(which, *ap, st) : gla_launch<64, 1>(which, *ap, st);
 }
 
 LMOE_API int lmoe_gla_combine(int rev, float* states, const float* gdecay, const float* seed, float* final_out, int BH,

@@ -108,6 +108,29 @@ def test_vector_decay_chunk_edges(D, T):
     check(got, want, ["o", "S", "dq", "dk", "dv", "dg", "dS0"])
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,chunks", [(2, 2, 1), (2, 2, 2), (2, 2, 3), (2, 2, 4), (2, 2, 5), (2, 2, 7), (40, 4, 1), (40, 4, 3)])
+def test_vector_decay_long_groups(B, H, chunks, D, monkeypatch):
+    """A group that walks `chunks` chunks of 64 tokens and a shorter one behind it with a ragged tail: double-buffered tiles, sums and
+    tables are used again.  160 sequences are more than an SM has CTAs of 64-wide heads.  The decays' gradient as in
+    test_scalar_decay_above_the_line, per channel."""
+    torch.manual_seed(0)
+    T = 64 * (2 * chunks - 1) - 19 if chunks > 1 else 100
+    G = -(-T // (64 * chunks))
+    monkeypatch.setattr(K, "lsm_groups", lambda *a: (G, chunks))
+    x, go = rand(B, T, H, 3 * D), rand(B, T, H, D, scale=1)
+    g = torch.nn.functional.logsigmoid(2 * torch.randn(B, T, H, D, device="cuda")) / 4
+    S0 = 0.3 * torch.randn(B, H, D, D, device="cuda")
+    got = run(lambda x, g, S: ops.lsm_vector(*x.split(D, dim=-1), g, None, S, None, 64), [x, g, S0], [go])
+    want = run(lambda x, g, S: RL.recurrent_lsm(*x.split(D, dim=-1), gk=g, initial_state=S), [x.float(), g, S0], [go.float()])
+    (dx, dg, dS), (wx, wg, wS) = got[1], want[1]
+    check((got[0], [dx, dS]), (want[0], [wx, wS]), ["o", "S", "dqkv", "dS0"])
+    q, k, _ = x.float().split(D, dim=-1)
+    dq, dk, _ = wx.split(D, dim=-1)
+    walk = ((q * dq).square() + (k * dk).square()).flip(1).cumsum(1).sqrt()
+    assert (dg - wg).norm() < GRAD * walk.norm()
+
+
 @pytest.mark.parametrize("h,f", [(128, 8), (200, 120), (256, 136), (512, 264)])
 @pytest.mark.parametrize("counts", [[512, 0, 256], [0, 0, 768], [256, 1024, 0]])
 def test_expert_mlp_epilogues(h, f, counts):
