@@ -2,15 +2,20 @@
 //
 // With a handful of rows the product is bound by reading W once (2 N K bytes); a 256 x 256 tensor-core tile would spend
 // its time on rows that do not exist.  Here a CTA owns 16 rows of W at a time and its eight warps split K.  Every lane brings
-// 16-byte pieces of two W rows into slots of shared memory of its own and from there, with one x row, into mma.sync.m16n8k16
+// 16-byte pieces of two W rows (into slots of shared memory of its own, or registers) and, with one x row, on into mma.sync.m16n8k16
 // fragments: the sum over k does not care about the order of k, so the eight consecutive elements a lane loads are used as the
 // k slots that lane owns in two MMA steps (the same assignment for the W and the x fragment), and nothing is transposed or
 // exchanged.  The eight partial tiles are added through shared memory.  No atomics: results are deterministic.
-// Two CTAs per SM walk the row blocks with 64 KB of copies in flight each, over the ends of row blocks too.  (One CTA per row block,
-// its loads in registers, drained the memory system at every block's end: W of 128256 x 2048 96 us, now 91, 16384 x 2048 16.4, now
-// 13.5.)  The kernel is launched with programmatic stream serialization: its first eight steps of W are in flight before it waits
-// for the kernel that produces x, so consecutive linears of a decode step keep HBM busy across the kernel boundaries (the small
-// kernels in between call griddepcontrol.launch_dependents at their start).
+// Two kernels differ in how W arrives, and give the same bits:
+//   gemm_skinny_kernel        two CTAs per SM walk the row blocks with 64 KB of copies in flight each, over the ends of row blocks too.
+//                             For many row blocks of short rows: a CTA per row block drains the memory system at every block's end.
+//                             (W of 128256 x 2048 96 us with a CTA per block, 91 so; 16384 x 2048 16.4 and 13.5.)
+//   gemm_skinny_block_kernel  a CTA (or cluster) per row block, its loads in registers.  For long rows, where the loop over K is what counts
+//                             (W of 32000 x 4096 50 us on the first kernel, 43 so; 8192 x 8192 27.9 and 23.8), and for few row blocks, where
+//                             there is no next block to copy for (2560 x 1024 behind a norm kernel 8.4 and 7.4).
+// use_ring below has the rule.  Both are launched with programmatic stream serialization: their first eight steps of W are in flight
+// before they wait for the kernel that produces x, so consecutive linears of a decode step keep HBM busy across the kernel
+// boundaries (the small kernels in between call griddepcontrol.launch_dependents at their start).
 #include <cstdlib>
 
 #include "common.cuh"
@@ -19,6 +24,7 @@
 namespace lmoe {
 namespace sk {
 
+__device__ __forceinline__ uint4 ld_stream(const bf16* p) { return __ldcs(reinterpret_cast<const uint4*>(p)); }
 // 16 bytes of global memory to shared memory, zeros where `ok` is false
 __device__ __forceinline__ void copy16(uint32_t dst, const bf16* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
@@ -52,12 +58,67 @@ __device__ __forceinline__ void put(void* y, long long i, float v) {
     else reinterpret_cast<float*>(y)[i] += v;
 }
 
+constexpr int PF = 8, STEP = 256;                                        // steps in flight; elements of K per step of the eight warps
+__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16(v)); }
+
+// The eight warps' partial tiles of a row block, added up and stored.
+template <int NTILES, int KS, int OUT>
+__device__ __forceinline__ void finish_block(const float (&acc)[NTILES][4], float (*red)[NTILES][32][4], float (*cred)[NTILES][32][4], uint32_t crank,
+                                             int row_lo, void* y, long long ldy, int M, int N) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, q = l & 3;
+    const int row_hi = row_lo + 8;
+    const bool lo_ok = row_lo < N, hi_ok = row_hi < N;
+#pragma unroll
+    for (int t = 0; t < NTILES; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) red[w][t][l][e] = acc[t][e];
+    __syncthreads();
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    if (w < NTILES) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] += red[i][w][l][e];
+    }
+    if (KS > 1) {
+        // the CTA's partial tile goes to slot `crank` of the first CTA; it adds the slots in rank order (deterministic)
+        if (w < NTILES) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) st_cluster_f32(&cred[crank][w][l][e], 0, s[e]);
+        }
+        sk_cluster_sync();
+        if (crank != 0) return;
+        if (w < NTILES) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                s[e] = 0.f;
+#pragma unroll
+                for (int i = 0; i < KS; ++i) s[e] += cred[i][w][l][e];
+            }
+        }
+    }
+    if (w < NTILES) {
+        const int n0 = 8 * w + 2 * q;                                   // batch rows n0, n0 + 1
+        if (OUT == OUT_SWIGLU) {                                        // of gate and up in bf16, as where they pass through memory
+            if (lo_ok && n0 < M) put<OUT_BF16>(y, (long long)n0 * ldy + row_lo, silu_f(bf16_round(s[0])) * bf16_round(s[2]));
+            if (lo_ok && n0 + 1 < M) put<OUT_BF16>(y, (long long)(n0 + 1) * ldy + row_lo, silu_f(bf16_round(s[1])) * bf16_round(s[3]));
+            return;
+        }
+        if (n0 < M) {
+            if (lo_ok) put<OUT>(y, (long long)n0 * ldy + row_lo, s[0]);
+            if (hi_ok) put<OUT>(y, (long long)n0 * ldy + row_hi, s[2]);
+        }
+        if (n0 + 1 < M) {
+            if (lo_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_lo, s[1]);
+            if (hi_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_hi, s[3]);
+        }
+    }
+}
+
 // A CTA, or a cluster of KS that split K, takes row blocks blockIdx.x / KS, + gridDim.x / KS, ...  A lane's pieces of W go through PF slots of
 // shared memory that only this lane writes and reads, so nothing but its own copies is waited for, and the next steps' copies stay
 // in flight over the reduction and the store of a row block.
 // ONE: a lane's piece of x (K / KS at most PF steps) stays in registers.
-constexpr int PF = 8, STEP = 256;                                        // slots; elements of K per step of the eight warps
-__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
 template <int NTILES, int KS, int OUT, bool ONE>
 __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long long ldx, const bf16* W,
@@ -113,8 +174,7 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long
     }
     int slot = 0, buf = 0;
     for (int block = blockIdx.x / KS; block < blocks; block += stride, buf ^= 1) {
-        const int row_lo = block * ROWS<OUT> + g, row_hi = row_lo + 8;
-        const bool lo_ok = row_lo < N, hi_ok = row_hi < N;
+        const int row_lo = block * ROWS<OUT> + g;
         float acc[NTILES][4];
 #pragma unroll
         for (int t = 0; t < NTILES; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
@@ -150,69 +210,82 @@ __global__ void __launch_bounds__(256, 2) gemm_skinny_kernel(const bf16* x, long
                 use(b);
             }
         }
-#pragma unroll
-        for (int t = 0; t < NTILES; ++t)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) red[buf][w][t][l][e] = acc[t][e];
-        __syncthreads();
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-        if (w < NTILES) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[e] += red[buf][i][w][l][e];
-        }
-        if (KS > 1) {
-            // the CTA's partial tile goes to slot `crank` of the first CTA; it adds the slots in rank order (deterministic)
-            if (w < NTILES) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) st_cluster_f32(&cred[buf][crank][w][l][e], 0, s[e]);
-            }
-            sk_cluster_sync();
-            if (crank != 0) continue;
-            if (w < NTILES) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    s[e] = 0.f;
-#pragma unroll
-                    for (int i = 0; i < KS; ++i) s[e] += cred[buf][i][w][l][e];
-                }
-            }
-        }
-        if (w < NTILES) {
-            const int n0 = 8 * w + 2 * q;                                   // batch rows n0, n0 + 1
-            if (OUT == OUT_SWIGLU) {                                        // of gate and up in bf16, as where they pass through memory
-                if (lo_ok && n0 < M) put<OUT_BF16>(y, (long long)n0 * ldy + row_lo, silu_f(bf16_round(s[0])) * bf16_round(s[2]));
-                if (lo_ok && n0 + 1 < M) put<OUT_BF16>(y, (long long)(n0 + 1) * ldy + row_lo, silu_f(bf16_round(s[1])) * bf16_round(s[3]));
-                continue;
-            }
-            if (n0 < M) {
-                if (lo_ok) put<OUT>(y, (long long)n0 * ldy + row_lo, s[0]);
-                if (hi_ok) put<OUT>(y, (long long)n0 * ldy + row_hi, s[2]);
-            }
-            if (n0 + 1 < M) {
-                if (lo_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_lo, s[1]);
-                if (hi_ok) put<OUT>(y, (long long)(n0 + 1) * ldy + row_hi, s[3]);
-            }
-        }
+        finish_block<NTILES, KS, OUT>(acc, red[buf], cred[buf], crank, row_lo, y, ldy, M, N);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// A CTA, or a cluster of KS that split K, per row block.  The first PF steps of W are requested ahead of the wait for x.
+template <int NTILES, int KS, int OUT>
+__global__ void __launch_bounds__(256) gemm_skinny_block_kernel(const bf16* x, long long ldx, const bf16* W, long long ldw, void* y, long long ldy,
+                                                                int M, int N, int K) {
+    __shared__ float red[8][NTILES][32][4];
+    __shared__ float cred[KS][NTILES][32][4];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int g = l >> 2, q = l & 3;
+    const uint32_t crank = KS > 1 ? sk_cluster_rank() : 0;
+    const int row_lo = (blockIdx.x / KS) * ROWS<OUT> + g, row_hi = OUT == OUT_SWIGLU ? row_lo + N : row_lo + 8;
+    const bool lo_ok = row_lo < N, hi_ok = OUT == OUT_SWIGLU ? lo_ok : row_hi < N;
+    const bf16* w_lo = W + (long long)(lo_ok ? row_lo : 0) * ldw + q * 8;
+    const bf16* w_hi = W + (long long)(hi_ok ? row_hi : 0) * ldw + q * 8;
+    const bf16* xr[NTILES];
+    bool x_ok[NTILES];
+#pragma unroll
+    for (int t = 0; t < NTILES; ++t) {
+        x_ok[t] = g + 8 * t < M;
+        xr[t] = x + (long long)(x_ok[t] ? g + 8 * t : 0) * ldx + q * 8;
+    }
+    float acc[NTILES][4];
+#pragma unroll
+    for (int t = 0; t < NTILES; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const int kslice = K / KS;                                           // a multiple of 32 (checked by the launcher)
+    const int k_beg = (int)crank * kslice + w * 32, k_end = (int)(crank + 1) * kslice;
+    uint4 a_lo[PF], a_hi[PF];
+#pragma unroll
+    for (int i = 0; i < PF; ++i) {
+        const int k = k_beg + i * STEP;
+        a_lo[i] = lo_ok && k < k_end ? ld_stream(w_lo + k) : zero;
+        a_hi[i] = hi_ok && k < k_end ? ld_stream(w_hi + k) : zero;
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     // the next kernel may start its own loads
+    // x is complete and visible from here on.  (No pointer of this kernel is __restrict__: loads through those may move ahead of the wait.)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    auto use = [&](const uint4& lo, const uint4& hi, int k) {
+        const uint32_t f1[4] = {lo.x, hi.x, lo.y, hi.y};
+        const uint32_t f2[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+        for (int t = 0; t < NTILES; ++t) {
+            const uint4 b = x_ok[t] ? *reinterpret_cast<const uint4*>(xr[t] + k) : zero;
+            mma16816(acc[t], f1, b.x, b.y);
+            mma16816(acc[t], f2, b.z, b.w);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < PF; ++i)
+        if (k_beg + i * STEP < k_end) use(a_lo[i], a_hi[i], k_beg + i * STEP);
+#pragma unroll 4
+    for (int k = k_beg + PF * STEP; k < k_end; k += STEP)
+        use(lo_ok ? ld_stream(w_lo + k) : zero, hi_ok ? ld_stream(w_hi + k) : zero, k);
+    finish_block<NTILES, KS, OUT>(acc, red, cred, crank, row_lo, y, ldy, M, N);
+}
+
 template <int NTILES, int KS, int OUT>
 static int launch_skinny(const bf16* x, long long ldx, const bf16* W, long long ldw, void* y, long long ldy, int M, int N, int K,
-                         int sms, cudaStream_t st) {
-    const int row_blocks = (N + ROWS<OUT> - 1) / ROWS<OUT>, blocks = min(row_blocks, 2 * sms / KS) * KS;       // two CTAs per SM
-    constexpr int SMEM = PF * 8192;
-    const bool one = K / KS <= PF * STEP;
-    const auto kernel = one ? gemm_skinny_kernel<NTILES, KS, OUT, true> : gemm_skinny_kernel<NTILES, KS, OUT, false>;
-    const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (rc) return rc;
+                         int sms, bool ring, cudaStream_t st) {
+    const int row_blocks = (N + ROWS<OUT> - 1) / ROWS<OUT>;
+    auto kernel = gemm_skinny_block_kernel<NTILES, KS, OUT>;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
+    cfg.gridDim = dim3(row_blocks * KS);
     cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = SMEM;
     cfg.stream = st;
+    if (ring) {
+        kernel = K / KS <= PF * STEP ? gemm_skinny_kernel<NTILES, KS, OUT, true> : gemm_skinny_kernel<NTILES, KS, OUT, false>;
+        cfg.gridDim = dim3(min(row_blocks, 2 * sms / KS) * KS);          // two CTAs per SM
+        cfg.dynamicSmemBytes = PF * 8192;
+        const int rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF * 8192);
+        if (rc) return rc;
+    }
     cudaLaunchAttribute attr[2];
     int na = 0;
     // the kernel may start while its predecessor in the stream is still running; it waits (griddepcontrol.wait) before it
@@ -235,21 +308,31 @@ static int launch_skinny(const bf16* x, long long ldx, const bf16* W, long long 
     return (int)cudaLaunchKernelEx(&cfg, kernel, x, ldx, W, ldw, y, ldy, M, N, K);
 }
 
+// Copies across row blocks (gemm_skinny_kernel) or a CTA per row block (gemm_skinny_block_kernel)?  Times in us, block / ring, of a small norm kernel
+// and the product that follows it, W from memory, as decode steps have them:
+//   K not split: the ring from the second wave of row blocks on while rows are short.  8 rows of x, 32000 of W: K = 1024 17.6 / 13.5, 2048 28.1 /
+//     23.8, 3072 41.0 / 44.2, 4096 49.7 / 56.9; 8192 of W: K = 2048 11.9 / 9.1, 3072 15.7 / 15.0, 4096 18.3 / 18.3, 8192 29.9 / 32.9, 14336 46.8 / 55.7;
+//     16 rows of x, 32000 of W: K = 3072 46.7 / 43.3, 4096 56.7 / 55.0.  One wave (4736 of W): K = 1024 4.9 / 5.2, 4096 12.2 / 13.7.
+//   K over a cluster: the ring where a CTA's slice of K is worth its slots, and while that fits them or clusters have two row blocks at most.  8 rows of x,
+//     2560 of W: K = 1024 7.4 / 8.4, 2048 8.7 / 9.7, 3072 10.8 / 10.3, 8192 18.3 / 15.3, 11008 25.8 / 29.1; 512 of W: K = 1024 3.5 / 3.5, 2048 4.0 /
+//     3.6; 2048 of W: K = 1024 5.9 / 6.0, 2048 6.8 / 7.0 (but a decode step of four 2048-wide layers 321 / 317), 8192 15.5 / 11.8, 14336 23.2 / 20.4.
+static bool use_ring(int M, int K, int row_blocks, int sms, bool split) {
+    if (split) return row_blocks <= sms ? K >= 2048 : K > 2560 && K <= 4 * PF * STEP;
+    return row_blocks > 2 * sms && (K <= 2560 || (K <= 4096 && (M > 8 || row_blocks <= 4 * sms)) || (K <= 5120 && row_blocks <= 3 * sms));
+}
+
 template <int OUT>
 static int dispatch(const bf16* x, long long ldx, const bf16* W, long long ldw, void* y, long long ldy, int M, int N, int K,
                     cudaStream_t st) {
-    // few row blocks: the four CTAs of a cluster split K so that the whole GPU streams W.  Clusters walk the row blocks too: as 512 CTAs in two waves
-    // W of 2048 x 2048 and 2048 x 8192 cost a decode step of four layers 6 us of 318 more than with the copies of both rounds in flight at once.
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    }
-    const bool split = (N + ROWS<OUT> - 1) / ROWS<OUT> < 2 * sms && K % 128 == 0;
-    if (M <= 8) return split ? launch_skinny<1, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st)
-                             : launch_skinny<1, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st);
-    return split ? launch_skinny<2, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st)
-                 : launch_skinny<2, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, st);
+    static const int sms = sm_count();
+    // few row blocks: the four CTAs of a cluster split K so that the whole GPU streams W
+    const int row_blocks = (N + ROWS<OUT> - 1) / ROWS<OUT>;
+    const bool split = row_blocks < 2 * sms && K % 128 == 0;
+    const bool ring = use_ring(M, K, row_blocks, sms, split);
+    if (M <= 8) return split ? launch_skinny<1, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, ring, st)
+                             : launch_skinny<1, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, ring, st);
+    return split ? launch_skinny<2, 4, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, ring, st)
+                 : launch_skinny<2, 1, OUT>(x, ldx, W, ldw, y, ldy, M, N, K, sms, ring, st);
 }
 
 }  // namespace sk

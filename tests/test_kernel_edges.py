@@ -327,6 +327,21 @@ def test_weight_streaming_edges(M, N, k):
     assert rel(acc, want) < 1e-5                                # fp32 sums of exact products: sqrt(K) 2^-24, K up to 8320
 
 
+@pytest.mark.parametrize("M,k,few,many", [(8, 2048, 4736, 4752), (16, 4096, 4736, 4752), (3, 2560, 4736, 8192), (8, 4224, 1024, 5400), (16, 4224, 1024, 2064),
+                                          (16, 8192, 512, 2048), (8, 9088, 1024, 2400), (8, 11008, 2368, 2384), (5, 96, 4000, 4800)])
+def test_weight_streaming_routes(M, k, few, many):
+    """A CTA per row block or row blocks walked with copies across their ends: the rule takes one for `few` rows of W and, for most of these, the
+    other for `many`, and the columns that both have are the same bits where K is split alike (else within the rounding of a result)."""
+    torch.manual_seed(0)
+    x, w = rand(M, k, scale=1), rand(many, k, scale=k ** -0.5)
+    a, b = K.linear_skinny(x, w[:few]), K.linear_skinny(x, w)
+    split = [(n + 15) // 16 < 2 * K.num_sms() and k % 128 == 0 for n in (few, many)]
+    assert torch.equal(a, b[:, :few]) if split[0] == split[1] else rel(a, b[:, :few]) < OUT
+    assert rel(b, x.double() @ w.double().t()) < OUT
+    for n in (few, many):
+        assert torch.equal(K.linear_skinny_swiglu(x, w[:n]), K.swiglu(K.linear_skinny(x, w[:n])))
+
+
 @pytest.mark.parametrize("M", [1, 8, 9, 16])
 @pytest.mark.parametrize("F,K_", [(8, 32), (24, 2048), (2504, 2048), (2400, 4096), (5000, 96)])
 def test_weight_streaming_swiglu(M, F, K_):
