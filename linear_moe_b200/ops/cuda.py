@@ -961,8 +961,14 @@ class _LsmArgs(ctypes.Structure):
 def _inner_contig(t):
     """Kernels need unit stride in the last dim and 16-byte aligned rows; other strides are free."""
     if t.stride(-1) != 1 or any(s % 8 for s in t.stride()[:-1]) or t.data_ptr() % 16:
-        return t.contiguous()
+        return _aligned(t)
     return t
+
+
+def _aligned(t):
+    """Contiguous and from a 16-byte boundary on: a contiguous view into a larger buffer need not start on one."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
 
 
 def lsm_groups(B, H, T):
@@ -1012,7 +1018,7 @@ def _scalar_groups(B, H, T, chunk):
 def _tma_view(t):
     """As :func:`_inner_contig`, for kernels that read through tensor maps: no repeated (stride zero) dimensions either."""
     if any(s <= 0 for s, n in zip(t.stride(), t.shape) if n > 1):
-        return t.contiguous()
+        return _aligned(t)
     return _inner_contig(t)
 
 
@@ -1091,7 +1097,7 @@ class _LsmScalar(torch.autograd.Function):
         q, k, v, gf, states, gdecay, final = ctx.saved_tensors
         B, T, H, D = q.shape
         G, cpg, chunk = ctx.grid
-        d_o = torch.zeros(B, T, H, D, dtype=q.dtype, device=q.device) if d_o is None else d_o.contiguous()
+        d_o = torch.zeros(B, T, H, D, dtype=q.dtype, device=q.device) if d_o is None else _aligned(d_o)
         if d_o.dtype != q.dtype:
             d_o = d_o.to(q.dtype)
         # dq | dk | dv are written straight into one [B,T,H,3D] buffer: when q,k,v were views of a fused
@@ -1257,7 +1263,7 @@ def _vector_forward(q, k, v, gk, scale, init):
     """Returns the output, the final state and what the backward pass needs: (tensors, (groups, chunks), exchange)."""
     B, T, H, D = q.shape
     q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
-    gf = gk.float().contiguous()
+    gf = _aligned(gk.float())
     G, cpg = lsm_groups(B, H, T)
     f32, dev = torch.float32, q.device
     states = torch.empty(B, H, G, D, D, dtype=f32, device=dev)
@@ -1292,7 +1298,7 @@ class _LsmVector(torch.autograd.Function):
         q, k, v, gf, states, gdecay, final = ctx.saved_tensors
         B, T, H, D = q.shape
         G, cpg = ctx.grid
-        d_o = torch.zeros(B, T, H, D, dtype=q.dtype, device=q.device) if d_o is None else d_o.contiguous().to(q.dtype)
+        d_o = torch.zeros(B, T, H, D, dtype=q.dtype, device=q.device) if d_o is None else _aligned(d_o).to(q.dtype)
         dqkv = torch.empty(B, T, H, 3 * D, dtype=q.dtype, device=q.device)
         dq, dk, dv = dqkv[..., :D], dqkv[..., D:2 * D], dqkv[..., 2 * D:]
         dstates = torch.empty_like(states)

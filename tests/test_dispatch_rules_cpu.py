@@ -41,3 +41,15 @@ def test_padded_tiles_own_their_rows():
             assert t.storage_offset() >= end and t.storage_offset() % 8 == 0
             end = t.storage_offset() + B * H * N * C * (n + 8)
             assert end * t.element_size() <= t.untyped_storage().nbytes()
+
+
+def test_views_that_start_off_a_boundary_are_copied():
+    """16-byte copies and tensor maps need 16-byte aligned bases; a contiguous view of a larger buffer is contiguous wherever it starts."""
+    n = 2 * 5 * 3 * 128
+    for start in (1, 4, 7):
+        t = torch.arange(n + start).bfloat16()[start:].view(2, 5, 3, 128)
+        for f in (K._inner_contig, K._tma_view, K._aligned):
+            c = f(t)
+            assert c.data_ptr() % 16 == 0 and c.is_contiguous() and torch.equal(c, t)
+    for t in (torch.zeros(2, 5, 3, 128), torch.zeros(n + 8).bfloat16()[8:].view(2, 5, 3, 128)):
+        assert K._aligned(t) is t
