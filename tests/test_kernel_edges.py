@@ -154,6 +154,38 @@ def test_expert_mlp_epilogues(h, f, counts):
     check(got, want, ["y", "dx", "dw1", "dw2"])
 
 
+@pytest.mark.parametrize("sms", [2, 6])
+@pytest.mark.parametrize("h,f", [(200, 120), (256, 264), (512, 136)])
+@pytest.mark.parametrize("counts", [[512, 0, 256, 0, 1024, 256], [0, 768, 0, 0, 256, 512]])
+def test_expert_mlp_many_tiles_per_pair(h, f, counts, sms, monkeypatch):
+    """One or three CTA pairs for all tiles: the search for the next tile's expert goes on from the last one, gate and up values are requested
+    for the next tile, both accumulator buffers are used again.  The same bits as with a pair per tile, and right."""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    E, rows = len(counts), sum(counts)
+    offs = torch.tensor([0] + counts, device="cuda").cumsum(0).int()
+    assert rows // 256 * -(-f // 128) > sms // 2 and rows // 256 * -(-h // 256) > sms // 2      # tiles of the products
+    x, w1, w2, go = rand(rows, h, scale=1), rand(E, h, 2 * f, scale=h ** -0.5), rand(E, f, h, scale=f ** -0.5), rand(rows, h, scale=1)
+
+    def kernel():
+        y, g = run(lambda x, w1, w2: gemm.expert_mlp(x, w1, w2, offs), [x, w1, w2], [go])
+        gemm.check_error()
+        return y, g
+    whole = kernel()
+    monkeypatch.setattr(K, "NUM_SMS", sms)
+    got = kernel()
+    for a, b in zip(got[0] + got[1], whole[0] + whole[1]):
+        assert torch.equal(a, b)
+
+    def plain(x, w1, w2):
+        ys = []
+        for e, xe in enumerate(x.split(counts)):
+            gate, up = (xe @ w1[e]).chunk(2, dim=-1)
+            ys.append((torch.nn.functional.silu(gate) * up) @ w2[e])
+        return torch.cat(ys)
+    check(got, run(plain, [t.float() for t in (x, w1, w2)], [go.float()]), ["y", "dx", "dw1", "dw2"])
+
+
 @pytest.mark.parametrize("T", [2, 127, 128, 129, 400])
 @pytest.mark.parametrize("decay", ["none", "head", "token"])
 @pytest.mark.parametrize("layout", ["fused", "heads first", "shared keys"])
@@ -272,6 +304,17 @@ def test_scalar_decay_above_the_line(B, T, H, decay):
         else:                                                   # the term of token i is in the sums of tokens 0 .. i
             walk = (step * torch.arange(1, T + 1, device="cuda").double().square()).sum().sqrt()
         assert (da[..., h] - dah).norm() < GRAD * (walk * g.detach()).norm()
+
+
+def test_long_model_against_64_bits():
+    """Loss and every weight's gradient of a two-layer model whose scans take the wide chunks by the rule.  The tolerance is the one of whole models
+    in perf/cases.py; measured 0.016 (geometric mean over the weights) and 0.02 (largest)."""
+    from perf import cases
+    case = dict(kind="train", B=1, T=38016, layers=2, hidden=512, ffn=1024, vocab=1000)
+    assert K._scalar_chunk(1, case["T"], case["hidden"] // 128, 128) == 128
+    got, want = cases.run(cases.prepare(case, 1)), cases.exact(case, 1)
+    for a, b in zip([got["loss"], *got["grads"]], [want["loss"], *want["grads"]]):
+        assert rel(a, b) < cases.tolerance(case)["rel"]
 
 
 def chunked64(q, k, v, g, C=100):
