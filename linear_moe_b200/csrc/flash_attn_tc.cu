@@ -12,7 +12,8 @@
 // units of a maximum that may lag behind by up to 2^LAG; only when a row runs ahead of that the output is rescaled there.  P_j goes
 // back over its scores in bf16 and is read as the A operand from tensor memory.
 // Tensor memory: 2 x 128 columns of scores, 2 x D of outputs.
-// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 190 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 66 us.
+// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 195 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 67 us.  (Of these an SM is
+// busy for 0.85 and 0.75: the longest tiles come first inside a head, not over all heads.)
 // Masking (causal with a query offset, sliding window, key length) is applied only on tiles that cross a boundary.
 // Every mbarrier wait is bounded (clock64 budget); on expiry the error word is set and the CTA drains and frees its
 // tensor memory.  Writes O (bf16) and the natural-log row log-sum-exp, which the backward kernels of flash_attn.cu use.
@@ -308,9 +309,10 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // and as an MN-major operand (rows = K) of the gradient GEMMs.  Same warp roles and bounded waits as the forward; all sixteen softmax
 // warps share a tile, four per 32 rows with 32 columns each.  The order of the products keeps the tensor core busy while
 // the warps work: a score GEMM is issued as soon as its scores have been read, ahead of the gradient GEMM of the tile before.
-// Issuing a product costs about 70 cycles whatever its width, so the 64-wide tiles that stood here first (24 instructions per
-// 128 x 64 scores, now 32 per 128 x 128) were bound by the issuing warp: 2650 - 2790 cycles per 128 x 64.
-// B=2, T=4096, 16 query and 4 kv heads of 128: dk / dv 514 -> 397 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125).
+// The 64-wide tiles that stood here first issued 24 instructions per 128 x 64 scores, these 32 per 128 x 128.  B=2, T=4096, 16 query and 4 kv heads of
+// 128 (16896 pairs of 128 x 128): dk / dv 514 -> 396 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125).  The tensor pipe is active for
+// 0.53 and 0.39 of the cycles of a busy SM, and an SM is busy for 0.61 and 0.86 of the launch: the tile is the fastest dimension of the
+// grid, so the last heads' longest tiles start late.
 // =====================================================================================================================
 struct BwdArgs {
     const float* lse;     // [B, Hq, Tq] natural-log sum-exp from the forward

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(NT + 32, 1) delta_scan_bwd_kernel(Args a) {
 // [[T0, 0], [-T1 (A10 T0), T1]] twice, with all threads on the small products.  A substitution over the whole chunk, one
 // column per thread, is a chain of 2016 multiply-adds on two warps; it was most of this kernel's time.
 // What bounds the kernel is the traffic of its tiles (120 KB in and out per chunk at D = 128); three CTAs of eight warps per SM
-// overlap one chunk's loads with another's products.  2 x 4096 tokens, 16 heads of 128: 110 -> 88 us (floor 37).
+// overlap one chunk's loads with another's products.  2 x 4096 tokens, 16 heads of 128: 110 -> 84 us (floor 37).
 // ---------------------------------------------------------------------------------------------------------------
 struct PrepArgs {
     const bf16 *q, *k, *v;             // [B,T,H,D] with the strides below (elements)

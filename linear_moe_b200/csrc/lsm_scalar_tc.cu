@@ -15,8 +15,10 @@
 // A factor e^{b_i - b_j} of a score is one exponential per element only in the 32 x 32 blocks on the diagonal; in the others it is a row
 // factor times a column factor around the block's edge, both at most one.
 //
-// What bounds them is memory: a chunk brings 96 - 128 KB of tiles and takes away 32 - 64 KB.  mma.sync fragments of 16 x 64 tiles read shared
-// memory 2.5 cycles per 2 cycles of tensor pipe with three to four barriers per 64 tokens: those kernels were at 18 - 22 % of DRAM.
+// A chunk brings 96 - 128 KB of tiles and takes away 32 - 64 KB, so memory is the bound that they approach: outputs and dq run at 0.49 of the DRAM
+// peak, dk / dv at 0.44, with the tensor pipe active for 0.3 of the cycles; between that and the bound stands a chunk's score products waiting for
+// the state of the chunk before.  mma.sync fragments of 16 x 64 tiles read shared memory 2.5 cycles per 2 cycles of tensor pipe with three
+// to four barriers per 64 tokens: those kernels were at 18 - 22 % of DRAM.
 // 16 heads of 16384 tokens: outputs 125 -> 59 us, dq 125 -> 63, dk / dv 232 -> 98, group summaries 50 -> 32 each.
 #include "flash_tc_utils.cuh"
 #include "lsm_scalar.cuh"
