@@ -210,8 +210,8 @@ def _skinny_ok(x, weight) -> bool:
 
 
 def linear_skinny(x, weight):
-    """``x W^T`` for up to 16 rows on ``gemm_skinny_kernel`` (csrc/gemm_skinny.cu): CTAs stream blocks of 16 rows of W through
-    lane-private slots of shared memory into mma.sync fragments, K split over the warps."""
+    """``x W^T`` for up to 16 rows on the kernels of csrc/gemm_skinny.cu: CTAs stream blocks of 16 rows of W, through lane-private
+    slots of shared memory or registers by a rule on the shapes, into mma.sync fragments, K split over the warps."""
     x2 = _rows(x)
     M, K = x2.shape
     N = weight.shape[0]
