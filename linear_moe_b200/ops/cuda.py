@@ -992,9 +992,9 @@ def _scalar_chunk(B, T, H, D):
     By shapes alone: a training pass and an evaluation of the same tokens have the same bits.  Trained decays need no exception.  Against 64
     bits, over 200 - 16384 tokens of 16 heads (geometric means of ten seeds), chunks of 64 are off by 0.0025 - 0.0030 (output) and 0.0025 - 0.0032
     (input gradients), chunks of 128 by 0.0024 - 0.0028 and 0.0024 - 0.0028; the gradient of a decay per token by 0.0095 / 0.0142 / 0.029 /
-    0.063 / 0.079 (200, 512, 2000, 9600, 16384 tokens) and 0.0085 / 0.0130 / 0.025 / 0.055 / 0.071; that of a decay per head, one sum over all
-    tokens that scatters by a factor of four from seed to seed, by 0.25 / 0.31 / 0.60 (12000, 16384, 32768 tokens, fifty seeds) and
-    0.20 / 0.29 / 0.47.
+    0.063 / 0.079 (200, 512, 2000, 9600, 16384 tokens) and 0.0085 / 0.0130 / 0.025 / 0.055 / 0.071, of 4 heads 0.120 / 0.155 (40000, 65536 tokens,
+    forty seeds) and 0.104 / 0.132; that of a decay per head, one sum over all tokens that scatters by a factor of four from seed to
+    seed, by 0.25 / 0.31 / 0.60 (12000, 16384, 32768 tokens, fifty seeds) and 0.20 / 0.29 / 0.47.
 
     Short sequences of many heads stay at 64 too: up to 192 tokens the chunks of 128 are mostly empty or few.  Forward pass of 170000
     rows, 64 / 128: 16 - 64 tokens 0.85 - 0.87 (256 x 64 tokens of 16 heads 941 and 1098 us), 96 and 128 tokens 0.95, 192 tokens 0.98; 224 tokens
