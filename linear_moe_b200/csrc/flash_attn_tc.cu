@@ -12,8 +12,7 @@
 // units of a maximum that may lag behind by up to 2^LAG; only when a row runs ahead of that the output is rescaled there.  P_j goes
 // back over its scores in bf16 and is read as the A operand from tensor memory.
 // Tensor memory: 2 x 128 columns of scores, 2 x D of outputs.
-// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 195 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 67 us.  (Of these an SM is
-// busy for 0.85 and 0.75: the longest tiles come first inside a head, not over all heads.)
+// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 180 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 61 us.
 // Masking (causal with a query offset, sliding window, key length) is applied only on tiles that cross a boundary.
 // Every mbarrier wait is bounded (clock64 budget); on expiry the error word is set and the CTA drains and frees its
 // tensor memory.  Writes O (bf16) and the natural-log row log-sum-exp, which the backward kernels of flash_attn.cu use.
@@ -48,18 +47,36 @@ struct __align__(1024) Smem {
     int abort_flag;
 };
 
+// Which tile a CTA takes.  CTAs start in the order of their index, so the longest tiles of all (batch, head) pairs come first and the short ones
+// fill the end: with the tile as the fastest dimension inside a head, the last heads' longest tiles started when the others were done
+// (SM busy for 0.61 of the dk / dv launch, 0.85 of the others).  Only `group` pairs are mixed at a time: their streamed rows share the L2.
+// B=2, T=4096, 16 / 4 heads of 128, forward and backward: 901 -> 752 us; 1531 queries over 2552 keys, 32 / 8 heads of 64: 67 -> 61.
+struct TileOf { int rank, pair; };
+__device__ __forceinline__ TileOf longest_first(int idx, int tiles, int pairs, int group) {
+    const int sec = idx / (tiles * group), rem = idx - sec * tiles * group;
+    const int n = min(group, pairs - sec * group);
+    return {rem / n, sec * group + rem % n};
+}
+// Pairs whose streamed tensors (two of `rows` x D bf16 per `share` pairs) stay within half of the L2 together.
+static int pairs_in_l2(int pairs, long long rows, int D, int share) {
+    const long long n = (64LL << 20) / max(rows * D * 4, 1LL);
+    return (int)min((long long)pairs, max(n, 1LL) * share);
+}
+
 template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                 const __grid_constant__ CUtensorMap tmV, Args a) {
+                 const __grid_constant__ CUtensorMap tmV, Args a, int group) {
     extern __shared__ uint8_t smem_raw[];
     Smem<D>& sm = *reinterpret_cast<Smem<D>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int DK = D / 64;                              // 64-element blocks along the head dimension
     constexpr uint32_t TMEM_COLS = 512;
     constexpr uint32_t O_COL = 2 * BN;                      // the groups' outputs behind the two score buffers
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qb = gridDim.x - 1 - blockIdx.x;              // long (late) query tiles first
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int n_qb = (a.Tq + BM - 1) / BM;
+    const TileOf t = longest_first(blockIdx.x, n_qb, a.B * a.Hq, group);
+    const int qb = n_qb - 1 - t.rank;                       // late query tiles see the most keys
+    const int h = t.pair % a.Hq, b = t.pair / a.Hq;
     const int hk = h / (a.Hq / a.Hkv);
     const int q0 = qb * BM;
     volatile int* abort_flag = &sm.abort_flag;
@@ -310,9 +327,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // warps share a tile, four per 32 rows with 32 columns each.  The order of the products keeps the tensor core busy while
 // the warps work: a score GEMM is issued as soon as its scores have been read, ahead of the gradient GEMM of the tile before.
 // The 64-wide tiles that stood here first issued 24 instructions per 128 x 64 scores, these 32 per 128 x 128.  B=2, T=4096, 16 query and 4 kv heads of
-// 128 (16896 pairs of 128 x 128): dk / dv 514 -> 396 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125).  The tensor pipe is active for
-// 0.53 and 0.39 of the cycles of a busy SM, and an SM is busy for 0.61 and 0.86 of the launch: the tile is the fastest dimension of the
-// grid, so the last heads' longest tiles start late.
+// 128 (16896 pairs of 128 x 128): dk / dv 514 -> 396 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125), with the tensor pipe active for
+// 0.53 and 0.39 of the cycles of a busy SM; the order of the tiles then took another 120 us off the two.
 // =====================================================================================================================
 struct BwdArgs {
     const float* lse;     // [B, Hq, Tq] natural-log sum-exp from the forward
@@ -396,7 +412,7 @@ struct __align__(1024) SmemDq {
 template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
-                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdArgs a) {
+                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdArgs a, int group) {
     extern __shared__ uint8_t smem_raw[];
     SmemDq<D>& sm = *reinterpret_cast<SmemDq<D>*>(smem_raw);
     if ((s32(smem_raw) & 1023u) != 0) {
@@ -405,8 +421,10 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     constexpr uint32_t TMEM_COLS = 512, DP = 256, DQ = 384;                  // two buffers of scores in front
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qb = gridDim.x - 1 - blockIdx.x;
-    const int h = blockIdx.y, b = blockIdx.z;
+    const int n_qb = (a.Tq + BM - 1) / BM;
+    const TileOf t = longest_first(blockIdx.x, n_qb, a.B * a.Hq, group);
+    const int qb = n_qb - 1 - t.rank;
+    const int h = t.pair % a.Hq, b = t.pair / a.Hq;
     const int hk = h / (a.Hq / a.Hkv);
     const int q0 = qb * BM;
     volatile int* abort_flag = &sm.abort_flag;
@@ -562,7 +580,7 @@ struct __align__(1024) SmemDkv {
 template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
 fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG,
-                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdArgs a) {
+                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, BwdArgs a, int group) {
     extern __shared__ uint8_t smem_raw[];
     SmemDkv<D>& sm = *reinterpret_cast<SmemDkv<D>*>(smem_raw);
     if ((s32(smem_raw) & 1023u) != 0) {
@@ -571,7 +589,8 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     constexpr uint32_t TMEM_COLS = 512, ST = 0, DP = 128, DV = 256, DKC = 384;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb_tile = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+    const TileOf t = longest_first(blockIdx.x, (a.Tk + BM - 1) / BM, a.B * a.Hkv, group);
+    const int kb_tile = t.rank, hk = t.pair % a.Hkv, b = t.pair / a.Hkv;      // early key tiles are seen by the most queries
     const int rep = a.Hq / a.Hkv;
     const int k0 = kb_tile * BM;
     volatile int* abort_flag = &sm.abort_flag;
@@ -746,23 +765,33 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
 }
 
-// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d]; one warp per (b,t,h)
+// delta[b,h,t] = sum_d dO[b,t,h,d] * O[b,t,h,d].  Bound by reading both tensors once: D / 8 lanes take a row 16 bytes at a time, and a thread asks
+// for its pieces of four rows before it uses the first (a warp per row with 4-byte loads had too little in flight).
 template <int D>
-__global__ void fa_delta_tc_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, float* __restrict__ delta, int B, int Tq, int Hq) {
-    const int l = threadIdx.x & 31;
-    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= (long long)B * Tq * Hq) return;
-    const int h = row % Hq;
-    const long long bt = row / Hq;
-    const int t = bt % Tq, b = bt / Tq;
-    float s = 0.f;
-    for (int c = l * 2; c < D; c += 64) {
-        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(o + row * D + c));
-        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(d_o + row * D + c));
-        s += x.x * y.x + x.y * y.y;
+__global__ void __launch_bounds__(256) fa_delta_tc_kernel(const bf16* __restrict__ o, const bf16* __restrict__ d_o, float* __restrict__ delta, int B, int Tq, int Hq) {
+    constexpr int LANES = D / 8, PER = 256 / LANES, U = 4;       // lanes of a row, rows of a block at a time
+    const int l = threadIdx.x % LANES;
+    const long long rows = (long long)B * Tq * Hq, row0 = (long long)blockIdx.x * (PER * U) + threadIdx.x / LANES;
+    Vec<bf16> x[U], y[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const long long at = min(row0 + u * PER, rows - 1) * D + l * 8;
+        x[u].load(o + at);
+        y[u].load(d_o + at);
     }
-    s = warp_sum(s);
-    if (l == 0) delta[((long long)b * Hq + h) * Tq + t] = s;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const long long row = row0 + u * PER;
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s += x[u].get(e) * y[u].get(e);
+#pragma unroll
+        for (int w = LANES / 2; w > 0; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
+        if (l == 0 && row < rows) {
+            const long long bt = row / Hq;
+            delta[((bt / Tq) * Hq + row % Hq) * Tq + bt % Tq] = s;
+        }
+    }
 }
 
 }  // namespace fatc
@@ -782,15 +811,16 @@ LMOE_API int lmoe_flash_attn_fwd_tc(const void* q, const long long* qs, const vo
     if (rc) return rc;
     rc = make_map_4d(&mv, v, a.B, a.Tk, a.Hkv, D, vs[0], vs[1], vs[2], 64);
     if (rc) return rc;
-    dim3 grid((a.Tq + BM - 1) / BM, a.Hq, a.B);
+    const unsigned grid = (unsigned)((a.Tq + BM - 1) / BM) * a.Hq * a.B;
+    const int group = pairs_in_l2(a.B * a.Hq, a.Tk, D, a.Hq / a.Hkv);
     if (D == 128) {
         const size_t smem = sizeof(Smem<128>) + 1024;
         cudaFuncSetAttribute(fa_fwd_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        fa_fwd_tc_kernel<128><<<grid, THREADS, smem, st>>>(mq, mk, mv, a);
+        fa_fwd_tc_kernel<128><<<grid, THREADS, smem, st>>>(mq, mk, mv, a, group);
     } else if (D == 64) {
         const size_t smem = sizeof(Smem<64>) + 1024;
         cudaFuncSetAttribute(fa_fwd_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        fa_fwd_tc_kernel<64><<<grid, THREADS, smem, st>>>(mq, mk, mv, a);
+        fa_fwd_tc_kernel<64><<<grid, THREADS, smem, st>>>(mq, mk, mv, a, group);
     } else return -1;
     return (int)cudaGetLastError();
 }
@@ -799,13 +829,17 @@ template <int D>
 static int launch_bwd_tc(const CUtensorMap& q, const CUtensorMap& g, const CUtensorMap& k, const CUtensorMap& v, const BwdArgs& a, const bf16* o,
                          const bf16* d_o, float* delta, cudaStream_t st) {
     const long long rows = (long long)a.B * a.Tq * a.Hq;
-    fa_delta_tc_kernel<D><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(o, d_o, delta, a.B, a.Tq, a.Hq);
+    constexpr int per_block = 4 * 256 / (D / 8);
+    fa_delta_tc_kernel<D><<<(unsigned)((rows + per_block - 1) / per_block), 256, 0, st>>>(o, d_o, delta, a.B, a.Tq, a.Hq);
     int rc = (int)cudaFuncSetAttribute(fa_bwd_dq_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemDq<D>));
     if (rc) return rc;
     rc = (int)cudaFuncSetAttribute(fa_bwd_dkv_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemDkv<D>));
     if (rc) return rc;
-    fa_bwd_dq_tc_kernel<D><<<dim3((a.Tq + BM - 1) / BM, a.Hq, a.B), THREADS, sizeof(SmemDq<D>), st>>>(q, g, k, v, a);
-    fa_bwd_dkv_tc_kernel<D><<<dim3((a.Tk + BM - 1) / BM, a.Hkv, a.B), THREADS, sizeof(SmemDkv<D>), st>>>(q, g, k, v, a);
+    fa_bwd_dq_tc_kernel<D><<<(unsigned)((a.Tq + BM - 1) / BM) * a.Hq * a.B, THREADS, sizeof(SmemDq<D>), st>>>(
+        q, g, k, v, a, pairs_in_l2(a.B * a.Hq, a.Tk, D, a.Hq / a.Hkv));
+    // a CTA goes through its query heads one after the other, so one of them counts
+    fa_bwd_dkv_tc_kernel<D><<<(unsigned)((a.Tk + BM - 1) / BM) * a.Hkv * a.B, THREADS, sizeof(SmemDkv<D>), st>>>(
+        q, g, k, v, a, pairs_in_l2(a.B * a.Hkv, a.Tq, D, 1));
     return (int)cudaGetLastError();
 }
 

@@ -57,6 +57,25 @@ def test_attention_tile_edges(D, Tq, Tk, window):
     check(got, want, ["o"] + ["dq", "dk", "dv"][-len(got[1]):])
 
 
+def test_attention_in_sections():
+    """Sequences so long that only two of three heads share the L2: the kernels' order over tiles and heads goes section by section, the last of them
+    with one head.  Gradients enter in three places, and with a window a slice around each of them is all that they depend on."""
+    from linear_moe_b200.ops import flash, gemm
+    torch.manual_seed(0)
+    T, H, D, W, n = 50000, 3, 128, 200, 400
+    q, k, v, go = rand(1, T, H, D, scale=1), rand(1, T, H, D, scale=1), rand(1, T, H, D, scale=1), torch.zeros(1, T, H, D, device="cuda").bfloat16()
+    starts = (0, 24960, T - n)
+    for lo in starts:
+        go[:, lo:lo + n] = rand(1, n, H, D, scale=1)
+    (o,), grads = run(lambda q, k, v: flash.FlashAttention.apply(q, k, v, D ** -0.5, 0, W), [q, k, v], [go])
+    gemm.check_error()
+    for lo in starts:
+        a = max(0, lo - W)
+        (want,), wg = run(lambda q, k, v: R.softmax_attention(q, k, v, D ** -0.5, True, 0, W), [t[:, a:lo + n].float() for t in (q, k, v)],
+                          [go[:, a:lo + n].float()])
+        check(([o[:, lo:lo + n]], [t[:, a:lo + n] for t in grads]), ([want[:, lo - a:]], wg), ["o", "dq", "dk", "dv"])
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("T", [1, 15, 63, 64, 65, 200])
 def test_delta_rule_chunk_edges(D, T):
