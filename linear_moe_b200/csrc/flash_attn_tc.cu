@@ -317,10 +317,10 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // Backward on tcgen05, two kernels that recompute the scores (7 GEMMs per tile pair instead of 5, no atomics), on tiles of
 // 128 queries x 128 keys:
 //   fa_bwd_dq_tc_kernel    one CTA = 128 queries of one head, looping over the key tiles:
-//                          S = Q K^T and dP = dO V^T into tensor memory -> dS = P (dP - delta) (softmax warps, thread = query row) ->
-//                          shared memory -> dQ += dS K accumulated in tensor memory.
+//                          S = Q K^T and dP = dO V^T into tensor memory -> dS = P (dP - delta) (softmax warps, thread = query row), in bf16
+//                          over S -> dQ += dS K accumulated in tensor memory.
 //   fa_bwd_dkv_tc_kernel   one CTA = 128 keys of one KV head, looping over the query heads of the group and their query
-//                          tiles: S^T = K Q^T and dP^T = V dO^T -> P^T, dS^T (thread = key row) -> shared memory ->
+//                          tiles: S^T = K Q^T and dP^T = V dO^T -> P^T, dS^T (thread = key row), in bf16 over the two ->
 //                          dV += P^T dO and dK += dS^T Q accumulated in tensor memory.
 // A tile of 128 rows loaded as D/64 boxes of {64 d, 128 rows} serves both as a K-major operand (rows = N) of the score GEMMs
 // and as an MN-major operand (rows = K) of the gradient GEMMs.  Same warp roles and bounded waits as the forward; all sixteen softmax
@@ -329,6 +329,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // The 64-wide tiles that stood here first issued 24 instructions per 128 x 64 scores, these 32 per 128 x 128.  B=2, T=4096, 16 query and 4 kv heads of
 // 128 (16896 pairs of 128 x 128): dk / dv 514 -> 396 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125), with the tensor pipe active for
 // 0.53 and 0.39 of the cycles of a busy SM; the order of the tiles then took another 120 us off the two.
+// P^T and dS as operands in tensor memory (a trip through shared memory before, with a fence and an eighth of the traffic of its products) leave room for
+// dO in two stages: forward and backward 752 -> 738 us, dk / dv 277, dq 247.
 // =====================================================================================================================
 struct BwdArgs {
     const float* lse;     // [B, Hq, Tq] natural-log sum-exp from the forward
@@ -362,24 +364,19 @@ __device__ __forceinline__ void score_product(uint32_t tmem_d, const uint8_t* A,
         umma_lo(tmem_d, al + off, bl + off, idesc_bf16<false, 128>(), kk > 0 ? 1u : 0u, issue);
     }
 }
-// [128 x D] (+)= A B over 128: A a K-major [128 x 128] tile, B's rows are K
+// [128 x D] (+)= A B over 128: A in tensor memory as the warps left it (16 packed columns at the beginning of every part's 32), B's rows are K
 template <int D>
-__device__ __forceinline__ void grad_product(uint32_t tmem_d, const uint8_t* A, const uint8_t* B, bool add, uint32_t issue) {
-    const uint32_t al = desc_lo<false>(s32(A)), bl = ((s32(B) >> 4) & 0x3FFFu) | ((uint32_t)(BLK >> 4) << 16);
+__device__ __forceinline__ void grad_product(uint32_t tmem_d, uint32_t tmem_a, const uint8_t* B, bool add, uint32_t issue) {
+    const uint32_t bl = ((s32(B) >> 4) & 0x3FFFu) | ((uint32_t)(BLK >> 4) << 16);
 #pragma unroll
     for (int kk = 0; kk < 128 / UMMA_K; ++kk)
-        umma_lo(tmem_d, al + (((kk / 4) * BLK + (kk % 4) * 32) >> 4), bl + ((kk * 2048) >> 4), idesc_bf16<true, D>(), (add || kk > 0) ? 1u : 0u, issue);
+        umma_ta(tmem_d, tmem_a + kk / 2 * 32 + kk % 2 * 8, bl + ((kk * 2048) >> 4), idesc_bf16<true, D>(), (add || kk > 0) ? 1u : 0u, issue);
 }
-// this thread's 32 columns (64 bytes) of row r of a [128 x 128] tile
-__device__ __forceinline__ void store_columns(uint8_t* tile, int r, int part, const uint32_t (&v)[16]) {
-    uint8_t* row = tile + (part >> 1) * BLK + r * 128;
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(row + ((((part & 1) * 4 + c) ^ (r & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-}
-__device__ __forceinline__ void hand_over(uint64_t* bar) {
+// this thread's 32 columns of an operand, over scores that it has read
+__device__ __forceinline__ void hand_over(uint32_t taddr, const uint32_t (&v)[16], uint64_t* bar) {
+    tmem_st16(taddr, v);
+    tmem_st_wait();
     tc_fence_before();
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
@@ -403,8 +400,8 @@ __device__ __forceinline__ void write_row(bf16* out, uint32_t taddr, float scale
 // kernels check before anything else.
 template <int D>
 struct __align__(1024) SmemDq {
-    uint8_t q[BM * D * 2], g[BM * D * 2], k[2][BM * D * 2], v[2][BM * D * 2], ds[BM * BM * 2];
-    uint64_t qg_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], dp_full, ds_ready, dq_done;
+    uint8_t q[BM * D * 2], g[BM * D * 2], k[2][BM * D * 2], v[2][BM * D * 2];
+    uint64_t qg_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], dp_full, ds_ready, dq_done, all_done;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -442,7 +439,7 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1);
             mbar_init(&sm.s_full[s], 1);
         }
-        mbar_init(&sm.dp_full, 1); mbar_init(&sm.ds_ready, 4 * SPLIT); mbar_init(&sm.dq_done, 1);
+        mbar_init(&sm.dp_full, 1); mbar_init(&sm.ds_ready, 4 * SPLIT); mbar_init(&sm.dq_done, 1); mbar_init(&sm.all_done, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -499,10 +496,11 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 if (!mbar_wait_suspend(&sm.ds_ready, j & 1, abort_flag, err, 0x4400)) break;
                 if (j + 1 < n_it && !dprobs(j + 1)) break;
                 tc_fence_after();
-                grad_product<D>(tmem_base + DQ, sm.ds, sm.k[s], j > 0, issue);
+                grad_product<D>(tmem_base + DQ, tmem_base + s * 128, sm.k[s], j > 0, issue);
                 umma_commit_if(&sm.k_empty[s], issue);
-                umma_commit_if(&sm.dq_done, issue);
-                if (j + 2 < n_it) ok = scores(j + 2);
+                umma_commit_if(j + 1 < n_it ? &sm.dq_done : &sm.all_done, issue);
+                // the next scores of this buffer go over dS_j: the product that reads it has to complete
+                if (j + 2 < n_it) ok = mbar_wait_suspend(&sm.dq_done, j & 1, abort_flag, err, 0x4600) && scores(j + 2);
             }
         }
     } else if (warp >= 4) {
@@ -524,37 +522,33 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                                    (a.window > 0 && tile_key0 <= a.q_offset + q0 + BM - 1 - a.window);
             if (!mbar_wait_suspend(&sm.s_full[s], (j >> 1) & 1, abort_flag, err, 0x4500 | s)) { alive = false; break; }
             tc_fence_after();
-            float p[32];
+            uint32_t v[32];
+            tmem_ld32(lane_addr + s * 128 + part * 32, v);
+            tmem_ld_wait();
+            if (need_mask) {
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + s * 128 + part * 32 + c, v);
-                tmem_ld_wait();
-                if (need_mask) {
+                for (int i = 0; i < 32; ++i)
+                    if (!visible(key0 + i, qi, a.Tk, a.window)) v[i] = 0xff800000u;              // -inf -> p = 0
+            }
+            float2 p[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (!visible(key0 + c + i, qi, a.Tk, a.window)) v[i] = 0xff800000u;      // -inf -> p = 0
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) p[c + i] = exp2f(fmaf(__uint_as_float(v[i]), sc, -lse2));
+            for (int i = 0; i < 16; ++i) {
+                const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(sc, sc), make_float2(-lse2, -lse2));
+                p[i] = make_float2(exp2f(x.x), exp2f(x.y));
             }
             if (!mbar_wait_suspend(&sm.dp_full, j & 1, abort_flag, err, 0x4510)) { alive = false; break; }
             tc_fence_after();
+            tmem_ld32(lane_addr + DP + part * 32, v);
+            tmem_ld_wait();
             uint32_t pk[16];
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + DP + part * 32 + c, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 16; i += 2)                                                // the softmax scale is applied to dQ at the end
-                    pk[(c + i) >> 1] = pack_bf16(p[c + i] * (__uint_as_float(v[i]) - dl), p[c + i + 1] * (__uint_as_float(v[i + 1]) - dl));
+            for (int i = 0; i < 16; ++i) {                                                       // the softmax scale is applied to dQ at the end
+                const float2 d = __fmul2_rn(p[i], __fadd2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(-dl, -dl)));
+                pk[i] = pack_bf16(d.x, d.y);
             }
-            if (j > 0 && !mbar_wait_suspend(&sm.dq_done, (j - 1) & 1, abort_flag, err, 0x4600)) { alive = false; break; }
-            store_columns(sm.ds, r, part, pk);
-            hand_over(&sm.ds_ready);
+            hand_over(lane_addr + s * 128 + part * 32, pk, &sm.ds_ready);
         }
-        if (alive) alive = mbar_wait_suspend(&sm.dq_done, (n_it - 1) & 1, abort_flag, err, 0x4700);
+        if (alive) alive = mbar_wait_suspend(&sm.all_done, 0, abort_flag, err, 0x4700);
         tc_fence_after();
         constexpr int OW = D / SPLIT;
         write_row<OW>(a.dq + (((long long)b * a.Tq + row) * a.Hq + h) * D + part * OW, lane_addr + DQ + part * OW, a.scale, row < a.Tq, !alive);
@@ -570,9 +564,9 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
 template <int D>
 struct __align__(1024) SmemDkv {
-    uint8_t k[BM * D * 2], v[BM * D * 2], q[2][BM * D * 2], g[BM * D * 2], p[BM * BM * 2], ds[BM * BM * 2];
+    uint8_t k[BM * D * 2], v[BM * D * 2], q[2][BM * D * 2], g[2][BM * D * 2];
     float lse2[2][BM], delta[2][BM];                                         // of the looped queries
-    uint64_t kv_full, q_full[2], q_empty[2], stat_full[2], g_full, g_empty, s_full, dp_full, p_ready, ds_ready, dv_done, dk_done;
+    uint64_t kv_full, q_full[2], q_empty[2], stat_full[2], g_full[2], g_empty[2], s_full, dp_full, p_ready, ds_ready, dv_done, dk_done, all_done;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -605,11 +599,13 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.kv_full, 1);
-        for (int s = 0; s < 2; ++s) { mbar_init(&sm.q_full[s], 1); mbar_init(&sm.q_empty[s], 1); mbar_init(&sm.stat_full[s], 1); }
-        mbar_init(&sm.g_full, 1); mbar_init(&sm.g_empty, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&sm.q_full[s], 1); mbar_init(&sm.q_empty[s], 1); mbar_init(&sm.stat_full[s], 1);
+            mbar_init(&sm.g_full[s], 1); mbar_init(&sm.g_empty[s], 1);
+        }
         mbar_init(&sm.s_full, 1); mbar_init(&sm.dp_full, 1);
         mbar_init(&sm.p_ready, 4 * SPLIT); mbar_init(&sm.ds_ready, 4 * SPLIT);
-        mbar_init(&sm.dv_done, 1); mbar_init(&sm.dk_done, 1);
+        mbar_init(&sm.dv_done, 1); mbar_init(&sm.dk_done, 1); mbar_init(&sm.all_done, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -633,9 +629,9 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 if (!mbar_wait_suspend(&sm.q_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, err, 0x5100 | s)) break;
                 mbar_expect_tx(&sm.q_full[s], BM * D * 2);
                 load_tile<D>(sm.q[s], &tmQ, &sm.q_full[s], h, q0, b);
-                if (!mbar_wait_suspend(&sm.g_empty, (it & 1) ^ 1, abort_flag, err, 0x5120)) break;
-                mbar_expect_tx(&sm.g_full, BM * D * 2);
-                load_tile<D>(sm.g, &tmG, &sm.g_full, h, q0, b);
+                if (!mbar_wait_suspend(&sm.g_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, err, 0x5120 | s)) break;
+                mbar_expect_tx(&sm.g_full[s], BM * D * 2);
+                load_tile<D>(sm.g[s], &tmG, &sm.g_full[s], h, q0, b);
             }
         }
     } else if (warp == 1) {
@@ -650,26 +646,30 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 return true;
             };
             auto dprobs = [&](int it) -> bool {
-                if (!mbar_wait_suspend(&sm.g_full, it & 1, abort_flag, err, 0x5310)) return false;
+                if (!mbar_wait_suspend(&sm.g_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5310 | (it & 1))) return false;
                 tc_fence_after();
-                score_product<D>(tmem_base + DP, sm.v, sm.g, issue);
+                score_product<D>(tmem_base + DP, sm.v, sm.g[it & 1], issue);
                 umma_commit_if(&sm.dp_full, issue);
                 return true;
             };
             if (ok) ok = scores(0) && dprobs(0);
             for (int it = 0; ok && it < n_it; ++it) {
                 if (!mbar_wait_suspend(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
-                if (it + 1 < n_it && !scores(it + 1)) break;
                 tc_fence_after();
-                grad_product<D>(tmem_base + DV, sm.p, sm.g, it > 0, issue);                  // dV += P^T dO
-                umma_commit_if(&sm.g_empty, issue);
-                umma_commit_if(&sm.dv_done, issue);
+                const bool more = it + 1 < n_it;
+                grad_product<D>(tmem_base + DV, tmem_base + ST, sm.g[it & 1], it > 0, issue);   // dV += P^T dO
+                umma_commit_if(&sm.g_empty[it & 1], issue);
+                if (more) {
+                    // the next scores go over P^T: the product that reads it has to complete
+                    umma_commit_if(&sm.dv_done, issue);
+                    if (!mbar_wait_suspend(&sm.dv_done, it & 1, abort_flag, err, 0x5600) || !scores(it + 1)) break;
+                }
                 if (!mbar_wait_suspend(&sm.ds_ready, it & 1, abort_flag, err, 0x5410)) break;
                 tc_fence_after();
-                grad_product<D>(tmem_base + DKC, sm.ds, sm.q[it & 1], it > 0, issue);        // dK += dS^T Q
+                grad_product<D>(tmem_base + DKC, tmem_base + DP, sm.q[it & 1], it > 0, issue);  // dK += dS^T Q
                 umma_commit_if(&sm.q_empty[it & 1], issue);
-                umma_commit_if(&sm.dk_done, issue);
-                if (it + 1 < n_it) ok = dprobs(it + 1);
+                umma_commit_if(more ? &sm.dk_done : &sm.all_done, issue);
+                if (more) ok = mbar_wait_suspend(&sm.dk_done, it & 1, abort_flag, err, 0x5610) && dprobs(it + 1);
             }
         }
     } else if (warp == 2) {                                      // log-sum-exp and delta of the looped queries
@@ -705,52 +705,41 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             if (!mbar_wait_suspend(&sm.stat_full[s], (it >> 1) & 1, abort_flag, err, 0x5510 | s)) { alive = false; break; }
             if (!mbar_wait_suspend(&sm.s_full, it & 1, abort_flag, err, 0x5500)) { alive = false; break; }
             tc_fence_after();
-            float p[32];
-            uint32_t pk[16];
+            uint32_t v[32], pk[16];
+            float2 p[16];
+            tmem_ld32(lane_addr + ST + part * 32, v);
+            tmem_ld_wait();
+            if (need_mask) {
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + ST + part * 32 + c, v);
-                tmem_ld_wait();
-                if (need_mask) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (!visible(key, a.q_offset + tile_q0 + part * 32 + c + i, a.Tk, a.window)) v[i] = 0xff800000u;
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i += 4) {
-                    const float4 l2 = *reinterpret_cast<const float4*>(&sm.lse2[s][part * 32 + c + i]);
-                    p[c + i] = exp2f(fmaf(__uint_as_float(v[i]), sc, -l2.x));
-                    p[c + i + 1] = exp2f(fmaf(__uint_as_float(v[i + 1]), sc, -l2.y));
-                    p[c + i + 2] = exp2f(fmaf(__uint_as_float(v[i + 2]), sc, -l2.z));
-                    p[c + i + 3] = exp2f(fmaf(__uint_as_float(v[i + 3]), sc, -l2.w));
-                    pk[(c + i) >> 1] = pack_bf16(p[c + i], p[c + i + 1]);
-                    pk[((c + i) >> 1) + 1] = pack_bf16(p[c + i + 2], p[c + i + 3]);
-                }
+                for (int i = 0; i < 32; ++i)
+                    if (!visible(key, a.q_offset + tile_q0 + part * 32 + i, a.Tk, a.window)) v[i] = 0xff800000u;
             }
-            if (it > 0 && !mbar_wait_suspend(&sm.dv_done, (it - 1) & 1, abort_flag, err, 0x5600)) { alive = false; break; }
-            store_columns(sm.p, r, part, pk);
-            hand_over(&sm.p_ready);
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                const float4 l2 = *reinterpret_cast<const float4*>(&sm.lse2[s][part * 32 + 2 * i]);
+                const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(sc, sc), make_float2(-l2.x, -l2.y));
+                const float2 y = __ffma2_rn(make_float2(__uint_as_float(v[2 * i + 2]), __uint_as_float(v[2 * i + 3])), make_float2(sc, sc), make_float2(-l2.z, -l2.w));
+                p[i] = make_float2(exp2f(x.x), exp2f(x.y));
+                p[i + 1] = make_float2(exp2f(y.x), exp2f(y.y));
+                pk[i] = pack_bf16(p[i].x, p[i].y);
+                pk[i + 1] = pack_bf16(p[i + 1].x, p[i + 1].y);
+            }
+            hand_over(lane_addr + ST + part * 32, pk, &sm.p_ready);
             if (!mbar_wait_suspend(&sm.dp_full, it & 1, abort_flag, err, 0x5520)) { alive = false; break; }
             tc_fence_after();
+            tmem_ld32(lane_addr + DP + part * 32, v);
+            tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(lane_addr + DP + part * 32 + c, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 16; i += 4) {                                              // scale applied to dK at the end
-                    const float4 dl = *reinterpret_cast<const float4*>(&sm.delta[s][part * 32 + c + i]);
-                    pk[(c + i) >> 1] = pack_bf16(p[c + i] * (__uint_as_float(v[i]) - dl.x), p[c + i + 1] * (__uint_as_float(v[i + 1]) - dl.y));
-                    pk[((c + i) >> 1) + 1] = pack_bf16(p[c + i + 2] * (__uint_as_float(v[i + 2]) - dl.z), p[c + i + 3] * (__uint_as_float(v[i + 3]) - dl.w));
-                }
+            for (int i = 0; i < 16; i += 2) {                                                   // scale applied to dK at the end
+                const float4 dl = *reinterpret_cast<const float4*>(&sm.delta[s][part * 32 + 2 * i]);
+                const float2 x = __fmul2_rn(p[i], __fadd2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(-dl.x, -dl.y)));
+                const float2 y = __fmul2_rn(p[i + 1], __fadd2_rn(make_float2(__uint_as_float(v[2 * i + 2]), __uint_as_float(v[2 * i + 3])), make_float2(-dl.z, -dl.w)));
+                pk[i] = pack_bf16(x.x, x.y);
+                pk[i + 1] = pack_bf16(y.x, y.y);
             }
-            if (it > 0 && !mbar_wait_suspend(&sm.dk_done, (it - 1) & 1, abort_flag, err, 0x5610)) { alive = false; break; }
-            store_columns(sm.ds, r, part, pk);
-            hand_over(&sm.ds_ready);
+            hand_over(lane_addr + DP + part * 32, pk, &sm.ds_ready);
         }
-        if (alive) alive = mbar_wait_suspend(&sm.dv_done, (n_it - 1) & 1, abort_flag, err, 0x5700) &&
-                           mbar_wait_suspend(&sm.dk_done, (n_it - 1) & 1, abort_flag, err, 0x5710);
+        if (alive) alive = mbar_wait_suspend(&sm.all_done, 0, abort_flag, err, 0x5700);        // covers dV, which was issued before dK
         tc_fence_after();
         constexpr int OW = D / SPLIT;
         const long long off = (((long long)b * a.Tk + key) * a.Hkv + hk) * D + part * OW;
