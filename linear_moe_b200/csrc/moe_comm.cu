@@ -351,9 +351,275 @@ __global__ void moe_dprobs_kernel(const bf16* __restrict__ rows, const bf16* __r
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// One rank: the same routing and exchange with plain pointers, without counts matrices, flags and waits.  Two launches build the routing
+// record (three and a fence between them before), one brings the rows, with the padding rows' zeros, and one takes the results; the gradient of
+// the combine forms the routing weights' gradient from the same rows of d_out that it sends, and reads the experts' results where they are
+// (a copy of them in token order was written by the forward pass for that: 134 MB at 8192 tokens x 8 of width 1024).
+// The three exchange kernels are bound by memory: a warp takes a token, reads its row once for all k destinations and has all its pieces in flight.
+// 8192 tokens x 8 of 64 experts, width 1024, in us: routing 57 -> 17, push 53 -> 28, combine 55 -> 45, its gradients 100 -> 74.
+// ---------------------------------------------------------------------------------------------------------------------
+struct MoeLocalArgs {
+    const long long* idx;       // [T * k] expert of every (token, slot) pair, outside [0, E) = dropped
+    int *hist;                  // [E][nchunks] scratch
+    int *offs, *real;           // [E + 1], [E] out
+    int *dest_rank, *dest_row;  // [T * k] out: 0 and the row, or -1 and -1
+    int* status;
+    const bf16* src;            // [T][h] rows to send
+    bf16* x;                    // [rows][h] where they go
+    const bf16* y;              // [rows][h] the experts' results
+    const float* w;             // [T * k] or null
+    bf16* out;                  // [T][h]
+    float* d_probs;             // [T * k]
+    int T, k, E, cap, h, pad, nchunks;
+};
+constexpr int LOCAL_CHUNK = 1024;                                    // assignments of a block: eight warps x four rounds of 32
+
+__global__ void __launch_bounds__(256) moe_local_count_kernel(MoeLocalArgs a) {
+    extern __shared__ int sh[];
+    for (int e = threadIdx.x; e < a.E; e += 256) sh[e] = 0;
+    __syncthreads();
+    const long long n = (long long)a.T * a.k, base = (long long)blockIdx.x * LOCAL_CHUNK;
+    long long e[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long long p = base + i * 256 + threadIdx.x;
+        e[i] = p < n ? a.idx[p] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (e[i] >= 0 && e[i] < a.E) atomicAdd(&sh[e[i]], 1);
+    __syncthreads();
+    for (int x = threadIdx.x; x < a.E; x += 256) a.hist[(long long)x * a.nchunks + blockIdx.x] = sh[x];
+}
+
+// Rows in the order of the assignments inside every expert's segment (a stable counting sort).  Every block sums the histograms itself.
+__global__ void __launch_bounds__(256) moe_local_assign_kernel(MoeLocalArgs a) {
+    extern __shared__ int sh[];
+    int *tot = sh, *base = sh + a.E, *cnt = sh + 2 * a.E;             // [E] rows of an expert, [E] first row of this block's, [8][E]
+    __shared__ int over;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    for (int e = w; e < a.E; e += 8) {
+        int all = 0, before = 0;
+        for (int c = l; c < a.nchunks; c += 32) {
+            const int x = a.hist[(long long)e * a.nchunks + c];
+            all += x;
+            if (c < (int)blockIdx.x) before += x;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) { all += __shfl_xor_sync(0xffffffffu, all, o); before += __shfl_xor_sync(0xffffffffu, before, o); }
+        if (l == 0) { tot[e] = all; base[e] = before; }
+    }
+    for (int i = threadIdx.x; i < 8 * a.E; i += 256) cnt[i] = 0;
+    __syncthreads();
+    if (w == 0) {                                                    // segments start at multiples of `pad` rows
+        long long run = 0;
+        for (int e0 = 0; e0 < a.E; e0 += 32) {
+            const int e = e0 + l, n = e < a.E ? tot[e] : 0;
+            const long long padded = ((long long)n + a.pad - 1) / a.pad * a.pad;
+            long long s = padded;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long x = __shfl_up_sync(0xffffffffu, s, o);
+                if (l >= o) s += x;
+            }
+            const long long first = run + s - padded;                // past the capacity the numbers are not used
+            if (e < a.E) {
+                base[e] += (int)min(first, (long long)a.cap);
+                if (blockIdx.x == 0) { a.offs[e] = (int)min(first, (long long)a.cap); a.real[e] = n; }
+            }
+            run += __shfl_sync(0xffffffffu, s, 31);
+        }
+        if (l == 0) {
+            over = run > a.cap;
+            if (blockIdx.x == 0) a.offs[a.E] = (int)min(run, (long long)a.cap);
+            if (run > a.cap) atomicCAS(a.status, 0, (9 << 24) | 7);  // receive buffer too small
+        }
+    }
+    __syncthreads();
+    if (over && blockIdx.x == 0) {
+        for (int e = threadIdx.x; e <= a.E; e += 256) { a.offs[e] = 0; if (e < a.E) a.real[e] = 0; }
+    }
+    const long long n = (long long)a.T * a.k, p0 = (long long)blockIdx.x * LOCAL_CHUNK + w * 128 + l;
+    int ev[4], pos[4], *mine = cnt + w * a.E;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long long p = p0 + i * 32, e = p < n ? a.idx[p] : -1;
+        ev[i] = e >= 0 && e < a.E ? (int)e : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t same = __match_any_sync(0xffffffffu, ev[i]);
+        const int rank = __popc(same & ((1u << l) - 1));
+        pos[i] = ev[i] >= 0 ? mine[ev[i]] + rank : 0;
+        __syncwarp();
+        if (ev[i] >= 0 && rank == 0) mine[ev[i]] += __popc(same);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < a.E; e += 256) {
+        int run = base[e];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) { const int c = cnt[r * a.E + e]; cnt[r * a.E + e] = run; run += c; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long long p = p0 + i * 32;
+        if (p >= n) break;
+        const bool sent = ev[i] >= 0 && !over;
+        a.dest_rank[p] = sent ? 0 : -1;
+        a.dest_row[p] = sent ? mine[ev[i]] + pos[i] : -1;
+    }
+}
+
+__device__ __forceinline__ uint4 times(uint4 v, float w) {
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]);
+        h[i] = __floats2bfloat162_rn(f.x * w, f.y * w);
+    }
+    return v;
+}
+__device__ __forceinline__ void add_dot(float& s, uint4 x, uint4 y) {
+    const __nv_bfloat162 *a = reinterpret_cast<const __nv_bfloat162*>(&x), *b = reinterpret_cast<const __nv_bfloat162*>(&y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(a[i]), g = __bfloat1622float2(b[i]);
+        s += f.x * g.x + f.y * g.y;
+    }
+}
+
+// Rows of src (times w) to their segments; DOT: also d_probs[t, j] = <y[row of (t, j)], src[t]> (zero for a dropped pair).  Then the padding rows.
+template <int KMAX, bool DOT>
+__global__ void __launch_bounds__(256) moe_local_push_kernel(MoeLocalArgs a) {
+    const int wpb = blockDim.x >> 5, l = threadIdx.x & 31, vecs = a.h / 8;
+    const long long warp = (long long)blockIdx.x * wpb + (threadIdx.x >> 5), warps = (long long)gridDim.x * wpb;
+    uint4* x = reinterpret_cast<uint4*>(a.x);
+    const uint4 *src = reinterpret_cast<const uint4*>(a.src), *y = reinterpret_cast<const uint4*>(a.y);
+    for (long long t = warp; t < a.T; t += warps) {
+        for (int j0 = 0; j0 < a.k; j0 += KMAX) {
+            const int kj = min(KMAX, a.k - j0);
+            const int my_row = l < kj ? a.dest_row[t * a.k + j0 + l] : -1;
+            const float my_w = a.w != nullptr && l < kj ? a.w[t * a.k + j0 + l] : 1.f;
+            int row[KMAX];
+            float wt[KMAX], dot[KMAX];
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j) { row[j] = __shfl_sync(0xffffffffu, my_row, j); wt[j] = __shfl_sync(0xffffffffu, my_w, j); dot[j] = 0.f; }
+            constexpr int U = DOT ? 2 : 4;                            // pieces of the row in flight (DOT: with KMAX rows of y each)
+            for (int c0 = l; c0 < vecs; c0 += 32 * U) {
+                uint4 v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = c0 + 32 * u < vecs ? __ldg(src + t * vecs + c0 + 32 * u) : make_uint4(0, 0, 0, 0);
+                if (DOT) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        uint4 r[KMAX];
+                        const int c = c0 + 32 * u;
+#pragma unroll
+                        for (int j = 0; j < KMAX; ++j) r[j] = row[j] >= 0 && c < vecs ? __ldcs(y + (long long)row[j] * vecs + c) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                        for (int j = 0; j < KMAX; ++j) add_dot(dot[j], r[j], v[u]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < KMAX; ++j)
+                    if (row[j] >= 0) {
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+                            if (c0 + 32 * u < vecs) x[(long long)row[j] * vecs + c0 + 32 * u] = a.w != nullptr ? times(v[u], wt[j]) : v[u];
+                    }
+            }
+            if (DOT) {
+#pragma unroll
+                for (int j = 0; j < KMAX; ++j) {
+                    const float s = warp_sum(dot[j]);
+                    if (l == 0 && j < kj) a.d_probs[t * a.k + j0 + j] = row[j] >= 0 ? s : 0.f;
+                }
+            }
+        }
+    }
+    constexpr int ROWS = 8;                                          // padding rows of a warp at a time
+    const int per = (a.pad + ROWS - 1) / ROWS;
+    for (long long u = warp; u < (long long)a.E * per; u += warps) {
+        const int e = (int)(u / per), lo = a.offs[e] + a.real[e] + (int)(u % per) * ROWS, hi = min(a.offs[e + 1], lo + ROWS);
+        for (long long i = (long long)lo * vecs + l; i < (long long)hi * vecs; i += 32) x[i] = make_uint4(0, 0, 0, 0);
+    }
+}
+
+// out[t] = sum_j w[t, j] y[row of (t, j)] in fp32
+template <int KMAX>
+__global__ void __launch_bounds__(256) moe_local_pull_kernel(MoeLocalArgs a) {
+    const int wpb = blockDim.x >> 5, l = threadIdx.x & 31, vecs = a.h / 8;
+    const uint4* y = reinterpret_cast<const uint4*>(a.y);
+    for (long long t = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); t < a.T; t += (long long)gridDim.x * wpb) {
+        const int my_row = l < a.k ? a.dest_row[t * a.k + l] : -1;
+        const float my_w = l < a.k ? (a.w != nullptr ? a.w[t * a.k + l] : 1.f) : 0.f;
+        int row[KMAX];
+        float wt[KMAX];
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j) {
+            row[j] = __shfl_sync(0xffffffffu, my_row, j);
+            wt[j] = row[j] >= 0 ? __shfl_sync(0xffffffffu, my_w, j) : 0.f;
+        }
+        for (int c = l; c < vecs; c += 32) {
+            uint4 v[KMAX];
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j) v[j] = row[j] >= 0 ? __ldcg(y + (long long)row[j] * vecs + c) : make_uint4(0, 0, 0, 0);
+            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j) {
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = __bfloat1622float2(h[i]);
+                    acc[2 * i] += wt[j] * f.x;
+                    acc[2 * i + 1] += wt[j] * f.y;
+                }
+            }
+            uint4 o;
+            __nv_bfloat162* ho = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ho[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+            reinterpret_cast<uint4*>(a.out)[t * vecs + c] = o;
+        }
+    }
+}
+
 }  // namespace lmoe
 
 using namespace lmoe;
+
+// The exchange of one rank.  which: 0 route, 1 push (with a.d_probs: and the routing weights' gradient), 2 pull.  h a multiple of 8, rows
+// 16-byte aligned.
+LMOE_API int lmoe_moe_local(int which, const MoeLocalArgs* ap, int num_sms, cudaStream_t st) {
+    const MoeLocalArgs a = *ap;
+    if (a.h % 8 != 0) return -2;
+    const int grid = (int)std::min<long long>(std::max<long long>(((long long)a.T + 7) / 8, 1), (long long)num_sms * 8);
+    if (which == 0) {
+        if ((size_t)256 * a.E * sizeof(unsigned short) > 200 * 1024) return -4;      // the limit of moe_assign_kernel
+        if (a.nchunks > 0) moe_local_count_kernel<<<a.nchunks, 256, a.E * sizeof(int), st>>>(a);
+        moe_local_assign_kernel<<<std::max(a.nchunks, 1), 256, 10 * a.E * sizeof(int), st>>>(a);
+    } else if (which == 1) {
+        if (a.d_probs != nullptr) {
+            if (a.k <= 2) moe_local_push_kernel<2, true><<<grid, 256, 0, st>>>(a);
+            else if (a.k <= 4) moe_local_push_kernel<4, true><<<grid, 256, 0, st>>>(a);
+            else moe_local_push_kernel<8, true><<<grid, 256, 0, st>>>(a);
+        } else {
+            if (a.k <= 2) moe_local_push_kernel<2, false><<<grid, 256, 0, st>>>(a);
+            else if (a.k <= 4) moe_local_push_kernel<4, false><<<grid, 256, 0, st>>>(a);
+            else moe_local_push_kernel<8, false><<<grid, 256, 0, st>>>(a);
+        }
+    } else if (which == 2) {
+        if (a.k <= 2) moe_local_pull_kernel<2><<<grid, 256, 0, st>>>(a);
+        else if (a.k <= 4) moe_local_pull_kernel<4><<<grid, 256, 0, st>>>(a);
+        else if (a.k <= 8) moe_local_pull_kernel<8><<<grid, 256, 0, st>>>(a);
+        else if (a.k <= 16) moe_local_pull_kernel<16><<<grid, 256, 0, st>>>(a);
+        else return -3;
+    } else return -1;
+    return (int)cudaGetLastError();
+}
 
 // which: 0 exchange, 1 assign, 2 push, 3 zero pads, 4 signal, 5 pull, 6 count
 LMOE_API int lmoe_moe_comm(int which, const MoeArgs* ap, int num_sms, cudaStream_t st) {

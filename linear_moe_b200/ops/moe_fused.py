@@ -33,7 +33,10 @@ class _Combine(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y_local, probs, ws, route):
         w = probs.float().contiguous()
-        out, rows = ws.pull(y_local, route, w, True)
+        local = ws.group is None                                 # then the results stay where they are
+        out, rows = ws.pull(y_local, route, w, not local)
+        if local:
+            rows = y_local
         ctx.ws, ctx.route = ws, route
         ctx.save_for_backward(rows, w)
         ctx.pdtype = probs.dtype
@@ -45,6 +48,9 @@ class _Combine(torch.autograd.Function):
         route = ctx.route
         d_out = d_out.contiguous()
         T, k = route.T, route.k
+        if ctx.ws.group is None:
+            d_y, d_probs = ctx.ws.push_combine_grad(d_out, rows, route, w)
+            return d_y, d_probs.to(ctx.pdtype), None, None
         from . import cuda as K
         d_probs = K.moe_dprobs(rows, d_out, route.dest_rank, T, k)
         d_y = ctx.ws.push(d_out, route, w.reshape(-1), keep=False)

@@ -401,6 +401,12 @@ class _MoeArgs(ctypes.Structure):
                 [("n_assign", ctypes.c_int), ("k", ctypes.c_int), ("pad", ctypes.c_int)])
 
 
+class _MoeLocalArgs(ctypes.Structure):
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("idx", "hist", "offs", "real", "dest_rank", "dest_row", "status", "src", "x", "y", "w", "out",
+                                                "d_probs")] +
+                [(n, ctypes.c_int) for n in ("T", "k", "E", "cap", "h", "pad", "nchunks")])
+
+
 class MoeWorkspace:
     """Receive buffer ``x [cap, h]``, result buffer ``y [cap, h]``, count matrix and flags of one expert-parallel group.
     ``group=None`` builds a one-rank workspace out of ordinary tensors (single-GPU use and tests)."""
@@ -460,6 +466,13 @@ class MoeWorkspace:
         flat = idx.reshape(-1).contiguous()
         if flat.dtype != torch.int64:
             flat = flat.to(torch.int64)
+        if self.group is None:
+            E, n, nch = self.E, T * k, (T * k + 1023) // 1024
+            offs, real, dest_rank, dest_row, hist = torch.empty(2 * E + 1 + 2 * n + nch * E, dtype=torch.int32, device=dev).split(
+                [E + 1, E, n, n, nch * E])
+            route = MoeRoute(T, k, dest_rank, dest_row, offs, real)
+            self._local(0, route, "moe_route", idx=flat, hist=hist, launches=2)
+            return route
         nch = (T * k + 4095) // 4096
         scratch = torch.empty(2 * nch * self.E + self.El + 1 + self.El + self.E + 2 * T * k, dtype=torch.int32, device=dev)
         o = 0
@@ -482,6 +495,30 @@ class MoeWorkspace:
         self._run(1, a, "moe_assign")
         return MoeRoute(T, k, dest_rank, dest_row, offs, real)
 
+    def _local(self, which: int, route: "MoeRoute", name: str, launches: int = 1, **tensors):
+        """One of the one-rank kernels (``lmoe_moe_local``) with the tensors it reads and writes."""
+        from ..ops import cuda as K
+        from ..ops import gemm
+        p = {n: t.data_ptr() for n, t in tensors.items() if t is not None}
+        a = _MoeLocalArgs(offs=route.offs.data_ptr(), real=route.real.data_ptr(), dest_rank=route.dest_rank.data_ptr(),
+                          dest_row=route.dest_row.data_ptr(), status=status_word(self.device).data_ptr(), T=route.T, k=route.k, E=self.E,
+                          cap=self.cap, h=self.h, pad=gemm.ROW_ALIGN, nchunks=(route.T * route.k + 1023) // 1024, **p)
+        K._check(K.lib().lmoe_moe_local(ctypes.c_int(which), ctypes.byref(a), ctypes.c_int(K.NUM_SMS), K._st()), name, launches)
+
+    def _receive_rows(self, route: "MoeRoute") -> int:
+        """Rows that the padded segments of a call can take (one rank)."""
+        from ..ops import gemm
+        return min(self.cap, (route.T * route.k + gemm.ROW_ALIGN * self.E + 255) // 256 * 256)
+
+    def push_combine_grad(self, d_out: torch.Tensor, y: torch.Tensor, route: "MoeRoute", weights: torch.Tensor):
+        """One rank: the gradients of ``out[t] = sum_k w[t, k] y[row(t, k)]``, ``(d_y, d_w [T, k])``, in one pass."""
+        assert self.group is None and d_out.dtype == y.dtype == torch.bfloat16 and d_out.shape == (route.T, self.h)
+        d_out, y = _aligned(d_out), _aligned(y)
+        d_y = torch.empty(self._receive_rows(route), self.h, dtype=torch.bfloat16, device=self.device)
+        d_w = torch.empty(route.T, route.k, dtype=torch.float32, device=self.device)
+        self._local(1, route, "moe_push_dprobs", src=d_out, x=d_y, y=y, w=weights, d_probs=d_w)
+        return d_y, d_w
+
     def result_holder(self):
         """The buffer the peers pull from, for a producer that writes into it directly (``None`` on one rank, where results
         are read where they are)."""
@@ -493,6 +530,11 @@ class MoeWorkspace:
         weight gradient), the shared buffer itself without (the backward pass consumes it before this rank signals its
         results, and no peer pushes again before it has pulled those)."""
         assert src.is_contiguous() and src.dtype == torch.bfloat16 and src.shape == (route.T, self.h)
+        if self.group is None:
+            # the receive buffer is a fresh tensor that the caller keeps, no copy out of a shared buffer
+            x = torch.empty(self._receive_rows(route), self.h, dtype=torch.bfloat16, device=self.device)
+            self._local(1, route, "moe_push", src=_aligned(src), x=x, w=weights)
+            return x
         self.ep_push += 1
         a = self._args()
         a.epoch = self.ep_push
@@ -501,13 +543,6 @@ class MoeWorkspace:
         a.dest_rank, a.dest_row = route.dest_rank.data_ptr(), route.dest_row.data_ptr()
         a.offs, a.real = route.offs.data_ptr(), route.real.data_ptr()
         a.n_assign, a.k = route.T * route.k, route.k
-        if self.group is None:
-            # one rank: the receive buffer is a fresh tensor that the caller keeps, no copy out of a shared buffer
-            x = torch.empty(self.cap, self.h, dtype=torch.bfloat16, device=self.device)
-            self.peer_x.fill_(x.data_ptr())
-            self._run(2, a, "moe_push")
-            self._run(3, a, "moe_zero_pads")
-            return x
         self._run(2, a, "moe_push")
         self._run(3, a, "moe_zero_pads")
         return self.x.clone() if keep else self.x
@@ -515,11 +550,13 @@ class MoeWorkspace:
     def pull(self, y_local: torch.Tensor, route: "MoeRoute", weights: Optional[torch.Tensor], save_rows: bool):
         """Publish this rank's expert results ``[cap, h]`` and gather, weight and sum every token's ``k`` rows from their
         owners.  Returns ``(out [T, h], rows [T*k, h] or None)``."""
+        if self.group is None:                                   # one rank: the results are read, and kept, where they are
+            assert not save_rows
+            out = torch.empty(route.T, self.h, dtype=torch.bfloat16, device=self.device)
+            self._local(2, route, "moe_pull", y=_aligned(y_local), w=weights, out=out)
+            return out, None
         self.ep_pull += 1
-        if self.group is None:
-            y_local = y_local.contiguous()
-            self.peer_y.fill_(y_local.data_ptr())                # one rank: read the results where they are
-        elif y_local.data_ptr() != self.y.data_ptr():
+        if y_local.data_ptr() != self.y.data_ptr():
             self.y.copy_(y_local)                                # (the grouped GEMM normally writes into self.y itself)
         a = self._args()
         a.epoch = self.ep_pull
@@ -532,6 +569,12 @@ class MoeWorkspace:
         self._run(4, a, "moe_signal")
         self._run(5, a, "moe_pull")
         return out, rows
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on a 16-byte boundary, for kernels that read 16 bytes at a time."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 class _BufHolder:
