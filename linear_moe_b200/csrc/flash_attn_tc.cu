@@ -72,7 +72,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     constexpr int DK = D / 64;                              // 64-element blocks along the head dimension
     constexpr uint32_t TMEM_COLS = 512;
     constexpr uint32_t O_COL = 2 * BN;                      // the groups' outputs behind the two score buffers
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
     const int n_qb = (a.Tq + BM - 1) / BM;
     const TileOf t = longest_first(blockIdx.x, n_qb, a.B * a.Hq, group);
     const int qb = n_qb - 1 - t.rank;                       // late query tiles see the most keys
@@ -107,7 +107,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sm.tmem_base;
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
@@ -137,10 +137,10 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const uint32_t issue = lane == 0 ? 1u : 0u;
             constexpr uint32_t idesc_s = idesc_bf16<false, BN>();
             constexpr uint32_t idesc_o = idesc_bf16<true, D>();
-            bool ok = mbar_wait_suspend(&sm.q_full, 0, abort_flag, err, 0x2000);
+            bool ok = fatc::mbar_wait_warp(&sm.q_full, 0, abort_flag, err, 0x2000);
             auto issue_s = [&](int j) -> bool {
                 const int s = j & 1;
-                if (!mbar_wait_suspend(&sm.k_full[s], (j >> 1) & 1, abort_flag, err, 0x2100 | s)) return false;
+                if (!fatc::mbar_wait_warp(&sm.k_full[s], (j >> 1) & 1, abort_flag, err, 0x2100 | s)) return false;
                 tc_fence_after();
                 const uint32_t ql = desc_lo<false>(s32(sm.q)), kl = desc_lo<false>(s32(sm.k[s]));
 #pragma unroll
@@ -157,12 +157,12 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int s = j & 1;
                 if (j + 1 < n_it) {
                     // the other score buffer holds P_{j-1}: its product has to complete
-                    if (j > 0 && !mbar_wait_suspend(&sm.pv_done[s ^ 1], ((j - 1) >> 1) & 1, abort_flag, err, 0x2400)) break;
+                    if (j > 0 && !fatc::mbar_wait_warp(&sm.pv_done[s ^ 1], ((j - 1) >> 1) & 1, abort_flag, err, 0x2400)) break;
                     ok = issue_s(j + 1);
                     if (!ok) break;
                 }
-                if (!mbar_wait_suspend(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x2200 | s)) break;
-                if (!mbar_wait_suspend(&sm.p_ready[s], (j >> 1) & 1, abort_flag, err, 0x2300 | s)) break;
+                if (!fatc::mbar_wait_warp(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x2200 | s)) break;
+                if (!fatc::mbar_wait_warp(&sm.p_ready[s], (j >> 1) & 1, abort_flag, err, 0x2300 | s)) break;
                 tc_fence_after();
                 const uint32_t vl = desc_lo<true>(s32(sm.v[s]));
 #pragma unroll
@@ -330,7 +330,9 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // 128 (16896 pairs of 128 x 128): dk / dv 514 -> 396 us, dq 335 -> 288 (at the measured 1654 TFLOP/s: 166 and 125), with the tensor pipe active for
 // 0.53 and 0.39 of the cycles of a busy SM; the order of the tiles then took another 120 us off the two.
 // P^T and dS as operands in tensor memory (a trip through shared memory before, with a fence and an eighth of the traffic of its products) leave room for
-// dO in two stages: forward and backward 752 -> 738 us, dk / dv 277, dq 247.
+// dO in two stages: forward and backward 752 -> 738 us, dk / dv 277, dq 247.  A third stage of K in the dq kernel (a tile's K is read by its first and its
+// last product, and the next scores waited for a load that could start only then), its exponentials ahead of the wait for dP instead of
+// behind it, where the compiler had moved them, and MMA operands that look uniform: 738 -> 695, dk / dv 257, dq 208.
 // =====================================================================================================================
 struct BwdArgs {
     const float* lse;     // [B, Hq, Tq] natural-log sum-exp from the forward
@@ -400,8 +402,8 @@ __device__ __forceinline__ void write_row(bf16* out, uint32_t taddr, float scale
 // kernels check before anything else.
 template <int D>
 struct __align__(1024) SmemDq {
-    uint8_t q[BM * D * 2], g[BM * D * 2], k[2][BM * D * 2], v[2][BM * D * 2];
-    uint64_t qg_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], dp_full, ds_ready, dq_done, all_done;
+    uint8_t q[BM * D * 2], g[BM * D * 2], k[3][BM * D * 2], v[2][BM * D * 2];      // K: read by a tile's first and last product
+    uint64_t qg_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], dp_full, ds_ready, dq_done, all_done;
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -417,7 +419,7 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         return;
     }
     constexpr uint32_t TMEM_COLS = 512, DP = 256, DQ = 384;                  // two buffers of scores in front
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
     const int n_qb = (a.Tq + BM - 1) / BM;
     const TileOf t = longest_first(blockIdx.x, n_qb, a.B * a.Hq, group);
     const int qb = n_qb - 1 - t.rank;
@@ -434,11 +436,8 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.qg_full, 1);
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1);
-            mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1);
-            mbar_init(&sm.s_full[s], 1);
-        }
+        for (int s = 0; s < 3; ++s) { mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1); mbar_init(&sm.s_full[s], 1); }
         mbar_init(&sm.dp_full, 1); mbar_init(&sm.ds_ready, 4 * SPLIT); mbar_init(&sm.dq_done, 1); mbar_init(&sm.all_done, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -450,7 +449,7 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sm.tmem_base;
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
@@ -458,12 +457,11 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             load_tile<D>(sm.q, &tmQ, &sm.qg_full, h, q0, b);
             load_tile<D>(sm.g, &tmG, &sm.qg_full, h, q0, b);
             for (int j = 0; j < n_it; ++j) {
-                const int s = j & 1, key0 = (nb_lo + j) * BN;
-                const uint32_t ph = ((j >> 1) & 1) ^ 1;
-                if (!mbar_wait_suspend(&sm.k_empty[s], ph, abort_flag, err, 0x4100 | s)) break;
-                mbar_expect_tx(&sm.k_full[s], BM * D * 2);
-                load_tile<D>(sm.k[s], &tmK, &sm.k_full[s], hk, key0, b);
-                if (!mbar_wait_suspend(&sm.v_empty[s], ph, abort_flag, err, 0x4110 | s)) break;
+                const int s = j & 1, s3 = j % 3, key0 = (nb_lo + j) * BN;
+                if (!mbar_wait_suspend(&sm.k_empty[s3], ((j / 3) & 1) ^ 1, abort_flag, err, 0x4100 | s3)) break;
+                mbar_expect_tx(&sm.k_full[s3], BM * D * 2);
+                load_tile<D>(sm.k[s3], &tmK, &sm.k_full[s3], hk, key0, b);
+                if (!mbar_wait_suspend(&sm.v_empty[s], ((j >> 1) & 1) ^ 1, abort_flag, err, 0x4110 | s)) break;
                 mbar_expect_tx(&sm.v_full[s], BM * D * 2);
                 load_tile<D>(sm.v[s], &tmV, &sm.v_full[s], hk, key0, b);
             }
@@ -471,18 +469,18 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     } else if (warp == 1) {
         if (n_it > 0) {
             const uint32_t issue = lane == 0 ? 1u : 0u;
-            bool ok = mbar_wait_suspend(&sm.qg_full, 0, abort_flag, err, 0x4200);
+            bool ok = fatc::mbar_wait_warp(&sm.qg_full, 0, abort_flag, err, 0x4200);
             auto scores = [&](int j) -> bool {
-                const int s = j & 1;
-                if (!mbar_wait_suspend(&sm.k_full[s], (j >> 1) & 1, abort_flag, err, 0x4300 | s)) return false;
+                const int s = j & 1, s3 = j % 3;
+                if (!fatc::mbar_wait_warp(&sm.k_full[s3], (j / 3) & 1, abort_flag, err, 0x4300 | s3)) return false;
                 tc_fence_after();
-                score_product<D>(tmem_base + s * 128, sm.q, sm.k[s], issue);
+                score_product<D>(tmem_base + s * 128, sm.q, sm.k[s3], issue);
                 umma_commit_if(&sm.s_full[s], issue);
                 return true;
             };
             auto dprobs = [&](int j) -> bool {
                 const int s = j & 1;
-                if (!mbar_wait_suspend(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x4310 | s)) return false;
+                if (!fatc::mbar_wait_warp(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x4310 | s)) return false;
                 tc_fence_after();
                 score_product<D>(tmem_base + DP, sm.g, sm.v[s], issue);
                 umma_commit_if(&sm.v_empty[s], issue);
@@ -493,14 +491,14 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             if (ok && n_it > 1) ok = scores(1);
             for (int j = 0; ok && j < n_it; ++j) {
                 const int s = j & 1;
-                if (!mbar_wait_suspend(&sm.ds_ready, j & 1, abort_flag, err, 0x4400)) break;
+                if (!fatc::mbar_wait_warp(&sm.ds_ready, j & 1, abort_flag, err, 0x4400)) break;
                 if (j + 1 < n_it && !dprobs(j + 1)) break;
                 tc_fence_after();
-                grad_product<D>(tmem_base + DQ, tmem_base + s * 128, sm.k[s], j > 0, issue);
-                umma_commit_if(&sm.k_empty[s], issue);
+                grad_product<D>(tmem_base + DQ, tmem_base + s * 128, sm.k[j % 3], j > 0, issue);
+                umma_commit_if(&sm.k_empty[j % 3], issue);
                 umma_commit_if(j + 1 < n_it ? &sm.dq_done : &sm.all_done, issue);
                 // the next scores of this buffer go over dS_j: the product that reads it has to complete
-                if (j + 2 < n_it) ok = mbar_wait_suspend(&sm.dq_done, j & 1, abort_flag, err, 0x4600) && scores(j + 2);
+                if (j + 2 < n_it) ok = fatc::mbar_wait_warp(&sm.dq_done, j & 1, abort_flag, err, 0x4600) && scores(j + 2);
             }
         }
     } else if (warp >= 4) {
@@ -535,6 +533,7 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             for (int i = 0; i < 16; ++i) {
                 const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), make_float2(sc, sc), make_float2(-lse2, -lse2));
                 p[i] = make_float2(exp2f(x.x), exp2f(x.y));
+                asm volatile("" : "+f"(p[i].x), "+f"(p[i].y));                                     // here, not behind the wait
             }
             if (!mbar_wait_suspend(&sm.dp_full, j & 1, abort_flag, err, 0x4510)) { alive = false; break; }
             tc_fence_after();
@@ -582,7 +581,7 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         return;
     }
     constexpr uint32_t TMEM_COLS = 512, ST = 0, DP = 128, DV = 256, DKC = 384;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
     const TileOf t = longest_first(blockIdx.x, (a.Tk + BM - 1) / BM, a.B * a.Hkv, group);
     const int kb_tile = t.rank, hk = t.pair % a.Hkv, b = t.pair / a.Hkv;      // early key tiles are seen by the most queries
     const int rep = a.Hq / a.Hkv;
@@ -616,7 +615,7 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sm.tmem_base;
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
@@ -637,16 +636,16 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     } else if (warp == 1) {
         if (n_it > 0) {
             const uint32_t issue = lane == 0 ? 1u : 0u;
-            bool ok = mbar_wait_suspend(&sm.kv_full, 0, abort_flag, err, 0x5200);
+            bool ok = fatc::mbar_wait_warp(&sm.kv_full, 0, abort_flag, err, 0x5200);
             auto scores = [&](int it) -> bool {
-                if (!mbar_wait_suspend(&sm.q_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5300 | (it & 1))) return false;
+                if (!fatc::mbar_wait_warp(&sm.q_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5300 | (it & 1))) return false;
                 tc_fence_after();
                 score_product<D>(tmem_base + ST, sm.k, sm.q[it & 1], issue);
                 umma_commit_if(&sm.s_full, issue);
                 return true;
             };
             auto dprobs = [&](int it) -> bool {
-                if (!mbar_wait_suspend(&sm.g_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5310 | (it & 1))) return false;
+                if (!fatc::mbar_wait_warp(&sm.g_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5310 | (it & 1))) return false;
                 tc_fence_after();
                 score_product<D>(tmem_base + DP, sm.v, sm.g[it & 1], issue);
                 umma_commit_if(&sm.dp_full, issue);
@@ -654,7 +653,7 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             };
             if (ok) ok = scores(0) && dprobs(0);
             for (int it = 0; ok && it < n_it; ++it) {
-                if (!mbar_wait_suspend(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
+                if (!fatc::mbar_wait_warp(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
                 tc_fence_after();
                 const bool more = it + 1 < n_it;
                 grad_product<D>(tmem_base + DV, tmem_base + ST, sm.g[it & 1], it > 0, issue);   // dV += P^T dO
@@ -662,14 +661,14 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 if (more) {
                     // the next scores go over P^T: the product that reads it has to complete
                     umma_commit_if(&sm.dv_done, issue);
-                    if (!mbar_wait_suspend(&sm.dv_done, it & 1, abort_flag, err, 0x5600) || !scores(it + 1)) break;
+                    if (!fatc::mbar_wait_warp(&sm.dv_done, it & 1, abort_flag, err, 0x5600) || !scores(it + 1)) break;
                 }
-                if (!mbar_wait_suspend(&sm.ds_ready, it & 1, abort_flag, err, 0x5410)) break;
+                if (!fatc::mbar_wait_warp(&sm.ds_ready, it & 1, abort_flag, err, 0x5410)) break;
                 tc_fence_after();
                 grad_product<D>(tmem_base + DKC, tmem_base + DP, sm.q[it & 1], it > 0, issue);  // dK += dS^T Q
                 umma_commit_if(&sm.q_empty[it & 1], issue);
                 umma_commit_if(more ? &sm.dk_done : &sm.all_done, issue);
-                if (more) ok = mbar_wait_suspend(&sm.dk_done, it & 1, abort_flag, err, 0x5610) && dprobs(it + 1);
+                if (more) ok = fatc::mbar_wait_warp(&sm.dk_done, it & 1, abort_flag, err, 0x5610) && dprobs(it + 1);
             }
         }
     } else if (warp == 2) {                                      // log-sum-exp and delta of the looped queries

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(STHREADS, 1)
 lsm_state_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, LsmArgs a) {
     extern __shared__ uint8_t smem_raw[];
     SmemState& sm = *reinterpret_cast<SmemState*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
     const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int nchunks = (a.T + CT - 1) / CT, cpg = a.cpg / 2;                    // cpg counts chunks of 64
     const int c_lo = grp * cpg, n = max(0, min(nchunks, c_lo + cpg) - c_lo);
@@ -217,7 +217,7 @@ lsm_state_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sm.tmem_base;
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -234,7 +234,7 @@ lsm_state_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
         bool ok = true;
         for (int i = 0; ok && i < n; ++i) {
             const int s = i % SSTAGES;
-            ok = mbar_wait_suspend(&sm.ready[s], (i / SSTAGES) & 1, abort_flag, err, 0x7200 | s);
+            ok = fatc::mbar_wait_warp(&sm.ready[s], (i / SSTAGES) & 1, abort_flag, err, 0x7200 | s);
             if (!ok) break;
             tc_fence_after();
             product<true, true>(tmem_base, sm.x[s], sm.y[s], i > 0, issue);
@@ -325,7 +325,7 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
         return;
     }
     constexpr uint32_t SC = 0, DS = 128, OUT = 256;                              // columns of tensor memory; two outputs take turns
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
     const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int nchunks = (a.T + CT - 1) / CT, cpg = a.cpg / 2;
     const int c_lo = grp * cpg, n = max(0, min(nchunks, c_lo + cpg) - c_lo);
@@ -345,7 +345,7 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sm.tmem_base;
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -362,13 +362,13 @@ lsm_sweep_tc_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
         const uint32_t issue = lane == 0 ? 1u : 0u;
         for (int i = 0; i < n; ++i) {
             const int s = i & 1;
-            if (!mbar_wait_suspend(&sm.full[s], (i >> 1) & 1, abort_flag, err, 0x8200 | s)) break;
-            if (!mbar_wait_suspend(&sm.sb_ready, i & 1, abort_flag, err, 0x8210)) break;
+            if (!fatc::mbar_wait_warp(&sm.full[s], (i >> 1) & 1, abort_flag, err, 0x8200 | s)) break;
+            if (!fatc::mbar_wait_warp(&sm.sb_ready, i & 1, abort_flag, err, 0x8210)) break;
             tc_fence_after();
             product<false, false>(tmem_base + SC, sm.t0[s], sm.t1[s], false, issue);
             product<false, MODE == 0>(tmem_base + OUT + s * 128, sm.t0[s], sm.sb, false, issue);      // X0 S: rows of S are K; X0 S^T: rows of S are N
             umma_commit_if(&sm.c1, issue);
-            if (!mbar_wait_suspend(&sm.p_ready, i & 1, abort_flag, err, 0x8220)) break;
+            if (!fatc::mbar_wait_warp(&sm.p_ready, i & 1, abort_flag, err, 0x8220)) break;
             tc_fence_after();
             if (MODE == 0) product<true, true>(tmem_base + DS, sm.t1[s], sm.t2[s], false, issue);
             else product<true, true>(tmem_base + DS, sm.t2[s], sm.t1[s], false, issue);
@@ -496,7 +496,7 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         return;
     }
     constexpr uint32_t AT = 0, BT = 128, DV = 256, DK = 384;                     // AT: K Q^T, P1, then the state increment
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
     const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int nchunks = (a.T + CT - 1) / CT, cpg = a.cpg / 2;
     const int c_lo = grp * cpg, n = max(0, min(nchunks, c_lo + cpg) - c_lo), c_last = c_lo + n - 1;
@@ -517,7 +517,7 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = sm.tmem_base;
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -547,10 +547,10 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const uint32_t issue = lane == 0 ? 1u : 0u;
         for (int i = 0; i < n; ++i) {
             const int s = i & 1;
-            if (!mbar_wait_suspend(&sm.qg_full[s], (i >> 1) & 1, abort_flag, err, 0x9200 | s)) break;
-            if (!mbar_wait_suspend(&sm.k_full, i & 1, abort_flag, err, 0x9210)) break;
-            if (!mbar_wait_suspend(&sm.v_full, i & 1, abort_flag, err, 0x9220)) break;
-            if (!mbar_wait_suspend(&sm.db_ready, i & 1, abort_flag, err, 0x9230)) break;       // also: the accumulators of chunk i - 1 have been read
+            if (!fatc::mbar_wait_warp(&sm.qg_full[s], (i >> 1) & 1, abort_flag, err, 0x9200 | s)) break;
+            if (!fatc::mbar_wait_warp(&sm.k_full, i & 1, abort_flag, err, 0x9210)) break;
+            if (!fatc::mbar_wait_warp(&sm.v_full, i & 1, abort_flag, err, 0x9220)) break;
+            if (!fatc::mbar_wait_warp(&sm.db_ready, i & 1, abort_flag, err, 0x9230)) break;       // also: the accumulators of chunk i - 1 have been read
             tc_fence_after();
             product<false, false>(tmem_base + AT, sm.k, sm.q[s], false, issue);                // K Q^T
             product<false, true>(tmem_base + DV, sm.k, sm.db, false, issue);                   // K dS
@@ -558,12 +558,12 @@ lsm_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             product<false, false>(tmem_base + BT, sm.v, sm.g[s], false, issue);                // V dO^T
             product<false, false>(tmem_base + DK, sm.v, sm.db, false, issue);                  // V dS^T
             umma_commit_if(&sm.c1, issue);
-            if (!mbar_wait_suspend(&sm.p_ready, i & 1, abort_flag, err, 0x9240)) break;
+            if (!fatc::mbar_wait_warp(&sm.p_ready, i & 1, abort_flag, err, 0x9240)) break;
             tc_fence_after();
             product_ta(tmem_base + DV, tmem_base + AT, sm.g[s], issue);                        // += P1 dO
             umma_commit_if(&sm.p1_done, issue);
             product_ta(tmem_base + DK, tmem_base + BT, sm.q[s], issue);                        // += P2 Q
-            if (!mbar_wait_suspend(&sm.p1_done, i & 1, abort_flag, err, 0x9250)) break;        // over P1 goes
+            if (!fatc::mbar_wait_warp(&sm.p1_done, i & 1, abort_flag, err, 0x9250)) break;        // over P1 goes
             product<true, true>(tmem_base + AT, sm.v, sm.g[s], false, issue);                  // (scaled Q)^T dO
             umma_commit_if(&sm.v_empty, issue);
             umma_commit_if(&sm.acc_full, issue);
