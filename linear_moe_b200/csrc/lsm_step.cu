@@ -106,7 +106,7 @@ lsm_delta_step_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k,
 
 // q, k, v: bf16, one token per (batch, head), element strides over batch and head, contiguous over D.  g: [B, H] log
 // decay of this token (batch stride gs_b, zero for one decay per head) or null; gk: [B*H, D] log decay per key channel or null.  s_in: [B*H, D, D] fp32 or null (zero
-// state); s_out is a different buffer.  o: [B*H, D] bf16.
+// state); s_out is another buffer or s_in (a thread reads its elements before it writes them, and no other's).  o: [B*H, D] bf16.
 LMOE_API int lmoe_lsm_scalar_step(const void* q, const void* k, const void* v, long long qs_b, long long qs_h, long long ks_b,
                                   long long ks_h, long long vs_b, long long vs_h, const float* g, long long gs_b, const float* gk,
                                   const float* s_in, float* s_out, void* o, int B, int H, int D, float scale,
@@ -122,7 +122,7 @@ LMOE_API int lmoe_lsm_scalar_step(const void* q, const void* k, const void* v, l
     return -1;
 }
 
-// Delta-rule step; beta: [B*H]; g: [B*H] log decay or null (plain DeltaNet).  Other arguments as above.
+// Delta-rule step; beta: [B*H]; g: [B*H] log decay or null (plain DeltaNet).  Other arguments as above, s_out = s_in too.
 LMOE_API int lmoe_lsm_delta_step(const void* q, const void* k, const void* v, long long qs_b, long long qs_h, long long ks_b,
                                  long long ks_h, long long vs_b, long long vs_h, const float* g, const float* beta,
                                  const float* s_in, float* s_out, void* o, int B, int H, int D, float scale,

@@ -95,6 +95,13 @@ def score_tokens(model, tokens: torch.Tensor) -> torch.Tensor:
     return PF.broadcast_from_last_stage(model, out, (B, T - 1), torch.float32, tokens.device)
 
 
+def _overwritable(state: torch.Tensor) -> torch.Tensor:
+    """An alias of a state that nobody reads behind the step it goes into: the step may write the new state over it."""
+    alias = state.detach()
+    alias.lmoe_overwritable = True
+    return alias
+
+
 class GraphedDecodeStep:
     """One-token decode step replayed from a CUDA graph.
 
@@ -102,7 +109,8 @@ class GraphedDecodeStep:
     updates) that the host cannot issue as fast as the GPU runs them.  Models whose every cache entry has a fixed size
     (all mixers linear sequence models or Mamba2: O(1) recurrent state, no growing KV cache) make the step static, so it
     is captured once and replayed: the token is copied into a static buffer, the graph runs the whole forward, and the
-    new states are copied back over the state buffers the graph reads.  Softmax-attention layers whose KV cache grows by one
+    new states go over the state buffers that the graph reads: the one-token kernels of the decayed mixers write them there, others are
+    copied back.  Softmax-attention layers whose KV cache grows by one
     row per token are not supported and fall back to eager decoding.  A ``SlotCache`` is updated in place by the step, so
     nothing is copied back; ``rows`` then holds the requests' positions and slots in device tensors that the caller fills."""
 
@@ -132,11 +140,14 @@ class GraphedDecodeStep:
         static = [] if self.rows is not None else [dict(c) for c in self.caches]                # the state tensors the graph will read and update
         graph = torch.cuda.CUDAGraph()
         try:
+            for c, st in zip(self.caches, static):
+                c.update({k: _overwritable(v) for k, v in st.items()})
             with torch.cuda.graph(graph):
                 self.logits = self._forward(self.tok)
-                for c, st in zip(self.caches, static):        # forward rebinds every entry to a new tensor
+                for c, st in zip(self.caches, static):        # forward rebinds every entry, mostly to a new tensor
                     for k, v in st.items():
-                        v.copy_(c[k])
+                        if c[k].data_ptr() != v.data_ptr() or c[k].shape != v.shape or c[k].dtype != v.dtype:
+                            v.copy_(c[k])
                         c[k] = v
         except Exception:
             # a layer that synchronises with the host (e.g. an expert dispatch that reads token counts) cannot be
