@@ -357,7 +357,7 @@ __global__ void moe_dprobs_kernel(const bf16* __restrict__ rows, const bf16* __r
 // the combine forms the routing weights' gradient from the same rows of d_out that it sends, and reads the experts' results where they are
 // (a copy of them in token order was written by the forward pass for that: 134 MB at 8192 tokens x 8 of width 1024).
 // The three exchange kernels are bound by memory: a warp takes a token, reads its row once for all k destinations and has all its pieces in flight.
-// 8192 tokens x 8 of 64 experts, width 1024, in us: routing 57 -> 17, push 53 -> 28, combine 55 -> 45, its gradients 100 -> 74.
+// 8192 tokens x 8 of 64 experts, width 1024, in us: routing 57 -> 17, push 53 -> 28, combine 55 -> 30, its gradients 100 -> 74.
 // ---------------------------------------------------------------------------------------------------------------------
 struct MoeLocalArgs {
     const long long* idx;       // [T * k] expert of every (token, slot) pair, outside [0, E) = dropped
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(256) moe_local_push_kernel(MoeLocalArgs a) {
             float wt[KMAX], dot[KMAX];
 #pragma unroll
             for (int j = 0; j < KMAX; ++j) { row[j] = __shfl_sync(0xffffffffu, my_row, j); wt[j] = __shfl_sync(0xffffffffu, my_w, j); dot[j] = 0.f; }
-            constexpr int U = DOT ? 2 : 4;                            // pieces of the row in flight (DOT: with KMAX rows of y each)
+            constexpr int U = DOT ? 1 : 4;                            // pieces of the row in flight (DOT: with KMAX rows of y each)
             for (int c0 = l; c0 < vecs; c0 += 32 * U) {
                 uint4 v[U];
 #pragma unroll
@@ -549,11 +549,15 @@ __global__ void __launch_bounds__(256) moe_local_push_kernel(MoeLocalArgs a) {
 }
 
 // out[t] = sum_j w[t, j] y[row of (t, j)] in fp32
+constexpr int PULL_SEG = 64;                                         // 16-byte pieces
 template <int KMAX>
 __global__ void __launch_bounds__(256) moe_local_pull_kernel(MoeLocalArgs a) {
     const int wpb = blockDim.x >> 5, l = threadIdx.x & 31, vecs = a.h / 8;
     const uint4* y = reinterpret_cast<const uint4*>(a.y);
-    for (long long t = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); t < a.T; t += (long long)gridDim.x * wpb) {
+    const int segs = (vecs + PULL_SEG - 1) / PULL_SEG;               // a warp takes a piece of a token: the last round of warps is short
+    for (long long at = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); at < (long long)a.T * segs; at += (long long)gridDim.x * wpb) {
+        const long long t = at / segs;
+        const int c_lo = (int)(at % segs) * PULL_SEG, c_hi = min(vecs, c_lo + PULL_SEG);
         const int my_row = l < a.k ? a.dest_row[t * a.k + l] : -1;
         const float my_w = l < a.k ? (a.w != nullptr ? a.w[t * a.k + l] : 1.f) : 0.f;
         int row[KMAX];
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(256) moe_local_pull_kernel(MoeLocalArgs a) {
             row[j] = __shfl_sync(0xffffffffu, my_row, j);
             wt[j] = row[j] >= 0 ? __shfl_sync(0xffffffffu, my_w, j) : 0.f;
         }
-        for (int c = l; c < vecs; c += 32) {
+        for (int c = c_lo + l; c < c_hi; c += 32) {
             uint4 v[KMAX];
 #pragma unroll
             for (int j = 0; j < KMAX; ++j) v[j] = row[j] >= 0 ? __ldcg(y + (long long)row[j] * vecs + c) : make_uint4(0, 0, 0, 0);
@@ -596,7 +600,8 @@ using namespace lmoe;
 LMOE_API int lmoe_moe_local(int which, const MoeLocalArgs* ap, int num_sms, cudaStream_t st) {
     const MoeLocalArgs a = *ap;
     if (a.h % 8 != 0) return -2;
-    const int grid = (int)std::min<long long>(std::max<long long>(((long long)a.T + 7) / 8, 1), (long long)num_sms * 8);
+    const long long warps = which == 2 ? (long long)a.T * ((a.h / 8 + PULL_SEG - 1) / PULL_SEG) : a.T;
+    const int grid = (int)std::min<long long>(std::max<long long>((warps + 7) / 8, 1), (long long)num_sms * 8);
     if (which == 0) {
         if ((size_t)256 * a.E * sizeof(unsigned short) > 200 * 1024) return -4;      // the limit of moe_assign_kernel
         if (a.nchunks > 0) moe_local_count_kernel<<<a.nchunks, 256, a.E * sizeof(int), st>>>(a);

@@ -95,3 +95,46 @@ def test_bounded_wait_expiry_and_overflow_are_reported():
     torch.cuda.synchronize()
     fused_comm.check_status("after")
     assert torch.isfinite(recv[: int(route.offs[-1])].float()).all()
+
+
+@pytest.mark.parametrize("T,k,E,hid", [(1, 1, 3, 8), (1023, 1, 64, 72), (512, 2, 5, 264), (700, 16, 40, 520), (1100, 12, 7, 64)])
+def test_one_rank_exchange_kernels(T, k, E, hid):
+    """Routing, push, combine and its gradients on one rank: around the 1024 assignments of a routing block, one expert with most of the rows and
+    one with none, dropped pairs, more slots than the push takes at a time, rows of one and of odd numbers of 16-byte pieces."""
+    from linear_moe_b200.ops import gemm
+    from linear_moe_b200.parallel import fused_comm
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(1)
+    pad = gemm.ROW_ALIGN
+    ws = fused_comm.MoeWorkspace(None, E, hid, T * k + pad * E, dev)
+    idx = torch.where(torch.rand(T, k, device=dev) < 0.5, torch.randint(0, E - 1, (T, k), device=dev), torch.zeros((), dtype=torch.int64, device=dev))
+    idx = torch.where(torch.rand(T, k, device=dev) < 0.1, torch.full_like(idx, -1), idx)                 # (expert E - 1 gets nothing)
+    route = ws.route(idx)
+    flat = idx.reshape(-1)
+    count = torch.bincount(flat[flat >= 0], minlength=E)
+    segs = torch.cat([count.new_zeros(1), ((count + pad - 1) // pad * pad).cumsum(0)])
+    assert torch.equal(route.real.long(), count) and torch.equal(route.offs.long(), segs)
+    rank_in = torch.empty_like(flat)                                                                      # a stable counting sort
+    for e in range(E):
+        m = flat == e
+        rank_in[m] = torch.arange(int(m.sum()), device=dev)
+    want = torch.where(flat >= 0, segs[flat.clamp(min=0)] + rank_in, torch.full_like(flat, -1))
+    assert torch.equal(route.dest_row.long(), want) and torch.equal(route.dest_rank >= 0, flat >= 0)
+    x, go = (torch.randn(T, hid, device=dev).bfloat16() for _ in range(2))
+    n, sent = int(segs[-1]), flat >= 0
+    recv = ws.push(x, route, None)
+    ref = torch.zeros(n, hid, dtype=torch.bfloat16, device=dev)
+    ref[want[sent]] = x.repeat_interleave(k, 0)[sent]
+    assert torch.equal(recv[:n], ref)                                                                     # the padding rows are zeros
+    w = torch.rand(T, k, device=dev)
+    y = torch.randn(recv.shape, device=dev).bfloat16()
+    rows = torch.where(sent[:, None], y[want.clamp(min=0)].float(), torch.zeros((), device=dev)).view(T, k, hid)
+    out, _ = ws.pull(y, route, w, False)
+    torch.testing.assert_close(out.float(), (rows * w[..., None]).sum(1), rtol=2 ** -8, atol=k * 2 ** -9)
+    d_y, d_w = ws.push_combine_grad(go, y, route, w)
+    ref = torch.zeros(n, hid, device=dev)
+    ref[want[sent]] = (go.float()[:, None] * w[..., None]).reshape(-1, hid)[sent]
+    torch.testing.assert_close(d_y[:n].float(), ref, rtol=2 ** -8, atol=0)
+    torch.testing.assert_close(d_w, (rows * go.float()[:, None]).sum(-1), rtol=1e-4, atol=1e-3)            # fp32 sums over `hid` products of size one
+    torch.cuda.synchronize()
+    fused_comm.check_status("one rank")
