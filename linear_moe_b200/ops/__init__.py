@@ -142,10 +142,13 @@ class _CachedLinearCE(torch.autograd.Function):
         wd = weight if weight.dtype == h.dtype else weight.to(h.dtype)
         Z = _K().mm_nt(h, wd)
         loss = torch.empty(T, dtype=torch.float32, device=h.device)
-        lse = torch.empty(T, dtype=torch.float32, device=h.device)
         K = _K()
-        K.softmax_ce_fwd(Z, labels, loss, lse, ignore_index)
-        K.softmax_ce_bwd(Z, labels, lse, torch.ones(T, dtype=torch.float32, device=h.device), ignore_index)
+        if K.softmax_ce_rows_ok(Z):
+            K.softmax_ce_rows(Z, labels, loss, ignore_index)
+        else:
+            lse = torch.empty(T, dtype=torch.float32, device=h.device)
+            K.softmax_ce_fwd(Z, labels, loss, lse, ignore_index)
+            K.softmax_ce_bwd(Z, labels, lse, torch.ones(T, dtype=torch.float32, device=h.device), ignore_index)
         ctx.save_for_backward(h, wd, Z)
         ctx.wdtype, ctx.weight = weight.dtype, weight
         return loss
@@ -153,9 +156,7 @@ class _CachedLinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gl):
         h, wd, Z = ctx.saved_tensors
-        g = gl.to(h.dtype)[:, None]
-        dh = _K().mm_nn(Z, wd) * g
-        hg = h * g
+        dh, hg = _K().scale_rows(_K().mm_nn(Z, wd), h, gl.to(h.dtype))
         if _K().wgrad_into_main_grad(ctx.weight, Z, hg):
             return dh, None, None, None
         dw = _K().mm_tn(Z, hg)

@@ -483,6 +483,14 @@ class _Embedding(torch.autograd.Function):
         idf = ids.reshape(-1).to(torch.int64).contiguous()
         mg = getattr(w, "main_grad", None)
         direct = mg is not None and mg.dtype == torch.float32 and mg.is_contiguous()
+        if not direct and 2 * idf.numel() <= V:          # few tokens for the table: fp32 rows for the shared ids only
+            dy2 = _aligned(dy2)
+            out = torch.empty(V, h, dtype=w.dtype, device=dy.device)
+            acc = torch.empty(idf.numel(), h, dtype=torch.float32, device=dy.device)
+            tables = torch.empty(2 * V, dtype=torch.int32, device=dy.device)
+            _check(lib().lmoe_embedding_dense_grad(_p(dy2), _p(idf), _p(out), _p(acc), _p(tables), _i64(idf.numel()), _i32(h), _i64(V),
+                                                   _i64(ctx.id_offset), _i32(_dt(dy2)), _i32(_dt(out)), _st()), "embedding_dense_grad", 3)
+            return None, out, None, None
         dst = mg if direct else torch.zeros(V, h, dtype=torch.float32, device=dy.device)
         _check(lib().lmoe_embedding_bwd(_p(dy2), _p(idf), _p(dst), _i64(dy2.shape[0]), _i32(h), _i64(V), _i64(ctx.id_offset),
                                         _i32(_dt(dy2)), _st()), "embedding_bwd")
@@ -767,6 +775,29 @@ def softmax_ce_bwd(logits, labels, lse, gloss, ignore_index):
     _check(lib().lmoe_softmax_ce_bwd(_p(logits), _p(labels.contiguous()), _p(lse), _p(gloss), _p(logits), _i64(rows),
                                      _i32(V), _i64(ignore_index), _i32(_dt(logits)), _st()), "softmax_ce_bwd")
     return logits
+
+
+def softmax_ce_rows_ok(logits) -> bool:
+    return (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.is_contiguous() and logits.shape[1] % 8 == 0
+            and logits.data_ptr() % 16 == 0)
+
+
+def softmax_ce_rows(logits, labels, loss_out, ignore_index):
+    """Loss of every row, and ``softmax - onehot(label)`` over the logits (:func:`softmax_ce_rows_ok`), in one pass."""
+    rows, V = logits.shape
+    _check(lib().lmoe_softmax_ce_rows(_p(logits), _p(labels.contiguous()), _p(loss_out), _i64(rows), _i32(V), _i64(ignore_index), _st()),
+           "softmax_ce_rows")
+
+
+def scale_rows(x, h, g):
+    """``x *= g`` in place and ``h * g``, bf16 rows times bf16 ``g [rows]``, in one pass (torch's broadcasting kernels take four times as long)."""
+    if not (x.is_cuda and x.dtype == h.dtype == g.dtype == torch.bfloat16 and x.dim() == 2 and x.shape == h.shape and x.is_contiguous()
+            and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0):
+        return x * g[:, None], h * g[:, None]
+    h, g = _aligned(h), g.contiguous()
+    y = torch.empty_like(h)
+    _check(lib().lmoe_scale_rows(_p(x), _p(h), _p(y), _p(g), _i64(x.shape[0]), _i32(x.shape[1]), _st()), "scale_rows")
+    return x, y
 
 
 # =====================================================================================

@@ -436,3 +436,63 @@ def test_early_launches_wait():
     for _ in range(20):
         for a, b in zip(chain(lambda: None), want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("V", [8, 4104, 32000, 65544])
+def test_cross_entropy_rows(V):
+    """Loss and softmax - onehot in one pass over the logits: fewer pieces than threads, ragged last rounds, ignored rows, a row of equal logits."""
+    torch.manual_seed(0)
+    x = rand(37, V, scale=3)
+    x[5] = 1.5
+    labels = torch.randint(0, V, (37,), device="cuda")
+    labels[3], labels[9] = -100, V - 1
+    z, loss = x.clone(), torch.empty(37, device="cuda")
+    K.softmax_ce_rows(z, labels, loss, -100)
+    ref = x.double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(ref, labels, ignore_index=-100, reduction="none")
+    g, = torch.autograd.grad(want.sum(), ref)
+    torch.testing.assert_close(loss.double(), want.detach(), rtol=1e-5, atol=1e-5)          # fp32 sums and exponentials
+    torch.testing.assert_close(z.double(), g, rtol=2 ** -8, atol=1e-6)                     # one rounding to bf16
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,V,h", [(1, 8, 8), (300, 1000, 264), (500, 1000, 1032)])
+def test_embedding_gradient_of_few_tokens(T, V, h, dtype):
+    """The dense gradient of a table, with ids that are their token's own, shared by two and by many tokens, and outside this shard of the table."""
+    torch.manual_seed(0)
+    w = torch.randn(V, h, device="cuda", dtype=dtype).requires_grad_(True)
+    ids = torch.randint(100, 100 + V, (T,), device="cuda")
+    if T > 1:
+        ids[: T // 3] = 100 + V - 1
+        ids[-1], ids[-2] = 3, 100 + V + 7
+    go = torch.randn(T, h, device="cuda", dtype=dtype)
+    got, = torch.autograd.grad(K.embedding(ids, w, 100, True), w, go)
+    inside = (ids >= 100) & (ids < 100 + V)
+    want = torch.zeros(V, h, device="cuda", dtype=torch.float64).index_add_(0, ids[inside] - 100, go[inside].double())
+    assert got.dtype == dtype and rel(got, want) < (U if dtype == torch.bfloat16 else 1e-6)
+
+
+def test_scaled_rows():
+    x, h, g = rand(13, 1032, scale=1), rand(13, 1032, scale=1), rand(13, scale=1)
+    wx, wh = x * g[:, None], h * g[:, None]
+    a, b = K.scale_rows(x, h, g)
+    assert a is x and torch.equal(a, wx) and torch.equal(b, wh)
+
+
+@pytest.mark.parametrize("kind", ["scalar", "vector", "delta"])
+def test_states_that_may_be_overwritten(kind):
+    """One-token steps: a new state beside the old one, or over a state that was given away for that, with the same bits."""
+    from linear_moe_b200.infer.generation import _overwritable
+    torch.manual_seed(0)
+    B, H, D = 3, 2, 128
+    q, k, v = rand(B, 1, H, D), torch.nn.functional.normalize(torch.randn(B, 1, H, D, device="cuda"), dim=-1).bfloat16(), rand(B, 1, H, D)
+    g, gk, beta = -torch.rand(B, 1, H, device="cuda"), -torch.rand(B, 1, H, D, device="cuda"), torch.rand(B, 1, H, device="cuda")
+    step = {"scalar": lambda S: ops.lsm_scalar(q, k, v, g, None, S), "vector": lambda S: ops.lsm_vector(q, k, v, gk, None, S),
+            "delta": lambda S: ops.lsm_delta(q, k, v, beta, g, None, S)}[kind]
+    with torch.no_grad():
+        S = torch.randn(B, H, D, D, device="cuda")
+        before = S.clone()
+        o, S1 = step(S)
+        assert torch.equal(S, before) and S1.data_ptr() != S.data_ptr()
+        o2, S2 = step(_overwritable(S))
+        assert S2.data_ptr() == S.data_ptr() and torch.equal(S, S1) and torch.equal(o, o2)
