@@ -2,8 +2,9 @@
 // with accumulators in tensor memory, operands staged by TMA (4-D tensor maps over [B, T, H, D], 128-byte swizzle).
 //
 // One CTA = 128 queries of one head.  640 threads:
-//   warp 0      TMA producer: Q once, then K_j / V_j tiles of 128 keys through two 2-stage rings
-//   warp 1      MMA issuer:   S_{j+1} = Q K_{j+1}^T is issued before O += P_j V_j
+//   warp 0      TMA producer: Q once, then K_j / V_j tiles of 128 keys through rings of three and two stages
+//   warps 1, 2  MMA issuers, one per softmax group: S_j = Q K_j^T, then O += P_j V_j.  (One warp for both spent 1.3 of 2.4 thousand cycles a tile waiting
+//               for one group's product to complete before it could issue the other group's next one.)
 //   warps 4..19 softmax, two groups of eight: group g works on the tiles j = g (mod 2), so that one group's exponentials run while the
 //               other one waits for its scores, exchanges maxima or hands over P.  (With all warps on the same tile every stage of
 //               it was exposed: 3900 cycles a tile against 1024 of exponentials.)  Inside a group the two warps with equal (w & 3) own the 32 rows
@@ -12,7 +13,7 @@
 // units of a maximum that may lag behind by up to 2^LAG; only when a row runs ahead of that the output is rescaled there.  P_j goes
 // back over its scores in bf16 and is read as the A operand from tensor memory.
 // Tensor memory: 2 x 128 columns of scores, 2 x D of outputs.
-// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 180 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 61 us.
+// B=2, T=4096, 16 query and 4 kv heads of 128: 242 -> 180 us; B=1, 1531 queries over 2552 keys, 32 / 8 heads of 64: 86 -> 60 us (with one issuing warp and two stages of K 63).
 // Masking (causal with a query offset, sliding window, key length) is applied only on tiles that cross a boundary.
 // Every mbarrier wait is bounded (clock64 budget); on expiry the error word is set and the CTA drains and frees its
 // tensor memory.  Writes O (bf16) and the natural-log row log-sum-exp, which the backward kernels of flash_attn.cu use.
@@ -38,9 +39,9 @@ constexpr float LAG = 8.f;            // how far, as a power of two, a row's wei
 template <int D>
 struct __align__(1024) Smem {
     uint8_t q[BM * D * 2];
-    uint8_t k[2][BN * D * 2];
+    uint8_t k[3][BN * D * 2];         // the scores of a tile wait for its K at once, its V only behind the exponentials
     uint8_t v[2][BN * D * 2];
-    uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done[2];
+    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done[2];
     float mx[2][2][2][BM];            // [parity of the group's tile][group][half of the columns]
     float ls[2][2][BM], ms[2][BM];    // sums and maxima at the end
     uint32_t tmem_base;
@@ -72,7 +73,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     constexpr int DK = D / 64;                              // 64-element blocks along the head dimension
     constexpr uint32_t TMEM_COLS = 512;
     constexpr uint32_t O_COL = 2 * BN;                      // the groups' outputs behind the two score buffers
-    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int n_qb = (a.Tq + BM - 1) / BM;
     const TileOf t = longest_first(blockIdx.x, n_qb, a.B * a.Hq, group);
     const int qb = n_qb - 1 - t.rank;                       // late query tiles see the most keys
@@ -91,8 +92,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.q_full, 1);
+        for (int s = 0; s < 3; ++s) { mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1); }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1);
             mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1);
             mbar_init(&sm.s_full[s], 1); mbar_init(&sm.pv_done[s], 1);
             mbar_init(&sm.p_ready[s], 8);
@@ -107,7 +108,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
+    const uint32_t tmem_base = uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
@@ -115,13 +116,13 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
             for (int kb = 0; kb < DK; ++kb) tma_load_4d(sm.q + kb * BM * 128, &tmQ, &sm.q_full, kb * 64, h, q0, b);
             for (int j = 0; j < n_it; ++j) {
-                const int s = j & 1;
+                const int s = j & 1, s3 = j % 3;
                 const uint32_t ph = (j >> 1) & 1;
                 const int key0 = (nb_lo + j) * BN;
-                if (!mbar_wait_suspend(&sm.k_empty[s], ph ^ 1, abort_flag, err, 0x1100 | s)) break;
-                mbar_expect_tx(&sm.k_full[s], BN * D * 2);
+                if (!mbar_wait_suspend(&sm.k_empty[s3], ((j / 3) & 1) ^ 1, abort_flag, err, 0x1100 | s3)) break;
+                mbar_expect_tx(&sm.k_full[s3], BN * D * 2);
 #pragma unroll
-                for (int kb = 0; kb < DK; ++kb) tma_load_4d(sm.k[s] + kb * BN * 128, &tmK, &sm.k_full[s], kb * 64, hk, key0, b);
+                for (int kb = 0; kb < DK; ++kb) tma_load_4d(sm.k[s3] + kb * BN * 128, &tmK, &sm.k_full[s3], kb * 64, hk, key0, b);
                 if (!mbar_wait_suspend(&sm.v_empty[s], ph ^ 1, abort_flag, err, 0x1200 | s)) break;
                 mbar_expect_tx(&sm.v_full[s], BN * D * 2);
                 // MN-major operand: per 64 keys, D/64 boxes of {64 d, 64 keys} (8 KiB each)
@@ -132,47 +133,44 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         tma_load_4d(sm.v[s] + (kk * DK + nb) * 8192, &tmV, &sm.v_full[s], nb * 64, hk, key0 + kk * 64, b);
             }
         }
-    } else if (warp == 1) {
-        if (n_it > 0) {
-            const uint32_t issue = lane == 0 ? 1u : 0u;
+    } else if (warp == 1 || warp == 2) {                       // a group's products, each group's in a warp of its own
+        const int g = warp - 1;
+        if (g < n_it) {
             constexpr uint32_t idesc_s = idesc_bf16<false, BN>();
             constexpr uint32_t idesc_o = idesc_bf16<true, D>();
-            bool ok = fatc::mbar_wait_warp(&sm.q_full, 0, abort_flag, err, 0x2000);
-            auto issue_s = [&](int j) -> bool {
-                const int s = j & 1;
-                if (!fatc::mbar_wait_warp(&sm.k_full[s], (j >> 1) & 1, abort_flag, err, 0x2100 | s)) return false;
+            bool ok = mbar_wait_warp(&sm.q_full, 0, abort_flag, err, 0x2000);
+            for (int j = g; ok && j < n_it; j += 2) {
+                const int s3 = j % 3;
+                const uint32_t ph = (j >> 1) & 1;
+                // the scores go over the group's last P: its product has to complete
+                ok = mbar_wait_warp(&sm.k_full[s3], (j / 3) & 1, abort_flag, err, 0x2100 | s3) &&
+                     (j < 2 || mbar_wait_warp(&sm.pv_done[g], ph ^ 1, abort_flag, err, 0x2400));
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t ql = desc_lo<false>(s32(sm.q)), kl = desc_lo<false>(s32(sm.k[s]));
+                if (elect_one()) {
+                    const uint32_t ql = desc_lo<false>(s32(sm.q)), kl = desc_lo<false>(s32(sm.k[s3]));
 #pragma unroll
-                for (int kk = 0; kk < D / UMMA_K; ++kk) {
-                    const uint32_t off = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4;
-                    umma_lo(tmem_base + s * BN, ql + off, kl + off, idesc_s, kk > 0 ? 1u : 0u, issue);
+                    for (int kk = 0; kk < D / UMMA_K; ++kk) {
+                        const uint32_t off = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4;
+                        umma_ss(tmem_base + g * BN, ql + off, kl + off, idesc_s, kk > 0);
+                    }
+                    umma_commit(&sm.k_empty[s3]);
+                    umma_commit(&sm.s_full[g]);
                 }
-                umma_commit_if(&sm.k_empty[s], issue);
-                umma_commit_if(&sm.s_full[s], issue);
-                return true;
-            };
-            if (ok) ok = issue_s(0);
-            for (int j = 0; ok && j < n_it; ++j) {
-                const int s = j & 1;
-                if (j + 1 < n_it) {
-                    // the other score buffer holds P_{j-1}: its product has to complete
-                    if (j > 0 && !fatc::mbar_wait_warp(&sm.pv_done[s ^ 1], ((j - 1) >> 1) & 1, abort_flag, err, 0x2400)) break;
-                    ok = issue_s(j + 1);
-                    if (!ok) break;
-                }
-                if (!fatc::mbar_wait_warp(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x2200 | s)) break;
-                if (!fatc::mbar_wait_warp(&sm.p_ready[s], (j >> 1) & 1, abort_flag, err, 0x2300 | s)) break;
+                ok = mbar_wait_warp(&sm.v_full[g], ph, abort_flag, err, 0x2200 | g) && mbar_wait_warp(&sm.p_ready[g], ph, abort_flag, err, 0x2300 | g);
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t vl = desc_lo<true>(s32(sm.v[s]));
+                if (elect_one()) {
+                    const uint32_t vl = desc_lo<true>(s32(sm.v[g]));
 #pragma unroll
-                for (int kk = 0; kk < BN / UMMA_K; ++kk) {
-                    // every half of the columns left its 32 columns of P at its beginning
-                    const uint32_t boff = ((kk / 4) * (DK * 8192) + (kk % 4) * 2048) >> 4;
-                    umma_ta(tmem_base + O_COL + s * D, tmem_base + s * BN + kk / 4 * 64 + kk % 4 * 8, vl + boff, idesc_o, (j > 1 || kk > 0) ? 1u : 0u, issue);
+                    for (int kk = 0; kk < BN / UMMA_K; ++kk) {
+                        // every half of the columns left its 32 columns of P at its beginning
+                        const uint32_t boff = ((kk / 4) * (DK * 8192) + (kk % 4) * 2048) >> 4;
+                        umma_ts(tmem_base + O_COL + g * D, tmem_base + g * BN + kk / 4 * 64 + kk % 4 * 8, vl + boff, idesc_o, j > 1 || kk > 0);
+                    }
+                    umma_commit(&sm.v_empty[g]);
+                    umma_commit(&sm.pv_done[g]);
                 }
-                umma_commit_if(&sm.v_empty[s], issue);
-                umma_commit_if(&sm.pv_done[s], issue);
             }
         }
     } else if (warp >= 4) {
@@ -358,21 +356,23 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
 }
 // [128 x 128] = A B^T over D, both tiles K-major
 template <int D>
-__device__ __forceinline__ void score_product(uint32_t tmem_d, const uint8_t* A, const uint8_t* B, uint32_t issue) {
+__device__ __forceinline__ void score_product(uint32_t tmem_d, const uint8_t* A, const uint8_t* B) {
+    if (!elect_one()) return;
     const uint32_t al = desc_lo<false>(s32(A)), bl = desc_lo<false>(s32(B));
 #pragma unroll
     for (int kk = 0; kk < D / UMMA_K; ++kk) {
         const uint32_t off = ((kk / 4) * BLK + (kk % 4) * 32) >> 4;
-        umma_lo(tmem_d, al + off, bl + off, idesc_bf16<false, 128>(), kk > 0 ? 1u : 0u, issue);
+        umma_ss(tmem_d, al + off, bl + off, idesc_bf16<false, 128>(), kk > 0);
     }
 }
 // [128 x D] (+)= A B over 128: A in tensor memory as the warps left it (16 packed columns at the beginning of every part's 32), B's rows are K
 template <int D>
-__device__ __forceinline__ void grad_product(uint32_t tmem_d, uint32_t tmem_a, const uint8_t* B, bool add, uint32_t issue) {
+__device__ __forceinline__ void grad_product(uint32_t tmem_d, uint32_t tmem_a, const uint8_t* B, bool add) {
+    if (!elect_one()) return;
     const uint32_t bl = ((s32(B) >> 4) & 0x3FFFu) | ((uint32_t)(BLK >> 4) << 16);
 #pragma unroll
     for (int kk = 0; kk < 128 / UMMA_K; ++kk)
-        umma_ta(tmem_d, tmem_a + kk / 2 * 32 + kk % 2 * 8, bl + ((kk * 2048) >> 4), idesc_bf16<true, D>(), (add || kk > 0) ? 1u : 0u, issue);
+        umma_ts(tmem_d, tmem_a + kk / 2 * 32 + kk % 2 * 8, bl + ((kk * 2048) >> 4), idesc_bf16<true, D>(), add || kk > 0);
 }
 // this thread's 32 columns of an operand, over scores that it has read
 __device__ __forceinline__ void hand_over(uint32_t taddr, const uint32_t (&v)[16], uint64_t* bar) {
@@ -419,7 +419,7 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         return;
     }
     constexpr uint32_t TMEM_COLS = 512, DP = 256, DQ = 384;                  // two buffers of scores in front
-    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int n_qb = (a.Tq + BM - 1) / BM;
     const TileOf t = longest_first(blockIdx.x, n_qb, a.B * a.Hq, group);
     const int qb = n_qb - 1 - t.rank;
@@ -449,7 +449,7 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
+    const uint32_t tmem_base = uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
@@ -468,37 +468,34 @@ fa_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
     } else if (warp == 1) {
         if (n_it > 0) {
-            const uint32_t issue = lane == 0 ? 1u : 0u;
-            bool ok = fatc::mbar_wait_warp(&sm.qg_full, 0, abort_flag, err, 0x4200);
+            bool ok = mbar_wait_warp(&sm.qg_full, 0, abort_flag, err, 0x4200);
             auto scores = [&](int j) -> bool {
                 const int s = j & 1, s3 = j % 3;
-                if (!fatc::mbar_wait_warp(&sm.k_full[s3], (j / 3) & 1, abort_flag, err, 0x4300 | s3)) return false;
+                if (!mbar_wait_warp(&sm.k_full[s3], (j / 3) & 1, abort_flag, err, 0x4300 | s3)) return false;
                 tc_fence_after();
-                score_product<D>(tmem_base + s * 128, sm.q, sm.k[s3], issue);
-                umma_commit_if(&sm.s_full[s], issue);
+                score_product<D>(tmem_base + s * 128, sm.q, sm.k[s3]);
+                if (elect_one()) umma_commit(&sm.s_full[s]);
                 return true;
             };
             auto dprobs = [&](int j) -> bool {
                 const int s = j & 1;
-                if (!fatc::mbar_wait_warp(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x4310 | s)) return false;
+                if (!mbar_wait_warp(&sm.v_full[s], (j >> 1) & 1, abort_flag, err, 0x4310 | s)) return false;
                 tc_fence_after();
-                score_product<D>(tmem_base + DP, sm.g, sm.v[s], issue);
-                umma_commit_if(&sm.v_empty[s], issue);
-                umma_commit_if(&sm.dp_full, issue);
+                score_product<D>(tmem_base + DP, sm.g, sm.v[s]);
+                if (elect_one()) { umma_commit(&sm.v_empty[s]); umma_commit(&sm.dp_full); }
                 return true;
             };
             if (ok) ok = scores(0) && dprobs(0);
             if (ok && n_it > 1) ok = scores(1);
             for (int j = 0; ok && j < n_it; ++j) {
                 const int s = j & 1;
-                if (!fatc::mbar_wait_warp(&sm.ds_ready, j & 1, abort_flag, err, 0x4400)) break;
+                if (!mbar_wait_warp(&sm.ds_ready, j & 1, abort_flag, err, 0x4400)) break;
                 if (j + 1 < n_it && !dprobs(j + 1)) break;
                 tc_fence_after();
-                grad_product<D>(tmem_base + DQ, tmem_base + s * 128, sm.k[j % 3], j > 0, issue);
-                umma_commit_if(&sm.k_empty[j % 3], issue);
-                umma_commit_if(j + 1 < n_it ? &sm.dq_done : &sm.all_done, issue);
+                grad_product<D>(tmem_base + DQ, tmem_base + s * 128, sm.k[j % 3], j > 0);
+                if (elect_one()) { umma_commit(&sm.k_empty[j % 3]); umma_commit(j + 1 < n_it ? &sm.dq_done : &sm.all_done); }
                 // the next scores of this buffer go over dS_j: the product that reads it has to complete
-                if (j + 2 < n_it) ok = fatc::mbar_wait_warp(&sm.dq_done, j & 1, abort_flag, err, 0x4600) && scores(j + 2);
+                if (j + 2 < n_it) ok = mbar_wait_warp(&sm.dq_done, j & 1, abort_flag, err, 0x4600) && scores(j + 2);
             }
         }
     } else if (warp >= 4) {
@@ -581,7 +578,7 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         return;
     }
     constexpr uint32_t TMEM_COLS = 512, ST = 0, DP = 128, DV = 256, DKC = 384;
-    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const TileOf t = longest_first(blockIdx.x, (a.Tk + BM - 1) / BM, a.B * a.Hkv, group);
     const int kb_tile = t.rank, hk = t.pair % a.Hkv, b = t.pair / a.Hkv;      // early key tiles are seen by the most queries
     const int rep = a.Hq / a.Hkv;
@@ -615,7 +612,7 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
+    const uint32_t tmem_base = uniform(sm.tmem_base);
 
     if (warp == 0) {
         if (lane == 0 && n_it > 0) {
@@ -635,40 +632,38 @@ fa_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
     } else if (warp == 1) {
         if (n_it > 0) {
-            const uint32_t issue = lane == 0 ? 1u : 0u;
-            bool ok = fatc::mbar_wait_warp(&sm.kv_full, 0, abort_flag, err, 0x5200);
+            bool ok = mbar_wait_warp(&sm.kv_full, 0, abort_flag, err, 0x5200);
             auto scores = [&](int it) -> bool {
-                if (!fatc::mbar_wait_warp(&sm.q_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5300 | (it & 1))) return false;
+                if (!mbar_wait_warp(&sm.q_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5300 | (it & 1))) return false;
                 tc_fence_after();
-                score_product<D>(tmem_base + ST, sm.k, sm.q[it & 1], issue);
-                umma_commit_if(&sm.s_full, issue);
+                score_product<D>(tmem_base + ST, sm.k, sm.q[it & 1]);
+                if (elect_one()) umma_commit(&sm.s_full);
                 return true;
             };
             auto dprobs = [&](int it) -> bool {
-                if (!fatc::mbar_wait_warp(&sm.g_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5310 | (it & 1))) return false;
+                if (!mbar_wait_warp(&sm.g_full[it & 1], (it >> 1) & 1, abort_flag, err, 0x5310 | (it & 1))) return false;
                 tc_fence_after();
-                score_product<D>(tmem_base + DP, sm.v, sm.g[it & 1], issue);
-                umma_commit_if(&sm.dp_full, issue);
+                score_product<D>(tmem_base + DP, sm.v, sm.g[it & 1]);
+                if (elect_one()) umma_commit(&sm.dp_full);
                 return true;
             };
             if (ok) ok = scores(0) && dprobs(0);
             for (int it = 0; ok && it < n_it; ++it) {
-                if (!fatc::mbar_wait_warp(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
+                if (!mbar_wait_warp(&sm.p_ready, it & 1, abort_flag, err, 0x5400)) break;
                 tc_fence_after();
                 const bool more = it + 1 < n_it;
-                grad_product<D>(tmem_base + DV, tmem_base + ST, sm.g[it & 1], it > 0, issue);   // dV += P^T dO
-                umma_commit_if(&sm.g_empty[it & 1], issue);
+                grad_product<D>(tmem_base + DV, tmem_base + ST, sm.g[it & 1], it > 0);   // dV += P^T dO
+                if (elect_one()) umma_commit(&sm.g_empty[it & 1]);
                 if (more) {
                     // the next scores go over P^T: the product that reads it has to complete
-                    umma_commit_if(&sm.dv_done, issue);
-                    if (!fatc::mbar_wait_warp(&sm.dv_done, it & 1, abort_flag, err, 0x5600) || !scores(it + 1)) break;
+                    if (elect_one()) umma_commit(&sm.dv_done);
+                    if (!mbar_wait_warp(&sm.dv_done, it & 1, abort_flag, err, 0x5600) || !scores(it + 1)) break;
                 }
-                if (!fatc::mbar_wait_warp(&sm.ds_ready, it & 1, abort_flag, err, 0x5410)) break;
+                if (!mbar_wait_warp(&sm.ds_ready, it & 1, abort_flag, err, 0x5410)) break;
                 tc_fence_after();
-                grad_product<D>(tmem_base + DKC, tmem_base + DP, sm.q[it & 1], it > 0, issue);  // dK += dS^T Q
-                umma_commit_if(&sm.q_empty[it & 1], issue);
-                umma_commit_if(more ? &sm.dk_done : &sm.all_done, issue);
-                if (more) ok = fatc::mbar_wait_warp(&sm.dk_done, it & 1, abort_flag, err, 0x5610) && dprobs(it + 1);
+                grad_product<D>(tmem_base + DKC, tmem_base + DP, sm.q[it & 1], it > 0);  // dK += dS^T Q
+                if (elect_one()) { umma_commit(&sm.q_empty[it & 1]); umma_commit(more ? &sm.dk_done : &sm.all_done); }
+                if (more) ok = mbar_wait_warp(&sm.dk_done, it & 1, abort_flag, err, 0x5610) && dprobs(it + 1);
             }
         }
     } else if (warp == 2) {                                      // log-sum-exp and delta of the looped queries

@@ -87,6 +87,23 @@ __device__ __forceinline__ void umma_commit_if(uint64_t* bar, uint32_t issue) {
     asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"
                  "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" :: "r"(s32(bar)), "r"(issue) : "memory");
 }
+// One lane of a converged warp, always the same one, in a form that the compiler knows: the products issued behind it keep their operands in uniform
+// registers.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r != 0;
+}
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo) { return ((uint64_t)DESC_HI << 32) | lo; }
+__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+                 :: "r"(tmem_d), "l"(desc_of(a_lo)), "l"(desc_of(b_lo)), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+}
+// D += A B with A in tensor memory: row r in lane r, two consecutive k per column
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+                 :: "r"(tmem_d), "r"(tmem_a), "l"(desc_of(b_lo)), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
