@@ -20,26 +20,15 @@
 // 512 threads, one CTA per SM (two where 64-wide heads have more CTAs than SMs): a warp owns 16 rows of every product and a quarter of its columns (of the state: half or a quarter).  For the
 // gates a thread owns two channels and VCH / GR consecutive tokens: running sums stay in registers, the GR groups of tokens meet in one
 // small table, and the next chunk's gates and tiles are on their way while this one is worked on.  (With eight warps, single buffers and a
-// 64-step running sum in 128 threads the chunks were bound by latency.)  8 x 2048 tokens, 8 heads of 128: outputs 135 -> 97 us, dq
-// 138 -> 102, dk / dv 187 -> 141, group summaries 82 and 71 -> 43 and 41.
+// 64-step running sum in 128 threads the chunks were bound by latency.)  8 x 2048 tokens, 8 heads of 128: group summaries 82 and 71 -> 43 and
+// 41 us.  The sweeps of 128-wide heads are in lsm_vector_tc.cu, those here are for 64-wide ones.
+#include "lsm_vector.cuh"
 #include "mma_utils.cuh"
 
 namespace lmoe {
 
 constexpr int VCH = 64;
 constexpr int VTHREADS = 512;
-
-struct GlaArgs {
-    const bf16 *q, *k, *v, *d_o;
-    int64_t qs_b, qs_t, qs_h, ks_b, ks_t, ks_h, vs_b, vs_t, vs_h;
-    bf16 *o, *dq, *dk, *dv;
-    int64_t dqs_b, dqs_t, dqs_h, dks_b, dks_t, dks_h, dvs_b, dvs_t, dvs_h;
-    const float* gk;               // [B,T,H,D] fp32 log decay
-    float scale;
-    int B, T, H, G, cpg;
-    float* states;                 // [B,H,G,D,D]
-    float* gdecay;                 // [B,H,G,D] total log decay of each group per channel
-};
 
 template <int D> struct VCfg {
     static constexpr int LD = D + 8, PLD = VCH + 8, TILE = VCH * LD;
@@ -249,36 +238,49 @@ __global__ void __launch_bounds__(VTHREADS, CTAS) gla_state_scan_kernel(GlaArgs 
     }
 }
 
-// 2. combine with a per-row (key channel) decay
-template <int REV>
-__global__ void gla_combine_kernel(float* __restrict__ states, const float* __restrict__ gdecay, const float* __restrict__ seed,
-                                   float* __restrict__ final_out, int G, int D) {
+// 2. combine with a per-row (key channel) decay; a thread owns V consecutive values of the state
+template <int REV, int V>
+__global__ void __launch_bounds__(256) gla_combine_kernel(float* __restrict__ states, const float* __restrict__ gdecay, const float* __restrict__ seed,
+                                                          float* __restrict__ final_out, int G, int D) {
+    struct __align__(4 * V) Vec { float x[V]; };
     const int bh = blockIdx.y;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     const int DD = D * D;
     if (e >= DD) return;
     const int row = e / D;
-    float carry = seed != nullptr ? seed[(int64_t)bh * DD + e] : 0.f;
+    auto load = [](const float* p) -> Vec {
+        Vec r;
+        if constexpr (V == 4) { const float4 v = __ldcg(reinterpret_cast<const float4*>(p)); r.x[0] = v.x; r.x[1] = v.y; r.x[2] = v.z; r.x[3] = v.w; }
+        else r.x[0] = __ldcg(p);
+        return r;
+    };
+    Vec carry;
+    if (seed != nullptr) carry = load(seed + (int64_t)bh * DD + e);
+    else
+#pragma unroll
+        for (int c = 0; c < V; ++c) carry.x[c] = 0.f;
     // batches of loads in flight together (a load per group that waits for the previous store is bound by memory latency)
     constexpr int NB = 8;
     for (int i0 = 0; i0 < G; i0 += NB) {
-        float m[NB], dec[NB];
+        Vec m[NB];
+        float dec[NB];
 #pragma unroll
         for (int j = 0; j < NB; ++j)
             if (i0 + j < G) {
                 const int g = REV ? G - 1 - (i0 + j) : i0 + j;
-                m[j] = __ldcg(states + ((int64_t)bh * G + g) * DD + e);
+                m[j] = load(states + ((int64_t)bh * G + g) * DD + e);
                 dec[j] = __expf(gdecay[((int64_t)bh * G + g) * D + row]);
             }
 #pragma unroll
         for (int j = 0; j < NB; ++j)
             if (i0 + j < G) {
                 const int g = REV ? G - 1 - (i0 + j) : i0 + j;
-                states[((int64_t)bh * G + g) * DD + e] = carry;
-                carry = dec[j] * carry + m[j];
+                *reinterpret_cast<Vec*>(states + ((int64_t)bh * G + g) * DD + e) = carry;
+#pragma unroll
+                for (int c = 0; c < V; ++c) carry.x[c] = dec[j] * carry.x[c] + m[j].x[c];
             }
     }
-    if (final_out != nullptr) final_out[(int64_t)bh * DD + e] = carry;
+    if (final_out != nullptr) *reinterpret_cast<Vec*>(final_out + (int64_t)bh * DD + e) = carry;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -508,17 +510,22 @@ static int gla_launch(int which, const GlaArgs& a, cudaStream_t st) {
     } while (0)
     if (which == 0) GLAUNCH((gla_state_scan_kernel<D, 0, CTAS>), gla_smem_scan<D>());
     else if (which == 1) GLAUNCH((gla_state_scan_kernel<D, 1, CTAS>), gla_smem_scan<D>());
-    else if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<D, 0, CTAS>), gla_smem_sweep<D>());
-    else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<D, 1, CTAS>), gla_smem_sweep<D>());
-    else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<D, CTAS>), gla_smem_dkv<D>());
-    else return -1;
+    else if constexpr (D == 64) {
+        if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<D, 0, CTAS>), gla_smem_sweep<D>());
+        else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<D, 1, CTAS>), gla_smem_sweep<D>());
+        else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<D, CTAS>), gla_smem_dkv<D>());
+        else return -1;
+    } else return -1;
 #undef GLAUNCH
     return (int)cudaGetLastError();
 }
 
 // which: 0 forward state scan, 1 reverse state scan, 2 forward output, 3 backward dq, 4 backward dk/dv
 LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t st) {
-    if (D == 128) return gla_launch<128, 1>(which, *ap, st);
+    // 128-wide heads: sweeps on the tensor cores of lsm_vector_tc.cu at every size (8 x 2048 tokens, 8 heads: outputs 97 -> 50 us, dq 102 -> 59, dk / dv
+    // 141 -> 76; 3 x 1111 of 16 heads, a whole forward 65 -> 46 and with its gradients 234 -> 170; one chunk of one head 14.8 and 15.3, 58.8 and 58.9).  The
+    // summaries, one product a chunk, stay here: there they took 41 and 64 us, here 43 and 42.
+    if (D == 128) return which >= 2 ? lvt::launch(which, *ap, st) : gla_launch<128, 1>(which, *ap, st);
     if (D != 64) return -2;
     // 64-wide heads, more CTAs than SMs: two per SM with 64 registers a thread overlap each other's steps.  Outputs, one and two per SM:
     // 64 x 256 tokens of 16 heads 216 and 185 us, 64 x 128 144 and 123, 32 x 64 56 and 50; where every CTA has an SM to itself the
@@ -528,9 +535,17 @@ LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t s
 
 LMOE_API int lmoe_gla_combine(int rev, float* states, const float* gdecay, const float* seed, float* final_out, int BH,
                               int G, int D, cudaStream_t st) {
-    dim3 grid((D * D + 255) / 256, BH);
-    if (rev) gla_combine_kernel<1><<<grid, 256, 0, st>>>(states, gdecay, seed, final_out, G, D);
-    else gla_combine_kernel<0><<<grid, 256, 0, st>>>(states, gdecay, seed, final_out, G, D);
+    // Four values a thread once that leaves a block for every SM.  Pairs x groups, forward, one and four values: 64 x 2 16.5 and 8.3 us, 32 x 4 10.4 and
+    // 6.3, 16 x 9 9.0 and 6.3, 9 x 16 8.5 and 8.4, 4 x 37 8.7 and 8.9 (reverse 8.4 and 12.4), 1 x 148 12.6 and 25.4.
+    const int v = (long long)BH * (D * D / 1024) >= sm_count() ? 4 : 1;
+    dim3 grid((D * D / v + 255) / 256, BH);
+    if (rev) {
+        if (v == 4) gla_combine_kernel<1, 4><<<grid, 256, 0, st>>>(states, gdecay, seed, final_out, G, D);
+        else gla_combine_kernel<1, 1><<<grid, 256, 0, st>>>(states, gdecay, seed, final_out, G, D);
+    } else {
+        if (v == 4) gla_combine_kernel<0, 4><<<grid, 256, 0, st>>>(states, gdecay, seed, final_out, G, D);
+        else gla_combine_kernel<0, 1><<<grid, 256, 0, st>>>(states, gdecay, seed, final_out, G, D);
+    }
     return (int)cudaGetLastError();
 }
 

@@ -1276,16 +1276,17 @@ class _GlaArgs(ctypes.Structure):
                 [(n, ctypes.c_int64) for n in ("dqs_b", "dqs_t", "dqs_h", "dks_b", "dks_t", "dks_h", "dvs_b", "dvs_t", "dvs_h")] +
                 [("gk", ctypes.c_void_p), ("scale", ctypes.c_float)] +
                 [(n, ctypes.c_int) for n in ("B", "T", "H", "G", "cpg")] +
-                [("states", ctypes.c_void_p), ("gdecay", ctypes.c_void_p)])
+                [("states", ctypes.c_void_p), ("gdecay", ctypes.c_void_p), ("err", ctypes.c_void_p)])
 
 
 def _gla_args(q, k, v, gk, scale, B, T, H, G, cpg, states, gdecay, d_o=None, o=None, dq=None, dk=None, dv=None):
+    from . import gemm
     grads = []
     for t in (dq, dk, dv):
         grads += (0, 0, 0) if t is None else t.stride()[:3]
     return _GlaArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(d_o), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
                     _ptr(o), _ptr(dq), _ptr(dk), _ptr(dv), *grads, gk.data_ptr(), float(scale), B, T, H, G, cpg,
-                    states.data_ptr(), _ptr(gdecay))
+                    states.data_ptr(), _ptr(gdecay), gemm._err(q.device).data_ptr())
 
 
 def _gla_launch(which, D, args):
@@ -1300,7 +1301,8 @@ def _gla_combine(rev, states, gdecay, seed, final_out, BH, G, D):
 def _vector_forward(q, k, v, gk, scale, init):
     """Returns the output, the final state and what the backward pass needs: (tensors, (groups, chunks), exchange)."""
     B, T, H, D = q.shape
-    q, k, v = _inner_contig(q), _inner_contig(k), _inner_contig(v)
+    fix = _tma_view if D == 128 else _inner_contig
+    q, k, v = fix(q), fix(k), fix(v)
     gf = _aligned(gk.float())
     G, cpg = lsm_groups(B, H, T)
     f32, dev = torch.float32, q.device
@@ -1315,7 +1317,7 @@ def _vector_forward(q, k, v, gk, scale, init):
         lasp.combine(0, states, None, final, B * H, H, G, cpg, T, D, gdecay=gdecay, dmode=2)
         _gla_launch(2, D, a)
     else:
-        seed = None if init is None else init.float().contiguous()
+        seed = None if init is None else _aligned(init.float())
         _check(lib().lmoe_gla_forward(D, ctypes.byref(a), _p(seed), _p(final), _st()), "gla", 3)
     return o, final, ((q, k, v, gf, states, gdecay, final), (G, cpg), lasp)
 
@@ -1345,7 +1347,7 @@ class _LsmVector(torch.autograd.Function):
         _gla_launch(3, D, a)
         a2 = _gla_args(q, k, v, gf, ctx.scale, B, T, H, G, cpg, dstates, None, d_o=d_o, dk=dk, dv=dv)
         _gla_launch(1, D, a2)
-        seed = None if dfinal is None else dfinal.float().contiguous()
+        seed = None if dfinal is None else _aligned(dfinal.float())
         if ctx.lasp is not None:
             r_out = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device)
             ctx.lasp.combine(1, dstates, None, None, B * H, H, G, cpg, T, D, gdecay=gdecay, dmode=2, r_out=r_out)

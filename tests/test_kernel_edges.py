@@ -496,3 +496,26 @@ def test_states_that_may_be_overwritten(kind):
         assert torch.equal(S, before) and S1.data_ptr() != S.data_ptr()
         o2, S2 = step(_overwritable(S))
         assert S2.data_ptr() == S.data_ptr() and torch.equal(S, S1) and torch.equal(o, o2)
+
+
+@pytest.mark.parametrize("B,H,T", [(1, 9, 700), (2, 5, 700), (1, 149, 70)])
+def test_vector_decay_views(B, H, T):
+    """128-wide heads from views that tensor maps or 16-byte loads could not take as they are (heads that repeat one another, a value that starts 2 bytes
+    behind a boundary, states 4 bytes behind one), with few and many sequences for the combine kernel: the same bits as from dense copies."""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    D = 128
+    q = rand(B, T, 1, D).expand(B, T, H, D)
+    k = rand(B, T, H, 3 * D)[..., D:2 * D]
+    v = rand(B * T * H * D + 1)[1:].view(B, T, H, D)
+    g = torch.nn.functional.logsigmoid(torch.randn(B, T, H, D, device="cuda")) / 4
+    S0, gS = (torch.randn(B * H * D * D + 1, device="cuda")[1:].view(B, H, D, D) for _ in range(2))
+    go = rand(B * T * H * D + 1, scale=1)[1:].view(B, T, H, D)
+    outs = []
+    for copy in (lambda t: t, lambda t: t.clone(memory_format=torch.contiguous_format)):
+        ins = [copy(t).detach().requires_grad_(True) for t in (q, k, v, g, S0)]
+        out = ops.lsm_vector(*ins[:4], None, ins[4], None, 64)
+        outs.append([*out, *torch.autograd.grad(list(out), ins, [copy(go), copy(gS)])])
+    gemm.check_error()
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
