@@ -1386,10 +1386,15 @@ class _DgArgs(ctypes.Structure):
 
 
 def _gla_dg(q, k, dq, dk):
-    """Reverse cumulative sum over time of ``q*dq - k*dk`` per channel -> fp32 ``[B,T,H,D]`` (two kernel launches)."""
+    """Reverse cumulative sum over time of ``q*dq - k*dk`` per channel -> fp32 ``[B,T,H,D]``.
+
+    One launch where a cluster per head needs at most two rounds of 1024 tokens or heads occupy most SMs, two over segments otherwise.  Two
+    launches and one, heads x tokens: 1 x 1024 37.9 and 14.3 us, 1 x 2048 37.9 and 20.5, 64 x 2048 99 and 59, 16 x 8192 108 and 82, 32 x 8192 192
+    and 105, but 4 x 16384 69 and 131."""
     B, T, H, D = q.shape
     dg = torch.empty(B, T, H, D, dtype=torch.float32, device=q.device)
-    nseg = (T + 255) // 256
+    one = T <= 2048 or B * H >= 16
+    nseg = 0 if one else (T + 255) // 256
     seg = torch.empty(B * H, nseg, D, dtype=torch.float32, device=q.device)
     a = _DgArgs()
     for name, t in (("q", q), ("k", k), ("dq", dq), ("dk", dk)):
@@ -1397,7 +1402,7 @@ def _gla_dg(q, k, dq, dk):
         setattr(a, name + "s_b", t.stride(0)), setattr(a, name + "s_t", t.stride(1)), setattr(a, name + "s_h", t.stride(2))
     a.dg, a.segsum = dg.data_ptr(), seg.data_ptr()
     a.B, a.T, a.H, a.D, a.nseg = B, T, H, D, nseg
-    _check(lib().lmoe_gla_dg(ctypes.byref(a), _st()), "gla_dg", 2)
+    _check(lib().lmoe_gla_dg(ctypes.byref(a), _st()), "gla_dg", 1 if one else 2)
     return dg
 
 

@@ -519,3 +519,17 @@ def test_vector_decay_views(B, H, T):
     gemm.check_error()
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 127, 3), (1, 129, 2), (1, 1024, 3), (1, 1025, 3), (3, 2500, 7), (1, 2049, 3)])
+def test_decay_gradient_sums(B, T, H, D):
+    """Sums from a token to the end, of a cluster in one round or several and of two launches, against 64 bits: n terms of up to three roundings
+    each, added in any order, are off by (n + 3) units of their absolute sum at most."""
+    torch.manual_seed(0)
+    qkv, d = rand(B, T, H, 3 * D, scale=1), rand(B, T, H, 3 * D, scale=1)
+    q, k, dq, dk = qkv[..., :D], qkv[..., D:2 * D], d[..., :D], d[..., D:2 * D]
+    got = K._gla_dg(q, k, dq, dk).double()
+    a, b = q.double() * dq.double(), k.double() * dk.double()
+    want, size = ((x.flip(1).cumsum(1).flip(1)) for x in (a - b, a.abs() + b.abs()))
+    assert ((got - want).abs() <= (T + 3) * 2.0 ** -24 * size).all()
