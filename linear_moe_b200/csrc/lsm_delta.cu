@@ -19,34 +19,16 @@
 //
 // Reference counterpart: fla.ops.gated_delta_rule / delta_rule chunk kernels called by
 // sequence_modeling/gated_deltanet/gated_deltanet.py:99-116 and deltanet/deltanet.py:127-130.
+#include <algorithm>
+#include "lsm_delta.cuh"
 #include "mma_utils.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace lmoe {
 namespace dr {
 
-constexpr int C = 64;            // chunk length
 constexpr int DVS = 32;          // value columns per CTA
 constexpr int NT = 256;          // threads
-
-struct Args {
-    const bf16 *W, *U, *Qd, *Kd, *A;   // [BH, N, C, dk] / [BH, N, C, dv] / [BH, N, C, C]
-    const float* gamma;                // [BH, N]
-    const float* S0;                   // [BH, dk, dv] or null
-    const bf16* dO;                    // backward: [B, T, H, dv] with the strides gs_*
-    const float* dSfinal;              // backward: [BH, dk, dv] or null
-    bf16* O;                           // forward: [B, T, H, dv] with the strides os_*, or null (not wanted)
-    bf16* Vn;                          // forward out: [BH, N, C, dv], or null (neither Vn nor Sn is kept)
-    bf16* Sn;                          // forward out: state entering chunk n, [BH, N, dk, dv]
-    float* Sfinal;                     // forward out: [BH, dk, dv]
-    bf16* dVn;                         // backward out: [BH, N, C, dv]
-    bf16* dSn;                         // backward out: gradient of the state leaving chunk n, [BH, N, dk, dv]
-    float* dS0;                        // backward out: [BH, dk, dv]
-    long long os_b, os_t, os_h, gs_b, gs_t, gs_h;
-    int N, dv, T, H;
-    int ldw, lda;                      // row strides of W, Qd, Kd and of A in memory: LDK and LDC of Cfg, or dk and C
-    int* err;                          // error word of the bounded waits
-};
 
 // Both walks are chains over the chunks, bound by the latency of a step: two products with a barrier behind each.  Eight warps share the
 // products and a ninth brings the tiles, up to two chunks ahead.  The tile kernel writes them with the padded rows they have in shared memory, so
@@ -613,15 +595,16 @@ __device__ __forceinline__ void store_rows_global(const float (&acc)[NTL][4], bf
 // the blocks on and below the diagonal are computed or read.  Sums over rows and columns stay in registers until the end: a
 // shared atomic per element and the substitution for T were two thirds of this kernel's time, T now comes from the tile kernel
 // that has just run.  Tiles arrive in the order they are needed.  Bound by shared-memory reads of the fragments (about 3 cycles per
-// 2 cycles of tensor pipe).  2 x 4096 tokens, 16 heads of 128: 580 -> 221 us.
+// 2 cycles of tensor pipe); a CTA goes on to the next chunk, whose tiles load while it works on this one.  2 x 4096 tokens, 16 heads of 128: 580 -> 224 us,
+// and with the loads ahead 213.
 constexpr int NTB = 512;
 
 template <int D>
 __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
     constexpr int LD = D + 8, LDC = C + 8, NQ = D / 32, QD = D / 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* Ks = reinterpret_cast<bf16*>(smem_raw);            // [C][LD]
-    bf16* Qs = Ks + C * LD;                                  // [C][LD]
+    bf16* K2 = reinterpret_cast<bf16*>(smem_raw);            // [2][C][LD] of this chunk and the next
+    bf16* Qs = K2 + 2 * C * LD;                              // [C][LD]
     bf16* Vs = Qs + C * LD;                                  // [C][LD]
     bf16* Gs = Vs + C * LD;                                  // [C][LD]  dO, later dW
     bf16* Ns = Gs + C * LD;                                  // [C][LD]  Vn
@@ -638,39 +621,64 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
     float* rbe = rdb + 4 * C;                                // [4][C] ... of the gradient of beta
     float* cdb = rbe + 4 * C;                                // [4][C] column sums, by row block
     float* tot = cdb + 4 * C;                                // [2][16] per warp: <dS'_n, S_n>, sum of <dKd_j, Kd_j>
-    const int n = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int t0 = n * C;
-    const int valid = min(C, a.T - t0);
-    const long long cn = (long long)bh * a.N + n;
     const int qd = w >> 2, m0 = 16 * (w & 3), r0 = m0 + (l >> 2), c0 = (l & 3) * 2;
     const bool gated = a.g != nullptr;
     const int nd = qd * QD;                                  // first column of this warp's quarter of a D-wide product
     const int nc = qd * 16;                                  // ... of a C-wide product
     const bool lower = nc <= m0;                             // does the warp's C x C block touch the lower triangle?
 
-    load_tile_async<C, D, LD>(Ks, a.k + b * a.ks_b + h * a.ks_h + (long long)t0 * a.ks_t, a.ks_t, valid);
-    load_tile_async<C, D, LD>(Qs, a.q + b * a.qs_b + h * a.qs_h + (long long)t0 * a.qs_t, a.qs_t, valid);
-    cp_async_commit();
-    load_tile_async<C, D, LD>(Gs, a.dO + b * a.gs_b + h * a.gs_h + (long long)t0 * a.gs_t, a.gs_t, valid);
-    load_tile_async<C, D, LD>(Ns, a.Vn + cn * C * D, D, C);
-    cp_async_commit();
-    load_tile_async<D, D, LD>(Sb, a.Sn + cn * D * D, D, D);
-    load_tile_async<C, D, LD>(Us, a.dVn + cn * C * D, D, C);
-    cp_async_commit();
-    load_tile_async<C, C, LDC>(Tb, a.Tinv + cn * C * C, C, C);
-    load_tile_async<C, D, LD>(Vs, a.v + b * a.vs_b + h * a.vs_h + (long long)t0 * a.vs_t, a.vs_t, valid);
-    load_tile_async<D, D, LD>(Db, a.dSn + cn * D * D, D, D);
-    cp_async_commit();
+    // A CTA goes through its chunks, and the next chunk's tiles come in as soon as this one's are done with, in four groups: (K, Q), (Vn, S_n, dS'_n),
+    // (dO, dVn, V), T.
+    const int total = a.N * a.B * a.H;
+    struct At { int b, h, t0, valid; long long cn; };
+    auto place = [&](int idx) -> At {
+        const int bh = idx / a.N, n = idx % a.N;
+        return {bh / a.H, bh % a.H, n * C, min(C, a.T - n * C), (long long)idx};
+    };
+    auto load_kq = [&](const At& x, bf16* Kd) {
+        load_tile_async<C, D, LD>(Kd, a.k + x.b * a.ks_b + x.h * a.ks_h + (long long)x.t0 * a.ks_t, a.ks_t, x.valid);
+        load_tile_async<C, D, LD>(Qs, a.q + x.b * a.qs_b + x.h * a.qs_h + (long long)x.t0 * a.qs_t, a.qs_t, x.valid);
+    };
+    auto load_states = [&](const At& x) {
+        load_tile_async<C, D, LD>(Ns, a.Vn + x.cn * C * D, D, C);
+        load_tile_async<D, D, LD>(Sb, a.Sn + x.cn * D * D, D, D);
+        load_tile_async<D, D, LD>(Db, a.dSn + x.cn * D * D, D, D);
+    };
+    auto load_grads = [&](const At& x) {
+        load_tile_async<C, D, LD>(Gs, a.dO + x.b * a.gs_b + x.h * a.gs_h + (long long)x.t0 * a.gs_t, a.gs_t, x.valid);
+        load_tile_async<C, D, LD>(Us, a.dVn + x.cn * C * D, D, C);
+        load_tile_async<C, D, LD>(Vs, a.v + x.b * a.vs_b + x.h * a.vs_h + (long long)x.t0 * a.vs_t, a.vs_t, x.valid);
+    };
+    auto load_t = [&](const At& x) { load_tile_async<C, C, LDC>(Tb, a.Tinv + x.cn * C * C, C, C); };
+    const int i0 = 2 * l, i1 = 2 * l + 1;
+    float g0 = 0.f, g1 = 0.f, be0 = 0.f, be1 = 0.f;                    // warp 0: decays and betas of two tokens, a chunk ahead
+    auto load_scalars = [&](const At& x) {
+        const long long o = ((long long)x.b * a.T + x.t0 + i0) * a.H + x.h;
+        const bool v0 = i0 < x.valid, v1 = i1 < x.valid;
+        be0 = v0 ? a.beta[o] : 0.f; be1 = v1 ? a.beta[o + a.H] : 0.f;
+        g0 = v0 && a.g != nullptr ? a.g[o] : 0.f; g1 = v1 && a.g != nullptr ? a.g[o + a.H] : 0.f;
+    };
+    {
+        const At x = place(blockIdx.x);
+        load_kq(x, K2); cp_async_commit();
+        load_states(x); cp_async_commit();
+        load_grads(x); cp_async_commit();
+        load_t(x); cp_async_commit();
+        if (w == 0) load_scalars(x);
+    }
+    for (int idx = blockIdx.x, turn = 0; idx < total; idx += gridDim.x, turn ^= 1) {
+    const At c = place(idx);
+    const int b = c.b, h = c.h, t0 = c.t0, valid = c.valid;
+    const bool more = idx + (int)gridDim.x < total;
+    const At nx = place(more ? idx + (int)gridDim.x : idx);
+    bf16 *Ks = K2 + turn * C * LD, *Kn = K2 + (turn ^ 1) * C * LD;
     if (w == 0) {
-        const int i0 = 2 * l, i1 = 2 * l + 1;
-        float g0 = 0.f, g1 = 0.f, be0 = 0.f, be1 = 0.f;
-        if (i0 < valid) { const long long o = ((long long)b * a.T + t0 + i0) * a.H + h; be0 = a.beta[o]; if (a.g != nullptr) g0 = a.g[o]; }
-        if (i1 < valid) { const long long o = ((long long)b * a.T + t0 + i1) * a.H + h; be1 = a.beta[o]; if (a.g != nullptr) g1 = a.g[o]; }
         float s = g0 + g1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const float x = __shfl_up_sync(0xffffffffu, s, o); if (l >= o) s += x; }
         bcum[i1] = s; bcum[i0] = s - g1; bet[i0] = be0; bet[i1] = be1;
+        if (more) load_scalars(nx);
     }
     cp_async_wait<3>();
     __syncthreads();
@@ -694,7 +702,7 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
             const int i = r0 + 8 * (e >> 1), j = nc + nt * 8 + c0 + (e & 1);
             gam[nt][e] = i >= j ? __expf(((e >> 1) ? b_hi : b_lo) - bcum[j]) : 0.f;             // Gamma_ij
         }
-    cp_async_wait<2>();
+    cp_async_wait<1>();
     __syncthreads();
     // ---- (2) dAqk = tril(dO Vn^T); P = scale Gamma . dAqk; decay gradients of Aqk ------------------------------------
     if (lower) {
@@ -715,8 +723,7 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
             *reinterpret_cast<__nv_bfloat162*>(Ps + (r0 + 8) * LDC + nc + nt * 8 + c0) = __floats2bfloat162_rn(pv[2], pv[3]);
         }
     }
-    cp_async_wait<1>();
-    __syncthreads();                                                   // Ps, S_n, dVn
+    __syncthreads();                                                   // Ps
     // ---- (3) dq = scale e^b (dO S^T) + P K; its decay gradient <dQd_i, Qd_i>; dk += P^T Q -----------------------------
     float acc_dk[NQ][4], acc[NQ][4];
     zero_acc<NQ>(acc_dk);
@@ -732,7 +739,9 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
     warp_gemm<NQ, D, false, false>(acc, Us, LD, m0, Sb, LD, nd);
     scale_rows<NQ>(acc, -1.f, -1.f);
     cp_async_wait<0>();
-    __syncthreads();                                                   // dO is free; T, V, dS'_n are here
+    __syncthreads();                                                   // dO and Q are free; T is here
+    if (more) load_kq(nx, Kn);
+    cp_async_commit();
     store_acc_bf16<NQ>(acc, Gs, LD, m0, nd);                           // Gs now holds dW
     // ---- (5) dgamma = <dS'_n, S_n>; dKd = Vn dS'^T -------------------------------------------------------------------
     float dgam = 0.f;
@@ -767,7 +776,9 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
     row_dot<NQ>(acc, Vs + nd, LD, m0, dbe_lo, dbe_hi);                // <dVb_i, v_i>
     scale_rows<NQ>(acc, be_lo, be_hi);
     store_rows_global<NQ>(acc, a.dv + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
-    __syncthreads();                                                   // dW complete
+    __syncthreads();                                                   // dW complete; Vn, S_n and dS'_n are free
+    if (more) load_states(nx);
+    cp_async_commit();
     // ---- (7) dKb = T^T dW: its part of dk, dbeta and db -------------------------------------------------------------
     zero_acc<NQ>(acc);
     for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<NQ, 16, true, true>(acc, Tb + k0 * LDC, LDC, m0, Gs + k0 * LD, LD, nd);
@@ -800,6 +811,8 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
         store_acc_bf16<2>(x, X1, LDC, m0, nc);
     }
     __syncthreads();
+    if (more) load_grads(nx);                                          // dW, dVn and V have been read
+    cp_async_commit();
     if (lower) {
         float x[2][4];
         zero_acc<2>(x);
@@ -850,19 +863,20 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
         for (int i = 0; i < 4; ++i) cdb[(w & 3) * C + nc + (i >> 1) * 8 + c0 + (i & 1)] = col[i];
     }
     if (l == 0) { tot[w] = dgam; tot[16 + w] = kd; }
-    __syncthreads();                                                   // Ps holds M; the sums are in
+    __syncthreads();                                                   // Ps holds M; the sums are in; T has been read
+    if (more) load_t(nx);
+    cp_async_commit();
     // ---- (9) dk += M K + M^T K; store ---------------------------------------------------------------------------------
     for (int k0 = 0; k0 <= m0; k0 += 16) warp_gemm<NQ, 16, false, true>(acc_dk, Ps + k0, LDC, m0, Ks + k0 * LD, LD, nd);
     for (int k0 = m0; k0 < C; k0 += 16) warp_gemm<NQ, 16, true, true>(acc_dk, Ps + k0 * LDC, LDC, m0, Ks + k0 * LD, LD, nd);
     store_rows_global<NQ>(acc_dk, a.dk + (((long long)b * a.T + t0) * a.H + h) * D + nd, (long long)a.H * D, m0, valid);
     // ---- (10) dbeta; dg_s = sum_{i >= s} db_i (b_C also gets the sum of <dKd_j, Kd_j> and dgamma gamma) -------------------
     if (w == 0) {
-        const int i0 = 2 * l, i1 = 2 * l + 1;
-        float x0 = 0.f, x1 = 0.f, be0 = 0.f, be1 = 0.f, last = 0.f;
+        float x0 = 0.f, x1 = 0.f, e0 = 0.f, e1 = 0.f, last = 0.f;
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
             x0 += rdb[p * C + i0] + cdb[p * C + i0]; x1 += rdb[p * C + i1] + cdb[p * C + i1];
-            be0 += rbe[p * C + i0]; be1 += rbe[p * C + i1];
+            e0 += rbe[p * C + i0]; e1 += rbe[p * C + i1];
         }
         if (l == 31) {
             const float gamma = __expf(btot);                          // gamma = e^{b_C}: d b_C += dgamma gamma
@@ -873,13 +887,14 @@ __global__ void __launch_bounds__(NTB, 1) delta_prep_bwd_kernel(PrepBwdArgs a) {
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const float y = __shfl_down_sync(0xffffffffu, s, o); if (l + o < 32) s += y; }
         const long long o0 = ((long long)b * a.T + t0 + i0) * a.H + h, o1 = o0 + a.H;
-        if (i0 < valid) { a.dbeta[o0] = be0; if (a.dg != nullptr) a.dg[o0] = s; }
-        if (i1 < valid) { a.dbeta[o1] = be1; if (a.dg != nullptr) a.dg[o1] = s - x0; }
+        if (i0 < valid) { a.dbeta[o0] = e0; if (a.dg != nullptr) a.dg[o0] = s; }
+        if (i1 < valid) { a.dbeta[o1] = e1; if (a.dg != nullptr) a.dg[o1] = s - x0; }
+    }
     }
 }
 
 template <int D> constexpr size_t prep_bwd_smem() {
-    return (size_t)(6 * C * (D + 8) + 2 * D * (D + 8) + 4 * C * (C + 8)) * 2 + (size_t)(14 * C + 32) * 4;
+    return (size_t)(7 * C * (D + 8) + 2 * D * (D + 8) + 4 * C * (C + 8)) * 2 + (size_t)(14 * C + 32) * 4;
 }
 
 template <int D> constexpr size_t prep_smem() { return (size_t)3 * C * (D + 8) * 2 + (size_t)(C * LDF + 2 * C) * 4; }
@@ -894,6 +909,7 @@ LMOE_API int lmoe_delta_scan(int dir, int dk, int BH, const dr::Args* ap, cudaSt
     const dr::Args a = *ap;
     if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0 || a.H <= 0 || a.err == nullptr) return -1;
     if (!(a.ldw == dk && a.lda == dr::C) && !(a.ldw == dk + 8 && a.lda == dr::C + 8)) return -1;
+    if (dk == dr::TC_DK && a.dv % dr::TC_DV == 0) return dr::scan_tc(dir, BH, a, st);
     dim3 grid(a.dv / dr::DVS, BH);
     const bool out = dir != 0 || a.O != nullptr;
 #define LMOE_DR_LAUNCH(KERNEL, DK)                                                                                     \
@@ -931,7 +947,7 @@ LMOE_API int lmoe_delta_prepare(int D, const dr::PrepArgs* ap, cudaStream_t st) 
 LMOE_API int lmoe_delta_prepare_bwd(int D, const dr::PrepBwdArgs* ap, cudaStream_t st) {
     const dr::PrepBwdArgs a = *ap;
     if (a.N <= 0 || a.B * a.H <= 0) return -1;
-    dim3 grid(a.N, a.B * a.H);
+    const int grid = (int)std::min<long long>((long long)a.N * a.B * a.H, sm_count());
     if (D == 128) {
         cudaError_t e = cudaFuncSetAttribute(dr::delta_prep_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dr::prep_bwd_smem<128>());
         if (e != cudaSuccess) return (int)e;

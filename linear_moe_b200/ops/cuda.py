@@ -1588,7 +1588,7 @@ def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, out=None, keep=True):
     Vn = torch.empty(B, H, N, C, dv, dtype=bf, device=dev) if keep else None
     Sn = torch.empty(B, H, N, dk, dv, dtype=bf, device=dev) if keep else None
     Sf = torch.empty(B, H, dk, dv, dtype=torch.float32, device=dev)
-    s0 = None if S0 is None else S0.float().contiguous()
+    s0 = None if S0 is None else _aligned(S0.float())
     o_strides, T = ((0, 0, 0), 0) if out is None else (out.stride()[:3], out.shape[1])
     a = _DeltaArgs(W.data_ptr(), U.data_ptr(), Qd.data_ptr(), Kd.data_ptr(), A.data_ptr(), gamma.data_ptr(), _ptr(s0), 0, 0, _ptr(out),
                    _ptr(Vn), _ptr(Sn), Sf.data_ptr(), 0, 0, 0, *o_strides, 0, 0, 0, N, dv, T, H, W.stride(3), A.stride(3),
@@ -1599,7 +1599,7 @@ def _delta_scan_fwd(W, U, Qd, Kd, A, gamma, S0, out=None, keep=True):
 
 def _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf):
     """``delta_scan_bwd_kernel``: the reverse recurrence ``dVn = A^T dO + Kd dS'``, ``dS = gamma dS' + Qd^T dO - W^T dVn`` for ``dO``
-    ``[B,T,H,dv]`` (:func:`_inner_contig`).  Returns ``dVn`` ``[B,H,N,C,dv]``, the gradient of the state leaving every chunk
+    ``[B,T,H,dv]``.  Returns ``dVn`` ``[B,H,N,C,dv]``, the gradient of the state leaving every chunk
     ``dSn`` ``[B,H,N,dk,dv]`` (bf16) and the gradient of the initial state (fp32)."""
     from . import gemm
     B, H, N, C, dk = W.shape
@@ -1609,7 +1609,8 @@ def _delta_scan_bwd(W, Qd, Kd, A, gamma, dO, dSf):
     dVn = torch.empty(B, H, N, C, dv, dtype=bf, device=dev)
     dSn = torch.empty(B, H, N, dk, dv, dtype=bf, device=dev)
     dS0 = torch.empty(B, H, dk, dv, dtype=torch.float32, device=dev)
-    dsf = None if dSf is None else dSf.float().contiguous()
+    dsf = None if dSf is None else _aligned(dSf.float())
+    dO = _tma_view(dO)
     a = _DeltaArgs()
     a.W, a.Qd, a.Kd, a.A, a.gamma = (t.data_ptr() for t in (W, Qd, Kd, A, gamma))
     a.U = 0

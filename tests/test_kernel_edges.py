@@ -533,3 +533,21 @@ def test_decay_gradient_sums(B, T, H, D):
     a, b = q.double() * dq.double(), k.double() * dk.double()
     want, size = ((x.flip(1).cumsum(1).flip(1)) for x in (a - b, a.abs() + b.abs()))
     assert ((got - want).abs() <= (T + 3) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("B,T,H,dv", [(2, 300, 2, 32), (2, 300, 2, 64), (2, 300, 2, 96), (2, 300, 2, 192), (2, 700, 16, 128), (1, 64, 149, 128)])
+def test_delta_rule_sizes(B, T, H, dv):
+    """128-wide keys with other value widths (multiples of 64 on the 5th-generation tensor cores, the others not), and more chunks than SMs: the
+    kernel of the tiles' gradients goes on to a next chunk while it works on one."""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    D = 128
+    q, k = rand(B, T, H, D), torch.nn.functional.normalize(torch.randn(B, T, H, D, device="cuda"), dim=-1).bfloat16()
+    v, beta = rand(B, T, H, dv), torch.rand(B, T, H, device="cuda")
+    g = torch.nn.functional.logsigmoid(torch.randn(B, T, H, device="cuda") + 2)
+    S0, go, gS = 0.2 * torch.randn(B, H, D, dv, device="cuda"), rand(B, T, H, dv, scale=1), 0.05 * torch.randn(B, H, D, dv, device="cuda")
+    ins = [q, k, v, beta, g, S0]
+    got = run(lambda q, k, v, beta, g, S: ops.lsm_delta(q, k, v, beta, g, None, S, 64), ins, [go, gS])
+    gemm.check_error()
+    want = run(lambda q, k, v, beta, g, S: RL.recurrent_lsm(q, k, v, beta=beta, g=g, initial_state=S), [t.float() for t in ins], [go.float(), gS])
+    check(got, want, ["o", "S", "dq", "dk", "dv", "dbeta", "dg", "dS0"])
