@@ -140,4 +140,15 @@ __device__ __forceinline__ float dsilu_f(float x) {
     return s * (1.f + x * (1.f - s));
 }
 
+// V consecutive fp32 values of a thread (V 4: from a 16-byte boundary on), read past L1
+template <int V> struct __align__(4 * V) Values { float x[V]; };
+template <int V>
+__device__ __forceinline__ Values<V> load_values(const float* p) {
+    static_assert(V == 1 || V == 4);
+    Values<V> r;
+    if constexpr (V == 4) { const float4 v = __ldcg(reinterpret_cast<const float4*>(p)); r.x[0] = v.x; r.x[1] = v.y; r.x[2] = v.z; r.x[3] = v.w; }
+    else r.x[0] = __ldcg(p);
+    return r;
+}
+
 }  // namespace lmoe

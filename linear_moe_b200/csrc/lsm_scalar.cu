@@ -150,25 +150,30 @@ __global__ void __launch_bounds__(NTHREADS) state_scan_kernel(LsmArgs a) {
 //    `final` <- state after the last group.  reverse: slot g <- state gradient leaving group g (entering from the
 //    right), `final` <- gradient wrt the initial state.  `seed` = initial state / final-state gradient (nullable).
 // ---------------------------------------------------------------------------------------------
-template <int REV>
-__global__ void combine_kernel(float* __restrict__ states, const float* __restrict__ gdecay, const float* __restrict__ gconst,
-                               const float* __restrict__ seed, float* __restrict__ final_out, int H, int G, int cpg, int T,
-                               int DD) {
+template <int REV, int V>
+__global__ void __launch_bounds__(256) combine_kernel(float* __restrict__ states, const float* __restrict__ gdecay, const float* __restrict__ gconst,
+                                                      const float* __restrict__ seed, float* __restrict__ final_out, int H, int G, int cpg, int T,
+                                                      int DD) {
     const int bh = blockIdx.y, h = bh % H;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;          // a thread owns V consecutive values
     if (e >= DD) return;
-    float carry = seed != nullptr ? seed[(int64_t)bh * DD + e] : 0.f;
+    Values<V> carry;
+    if (seed != nullptr) carry = load_values<V>(seed + (int64_t)bh * DD + e);
+    else
+#pragma unroll
+        for (int c = 0; c < V; ++c) carry.x[c] = 0.f;
     // the summaries of a batch of groups are loaded before any of them is overwritten, so that the loads of a thread are
     // in flight together (one dependent load per group would leave the kernel bound by memory latency)
     constexpr int NB = 8;
     for (int i0 = 0; i0 < G; i0 += NB) {
-        float m[NB], dec[NB];
+        Values<V> m[NB];
+        float dec[NB];
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
             const int i = i0 + j;
             if (i < G) {
                 const int g = REV ? G - 1 - i : i;
-                m[j] = __ldcg(states + ((int64_t)bh * G + g) * DD + e);
+                m[j] = load_values<V>(states + ((int64_t)bh * G + g) * DD + e);
                 float a;
                 if (gdecay != nullptr) a = gdecay[(int64_t)bh * G + g];
                 else if (gconst != nullptr) {
@@ -183,12 +188,13 @@ __global__ void combine_kernel(float* __restrict__ states, const float* __restri
             const int i = i0 + j;
             if (i < G) {
                 const int g = REV ? G - 1 - i : i;
-                states[((int64_t)bh * G + g) * DD + e] = carry;
-                carry = dec[j] * carry + m[j];
+                *reinterpret_cast<Values<V>*>(states + ((int64_t)bh * G + g) * DD + e) = carry;
+#pragma unroll
+                for (int c = 0; c < V; ++c) carry.x[c] = dec[j] * carry.x[c] + m[j].x[c];
             }
         }
     }
-    if (final_out != nullptr) final_out[(int64_t)bh * DD + e] = carry;
+    if (final_out != nullptr) *reinterpret_cast<Values<V>*>(final_out + (int64_t)bh * DD + e) = carry;
 }
 
 // Copy a staged [CH x D] bf16 tile from shared memory to global rows with stride `row_stride`.
@@ -493,10 +499,17 @@ LMOE_API int lmoe_lsm_scalar_launch(int which, int D, const LsmArgs* ap, cudaStr
 // (seed = gradient of the final state, final_out = gradient of the initial state).
 LMOE_API int lmoe_lsm_scalar_combine(int rev, float* states, const float* gdecay, const float* gconst, const float* seed,
                                      float* final_out, int BH, int H, int G, int cpg, int T, int D, cudaStream_t st) {
-    int DD = D * D;
-    dim3 grid((DD + 255) / 256, BH);
-    if (rev) combine_kernel<1><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
-    else combine_kernel<0><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
+    // Four values a thread once that leaves a block for every SM.  16 pairs x 9 groups: 8.2 (reverse 10.8) -> 6.6 us; below the line one value keeps more
+    // SMs busy (measured for the same kernel in lsm_vector.cu: 4 pairs x 37 groups reverse 8.4 and, with four, 12.4).
+    const int DD = D * D, v = (long long)BH * (DD / 1024) >= sm_count() ? 4 : 1;
+    const dim3 grid((DD / v + 255) / 256, BH);
+    if (rev) {
+        if (v == 4) combine_kernel<1, 4><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
+        else combine_kernel<1, 1><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
+    } else {
+        if (v == 4) combine_kernel<0, 4><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
+        else combine_kernel<0, 1><<<grid, 256, 0, st>>>(states, gdecay, gconst, seed, final_out, H, G, cpg, T, DD);
+    }
     return (int)cudaGetLastError();
 }
 

@@ -242,45 +242,38 @@ __global__ void __launch_bounds__(VTHREADS, CTAS) gla_state_scan_kernel(GlaArgs 
 template <int REV, int V>
 __global__ void __launch_bounds__(256) gla_combine_kernel(float* __restrict__ states, const float* __restrict__ gdecay, const float* __restrict__ seed,
                                                           float* __restrict__ final_out, int G, int D) {
-    struct __align__(4 * V) Vec { float x[V]; };
     const int bh = blockIdx.y;
     const int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     const int DD = D * D;
     if (e >= DD) return;
     const int row = e / D;
-    auto load = [](const float* p) -> Vec {
-        Vec r;
-        if constexpr (V == 4) { const float4 v = __ldcg(reinterpret_cast<const float4*>(p)); r.x[0] = v.x; r.x[1] = v.y; r.x[2] = v.z; r.x[3] = v.w; }
-        else r.x[0] = __ldcg(p);
-        return r;
-    };
-    Vec carry;
-    if (seed != nullptr) carry = load(seed + (int64_t)bh * DD + e);
+    Values<V> carry;
+    if (seed != nullptr) carry = load_values<V>(seed + (int64_t)bh * DD + e);
     else
 #pragma unroll
         for (int c = 0; c < V; ++c) carry.x[c] = 0.f;
     // batches of loads in flight together (a load per group that waits for the previous store is bound by memory latency)
     constexpr int NB = 8;
     for (int i0 = 0; i0 < G; i0 += NB) {
-        Vec m[NB];
+        Values<V> m[NB];
         float dec[NB];
 #pragma unroll
         for (int j = 0; j < NB; ++j)
             if (i0 + j < G) {
                 const int g = REV ? G - 1 - (i0 + j) : i0 + j;
-                m[j] = load(states + ((int64_t)bh * G + g) * DD + e);
+                m[j] = load_values<V>(states + ((int64_t)bh * G + g) * DD + e);
                 dec[j] = __expf(gdecay[((int64_t)bh * G + g) * D + row]);
             }
 #pragma unroll
         for (int j = 0; j < NB; ++j)
             if (i0 + j < G) {
                 const int g = REV ? G - 1 - (i0 + j) : i0 + j;
-                *reinterpret_cast<Vec*>(states + ((int64_t)bh * G + g) * DD + e) = carry;
+                *reinterpret_cast<Values<V>*>(states + ((int64_t)bh * G + g) * DD + e) = carry;
 #pragma unroll
                 for (int c = 0; c < V; ++c) carry.x[c] = dec[j] * carry.x[c] + m[j].x[c];
             }
     }
-    if (final_out != nullptr) *reinterpret_cast<Vec*>(final_out + (int64_t)bh * DD + e) = carry;
+    if (final_out != nullptr) *reinterpret_cast<Values<V>*>(final_out + (int64_t)bh * DD + e) = carry;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1109,7 +1109,7 @@ def _scalar_forward(q, k, v, g, scale, init):
                      gdecay=gdecay, dmode=1 if gmode == 2 else 0)
         _lsm_launch(2, D, a)
     else:
-        seed = None if init is None else init.float().contiguous()
+        seed = None if init is None else _aligned(init.float())
         _check(lib().lmoe_lsm_scalar_forward(D, ctypes.byref(a), _p(gf if gmode == 1 else None), _p(seed), _p(final), _st()), "lsm_scalar", 3)
     return o, final, ((q, k, v, gf, states, gdecay, final), gmode, (G, cpg, chunk), lasp)
 
@@ -1146,7 +1146,7 @@ class _LsmScalar(torch.autograd.Function):
         # reverse-direction: group summaries of dS, suffix combine, dk/dv sweep
         a2 = _lsm_args(q, k, v, gf, ctx.gmode, ctx.scale, B, T, H, G, cpg, dstates, None, chunk, d_o=d_o, dk=dk, dv=dv)
         _lsm_launch(1, D, a2)
-        seed = None if dfinal is None else dfinal.float().contiguous()
+        seed = None if dfinal is None else _aligned(dfinal.float())
         if ctx.lasp is not None:
             # the gradient of the state that leaves this rank arrives from the ranks after it; the decay gradient needs it
             need_r = ctx.gmode == 2 or (ctx.gmode == 1 and ctx.needs_input_grad[ctx.g_input])
