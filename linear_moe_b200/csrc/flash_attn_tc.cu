@@ -2,7 +2,7 @@
 // with accumulators in tensor memory, operands staged by TMA (4-D tensor maps over [B, T, H, D], 128-byte swizzle).
 //
 // One CTA = 128 queries of one head.  640 threads:
-//   warp 0      TMA producer: Q once, then K_j / V_j tiles of 128 keys through rings of three and two stages
+//   warp 0      TMA producer: Q once, then K_j / V_j tiles of 128 keys through rings of four (D 128: two) and two stages
 //   warps 1, 2  MMA issuers, one per softmax group: S_j = Q K_j^T, then O += P_j V_j.  (One warp for both spent 1.3 of 2.4 thousand cycles a tile waiting
 //               for one group's product to complete before it could issue the other group's next one.)
 //   warps 4..19 softmax, two groups of eight: group g works on the tiles j = g (mod 2), so that one group's exponentials run while the
@@ -39,9 +39,12 @@ constexpr float LAG = 8.f;            // how far, as a power of two, a row's wei
 template <int D>
 struct __align__(1024) Smem {
     uint8_t q[BM * D * 2];
-    uint8_t k[3][BN * D * 2];         // the scores of a tile wait for its K at once, its V only behind the exponentials
+    // The scores of a tile wait for its K at once, its V only behind the exponentials.  An even number of stages: a stage's tiles are all of one group, whose
+    // warp has waited for the one before (else a wait by parity could take the tile before for this one).
+    static constexpr int KS = D == 64 ? 4 : 2;
+    uint8_t k[KS][BN * D * 2];
     uint8_t v[2][BN * D * 2];
-    uint64_t q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done[2];
+    uint64_t q_full, k_full[KS], k_empty[KS], v_full[2], v_empty[2], s_full[2], p_ready[2], pv_done[2];
     float mx[2][2][2][BM];            // [parity of the group's tile][group][half of the columns]
     float ls[2][2][BM], ms[2][BM];    // sums and maxima at the end
     uint32_t tmem_base;
@@ -70,6 +73,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmV, Args a, int group) {
     extern __shared__ uint8_t smem_raw[];
     Smem<D>& sm = *reinterpret_cast<Smem<D>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr int KS = Smem<D>::KS;
     constexpr int DK = D / 64;                              // 64-element blocks along the head dimension
     constexpr uint32_t TMEM_COLS = 512;
     constexpr uint32_t O_COL = 2 * BN;                      // the groups' outputs behind the two score buffers
@@ -92,7 +96,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
     if (threadIdx.x == 0) {
         mbar_init(&sm.q_full, 1);
-        for (int s = 0; s < 3; ++s) { mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1); }
+        for (int s = 0; s < KS; ++s) { mbar_init(&sm.k_full[s], 1); mbar_init(&sm.k_empty[s], 1); }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&sm.v_full[s], 1); mbar_init(&sm.v_empty[s], 1);
             mbar_init(&sm.s_full[s], 1); mbar_init(&sm.pv_done[s], 1);
@@ -116,13 +120,13 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
             for (int kb = 0; kb < DK; ++kb) tma_load_4d(sm.q + kb * BM * 128, &tmQ, &sm.q_full, kb * 64, h, q0, b);
             for (int j = 0; j < n_it; ++j) {
-                const int s = j & 1, s3 = j % 3;
+                const int s = j & 1, sk = j % KS;
                 const uint32_t ph = (j >> 1) & 1;
                 const int key0 = (nb_lo + j) * BN;
-                if (!mbar_wait_suspend(&sm.k_empty[s3], ((j / 3) & 1) ^ 1, abort_flag, err, 0x1100 | s3)) break;
-                mbar_expect_tx(&sm.k_full[s3], BN * D * 2);
+                if (!mbar_wait_suspend(&sm.k_empty[sk], ((j / KS) & 1) ^ 1, abort_flag, err, 0x1100 | sk)) break;
+                mbar_expect_tx(&sm.k_full[sk], BN * D * 2);
 #pragma unroll
-                for (int kb = 0; kb < DK; ++kb) tma_load_4d(sm.k[s3] + kb * BN * 128, &tmK, &sm.k_full[s3], kb * 64, hk, key0, b);
+                for (int kb = 0; kb < DK; ++kb) tma_load_4d(sm.k[sk] + kb * BN * 128, &tmK, &sm.k_full[sk], kb * 64, hk, key0, b);
                 if (!mbar_wait_suspend(&sm.v_empty[s], ph ^ 1, abort_flag, err, 0x1200 | s)) break;
                 mbar_expect_tx(&sm.v_full[s], BN * D * 2);
                 // MN-major operand: per 64 keys, D/64 boxes of {64 d, 64 keys} (8 KiB each)
@@ -140,21 +144,21 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             constexpr uint32_t idesc_o = idesc_bf16<true, D>();
             bool ok = mbar_wait_warp(&sm.q_full, 0, abort_flag, err, 0x2000);
             for (int j = g; ok && j < n_it; j += 2) {
-                const int s3 = j % 3;
+                const int sk = j % KS;
                 const uint32_t ph = (j >> 1) & 1;
                 // the scores go over the group's last P: its product has to complete
-                ok = mbar_wait_warp(&sm.k_full[s3], (j / 3) & 1, abort_flag, err, 0x2100 | s3) &&
+                ok = mbar_wait_warp(&sm.k_full[sk], (j / KS) & 1, abort_flag, err, 0x2100 | sk) &&
                      (j < 2 || mbar_wait_warp(&sm.pv_done[g], ph ^ 1, abort_flag, err, 0x2400));
                 if (!ok) break;
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint32_t ql = desc_lo<false>(s32(sm.q)), kl = desc_lo<false>(s32(sm.k[s3]));
+                    const uint32_t ql = desc_lo<false>(s32(sm.q)), kl = desc_lo<false>(s32(sm.k[sk]));
 #pragma unroll
                     for (int kk = 0; kk < D / UMMA_K; ++kk) {
                         const uint32_t off = ((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4;
                         umma_ss(tmem_base + g * BN, ql + off, kl + off, idesc_s, kk > 0);
                     }
-                    umma_commit(&sm.k_empty[s3]);
+                    umma_commit(&sm.k_empty[sk]);
                     umma_commit(&sm.s_full[g]);
                 }
                 ok = mbar_wait_warp(&sm.v_full[g], ph, abort_flag, err, 0x2200 | g) && mbar_wait_warp(&sm.p_ready[g], ph, abort_flag, err, 0x2300 | g);
