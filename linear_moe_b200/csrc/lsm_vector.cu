@@ -17,11 +17,12 @@
 //   dS <- diag(e^{b_m}) [ diag(e^{b_C - b_m}) dS + scale q~^T dO ]
 // The gate gradient is d g = reverse-cumsum_t (q . dq - k . dk) per channel (the kernels at the end of this file).
 //
-// 512 threads, one CTA per SM (two where 64-wide heads have more CTAs than SMs): a warp owns 16 rows of every product and a quarter of its columns (of the state: half or a quarter).  For the
+// These kernels take 64-wide heads; those for 128-wide ones are in lsm_vector_tc.cu.
+//
+// 512 threads, one CTA per SM, or two where there are more CTAs than SMs: a warp owns 16 rows of every product and a quarter of its columns (of the state: a half).  For the
 // gates a thread owns two channels and VCH / GR consecutive tokens: running sums stay in registers, the GR groups of tokens meet in one
 // small table, and the next chunk's gates and tiles are on their way while this one is worked on.  (With eight warps, single buffers and a
-// 64-step running sum in 128 threads the chunks were bound by latency.)  8 x 2048 tokens, 8 heads of 128: group summaries 82 and 71 -> 43 and
-// 41 us.  The sweeps of 128-wide heads are in lsm_vector_tc.cu, those here are for 64-wide ones.
+// 64-step running sum in 128 threads the chunks were bound by latency.)
 #include "lsm_vector.cuh"
 #include "mma_utils.cuh"
 
@@ -503,22 +504,19 @@ static int gla_launch(int which, const GlaArgs& a, cudaStream_t st) {
     } while (0)
     if (which == 0) GLAUNCH((gla_state_scan_kernel<D, 0, CTAS>), gla_smem_scan<D>());
     else if (which == 1) GLAUNCH((gla_state_scan_kernel<D, 1, CTAS>), gla_smem_scan<D>());
-    else if constexpr (D == 64) {
-        if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<D, 0, CTAS>), gla_smem_sweep<D>());
-        else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<D, 1, CTAS>), gla_smem_sweep<D>());
-        else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<D, CTAS>), gla_smem_dkv<D>());
-        else return -1;
-    } else return -1;
+    else if (which == 2) GLAUNCH((gla_fwd_sweep_kernel<D, 0, CTAS>), gla_smem_sweep<D>());
+    else if (which == 3) GLAUNCH((gla_fwd_sweep_kernel<D, 1, CTAS>), gla_smem_sweep<D>());
+    else if (which == 4) GLAUNCH((gla_bwd_dkv_kernel<D, CTAS>), gla_smem_dkv<D>());
+    else return -1;
 #undef GLAUNCH
     return (int)cudaGetLastError();
 }
 
 // which: 0 forward state scan, 1 reverse state scan, 2 forward output, 3 backward dq, 4 backward dk/dv
 LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t st) {
-    // 128-wide heads: sweeps on the tensor cores of lsm_vector_tc.cu at every size (8 x 2048 tokens, 8 heads: outputs 97 -> 50 us, dq 102 -> 59, dk / dv
-    // 141 -> 76; 3 x 1111 of 16 heads, a whole forward 65 -> 46 and with its gradients 234 -> 170; one chunk of one head 14.8 and 15.3, 58.8 and 58.9).  The
-    // summaries, one product a chunk, stay here: there they took 41 and 64 us, here 43 and 42.
-    if (D == 128) return which >= 2 ? lvt::launch(which, *ap, st) : gla_launch<128, 1>(which, *ap, st);
+    // 128-wide heads: the tensor cores of lsm_vector_tc.cu at every size.  Kernels of a forward pass and with all gradients, here and there: 8 x 2048 tokens of
+    // 8 heads 155 and 88 us, 560 and 303; 3 x 1111 of 16 heads 65 and 41, 234 and 159; one chunk of one head 14.8 and 16.6, 58.8 and 49.1.
+    if (D == 128) return lvt::launch(which, *ap, st);
     if (D != 64) return -2;
     // 64-wide heads, more CTAs than SMs: two per SM with 64 registers a thread overlap each other's steps.  Outputs, one and two per SM:
     // 64 x 256 tokens of 16 heads 216 and 185 us, 64 x 128 144 and 123, 32 x 64 56 and 50; where every CTA has an SM to itself the

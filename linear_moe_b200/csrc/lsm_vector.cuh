@@ -18,7 +18,7 @@ struct GlaArgs {
 };
 
 namespace lvt {
-// which 2 .. 4 of lmoe_gla_launch for 128-wide heads
+// lmoe_gla_launch for 128-wide heads
 int launch(int which, const GlaArgs& a, cudaStream_t st);
 }  // namespace lvt
 

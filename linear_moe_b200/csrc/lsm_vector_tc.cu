@@ -4,6 +4,7 @@
 // accumulator holds the tile's rows, the upper half products of whatever follows the tile in shared memory, and nobody reads it (an
 // instruction with 64 rows takes as long).
 //
+//   gla_state_tc_kernel   group summaries.
 //   gla_sweep_tc_kernel   outputs and dq, chunks in order.
 //   gla_dkv_tc_kernel     dk and dv, chunks in reverse order.
 //
@@ -12,9 +13,10 @@
 // the chain over the chunks: the state lives in tensor memory, is scaled there row by row and published as a bf16 tile, and the chunk's
 // increment accumulates onto it.  (Four of them for the state alone and four for scores and outputs took as long: a row's 128 columns then come
 // one half after the other.)
-// Bound by the latency of a chunk, 4000 - 5000 cycles of which the tensor cores need 2000 - 3500; a group has only cpg chunks.  8 x 2048 tokens of 8
-// heads, against mma.sync: outputs 97 -> 50 us (201 MB, 31 us at the copy rate), dq 102 -> 59, dk and dv 141 -> 76.  Gates in registers
-// and the walks written out: 67, 73 and 82.
+// The summaries' chain is one product a chunk onto the state, which eight warps scale row by row in between.
+// Sweeps are bound by the latency of a chunk, 4000 - 5000 cycles of which the tensor cores need 2000 - 3500 (a group has only cpg chunks), summaries
+// by memory.  8 x 2048 tokens of 8 heads, against mma.sync: outputs 97 -> 49 us (201 MB, 31 us at the copy rate), dq 102 -> 58, dk and dv
+// 141 -> 73, summaries 43 -> 31 and 41 -> 27 (134 MB, 20 us).  With gates in registers and the walks written out: 67, 73 and 82, summaries 41 and 64.
 #include <cstddef>
 #include "flash_tc_utils.cuh"
 #include "lsm_vector.cuh"
@@ -220,7 +222,161 @@ __device__ __forceinline__ void operand_warps(int tid, F f) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-constexpr int FS = 2, GTILE = CT * D * 4;      // stages; bytes of a chunk's gates
+constexpr int SS = 3, GTILE = CT * D * 4;                                // stages of the summaries; bytes of a chunk's gates
+constexpr int ST_E0 = 2, ST_C0 = ST_E0 + 8, ST_THREADS = 32 * (ST_C0 + 8);   // warps 0: TMA, 1: MMA, then two sets of operand warps, then the state
+struct __align__(1024) SmemState {
+    uint8_t x[SS][TILE], y[SS][TILE], gk[SS][GTILE];
+    float tab[SS][D];                               // the sum of a chunk's gates
+    uint64_t full[SS], empty[SS], e_ready[SS], s_ready, s_done;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+// The operand of a summary: 32 rows of a tile times e^ the sum of the gates between them and the chunk's end (REV 0, without their own) or its start (REV 1,
+// with their own, times `mul` too), in the order away from there.  FAR: the rows behind the other 32, whose gates are summed first.  Returns the sum.
+template <int REV>
+__device__ __forceinline__ float2 summary_rows(uint32_t tile, uint32_t gates, int pair, bool far, float mul) {
+    constexpr uint32_t STEP = REV ? 1024u : 0u - 1024u;
+    const uint32_t at = (pair >> 5) * BLOCK + ((pair & 31) >> 2 << 4) + (pair & 3) * 4, first = (REV ? 0 : 63);
+    uint32_t gp = gates + first * 512 + pair * 8;
+    float2 z = make_float2(0.f, 0.f);
+    auto gate = [&](int e) { return lds64(gp + (REV ? (uint32_t)(e * 512) : 0u - (uint32_t)(e * 512))); };
+    if (far) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j, gp += 4 * STEP) {
+            float2 g[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) g[e] = gate(e);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { z.x += g[e].x; z.y += g[e].y; }
+        }
+    }
+    uint32_t p[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) p[e] = tile + (at ^ ((REV ? e : 7 - e) << 4)) + (REV ? e : 63 - e) * 128 + (far ? 4 * STEP : 0u);
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j, gp += 4 * STEP) {
+        float2 g[8];
+        uint32_t v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) g[e] = gate(e);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = lds32(p[e]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (REV) { z.x += g[e].x; z.y += g[e].y; }
+            sts32(p[e], REV ? times(v[e], __expf(z.x) * mul, __expf(z.y) * mul) : times(v[e], __expf(z.x), __expf(z.y)));
+            if (!REV) { z.x += g[e].x; z.y += g[e].y; }
+            p[e] += STEP;
+        }
+    }
+    return z;
+}
+
+// Group summaries.  REV 0: S <- e^{b_C} S + (e^{b_C - b_j} K)^T V.  REV 1: dS <- e^{b_C} dS + (scale e^{b_i} Q)^T dO, chunks in reverse order.
+template <int REV>
+__global__ void __launch_bounds__(ST_THREADS, 1)
+gla_state_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmGk, GlaArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    SmemState& sm = *reinterpret_cast<SmemState*>(smem_raw + ((1024 - (s32(smem_raw) & 1023)) & 1023));
+    const int warp = fatc::uniform_warp(), lane = threadIdx.x & 31;
+    const int grp = blockIdx.x, bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
+    const int chunks = (a.T + CT - 1) / CT, c_lo = grp * a.cpg, n = max(0, min(chunks, c_lo + a.cpg) - c_lo);
+    volatile int* abort_flag = &sm.abort_flag;
+    int* err = a.err;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SS; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); mbar_init(&sm.e_ready[s], 4); }
+        mbar_init(&sm.s_ready, 8); mbar_init(&sm.s_done, 1);
+        sm.abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    init_tmem(&sm.tmem_base, warp, 128);
+    const uint32_t tmem_base = fatc::uniform(sm.tmem_base);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int i = 0; i < n; ++i) {
+                const int s = i % SS, t0 = (REV ? c_lo + n - 1 - i : c_lo + i) * CT;
+                if (!mbar_wait_suspend(&sm.empty[s], ((i / SS) & 1) ^ 1, abort_flag, err, 0xa100 | s)) break;
+                mbar_expect_tx(&sm.full[s], 2 * TILE + GTILE);
+                tma_load_4d(sm.gk[s], &tmGk, &sm.full[s], 0, h, t0, b);
+                tma_tile(sm.x[s], &tmX, &sm.full[s], h, t0, b);
+                tma_tile(sm.y[s], &tmY, &sm.full[s], h, t0, b);
+            }
+        }
+    } else if (warp == 1) {
+        for (int i = 0; i < n; ++i) {
+            const int s = i % SS;
+            if (!fatc::mbar_wait_warp(&sm.e_ready[s], (i / SS) & 1, abort_flag, err, 0xa200 | s)) break;
+            if (!fatc::mbar_wait_warp(&sm.full[s], (i / SS) & 1, abort_flag, err, 0xa210 | s)) break;
+            if (!fatc::mbar_wait_warp(&sm.s_ready, i & 1, abort_flag, err, 0xa220)) break;
+            tc_fence_after();
+            product<true, true, 128, 4, BLOCK>(tmem_base, sm.x[s], sm.y[s], i > 0);
+            if (elect_one()) { umma_commit(&sm.empty[s]); umma_commit(&sm.s_done); }
+        }
+    } else if (warp < ST_C0) {                      // rescaled operands; a set of four warps takes every other chunk
+        const int tid = threadIdx.x - ST_E0 * 32, pair = tid & 63, set = tid >> 7;
+        const bool far = (tid >> 6) & 1;
+        for (int i = set; i < n; i += 2) {
+            const int s = i % SS;
+            // The other set has this stage's chunk before: until that one's tiles are there, full[s] looks as it will when this one's are.
+            if (i >= SS && !mbar_wait_suspend(&sm.e_ready[s], (i / SS - 1) & 1, abort_flag, err, 0xa310 | s)) break;
+            if (!mbar_wait_suspend(&sm.full[s], (i / SS) & 1, abort_flag, err, 0xa300 | s)) break;
+            const float2 sum = summary_rows<REV>(s32(sm.x[s]), s32(sm.gk[s]), pair, far, a.scale);
+            if (far) *reinterpret_cast<float2*>(&sm.tab[s][2 * pair]) = sum;
+            fence_async();
+            arrive(&sm.e_ready[s]);
+        }
+    } else {
+        const int qd = warp & 3, part = (warp - ST_C0) >> 2, r = qd * 32 + lane;
+        const uint32_t st = tmem_base + ((uint32_t)(qd * 32) << 16) + part * 64;
+        float decay = 0.f;
+        bool ok = true;
+        for (int i = 0; ok && i < n; ++i) {
+            const int s = i % SS;
+            ok = mbar_wait_suspend(&sm.e_ready[s], (i / SS) & 1, abort_flag, err, 0xa400 | s);
+            if (!ok) break;
+            const float sum = sm.tab[s][r], f = __expf(sum);
+            decay += sum;
+            if (i > 0) {
+                ok = mbar_wait_suspend(&sm.s_done, (i - 1) & 1, abort_flag, err, 0xa410);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int c = 0; c < 64; c += 32) {
+                    uint32_t x[32];
+                    tmem_ld32(st + c, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) x[e] = __float_as_uint(f * __uint_as_float(x[e]));
+                    tmem_st16(st + c, reinterpret_cast<uint32_t(&)[16]>(x[0]));
+                    tmem_st16(st + c + 16, reinterpret_cast<uint32_t(&)[16]>(x[16]));
+                }
+                tmem_st_wait();
+                tc_fence_before();
+            }
+            arrive(&sm.s_ready);
+        }
+        if (ok && n > 0) ok = mbar_wait_suspend(&sm.s_done, (n - 1) & 1, abort_flag, err, 0xa420);
+        tc_fence_after();
+        float* out = a.states + (((int64_t)bh * a.G + grp) * D + r) * D + part * 64;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 32) {
+            uint32_t v[32];
+            tmem_ld32(st + c, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+                *reinterpret_cast<float4*>(out + c + e) = n > 0 ? make_float4(__uint_as_float(v[e]), __uint_as_float(v[e + 1]), __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]))
+                                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (a.gdecay != nullptr && part == 0) a.gdecay[((int64_t)bh * a.G + grp) * D + r] = decay;
+    }
+    free_tmem(tmem_base, warp, 128);
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int FS = 2;              // stages, one for each set of operand warps
 struct __align__(1024) SmemSweep {
     uint8_t t0[FS][TILE], k[FS][TILE], v[FS][TILE], sb[STILE], gk[FS][GTILE];
     float tab[FS][2][D];                            // e^{b_m}, e^{b_C - b_m}
@@ -531,21 +687,26 @@ static int gates_map(CUtensorMap* m, const GlaArgs& a) {
 template <typename K>
 static int set_smem(K kernel, size_t bytes) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
 
-// which: 2 .. 4 of lmoe_gla_launch (the summaries, which only multiply once per chunk, stay in lsm_vector.cu); positive strides
+// which as in lmoe_gla_launch; positive strides
 int launch(int which, const GlaArgs& a, cudaStream_t st) {
     if (a.err == nullptr) return -1;
     dim3 grid(a.G, a.B * a.H);
     CUtensorMap q, k, v, g, o, dk, dv, gk;
     int rc = gates_map(&gk, a);
-    if (which == 2 || which == 4) rc |= map_of(&q, a.q, a, a.qs_b, a.qs_t, a.qs_h);
-    rc |= map_of(&k, a.k, a, a.ks_b, a.ks_t, a.ks_h);
-    rc |= map_of(&v, a.v, a, a.vs_b, a.vs_t, a.vs_h);
-    if (which == 3 || which == 4) rc |= map_of(&g, a.d_o, a, (int64_t)a.T * a.H * D, (int64_t)a.H * D, D);
+    if (which == 1 || which == 2 || which == 4) rc |= map_of(&q, a.q, a, a.qs_b, a.qs_t, a.qs_h);
+    if (which != 1) { rc |= map_of(&k, a.k, a, a.ks_b, a.ks_t, a.ks_h); rc |= map_of(&v, a.v, a, a.vs_b, a.vs_t, a.vs_h); }
+    if (which == 1 || which == 3 || which == 4) rc |= map_of(&g, a.d_o, a, (int64_t)a.T * a.H * D, (int64_t)a.H * D, D);
     if (which == 2) rc |= map_of(&o, a.o, a, (int64_t)a.T * a.H * D, (int64_t)a.H * D, D);
     if (which == 3) rc |= map_of(&o, a.dq, a, a.dqs_b, a.dqs_t, a.dqs_h);
     if (which == 4) { rc |= map_of(&dk, a.dk, a, a.dks_b, a.dks_t, a.dks_h); rc |= map_of(&dv, a.dv, a, a.dvs_b, a.dvs_t, a.dvs_h); }
     if (rc) return -11;
-    if (which == 2 || which == 3) {
+    if (which == 0 || which == 1) {
+        const size_t smem = sizeof(SmemState) + 1024;
+        rc = which == 0 ? set_smem(gla_state_tc_kernel<0>, smem) : set_smem(gla_state_tc_kernel<1>, smem);
+        if (rc) return rc;
+        if (which == 0) gla_state_tc_kernel<0><<<grid, ST_THREADS, smem, st>>>(k, v, gk, a);
+        else gla_state_tc_kernel<1><<<grid, ST_THREADS, smem, st>>>(q, g, gk, a);
+    } else if (which == 2 || which == 3) {
         const size_t smem = sizeof(SmemSweep) + 1024;
         rc = which == 2 ? set_smem(gla_sweep_tc_kernel<0>, smem) : set_smem(gla_sweep_tc_kernel<1>, smem);
         if (rc) return rc;

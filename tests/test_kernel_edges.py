@@ -521,6 +521,20 @@ def test_vector_decay_views(B, H, T):
         assert torch.equal(a, b)
 
 
+def test_vector_decay_repeats():
+    """Sixteen chunks in a row on most SMs, several times: the same bits.  (Two sets of warps take turns with the stages of a ring.)"""
+    torch.manual_seed(0)
+    B, T, H, D = 8, 2048, 8, 128
+    x, go = rand(B, T, H, 3 * D), rand(B, T, H, D, scale=1)
+    g = torch.nn.functional.logsigmoid(torch.randn(B, T, H, D, device="cuda")) / 4
+    first = None
+    for _ in range(6):
+        (o, S), grads = run(lambda x, g: ops.lsm_vector(*x.split(D, dim=-1), g, None, None, None, 64), [x, g], [go])
+        first = first or [o, S, *grads]
+        for a, b in zip(first, [o, S, *grads]):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 127, 3), (1, 129, 2), (1, 1024, 3), (1, 1025, 3), (3, 2500, 7), (1, 2049, 3)])
 def test_decay_gradient_sums(B, T, H, D):
