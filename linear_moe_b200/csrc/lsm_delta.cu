@@ -909,7 +909,10 @@ LMOE_API int lmoe_delta_scan(int dir, int dk, int BH, const dr::Args* ap, cudaSt
     const dr::Args a = *ap;
     if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0 || a.H <= 0 || a.err == nullptr) return -1;
     if (!(a.ldw == dk && a.lda == dr::C) && !(a.ldw == dk + 8 && a.lda == dr::C + 8)) return -1;
-    if (dk == dr::TC_DK && a.dv % dr::TC_DV == 0) return dr::scan_tc(dir, BH, a, st);
+    // The kernels of lsm_delta_tc.cu have half as many CTAs and shorter steps, but start later, and their tensor maps cost the host time: for long chains, or
+    // where the CTAs here are more than SMs.  Here and there, sequences x chunks: 64 x 32 forward and backward scans 167 + 97 and 97 + 52 us, 256 x 5 120 + 72 and
+    // 88 + 57, 16 x 64 175 + 95 and 171 + 89; 16 x 16 47 + 27 and 49 + 27, 4 x 8 26 + 14 and 28 + 16.
+    if (dk == dr::TC_DK && a.dv % dr::TC_DV == 0 && ((long long)BH * (a.dv / dr::DVS) > sm_count() || a.N >= 32)) return dr::scan_tc(dir, BH, a, st);
     dim3 grid(a.dv / dr::DVS, BH);
     const bool out = dir != 0 || a.O != nullptr;
 #define LMOE_DR_LAUNCH(KERNEL, DK)                                                                                     \

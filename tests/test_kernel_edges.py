@@ -549,9 +549,9 @@ def test_decay_gradient_sums(B, T, H, D):
     assert ((got - want).abs() <= (T + 3) * 2.0 ** -24 * size).all()
 
 
-@pytest.mark.parametrize("B,T,H,dv", [(2, 300, 2, 32), (2, 300, 2, 64), (2, 300, 2, 96), (2, 300, 2, 192), (2, 700, 16, 128), (1, 64, 149, 128)])
+@pytest.mark.parametrize("B,T,H,dv", [(2, 300, 2, 32), (2, 300, 2, 64), (1, 150, 60, 96), (1, 150, 75, 64), (1, 130, 25, 192), (2, 300, 32, 128), (1, 2050, 2, 128), (1, 64, 149, 128)])
 def test_delta_rule_sizes(B, T, H, dv):
-    """128-wide keys with other value widths (multiples of 64 on the 5th-generation tensor cores, the others not), and more chunks than SMs: the
+    """128-wide keys with other value widths (multiples of 64 on the 5th-generation tensor cores, with many heads or chunks), and more chunks than SMs: the
     kernel of the tiles' gradients goes on to a next chunk while it works on one."""
     from linear_moe_b200.ops import gemm
     torch.manual_seed(0)
