@@ -96,7 +96,8 @@ def score_tokens(model, tokens: torch.Tensor) -> torch.Tensor:
 
 
 def _overwritable(state: torch.Tensor) -> torch.Tensor:
-    """An alias of a state that nobody reads behind the step it goes into: the step may write the new state over it."""
+    """An alias of a state that its owner reads no more: the operator it goes into may write the new state over it, and then reads what it still wants
+    of the old one first."""
     alias = state.detach()
     alias.lmoe_overwritable = True
     return alias

@@ -1432,12 +1432,12 @@ def _lsm_vector_bonus(q, k, v, gk, scale, initial_state, bonus, chunk_size):
     B, T, H, D = q.shape
     if T > 1:
         _note_strong_decay(gk)            # RWKV6 decays -exp(.) are not bounded the way GLA's normalised log-sigmoids are
+    if initial_state is None:
+        first = q.new_zeros(B, 1, H, v.shape[-1])
+    else:                                 # ahead of the kernels: a single step may write the new state over this one
+        first = (scale * torch.einsum("bhk,bhkv->bhv", q[:, 0].float(), initial_state.float())).to(q.dtype)[:, None]
     q_shift = torch.cat([q[:, 1:], q.new_zeros(B, 1, H, D)], 1)
     out_s, S = lsm_vector(q_shift, k, v, gk, scale, initial_state, None, chunk_size)
-    if initial_state is None:
-        first = out_s.new_zeros(B, 1, H, v.shape[-1])
-    else:
-        first = (scale * torch.einsum("bhk,bhkv->bhv", q[:, 0].float(), initial_state.float())).to(out_s.dtype)[:, None]
     o_state = torch.cat([first, out_s[:, :-1]], 1)
     diag = (q.float() * k.float() * bonus.float()[None, None]).sum(-1, keepdim=True) * scale
     return o_state + (diag * v.float()).to(o_state.dtype), S

@@ -498,6 +498,26 @@ def test_states_that_may_be_overwritten(kind):
         assert S2.data_ptr() == S.data_ptr() and torch.equal(S, S1) and torch.equal(o, o2)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_bonus_step_over_its_state(D):
+    """One token with a bonus (RWKV6), whose output needs the state in front of it: the same bits beside the old state and over it, and as the
+    definition has it."""
+    from linear_moe_b200.infer.generation import _overwritable
+    torch.manual_seed(0)
+    B, H = 3, 2
+    q, k, v, u = rand(B, 1, H, D), rand(B, 1, H, D), rand(B, 1, H, D), torch.randn(H, D, device="cuda")
+    gk, S = -torch.rand(B, 1, H, D, device="cuda"), torch.randn(B, H, D, D, device="cuda")
+    with torch.no_grad():
+        o, S1 = ops.lsm_vector(q, k, v, gk, None, S, u)
+        q0, k0, v0 = (t[:, 0].double() for t in (q, k, v))
+        kv = k0[..., None] * v0[..., None, :]
+        want = D ** -0.5 * torch.einsum("bhk,bhkv->bhv", q0, S.double() + u.double()[..., None] * kv)
+        # three roundings to bf16: of the two terms and of their sum
+        assert rel(o[:, 0], want) < 4 * U and rel(S1, gk[:, 0].double().exp()[..., None] * S.double() + kv) < 1e-5
+        o2, S2 = ops.lsm_vector(q, k, v, gk, None, _overwritable(S), u)
+        assert torch.equal(o, o2) and torch.equal(S1, S2)
+
+
 @pytest.mark.parametrize("B,H,T", [(1, 9, 700), (2, 5, 700), (1, 149, 70)])
 def test_vector_decay_views(B, H, T):
     """128-wide heads from views that tensor maps or 16-byte loads could not take as they are (heads that repeat one another, a value that starts 2 bytes

@@ -214,6 +214,37 @@ def test_cuda_graph_decode_matches_eager(la):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["lightning_attention", "gla", "gated_deltanet", "rwkv6", "hgrn2", "gsa", "mamba2"])
+def test_cuda_graph_steps_match_eager_steps(kind):
+    """Logits and cached states of a replayed one-token step are those of the eager step, for mixers whose outputs need the state in front of the token and
+    those that need the one behind it, and with several states per layer."""
+    from linear_moe_b200.infer.generation import GraphedDecodeStep
+    torch.manual_seed(0)
+    kw = dict(hybrid_override_pattern="MM", mamba_head_dim=64, mamba_d_state=128, mamba_ngroups=2) if kind == "mamba2" else dict(layer_type_list="LL")
+    cfg = ModelConfig(num_layers=2, hidden_size=256, num_attention_heads=2, ffn_hidden_size=512, vocab_size=512, use_la_module=True, la_module=kind,
+                      params_dtype=torch.bfloat16, **kw)
+    m = CausalLM(cfg, device="cuda").cuda().eval()
+    ids = torch.randint(0, 512, (2, 18), device="cuda")
+    with torch.no_grad():
+        for n, p in m.named_parameters():
+            if n.endswith("bonus"):
+                p.normal_()
+        eager, captured = m.new_cache(), m.new_cache()
+        for caches in (eager, captured):
+            m(ids[:, :12], caches=caches)
+            m(ids[:, 12:13], caches=caches, position_offset=12)
+        assert GraphedDecodeStep.supported(m, captured, ids.device)
+        step = GraphedDecodeStep(m, captured, 2, ids.device)
+        for t in range(13, 18):
+            tok = ids[:, t:t + 1].contiguous()
+            want = m(tok, caches=eager, position_offset=t)
+            assert torch.equal(step(tok), want)
+            for a, b in zip(eager, captured):
+                assert a.keys() == b.keys() and all(torch.equal(a[k], b[k]) for k in a)
+        assert step.graph is not None
+
+
+@pytest.mark.gpu
 def test_cuda_graph_decode_with_moe_layers():
     """A linear-attention + MoE model decodes to the same tokens with ``cuda_graph=True``, whether the expert layer can be
     captured or the step falls back to eager launches."""
