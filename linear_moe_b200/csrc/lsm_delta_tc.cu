@@ -103,16 +103,23 @@ template <bool OUT>
 struct __align__(1024) Smem {
     Stage<OUT> st[STAGES];
     uint8_t sb[SBLOCK], vb[BLOCK], vneg[BLOCK];
-    uint64_t full[STAGES], empty[STAGES], sb_ready, x_full, v_ready, s_full, o_full, o_ready, kept;
+    // Every wait goes by the parity of a phase, so a barrier must not be two phases ahead of whoever waits for it.  What keeps it from that, chunk n:
+    //   full     its next phase wants empty, which comes behind everybody's use of the stage; empty: behind the one load that waits for it
+    //   sb_ready the next is for chunk n + 1 and wants s_full (from the warp that issues products) and, where Sn and Vn are kept, kept (from the one that
+    //            stores them); x_full, s_full, kept: the next wants sb_ready n + 1, where all eight warps of threads arrive behind these waits
+    //   v_ready  the next wants x_full n + 1, and kept, so both of its waiters; o_full: the next wants v_ready n + 1, behind the outputs of chunk n
+    //   o_ready  one per stage: the next of a stage wants full, so empty, so the store of the stage's outputs.  (With one for all of them the threads could get two
+    //            chunks ahead of a slow store, which then waited for ever.)
+    uint64_t full[STAGES], empty[STAGES], sb_ready, x_full, v_ready, s_full, o_full, o_ready[STAGES], kept;
     uint32_t tmem_base;
     int abort_flag;
 };
 template <bool OUT>
 __device__ __forceinline__ uint32_t setup(Smem<OUT>& sm, int warp) {
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); mbar_init(&sm.o_ready[s], WORKERS / 2); }
         mbar_init(&sm.sb_ready, WORKERS); mbar_init(&sm.x_full, 1); mbar_init(&sm.v_ready, WORKERS / 2); mbar_init(&sm.s_full, 1);
-        mbar_init(&sm.o_full, 1); mbar_init(&sm.o_ready, WORKERS / 2); mbar_init(&sm.kept, 1);
+        mbar_init(&sm.o_full, 1); mbar_init(&sm.kept, 1);
         sm.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -202,7 +209,7 @@ __global__ void __launch_bounds__(THREADS, 1) delta_scan_fwd_tc_kernel(const __g
         if constexpr (OUT) {
             for (int n = 0; n < a.N; ++n) {
                 const int s = n % STAGES;
-                if (!mbar_wait_suspend(&sm.o_ready, n & 1, abort_flag, err, 0xd400)) break;
+                if (!mbar_wait_suspend(&sm.o_ready[s], (n / STAGES) & 1, abort_flag, err, 0xd400 | s)) break;
                 if (lane == 0) {
                     fatc::tma_store_4d(&m.o, sm.st[s].x, col0, bh % a.H, n * C, bh / a.H);       // rows behind T are cut off
                     fatc::tma_store_commit();
@@ -228,7 +235,7 @@ __global__ void __launch_bounds__(THREADS, 1) delta_scan_fwd_tc_kernel(const __g
                 store32(sm.st[n % STAGES].x, r, part, o);
                 fence_async();
                 tc_fence_before();
-                arrive(&sm.o_ready);
+                arrive(&sm.o_ready[n % STAGES]);
             }
             return true;
         };

@@ -585,3 +585,20 @@ def test_delta_rule_sizes(B, T, H, dv):
     gemm.check_error()
     want = run(lambda q, k, v, beta, g, S: RL.recurrent_lsm(q, k, v, beta=beta, g=g, initial_state=S), [t.float() for t in ins], [go.float(), gS])
     check(got, want, ["o", "S", "dq", "dk", "dv", "dbeta", "dg", "dS0"])
+
+
+def test_delta_prompt_repeats():
+    """Forward calls without gradients, chains of 33 and 34 chunks on most SMs, several times: the same bits, and every wait came to its end.  (Outputs are
+    stored by a warp of their own, from a ring of stages.)"""
+    from linear_moe_b200.ops import gemm
+    torch.manual_seed(0)
+    B, H, D = 4, 18, 128
+    for T in (2100, 2176):
+        q, k = rand(B, T, H, D), torch.nn.functional.normalize(torch.randn(B, T, H, D, device="cuda"), dim=-1).bfloat16()
+        v, beta = rand(B, T, H, D), torch.rand(B, T, H, device="cuda")
+        with torch.no_grad():
+            o, S = ops.lsm_delta(q, k, v, beta, None, None, None, 64)
+            for _ in range(8):
+                o2, S2 = ops.lsm_delta(q, k, v, beta, None, None, None, 64)
+                assert torch.equal(o, o2) and torch.equal(S, S2)
+        gemm.check_error()
