@@ -551,10 +551,12 @@ class MoeWorkspace:
         """Publish this rank's expert results ``[cap, h]`` and gather, weight and sum every token's ``k`` rows from their
         owners.  Returns ``(out [T, h], rows [T*k, h] or None)``."""
         if self.group is None:                                   # one rank: the results are read, and kept, where they are
-            assert not save_rows
             out = torch.empty(route.T, self.h, dtype=torch.bfloat16, device=self.device)
             self._local(2, route, "moe_pull", y=_aligned(y_local), w=weights, out=out)
-            return out, None
+            if not save_rows:
+                return out, None
+            rows = y_local[route.dest_row.clamp(min=0).long()]
+            return out, rows.masked_fill_((route.dest_row < 0)[:, None], 0)
         self.ep_pull += 1
         if y_local.data_ptr() != self.y.data_ptr():
             self.y.copy_(y_local)                                # (the grouped GEMM normally writes into self.y itself)

@@ -138,3 +138,22 @@ def test_one_rank_exchange_kernels(T, k, E, hid):
     torch.testing.assert_close(d_w, (rows * go.float()[:, None]).sum(-1), rtol=1e-4, atol=1e-3)            # fp32 sums over `hid` products of size one
     torch.cuda.synchronize()
     fused_comm.check_status("one rank")
+
+
+@pytest.mark.parametrize("T,k,E,hid,drop", [(1, 1, 3, 8, False), (300, 2, 4, 72, True), (0, 2, 4, 64, False)])
+def test_one_rank_pull_with_the_gathered_rows(T, k, E, hid, drop):
+    """The rows that a combine gathers, unweighted and in token order, zeros for dropped pairs; the sum is that of a pull without them."""
+    from linear_moe_b200.ops import gemm
+    from linear_moe_b200.parallel import fused_comm
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(2)
+    ws = fused_comm.MoeWorkspace(None, E, hid, T * k + gemm.ROW_ALIGN * E, dev)
+    idx = torch.randint(-1 if drop else 0, E, (T, k), device=dev)
+    route = ws.route(idx)
+    y, w = torch.randn(ws.cap, hid, device=dev).bfloat16(), torch.rand(T, k, device=dev)
+    out, rows = ws.pull(y, route, w, True)
+    sent = (idx.reshape(-1) >= 0)[:, None]
+    assert rows.shape == (T * k, hid) and torch.equal(rows, torch.where(sent, y[route.dest_row.clamp(min=0).long()], torch.zeros_like(rows)))
+    assert torch.equal(out, ws.pull(y, route, w, False)[0])
+    torch.cuda.synchronize()
+    fused_comm.check_status("pull")
