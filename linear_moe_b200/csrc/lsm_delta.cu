@@ -909,12 +909,16 @@ LMOE_API int lmoe_delta_scan(int dir, int dk, int BH, const dr::Args* ap, cudaSt
     const dr::Args a = *ap;
     if (a.dv % dr::DVS || (dk != 64 && dk != 128) || BH <= 0 || a.H <= 0 || a.err == nullptr) return -1;
     if (!(a.ldw == dk && a.lda == dr::C) && !(a.ldw == dk + 8 && a.lda == dr::C + 8)) return -1;
-    // The kernels of lsm_delta_tc.cu have half as many CTAs and shorter steps, but start later, and their tensor maps cost the host time: for long chains, or
-    // where the CTAs here are more than SMs.  Here and there, sequences x chunks: 64 x 32 forward and backward scans 167 + 97 and 97 + 52 us, 256 x 5 120 + 72 and
-    // 88 + 57, 16 x 64 175 + 95 and 171 + 89; 16 x 16 47 + 27 and 49 + 27, 4 x 8 26 + 14 and 28 + 16.
-    if (dk == dr::TC_DK && a.dv % dr::TC_DV == 0 && ((long long)BH * (a.dv / dr::DVS) > sm_count() || a.N >= 32)) return dr::scan_tc(dir, BH, a, st);
-    dim3 grid(a.dv / dr::DVS, BH);
+    // The kernels of lsm_delta_tc.cu have half as many CTAs.  Where the CTAs here are more than SMs, that alone decides; sequences x chunks, here and there in us:
+    // outputs 64 x 26 82 and 42, 38 x 8 28 and 16, 256 x 2 38 and 28; Vn and the states only (the backward pass rebuilds them) 55 and 37, 19 and 14, 24 and 22;
+    // reverse 80 and 42, 28 and 16, 38 and 26.  With an SM for every CTA it is the latency of a step: theirs is shorter with outputs (2 x 32 49.7 and 46.2, 2 x 128
+    // 189 and 170, 32 x 64 97 and 90) and in the reverse scan (48.9 and 46.1, 186 and 169, 95 and 89), enough from 32 chunks on for their later start and the
+    // host's time for their tensor maps (37 x 8 15.4 and 16.0, 15.2 and 16.2), and longer where Vn and the states are all that is wanted
+    // (37.0 and 42.7, 138 and 159, 82 and 82).
     const bool out = dir != 0 || a.O != nullptr;
+    const bool shared = (long long)BH * (a.dv / dr::DVS) > sm_count();
+    if (dk == dr::TC_DK && a.dv % dr::TC_DV == 0 && (shared || (out && a.N >= 32))) return dr::scan_tc(dir, BH, a, st);
+    dim3 grid(a.dv / dr::DVS, BH);
 #define LMOE_DR_LAUNCH(KERNEL, DK)                                                                                     \
     do {                                                                                                               \
         auto kernel = KERNEL;                                                                                          \

@@ -10,9 +10,9 @@
 // many CTAs), and the outputs are made while the next step's first product runs.
 // A tile of 64 rows stands where an instruction wants 128: the upper half of its accumulator holds products of what follows the tile in shared
 // memory, and nobody reads it.
-// 2 x 4096 tokens, 16 heads of 128 (64 CTAs, 64 chunks each): forward with Vn and the states kept 96 -> 89 us, reverse 98 -> 90, outputs alone
-// 83 -> 82; 2700 cycles a chunk, of which the two products of the chain and their latencies are about half.  4 x 2000 tokens, 16 heads (128 CTAs against
-// 256): both forward scans 167 -> 97, reverse 97 -> 52.
+// 2 x 4096 tokens, 16 heads of 128 (64 CTAs, 64 chunks each): outputs 97 -> 90 us, reverse 95 -> 89, Vn and the states alone 82 -> 82 (with fewer heads, 2 x 64
+// chunks, 71 -> 81: such scans stay with lsm_delta.cu); 2700 cycles a chunk, of which the two products of the chain and their latencies are about half.
+// 64 heads x 26 chunks (128 CTAs against 256): outputs 82 -> 42, reverse 80 -> 42, Vn and the states 55 -> 37.
 #include "flash_tc_utils.cuh"
 #include "lsm_delta.cuh"
 

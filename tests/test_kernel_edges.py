@@ -602,3 +602,33 @@ def test_delta_prompt_repeats():
                 o2, S2 = ops.lsm_delta(q, k, v, beta, None, None, None, 64)
                 assert torch.equal(o, o2) and torch.equal(S, S2)
         gemm.check_error()
+
+
+@pytest.mark.parametrize("H,N,dv,tc", [(2, 31, 128, ""), (2, 32, 128, "output reverse"), (37, 40, 128, "output reverse"), (38, 3, 128, "output states reverse"),
+                                       (50, 2, 96, ""), (50, 2, 192, "output states reverse")])
+def test_delta_scan_routes(H, N, dv, tc):
+    """Which scans of 128-wide keys run on tcgen05: those with outputs and the reverse one from 32 chunks on, those that only rebuild the increments and
+    states (a step with few heads takes longer there) where the CTAs of the others are more than SMs.  Both give the increments and states of the definition."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines go by 148 SMs")
+    torch.manual_seed(0)
+    D = 128
+    kw = dict(device="cuda", dtype=torch.bfloat16)
+    W, Qd, Kd = (0.05 * torch.randn(1, H, N, 64, D, **kw) for _ in range(3))              # small enough for roundings to fade over the chunks
+    U, A, dO = torch.randn(1, H, N, 64, dv, **kw), 0.1 * torch.randn(1, H, N, 64, 64, **kw).tril(), torch.randn(1, N * 64, H, dv, **kw)
+    gamma, o = torch.full((1, H, N), 0.5, device="cuda"), torch.empty(1, N * 64, H, dv, **kw)
+    calls = {"output": lambda: K._delta_scan_fwd(W, U, Qd, Kd, A, gamma, None, o, keep=False), "states": lambda: K._delta_scan_fwd(W, U, Qd, Kd, A, gamma, None),
+             "reverse": lambda: K._delta_scan_bwd(W, Qd, Kd, A, gamma, dO, None)}
+    for name, f in calls.items():
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+            res = f()
+            torch.cuda.synchronize()
+        scans = [e.key for e in p.key_averages() if "delta_scan" in e.key]
+        assert len(scans) == 1 and ("_tc_kernel" in scans[0]) == (name in tc.split()), (name, scans)
+        if name == "states":
+            S = torch.zeros(1, H, D, dv, dtype=torch.float64, device="cuda")
+            for n in range(N):
+                vn = U[:, :, n].double() - W[:, :, n].double() @ S
+                assert n == 0 or rel(res[1][:, :, n], S) < 8 * 2.0 ** -9
+                assert rel(res[0][:, :, n], vn) < 8 * 2.0 ** -9
+                S = 0.5 * S + Kd[:, :, n].double().transpose(-1, -2) @ vn
