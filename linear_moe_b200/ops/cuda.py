@@ -35,6 +35,7 @@ def __getattr__(name):                       # ``K.NUM_SMS`` for the callers in 
     if name == "NUM_SMS":
         return num_sms()
     raise AttributeError(name)
+_GEMM = None              # the module of the tcgen05 products, once asked for
 launch_count = 0          # kernels of this library launched since the last reset (bench.py reports it)
 
 
@@ -1051,9 +1052,18 @@ def _scalar_groups(B, H, T, chunk):
 
 def _tma_view(t):
     """As :func:`_inner_contig`, for kernels that read through tensor maps: no repeated (stride zero) dimensions either."""
-    if any(s <= 0 for s, n in zip(t.stride(), t.shape) if n > 1):
+    if 0 in t.stride() and any(s == 0 for s, n in zip(t.stride(), t.shape) if n > 1):        # (the first test alone takes a tenth of the time)
         return _aligned(t)
     return _inner_contig(t)
+
+
+def _error_word(device) -> int:
+    """Where the tcgen05 kernels report a wait that ran out."""
+    global _GEMM
+    if _GEMM is None:                     # (an import statement costs a short call a microsecond each time)
+        from . import gemm
+        _GEMM = gemm
+    return _GEMM._err(device).data_ptr()
 
 
 def _lsm_args(q, k, v, g, gmode, scale, B, T, H, G, cpg, states, gdecay, chunk, d_o=None, o=None, dq=None, dk=None, dv=None):
@@ -1280,13 +1290,12 @@ class _GlaArgs(ctypes.Structure):
 
 
 def _gla_args(q, k, v, gk, scale, B, T, H, G, cpg, states, gdecay, d_o=None, o=None, dq=None, dk=None, dv=None):
-    from . import gemm
     grads = []
     for t in (dq, dk, dv):
         grads += (0, 0, 0) if t is None else t.stride()[:3]
     return _GlaArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(d_o), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
                     _ptr(o), _ptr(dq), _ptr(dk), _ptr(dv), *grads, gk.data_ptr(), float(scale), B, T, H, G, cpg,
-                    states.data_ptr(), _ptr(gdecay), gemm._err(q.device).data_ptr())
+                    states.data_ptr(), _ptr(gdecay), _error_word(q.device))
 
 
 def _gla_launch(which, D, args):
