@@ -17,9 +17,9 @@
 //   dS <- diag(e^{b_m}) [ diag(e^{b_C - b_m}) dS + scale q~^T dO ]
 // The gate gradient is d g = reverse-cumsum_t (q . dq - k . dk) per channel (the kernels at the end of this file).
 //
-// These kernels take 64-wide heads; those for 128-wide ones are in lsm_vector_tc.cu.
+// These kernels take 64-wide heads, and 128-wide ones where a group has one chunk; the others are in lsm_vector_tc.cu.
 //
-// 512 threads, one CTA per SM, or two where there are more CTAs than SMs: a warp owns 16 rows of every product and a quarter of its columns (of the state: a half).  For the
+// 512 threads, one CTA per SM (two where 64-wide heads have more CTAs than SMs): a warp owns 16 rows of every product and a quarter of its columns (of the state: half or a quarter).  For the
 // gates a thread owns two channels and VCH / GR consecutive tokens: running sums stay in registers, the GR groups of tokens meet in one
 // small table, and the next chunk's gates and tiles are on their way while this one is worked on.  (With eight warps, single buffers and a
 // 64-step running sum in 128 threads the chunks were bound by latency.)
@@ -512,16 +512,19 @@ static int gla_launch(int which, const GlaArgs& a, cudaStream_t st) {
     return (int)cudaGetLastError();
 }
 
-// which: 0 forward state scan, 1 reverse state scan, 2 forward output, 3 backward dq, 4 backward dk/dv
-LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t st) {
-    // 128-wide heads: the tensor cores of lsm_vector_tc.cu at every size.  Kernels of a forward pass and with all gradients, here and there: 8 x 2048 tokens of
-    // 8 heads 155 and 88 us, 560 and 303; 3 x 1111 of 16 heads 65 and 41, 234 and 159; one chunk of one head 14.8 and 16.6, 58.8 and 49.1.
-    if (D == 128) return lvt::launch(which, *ap, st);
+static int gla_launch(int which, int D, const GlaArgs& a, lvt::Maps& maps, cudaStream_t st) {
+    if (D == 128) return a.wide ? lvt::launch(which, a, maps, st) : gla_launch<128, 1>(which, a, st);
     if (D != 64) return -2;
     // 64-wide heads, more CTAs than SMs: two per SM with 64 registers a thread overlap each other's steps.  Outputs, one and two per SM:
     // 64 x 256 tokens of 16 heads 216 and 185 us, 64 x 128 144 and 123, 32 x 64 56 and 50; where every CTA has an SM to itself the
     // registers are worth more (8 x 2048 of 8 heads, 128 CTAs: 81 and 91).
-    return (long long)ap->G * ap->B * ap->H > sm_count() ? gla_launch<64, 2>(which, *ap, st) : gla_launch<64, 1>(which, *ap, st);
+    return (long long)a.G * a.B * a.H > sm_count() ? gla_launch<64, 2>(which, a, st) : gla_launch<64, 1>(which, a, st);
+}
+
+// which: 0 forward state scan, 1 reverse state scan, 2 forward output, 3 backward dq, 4 backward dk/dv
+LMOE_API int lmoe_gla_launch(int which, int D, const GlaArgs* ap, cudaStream_t st) {
+    lvt::Maps maps;
+    return gla_launch(which, D, *ap, maps, st);
 }
 
 LMOE_API int lmoe_gla_combine(int rev, float* states, const float* gdecay, const float* seed, float* final_out, int BH,
@@ -542,11 +545,25 @@ LMOE_API int lmoe_gla_combine(int rev, float* states, const float* gdecay, const
 
 // Summaries, combine and outputs of a forward call: the three launches behind one host call.
 LMOE_API int lmoe_gla_forward(int D, const GlaArgs* ap, const float* seed, float* final_out, cudaStream_t st) {
-    int rc = lmoe_gla_launch(0, D, ap, st);
+    lvt::Maps maps;
+    int rc = gla_launch(0, D, *ap, maps, st);
     if (rc) return rc;
     rc = lmoe_gla_combine(0, ap->states, ap->gdecay, seed, final_out, ap->B * ap->H, ap->G, D, st);
     if (rc) return rc;
-    return lmoe_gla_launch(2, D, ap, st);
+    return gla_launch(2, D, *ap, maps, st);
+}
+
+// dq (of `ap`, with the entering states), summaries of the state's gradient, combine, dk and dv (of `bp`, whose states are the gradient's): four launches
+// behind one host call.  gdecay: of the forward call.
+LMOE_API int lmoe_gla_backward(int D, const GlaArgs* ap, const GlaArgs* bp, const float* gdecay, const float* seed, float* dinit, cudaStream_t st) {
+    lvt::Maps maps;
+    int rc = gla_launch(3, D, *ap, maps, st);
+    if (rc) return rc;
+    rc = gla_launch(1, D, *bp, maps, st);
+    if (rc) return rc;
+    rc = lmoe_gla_combine(1, bp->states, gdecay, seed, dinit, bp->B * bp->H, bp->G, D, st);
+    if (rc) return rc;
+    return gla_launch(4, D, *bp, maps, st);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -1,5 +1,6 @@
 // Arguments of the kernels for linear attention with a decay per key channel (lsm_vector.cu, lsm_vector_tc.cu).
 #pragma once
+#include <cuda.h>
 #include "common.cuh"
 
 namespace lmoe {
@@ -15,11 +16,14 @@ struct GlaArgs {
     float* states;                 // [B,H,G,D,D]
     float* gdecay;                 // [B,H,G,D] total log decay of each group per channel
     int* err;                      // error word of the bounded waits (lsm_vector_tc.cu)
+    int wide;                      // 128-wide heads: the kernels of lsm_vector_tc.cu
 };
 
 namespace lvt {
-// lmoe_gla_launch for 128-wide heads
-int launch(int which, const GlaArgs& a, cudaStream_t st);
+// The tensor maps of a call's inputs, made when a launch first wants them
+struct Maps { CUtensorMap q, k, v, g, gk; unsigned made = 0; };
+// lmoe_gla_launch for `wide`; the launches that share `m` have the same inputs
+int launch(int which, const GlaArgs& a, Maps& m, cudaStream_t st);
 }  // namespace lvt
 
 }  // namespace lmoe

@@ -1,4 +1,4 @@
-// The kernels of lsm_vector.cu for 128-wide heads on the 5th-generation tensor cores: chunks of 64 tokens, tiles by TMA, products as tcgen05.mma
+// The kernels of lsm_vector.cu for 128-wide heads and groups of several chunks on the 5th-generation tensor cores: chunks of 64 tokens, tiles by TMA, products as tcgen05.mma
 // with accumulators in tensor memory.  The arithmetic is the same, operands rescaled around the middle of a chunk: with chunks of 128 the factors
 // e^{+-(b_i - b_m)} would overflow twice as early.  A tile of 64 tokens stands where an instruction wants 128 rows: the lower half of its
 // accumulator holds the tile's rows, the upper half products of whatever follows the tile in shared memory, and nobody reads it (an
@@ -688,14 +688,19 @@ template <typename K>
 static int set_smem(K kernel, size_t bytes) { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); }
 
 // which as in lmoe_gla_launch; positive strides
-int launch(int which, const GlaArgs& a, cudaStream_t st) {
+int launch(int which, const GlaArgs& a, Maps& m, cudaStream_t st) {
     if (a.err == nullptr) return -1;
     dim3 grid(a.G, a.B * a.H);
-    CUtensorMap q, k, v, g, o, dk, dv, gk;
-    int rc = gates_map(&gk, a);
-    if (which == 1 || which == 2 || which == 4) rc |= map_of(&q, a.q, a, a.qs_b, a.qs_t, a.qs_h);
-    if (which != 1) { rc |= map_of(&k, a.k, a, a.ks_b, a.ks_t, a.ks_h); rc |= map_of(&v, a.v, a, a.vs_b, a.vs_t, a.vs_h); }
-    if (which == 1 || which == 3 || which == 4) rc |= map_of(&g, a.d_o, a, (int64_t)a.T * a.H * D, (int64_t)a.H * D, D);
+    CUtensorMap o, dk, dv;
+    int rc = 0;
+    auto want = [&](unsigned bit, auto make) { if (!(m.made & bit)) { rc |= make(); m.made |= bit; } };
+    want(1, [&] { return gates_map(&m.gk, a); });
+    if (which == 1 || which == 2 || which == 4) want(2, [&] { return map_of(&m.q, a.q, a, a.qs_b, a.qs_t, a.qs_h); });
+    if (which != 1) {
+        want(4, [&] { return map_of(&m.k, a.k, a, a.ks_b, a.ks_t, a.ks_h); });
+        want(8, [&] { return map_of(&m.v, a.v, a, a.vs_b, a.vs_t, a.vs_h); });
+    }
+    if (which == 1 || which == 3 || which == 4) want(16, [&] { return map_of(&m.g, a.d_o, a, (int64_t)a.T * a.H * D, (int64_t)a.H * D, D); });
     if (which == 2) rc |= map_of(&o, a.o, a, (int64_t)a.T * a.H * D, (int64_t)a.H * D, D);
     if (which == 3) rc |= map_of(&o, a.dq, a, a.dqs_b, a.dqs_t, a.dqs_h);
     if (which == 4) { rc |= map_of(&dk, a.dk, a, a.dks_b, a.dks_t, a.dks_h); rc |= map_of(&dv, a.dv, a, a.dvs_b, a.dvs_t, a.dvs_h); }
@@ -704,19 +709,19 @@ int launch(int which, const GlaArgs& a, cudaStream_t st) {
         const size_t smem = sizeof(SmemState) + 1024;
         rc = which == 0 ? set_smem(gla_state_tc_kernel<0>, smem) : set_smem(gla_state_tc_kernel<1>, smem);
         if (rc) return rc;
-        if (which == 0) gla_state_tc_kernel<0><<<grid, ST_THREADS, smem, st>>>(k, v, gk, a);
-        else gla_state_tc_kernel<1><<<grid, ST_THREADS, smem, st>>>(q, g, gk, a);
+        if (which == 0) gla_state_tc_kernel<0><<<grid, ST_THREADS, smem, st>>>(m.k, m.v, m.gk, a);
+        else gla_state_tc_kernel<1><<<grid, ST_THREADS, smem, st>>>(m.q, m.g, m.gk, a);
     } else if (which == 2 || which == 3) {
         const size_t smem = sizeof(SmemSweep) + 1024;
         rc = which == 2 ? set_smem(gla_sweep_tc_kernel<0>, smem) : set_smem(gla_sweep_tc_kernel<1>, smem);
         if (rc) return rc;
-        if (which == 2) gla_sweep_tc_kernel<0><<<grid, THREADS, smem, st>>>(q, k, v, o, gk, a);
-        else gla_sweep_tc_kernel<1><<<grid, THREADS, smem, st>>>(g, k, v, o, gk, a);
+        if (which == 2) gla_sweep_tc_kernel<0><<<grid, THREADS, smem, st>>>(m.q, m.k, m.v, o, m.gk, a);
+        else gla_sweep_tc_kernel<1><<<grid, THREADS, smem, st>>>(m.g, m.k, m.v, o, m.gk, a);
     } else if (which == 4) {
         const size_t smem = sizeof(SmemDkv);
         rc = set_smem(gla_dkv_tc_kernel, smem);
         if (rc) return rc;
-        gla_dkv_tc_kernel<<<grid, THREADS, smem, st>>>(q, k, v, g, dk, dv, gk, a);
+        gla_dkv_tc_kernel<<<grid, THREADS, smem, st>>>(m.q, m.k, m.v, m.g, dk, dv, m.gk, a);
     } else return -1;
     return (int)cudaGetLastError();
 }

@@ -1286,7 +1286,17 @@ class _GlaArgs(ctypes.Structure):
                 [(n, ctypes.c_int64) for n in ("dqs_b", "dqs_t", "dqs_h", "dks_b", "dks_t", "dks_h", "dvs_b", "dvs_t", "dvs_h")] +
                 [("gk", ctypes.c_void_p), ("scale", ctypes.c_float)] +
                 [(n, ctypes.c_int) for n in ("B", "T", "H", "G", "cpg")] +
-                [("states", ctypes.c_void_p), ("gdecay", ctypes.c_void_p), ("err", ctypes.c_void_p)])
+                [("states", ctypes.c_void_p), ("gdecay", ctypes.c_void_p), ("err", ctypes.c_void_p), ("wide", ctypes.c_int)])
+
+
+def _gla_wide(D, cpg) -> bool:
+    """Whether 128-wide heads take the tcgen05 kernels (csrc/lsm_vector_tc.cu): where a group has several chunks.
+
+    They shorten the step from chunk to chunk, start later, and their tensor maps cost the host time.  Kernels of a forward call, those of
+    csrc/lsm_vector.cu and these, heads x tokens: groups of one chunk 1 x 64 15.5 and 17.2 us, 8 x 1024 20.1 and 23.0, 300 x 64 62 and 65; of two
+    16 x 1024 27.1 and 23.9, 8 x 2048 26.5 and 26.2, 256 x 128 65 and 59; of three 16 x 1280 32 and 27; 48 x 2048 111 and 69.  Whole
+    calls, among others: 1 x 64 29.0 and 32.8, 16 x 1024 34.0 and 32.1; with gradients 188 and 194, 201 and 193."""
+    return D == 128 and cpg > 1
 
 
 def _gla_args(q, k, v, gk, scale, B, T, H, G, cpg, states, gdecay, d_o=None, o=None, dq=None, dk=None, dv=None):
@@ -1295,25 +1305,20 @@ def _gla_args(q, k, v, gk, scale, B, T, H, G, cpg, states, gdecay, d_o=None, o=N
         grads += (0, 0, 0) if t is None else t.stride()[:3]
     return _GlaArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(d_o), *q.stride()[:3], *k.stride()[:3], *v.stride()[:3],
                     _ptr(o), _ptr(dq), _ptr(dk), _ptr(dv), *grads, gk.data_ptr(), float(scale), B, T, H, G, cpg,
-                    states.data_ptr(), _ptr(gdecay), _error_word(q.device))
+                    states.data_ptr(), _ptr(gdecay), *((_error_word(q.device), 1) if _gla_wide(q.shape[-1], cpg) else (0, 0)))
 
 
 def _gla_launch(which, D, args):
     _check(lib().lmoe_gla_launch(_i32(which), _i32(D), ctypes.byref(args), _st()), f"gla[{which}]")
 
 
-def _gla_combine(rev, states, gdecay, seed, final_out, BH, G, D):
-    _check(lib().lmoe_gla_combine(_i32(rev), _p(states), _p(gdecay), _p(seed), _p(final_out), _i32(BH), _i32(G), _i32(D),
-                                  _st()), "gla_combine")
-
-
 def _vector_forward(q, k, v, gk, scale, init):
     """Returns the output, the final state and what the backward pass needs: (tensors, (groups, chunks), exchange)."""
     B, T, H, D = q.shape
-    fix = _tma_view if D == 128 else _inner_contig
+    G, cpg = lsm_groups(B, H, T)
+    fix = _tma_view if _gla_wide(D, cpg) else _inner_contig
     q, k, v = fix(q), fix(k), fix(v)
     gf = _aligned(gk.float())
-    G, cpg = lsm_groups(B, H, T)
     f32, dev = torch.float32, q.device
     states = torch.empty(B, H, G, D, D, dtype=f32, device=dev)
     gdecay = torch.empty(B, H, G, D, dtype=f32, device=dev)
@@ -1353,17 +1358,17 @@ class _LsmVector(torch.autograd.Function):
         dstates = torch.empty_like(states)
         dinit = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device) if ctx.has_init else None
         a = _gla_args(q, k, v, gf, ctx.scale, B, T, H, G, cpg, states, None, d_o=d_o, dq=dq)
-        _gla_launch(3, D, a)
         a2 = _gla_args(q, k, v, gf, ctx.scale, B, T, H, G, cpg, dstates, None, d_o=d_o, dk=dk, dv=dv)
-        _gla_launch(1, D, a2)
-        seed = None if dfinal is None else _aligned(dfinal.float())
         if ctx.lasp is not None:
+            _gla_launch(3, D, a)
+            _gla_launch(1, D, a2)
             r_out = torch.empty(B, H, D, D, dtype=torch.float32, device=q.device)
             ctx.lasp.combine(1, dstates, None, None, B * H, H, G, cpg, T, D, gdecay=gdecay, dmode=2, r_out=r_out)
             dfinal = r_out         # gradient of the state leaving this rank, folded from the ranks after it
+            _gla_launch(4, D, a2)
         else:
-            _gla_combine(1, dstates, gdecay, seed, dinit, B * H, G, D)
-        _gla_launch(4, D, a2)
+            seed = None if dfinal is None else _aligned(dfinal.float())
+            _check(lib().lmoe_gla_backward(D, ctypes.byref(a), ctypes.byref(a2), _p(gdecay), _p(seed), _p(dinit), _st()), "gla_backward", 4)
         # d gk_t = sum_{i>=t} q_i . dq_i - sum_{j>=t} k_j . dk_j per channel (+ <S_T, dS_T> rows with a final-state gradient)
         # (the scan runs along the innermost dimension of a [B,H,D,T] copy: a scan over an outer dimension is ~10x slower)
         dg = _gla_dg(q, k, dq, dk)

@@ -632,3 +632,27 @@ def test_delta_scan_routes(H, N, dv, tc):
                 assert n == 0 or rel(res[1][:, :, n], S) < 8 * 2.0 ** -9
                 assert rel(res[0][:, :, n], vn) < 8 * 2.0 ** -9
                 S = 0.5 * S + Kd[:, :, n].double().transpose(-1, -2) @ vn
+
+
+@pytest.mark.parametrize("B,H,T,chunks", [(1, 9, 700, 4), (2, 5, 700, 11), (1, 149, 130, 3)])
+def test_vector_decay_views_in_groups(B, H, T, chunks, monkeypatch):
+    """As test_vector_decay_views, in groups of several chunks (the tcgen05 kernels)."""
+    monkeypatch.setattr(K, "lsm_groups", lambda *a: (-(-T // (64 * chunks)), chunks))
+    test_vector_decay_views(B, H, T)
+
+
+@pytest.mark.parametrize("B,T,H,D,tc", [(1, 2, 1, 128, False), (1, 64 * 74, 2, 128, False), (1, 64 * 74 + 1, 2, 128, True), (150, 64, 1, 128, False),
+                                        (150, 65, 1, 128, True), (2, 64 * 200, 1, 64, False)])
+def test_vector_decay_routes(B, T, H, D, tc):
+    """128-wide heads run on tcgen05 where a group has several chunks, forward and backward; a call with one chunk per group does not pay for tensor maps and
+    the later start."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line goes by 148 SMs")
+    torch.manual_seed(0)
+    ins = [rand(B, T, H, D).requires_grad_(True) for _ in range(3)] + [-torch.rand(B, T, H, D, device="cuda").requires_grad_(True)]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        o, _ = ops.lsm_vector(*ins, None, None, None, 64)
+        torch.autograd.grad(o, ins, torch.ones_like(o))
+        torch.cuda.synchronize()
+    names = [e.key for e in p.key_averages() if "gla_" in e.key and "combine" not in e.key and "gla_dg" not in e.key]
+    assert len(names) == 5 and all(("_tc_kernel" in n) == tc for n in names), names
