@@ -381,8 +381,8 @@ _MOE_LOCAL: Dict[tuple, "MoeWorkspace"] = {}
 
 
 def local_moe_workspace(num_experts: int, hidden: int, rows: int, device) -> "MoeWorkspace":
-    """One-rank workspace (ordinary tensors) for a MoE layer without expert parallelism: the same push / pull kernels
-    replace the index_select / index_add_ permutation, which is several times slower in both directions."""
+    """One-rank workspace for a MoE layer without expert parallelism: push and pull kernels on plain tensors replace the
+    index_select / index_add_ permutation, which is several times slower in both directions."""
     key = (str(device), num_experts, hidden)
     ws = _MOE_LOCAL.get(key)
     if ws is None or ws.cap < rows:
@@ -409,7 +409,8 @@ class _MoeLocalArgs(ctypes.Structure):
 
 class MoeWorkspace:
     """Receive buffer ``x [cap, h]``, result buffer ``y [cap, h]``, count matrix and flags of one expert-parallel group.
-    ``group=None`` builds a one-rank workspace out of ordinary tensors (single-GPU use and tests)."""
+    ``group=None``: a one-rank workspace.  Its routing, push and pull work on tensors of the call, so it holds no buffers until
+    somebody asks for the arguments of the exchange kernels (:meth:`_args`)."""
 
     def __init__(self, group, num_experts: int, hidden: int, cap_rows: int, device, spin_limit: Optional[int] = None):
         self.group, self.device = group, device
@@ -418,6 +419,16 @@ class MoeWorkspace:
         assert num_experts % W == 0 and hidden % 8 == 0
         self.E, self.El, self.h = num_experts, num_experts // W, hidden
         self.cap = (cap_rows + 255) // 256 * 256
+        if group is not None:
+            self._make_buffers()
+        self.ep_exchange = self.ep_push = self.ep_pull = 0
+        self.spin_limit = default_spin_limit() if spin_limit is None else spin_limit
+        torch.cuda.synchronize()
+        if group is not None:
+            dist.barrier(group=group.pg)
+
+    def _make_buffers(self):
+        group, W, hidden, num_experts, device = self.group, self.W, self.h, self.E, self.device
         if group is not None:
             self.x, hx = _symm_empty(self.cap * hidden, torch.bfloat16, device, group)
             self.y, hy = _symm_empty(self.cap * hidden, torch.bfloat16, device, group)
@@ -437,13 +448,10 @@ class MoeWorkspace:
         self.peer_x, self.peer_y, self.peer_cnt, self.peer_flags = [
             torch.tensor(p, dtype=torch.int64, device=device) for p in ptrs]
         self.done_ctr = torch.zeros(1, dtype=torch.int32, device=device)
-        self.ep_exchange = self.ep_push = self.ep_pull = 0
-        self.spin_limit = default_spin_limit() if spin_limit is None else spin_limit
-        torch.cuda.synchronize()
-        if group is not None:
-            dist.barrier(group=group.pg)
 
     def _args(self) -> _MoeArgs:
+        if self.group is None and not hasattr(self, "x"):
+            self._make_buffers()
         a = _MoeArgs()
         a.peer_cnt, a.peer_flags = self.peer_cnt.data_ptr(), self.peer_flags.data_ptr()
         a.peer_x, a.peer_y = self.peer_x.data_ptr(), self.peer_y.data_ptr()
@@ -528,7 +536,7 @@ class MoeWorkspace:
         """Send every (token, slot) row of ``src [T, h]`` (times ``weights [T*k]``) to its expert's rank; returns this
         rank's receive buffer ``[cap, h]`` with zeroed padding rows: a copy with ``keep`` (the forward pass saves it for the
         weight gradient), the shared buffer itself without (the backward pass consumes it before this rank signals its
-        results, and no peer pushes again before it has pulled those)."""
+        results, and no peer pushes again before it has pulled those).  One rank: a fresh tensor of the rows that this call can take."""
         assert src.is_contiguous() and src.dtype == torch.bfloat16 and src.shape == (route.T, self.h)
         if self.group is None:
             # the receive buffer is a fresh tensor that the caller keeps, no copy out of a shared buffer

@@ -157,3 +157,21 @@ def test_one_rank_pull_with_the_gathered_rows(T, k, E, hid, drop):
     assert torch.equal(out, ws.pull(y, route, w, False)[0])
     torch.cuda.synchronize()
     fused_comm.check_status("pull")
+
+
+def test_one_rank_workspace_holds_no_buffers():
+    """A workspace for many rows takes no device memory of its own on one rank, and a call with it leaves none behind."""
+    from linear_moe_b200.ops.moe_fused import fused_moe
+    from linear_moe_b200.parallel import fused_comm
+    dev = torch.device("cuda", 0)
+    T, k, E, hid, f = 64, 2, 4, 256, 64
+    w1, w2 = torch.randn(E, hid, 2 * f, device=dev).bfloat16(), torch.randn(E, f, hid, device=dev).bfloat16()
+    h, probs, idx = torch.randn(T, hid, device=dev).bfloat16(), torch.rand(T, k, device=dev), torch.randint(0, E, (T, k), device=dev)
+    ws = fused_comm.MoeWorkspace(None, E, hid, 256 * E + T * k, dev)
+    fused_moe(h, probs, idx, w1, w2, ws)                     # scratch and status words of the process
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    ws = fused_comm.MoeWorkspace(None, E, hid, 1 << 18, dev)
+    out = fused_moe(h, probs, idx, w1, w2, ws)
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() - before <= out.numel() * 2 + 65536
